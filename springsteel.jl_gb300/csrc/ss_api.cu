@@ -112,6 +112,7 @@ static void free_grid(ss_grid *g) {
     if (g->copy_stream) cudaStreamSynchronize(g->copy_stream);
     for (cudaEvent_t e : g->ev_pool) cudaEventDestroy(e);
     for (cudaEvent_t e : g->chunk_ev) cudaEventDestroy(e);
+    digit_free(g);
     for (void *p : g->allocs) cudaFree(p);
     if (g->copy_stream) cudaStreamDestroy(g->copy_stream);
     if (g->stream) cudaStreamDestroy(g->stream);
@@ -348,10 +349,11 @@ static int32_t build_grid(ss_grid *g) {
     }
 
     // ---- Chebyshev columns (src/factory.jl:722-728)
+    std::vector<ChebHost> cheb(g->rlz ? nv : 0);
     if (g->rlz) {
         std::vector<ChebDev> cdev(nv);
         for (int v = 0; v < nv; v++) {
-            ChebHost ch;
+            ChebHost &ch = cheb[v];
             st = build_cheb(kz, bk, g->bcb[v], g->bct[v], p.kMin, p.kMax, ch);
             if (st) return st;
             ChebDev &cd = cdev[v];
@@ -455,7 +457,8 @@ static int32_t build_grid(ss_grid *g) {
     }
     fft_init_constants();
     CUDA_TRY(cudaStreamSynchronize(g->stream));
-    return SS_OK;
+    if ((st = digit_build(g, rings))) return st;
+    return digit_columns_build(g, cheb);
 }
 
 // ---------------------------------------------------------------- launches
@@ -552,8 +555,14 @@ SaLaunch sa_record(const ss_grid *g, int coeffs, size_t *smem_generic) {
 
 template <typename P, typename T>
 static int32_t fwd_rings(ss_grid *g, cudaStream_t st, int chunk) {
-    RingLaunch L = ring_record(g, false);
     StageScope sc(g, SS_STAGE_RING_FWD, st);
+    if (g->digit.on && g->tl == TL_F64) {
+        int launches = 0;
+        const int32_t rc = digit_ring_forward(g, st, chunk, &launches);
+        g->launches[SS_STAGE_RING_FWD] += launches;
+        return rc;
+    }
+    RingLaunch L = ring_record(g, false);
     return for_ring_segments(g, chunk, [&](const int *list, int count, const RingBucket &bkt) -> int32_t {
         L.ring_list = list;
         const size_t smem = ring_item_smem(g, bkt, false);
@@ -601,8 +610,15 @@ static int32_t inv_sa(ss_grid *g, cudaStream_t st, int coeffs, const void *spec_
 
 template <typename P, typename T>
 static int32_t inv_rings(ss_grid *g, cudaStream_t st, int chunk) {
-    RingLaunch L = ring_record(g, true);
     StageScope sc(g, SS_STAGE_RING_INV, st);
+    if (g->digit.on) {
+        int launches = 0;
+        const int32_t rc = digit_ring_inverse(g, st, chunk, &launches);
+        g->launches[SS_STAGE_RING_INV] += launches;
+        if (rc || g->tl == TL_F64) return rc;
+    }
+    RingLaunch L = ring_record(g, true);
+    L.value_only = g->digit.on;
     return for_ring_segments(g, chunk, [&](const int *list, int count, const RingBucket &bkt) -> int32_t {
         L.ring_list = list;
         const size_t sm = ring_item_smem(g, bkt, true);
@@ -622,6 +638,10 @@ static int32_t inv_columns(ss_grid *g, cudaStream_t st, int chunk) {
     Cl.col0 = chunk_col(g, chunk, 0); Cl.col1 = chunk_col(g, chunk, 1);
     const int N = (int)d.kDim;
     StageScope sc(g, SS_STAGE_CHEB_INV, st);
+    if (g->digit.columns.on) {
+        g->launches[SS_STAGE_CHEB_INV]++;
+        return digit_columns_inverse(g, st, chunk);
+    }
     CUDA_TRY((launch_cheb_inverse<P, T>(Cl, 0, st, N)));
     g->launches[SS_STAGE_CHEB_INV]++;
     return SS_OK;
@@ -1045,6 +1065,11 @@ int32_t ss_grid_synchronize(ss_grid *g) {
     CHECK_GRID(g);
     CUDA_TRY(cudaStreamSynchronize(g->stream));
     CUDA_TRY(cudaGetLastError());
+    if (g->digit.err && *(volatile int *)g->digit.err) {
+        *g->digit.err = 0;
+        set_error("ring product: a bounded device wait gave up");
+        return SS_DEVICE_TIMEOUT;
+    }
     return SS_OK;
 }
 

@@ -1,0 +1,899 @@
+// ss_digit.cu — the ring DFTs of RLZ grids on the tensor cores, by exact
+// products of digit slices.
+//
+// A ring of L = 4n points carries the wavenumbers k ≤ n − 1 only, and its points
+// are symmetric about 0 and π/2, so HC2R of a column folds into four real
+// products of quadrant size (cos / sin × even / odd k, n × n/2 each).  One ring
+// holds nvars · b_kDim · 5 columns, so each product is a GEMM of the ring's own
+// cosine matrix with the columns of all items.  FP64 runs at 2 FMA per clock and
+// SM on this GPU and the mixed-radix FFT of the arbitrary lengths 4 + 4ri spends
+// 2.3 times the conventional operations on prime factors; a binary16 tensor-core
+// product with binary32 accumulation is exact while the operands are integers
+// and the sums stay below 2^24.  So each column is scaled by the exponent of its
+// largest entry to a fixed-point number and cut into balanced digits (Ozaki et
+// al. 2012, error-free splitting), the matrix likewise once per grid, and
+//     Σ_k Y[m][k] X[k][c] = Σ_s 2^{−9s} D_s,   D_s = Σ_{i+j=s} Σ_k y_i x_j,
+// keeps s ≤ 6 (binary64; 26 of the 36 products, the rest is below 2^−60 of the
+// column's scale) or s ≤ 2 (binary32).  The D_s are combined as integers in
+// 64-bit fixed point (binary64) or in binary32.
+//
+// The reference turns each coefficient by cos, sin of the Float64 product k·ymin;
+// the folded matrices hold the exact angles, and the difference δ_k (up to 1e-13)
+// is applied to the fixed-point coefficients, so both agree to their last bits.
+//
+// Measured on the 200-cell, 32-level, 5-variable FP64 grid: ring_inverse 34.1 →
+// 5.3 ms and ring_forward 7.1 → 1.9 ms, each with an error against 64-bit ring sums
+// no larger than the FFT kernels' (9.2e-16 against 9.6e-16 of f, 3.0e-16 against
+// 3.3e-16 of the spectral array at 200 cells).
+//
+// digit_split   G (spectra at the mish points) → column exponents and digit
+//               planes in the MMA operand layout
+// digit_gemm    persistent, warp-specialised: bulk copies → 8-slot (6-slot) ring
+//               of K-steps → two issuing warps, one per accumulator half → two
+//               warpgroups drain and combine
+// digit_unfold  quadrant parts → ring points, in place
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstdlib>
+#include <cstring>
+
+#include "ss_digit.h"
+#include "ss_digit_dev.cuh"
+#include "ss_grid.h"
+#include "ss_internal.h"
+#include "ss_types.cuh"
+
+using namespace ss;
+
+#define CUDA_TRY(expr)                                                                      \
+    do {                                                                                    \
+        cudaError_t _e = (expr);                                                            \
+        if (_e != cudaSuccess) {                                                            \
+            set_error("%s failed: %s", #expr, cudaGetErrorString(_e));                      \
+            return (_e == cudaErrorMemoryAllocation) ? SS_OUT_OF_MEMORY : SS_CUDA_ERROR;   \
+        }                                                                                   \
+    } while (0)
+
+namespace ss {
+
+// ------------------------------------------------------------ tables
+// cos(2πt/8n), t = 0..2n, of every ring
+__global__ void digit_cos_kernel(const DigitRing *rings, double *cosq) {
+    const DigitRing r = rings[blockIdx.x];
+    const double inv = 1.0 / (4.0 * r.n);
+    for (int t = threadIdx.x; t <= 2 * r.n; t += blockDim.x)
+        cosq[r.cosofs + t] = t <= r.n ? cospi(t * inv) : sinpi((2 * r.n - t) * inv);
+}
+__device__ __forceinline__ double quarter_cos(const double *c, int n, int t) {  // cos(2πt/8n), 0 ≤ t < 8n
+    if (t > 4 * n) t = 8 * n - t;
+    return t > 2 * n ? -c[4 * n - t] : c[t];
+}
+// entry of part `part` at row m, wavenumber k (half weight at k = 0: the result is doubled)
+__device__ __forceinline__ double dft_entry(const DigitRing &r, const double *c, int part, int m, int k) {
+    if (k > r.kmax || m >= r.n + 1 - r.half) return 0.0;
+    const int per = 8 * r.n;
+    int t = (int)((long long)k * (2 * m + r.half) % per);
+    if (part >= 2) {  // −sin = −cos(t − 2n)
+        t = t - 2 * r.n;
+        if (t < 0) t += per;
+        return -quarter_cos(c, r.n, t);
+    }
+    const double v = quarter_cos(c, r.n, t);
+    return k == 0 ? 0.5 * v : v;
+}
+
+// digit planes of the inverse matrices: A tile = [digit][row group][K core][8 rows][8 k]
+// (forward: rows are wavenumbers and K the quadrant positions, without the half weight)
+template <typename T, bool kForward>
+__global__ void __launch_bounds__(256) digit_matrix_kernel(const DigitRing *rings, const double *cosq, uint8_t *A) {
+    const DigitRing r = rings[blockIdx.x];
+    const double *c = cosq + r.cosofs;
+    const int64_t ntile = kForward ? (int64_t)4 * r.rtf * r.tm : (int64_t)r.rt * 2 * (r.te + r.to);
+    for (int64_t e = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; e < ntile * 256; e += (int64_t)gridDim.y * blockDim.x) {
+        const int64_t tile = e >> 8;
+        const int row = (int)(e & 127), kg = (int)((e >> 7) & 1);
+        int part = 0;
+        int64_t q = tile;
+        int steps = r.tm;
+        if (kForward) {
+            part = (int)(tile / (r.rtf * r.tm));
+            q = tile - (int64_t)part * r.rtf * r.tm;
+        } else {
+            while (part < 3 && tile >= digit_part_base(r, part + 1, r.rt)) part++;
+            steps = digit_steps(r, part);
+            q = tile - digit_part_base(r, part, r.rt);
+        }
+        const int m = (int)(q / steps) * kDigitRows + row, j0 = (int)(q % steps) * 16 + kg * 8;
+        auto entry = [&](int i) {
+            if (!kForward) return dft_entry(r, c, part, m, 2 * (j0 + i) + (part & 1));
+            const int k = 2 * m + (part & 1);
+            const double v = dft_entry(r, c, part, j0 + i, k);
+            return k == 0 ? 2.0 * v : v;
+        };
+        uint8_t *dst = A + ((kForward ? r.af_tile : r.a_tile) + tile) * digit_a_bytes<T>() + (row >> 3) * 256 + kg * 128 + (row & 7) * 16;
+        if constexpr (std::is_same<T, double>::value) {
+            unsigned long long U[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                U[i] = (unsigned long long)__double2ll_rn(entry(i) * 0x1p53) + kDigitBias;
+            uint4 w[6];
+            planes8(U, w);
+#pragma unroll
+            for (int i = 0; i < 6; i++) *reinterpret_cast<uint4 *>(dst + i * kDigitPlane) = w[i];
+        } else {
+            // the digits of the binary64 entry itself, not of its binary32 rounding
+            uint32_t w[3][4];
+#pragma unroll
+            for (int q2 = 0; q2 < 4; q2++) {
+                float d[3][2];
+#pragma unroll
+                for (int p = 0; p < 2; p++) {
+                    double v = entry(2 * q2 + p) * 256.0;
+                    for (int i = 0; i < 3; i++) {
+                        const double d0 = rint(v);
+                        d[i][p] = (float)d0;
+                        v = (v - d0) * 1024.0;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    const __half2 h = __floats2half2_rn(d[i][0], d[i][1]);
+                    w[i][q2] = *reinterpret_cast<const uint32_t *>(&h);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 3; i++)
+                *reinterpret_cast<uint4 *>(dst + i * kDigitPlane) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+        }
+    }
+}
+
+// ------------------------------------------------------------ split
+// CTA = (ring of the span, group of 8 items).  Pass 1: a warp per item finds the
+// largest exponent of each variant's column (k·X and k²·X for ∂λ, ∂λλ); pass 2:
+// a thread per (item, source, 16 wavenumbers), source = real or imaginary parts
+// of even or odd k, writes 8 K entries of each plane as 16 bytes; the 8 items of
+// a group are the 8 rows of one core matrix, so a warp's stores are 128-byte
+// runs.  Column of (item, variant): (item / 8)·8·kVars + variant·8 + item mod 8.
+struct SplitArgs {
+    const void *G;
+    const DigitRing *rings;
+    const int64_t *btile;
+    uint8_t *B;
+    int *expo;
+    const int *delta;
+    int64_t frows;
+    int r0, nitems, iDim, col_tiles;
+};
+
+__device__ __forceinline__ uint32_t mag_bits(double v) { return (uint32_t)__double2hiint(v) & 0x7fffffffu; }
+__device__ __forceinline__ uint32_t mag_bits(float v) { return (uint32_t)__float_as_int(v) & 0x7fffffffu; }
+template <typename T>
+__device__ __forceinline__ int mag_expo(uint32_t bits) {  // biased exponent ≥ 1, or kNanColumn
+    if constexpr (std::is_same<T, double>::value) {
+        const int e = (int)(bits >> 20);
+        return e == 0x7ff ? kNanColumn : (e > 0 ? e : 1);
+    } else {
+        const int e = (int)(bits >> 23);
+        return e == 0xff ? kNanColumn : (e > 0 ? e : 1);
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, 2) digit_split_kernel(SplitArgs S) {
+    using F = DigitFormat<T>;
+    constexpr int V0 = kDigitVariants - F::kVars;
+    __shared__ int ex[kDigitGroup][kDigitVariants];
+    const int ring = S.r0 + (int)(gridDim.y - 1 - blockIdx.y);  // largest rings first
+    const DigitRing r = S.rings[ring];
+    const int grp = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const T *G = (const T *)S.G;
+    const size_t plane = (size_t)S.nitems * S.frows;
+    {
+        const int item = grp * kDigitGroup + warp;
+        uint32_t mx[kDigitVariants] = {0, 0, 0, 0, 0};
+        if (item < S.nitems) {
+            const T *g0 = G + (size_t)item * S.frows + r.fofs;
+            for (int s = lane; s < 1 + 2 * r.kmax; s += 32) {
+                const T k = (T)((s + 1) >> 1);
+                const T v = g0[s];
+                mx[0] = max(mx[0], mag_bits(v));
+                mx[1] = max(mx[1], mag_bits(v * k));
+                mx[2] = max(mx[2], mag_bits(v * k * k));
+                mx[3] = max(mx[3], mag_bits(g0[s + plane]));
+                mx[4] = max(mx[4], mag_bits(g0[s + 2 * plane]));
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kDigitVariants; q++) {
+            const int e = mag_expo<T>(__reduce_max_sync(0xffffffffu, mx[q]));
+            if (lane == 0) {
+                ex[warp][q] = e;
+                if (item < S.nitems) S.expo[((size_t)q * S.nitems + item) * S.iDim + ring] = e;
+            }
+        }
+    }
+    __syncthreads();
+    // warp-uniform control flow: lanes exchange values; idle ones (no such item, no
+    // such odd step) read item 0 and store nothing
+    const int il = threadIdx.x & 7;
+    const bool real = grp * kDigitGroup + il < S.nitems;
+    const int item = real ? grp * kDigitGroup + il : 0;
+    const int par = (threadIdx.x >> 3) & 1, imag = (threadIdx.x >> 4) & 1;
+    const int64_t bt = S.btile[ring];
+    const T *g = G + (size_t)item * S.frows + r.fofs;
+    const int steps = par ? r.to : r.te;
+    for (int kg = warp; kg < 2 * r.te; kg += 8) {
+        const bool store = real && kg < 2 * steps;
+        const int k0 = 16 * kg + par;
+        int dk[8];
+        if constexpr (std::is_same<T, double>::value) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int k = k0 + 2 * i;
+                dk[i] = (k > 0 && k <= r.kmax) ? S.delta[r.dofs + k - 1] : 0;
+            }
+        }
+#pragma unroll 1
+        for (int d = 0; d < 3; d++) {
+            T x[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int k = k0 + 2 * i;
+                x[i] = (k <= r.kmax && (k > 0 || !imag)) ? g[d * plane + (k > 0 ? 2 * k - 1 + imag : 0)] : T(0);
+            }
+#pragma unroll 1
+            for (int dl = 0; dl < (d == 0 ? 3 : 1); dl++) {
+                if (dl > 0) {  // ×ik: (re, im) → (−k im, k re)
+                    const bool neg = (dl == 1) == (imag != 0);
+#pragma unroll
+                    for (int i = 0; i < 8; i++) x[i] *= (T)(neg ? -(k0 + 2 * i) : k0 + 2 * i);
+                }
+                const int var = d == 0 ? dl : d + 2;
+                if (var < V0) continue;
+                const int part = ((imag ^ (dl & 1)) << 1) + par;
+                const int e = ex[il][var];
+                const int col = (grp * F::kVars + var - V0) * kDigitGroup + il;
+                const int ct = col / (2 * F::kCols), cl = col % (2 * F::kCols);
+                const int h = cl / F::kCols, c = cl % F::kCols;
+                uint4 w[F::kDigits];
+                if constexpr (std::is_same<T, double>::value) {
+                    // cos entries −= δ·sin entries, sin += δ·cos: the partner lane holds the
+                    // other half of the same wavenumbers
+                    unsigned long long U[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        const long long X = fixed_point<54>(x[i], e);
+                        const int other = __shfl_xor_sync(0xffffffffu, (int)(X >> 23), 16);
+                        const int turn = (__mulhi(other, dk[i]) + (1 << 14)) >> 15;
+                        U[i] = kDigitBias + (unsigned long long)(part < 2 ? X - turn : X + turn);
+                    }
+                    planes8(U, w);
+                } else {
+                    float y[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) y[i] = scale2(x[i], 8 - (e - 126));
+                    planes8(y, w);
+                }
+                const int64_t tile = bt + digit_part_base(r, part, S.col_tiles) + (int64_t)ct * steps + (kg >> 1);
+                uint8_t *dst = S.B + tile * digit_b_bytes<T>() + h * digit_half_bytes<T>() + (kg & 1) * 128 + (c & 7) * 16;
+                if (store)
+#pragma unroll
+                    for (int i = 0; i < F::kDigits; i++)
+                        *reinterpret_cast<uint4 *>(dst + ((i * F::kCols + c) >> 3) * 256) = w[i];
+            }
+        }
+    }
+}
+
+// ------------------------------------------------------------ product
+struct GemmDigitArgs {
+    const uint8_t *A, *B;
+    const DigitItem *items;
+    int nwork;
+    const DigitRing *rings;
+    const int *expo;
+    void *out;
+    int64_t jDim, frows;
+    int nitems, nvars, bk, iDim;
+    int *err;
+};
+
+constexpr int kDrainWarps = 16;
+constexpr int kDigitThreads = (kDrainWarps + 3) * 32;  // and 1 copying, 2 issuing warps
+
+// One CTA per SM (shared-memory ring, 2 × kSums·kCols accumulator columns).
+// Each accumulator half has its own issuing warp and warpgroup, so one half
+// computes while the other drains.
+template <typename T, bool kForward>
+__global__ void __launch_bounds__(kDigitThreads, 1) digit_gemm_kernel(GemmDigitArgs g) {
+    using F = DigitFormat<T>;
+    constexpr int ND = F::kDigits, W = F::kCols, ST = F::kStages;
+    constexpr uint32_t AB = digit_a_bytes<T>(), HB = digit_half_bytes<T>(), BB = digit_b_bytes<T>();
+    extern __shared__ __align__(1024) uint8_t dsm[];
+    __shared__ __align__(8) uint64_t full[ST], empty[ST], accf[2], acce[2], drain[2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile int quit;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_slot)), "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < ST; i++) {
+            bar_init(&full[i], 1);
+            bar_init(&empty[i], 2);
+        }
+        for (int h = 0; h < 2; h++) {
+            bar_init(&accf[h], 1);
+            bar_init(&acce[h], kDrainWarps * 16);
+            bar_init(&drain[h], 1);
+        }
+        quit = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+
+    if (warp == kDrainWarps) {
+        if (lane == 0) {
+            uint32_t it = 0;
+            bool ok = true;
+            DigitItem next = g.items[blockIdx.x];
+            for (int w = blockIdx.x; ok && w < g.nwork; w += gridDim.x) {
+                const DigitItem d = next;
+                if (w + gridDim.x < g.nwork) next = g.items[w + gridDim.x];
+                const uint8_t *a = g.A + d.a_tile * AB, *b = g.B + d.b_tile * BB;
+                for (int k = 0; k < d.steps; k++, it++) {
+                    const uint32_t s = it % ST;
+                    if (!(ok = bar_wait(&empty[s], ((it / ST) & 1) ^ 1, &quit))) break;
+                    const uint32_t dst = smem_addr(dsm + s * (AB + BB)), bar = smem_addr(&full[s]);
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(AB + BB) : "memory");
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                                 "l"(a + (size_t)k * AB), "r"(AB), "r"(bar)
+                                 : "memory");
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst + AB),
+                                 "l"(b + (size_t)k * BB), "r"(BB), "r"(bar)
+                                 : "memory");
+                }
+            }
+            if (!ok) {  // copies in flight land before the CTA leaves
+                int never = 0;
+                for (uint32_t q = it > ST ? it - ST : 0; q < it; q++) bar_wait(&full[q % ST], (q / ST) & 1, &never);
+            }
+        }
+    } else if (warp > kDrainWarps) {
+        if (lane == 0) {
+            const int h = warp - kDrainWarps - 1;
+            const uint32_t tacc = tmem + h * 256;
+            uint32_t it = 0, ch = 0;
+            bool ok = true;
+            int next = g.items[blockIdx.x].steps;
+            for (int w = blockIdx.x; ok && w < g.nwork; w += gridDim.x) {
+                const int steps = next;
+                if (w + gridDim.x < g.nwork) next = g.items[w + gridDim.x].steps;
+                const int nch = (steps + F::kChunk - 1) / F::kChunk, len = (steps + nch - 1) / nch;
+                for (int k0 = 0; ok && k0 < steps; k0 += len, ch++) {
+                    if (!(ok = bar_wait(&acce[h], (ch & 1) ^ 1, &quit))) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const int ke = min(len, steps - k0);
+                    for (int k = 0; k < ke; k++, it++) {
+                        const uint32_t s = it % ST;
+                        if (!(ok = bar_wait(&full[s], (it / ST) & 1, &quit))) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const uint32_t sa = smem_addr(dsm + s * (AB + BB));
+                        const uint64_t bd = operand_desc(sa + AB + h * HB);
+                        if constexpr (F::kSums > ND) {
+                            // digit i of the matrix times the data digits j ≤ kSums − 1 − i; the
+                            // first step writes D_1..D_6 by i = 1, then D_0, then adds the rest of i = 0
+                            static_assert(F::kSums == ND + 1, "D_6 is the only sum without a digit-0 term");
+                            const bool first = k == 0;
+                            if (first) {
+                                mma_f16(tacc + W, operand_desc(sa + kDigitPlane), bd, mma_idesc(ND * W), 0u);
+                                mma_f16(tacc, operand_desc(sa), bd, mma_idesc(W), 0u);
+                                mma_f16(tacc + W, operand_desc(sa), operand_desc(sa + AB + h * HB + W * 32), mma_idesc((ND - 1) * W), 1u);
+                            } else {
+                                mma_f16(tacc, operand_desc(sa), bd, mma_idesc(ND * W), 1u);
+                                mma_f16(tacc + W, operand_desc(sa + kDigitPlane), bd, mma_idesc(ND * W), 1u);
+                            }
+#pragma unroll
+                            for (int i = 2; i < ND; i++)
+                                mma_f16(tacc + i * W, operand_desc(sa + i * kDigitPlane), bd, mma_idesc((F::kSums - i) * W), 1u);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < ND; i++)
+                                mma_f16(tacc + i * W, operand_desc(sa + i * kDigitPlane), bd, mma_idesc((ND - i) * W),
+                                        (k > 0 || i > 0) ? 1u : 0u);
+                        }
+                        mma_commit(&empty[s]);
+                    }
+                    mma_commit(&accf[h]);
+                }
+            }
+            if (!ok) {
+                int never = 0;
+                mma_commit(&drain[h]);
+                bar_wait(&drain[h], 0, &never);
+            }
+        }
+    } else {
+        // two warpgroups per half, each with half of its columns
+        constexpr int WC = W / 2;
+        const int h = warp >> 3, cb = ((warp >> 2) & 1) * WC;
+        const uint32_t tacc = tmem + ((uint32_t)((warp & 3) * 32) << 16) + h * 256 + cb;
+        uint32_t ch = 0;
+        bool ok = true;
+        for (int w = blockIdx.x; ok && w < g.nwork; w += gridDim.x) {
+            const DigitItem d = g.items[w];
+            const int nch = (d.steps + F::kChunk - 1) / F::kChunk;
+            const DigitRing *r = g.rings + d.ring;
+            const int row = d.row_tile * kDigitRows + (warp & 3) * 32 + lane;
+            // forward rows: wavenumber k = 2·row + parity ≤ ri, stored at slot 2k − 1 (re), 2k (im)
+            const int k = 2 * row + (d.part & 1);
+            const int m = kForward ? max(2 * k - 1 + (d.part >> 1), 0) : row - r->lo[d.part];
+            const bool live = kForward ? k < r->n && (k > 0 || d.part == 0) : m >= 0 && m < r->cnt[d.part];
+            // lane c's column of this warp: its output base (−1 for padding) and exponent
+            auto col_base = [&](int c, int &e) -> int64_t {
+                constexpr int V0 = kDigitVariants - F::kVars;
+                const int col = (d.col_tile * 2 + h) * W + cb + c;
+                const int item = col / (kDigitGroup * F::kVars) * kDigitGroup + col % kDigitGroup;
+                const int var = col / kDigitGroup % F::kVars + V0;
+                e = 0;
+                if constexpr (kForward) {
+                    if (c >= WC || col >= g.nitems) return -1;
+                    e = g.expo[(size_t)col * g.iDim + d.ring];
+                    return (int64_t)col * g.frows + r->fofs;
+                }
+                if (c >= WC || item >= g.nitems) return -1;
+                e = g.expo[((size_t)var * g.nitems + item) * g.iDim + d.ring];
+                return ((int64_t)var * g.nvars + item / g.bk) * g.bk * g.jDim + (int64_t)g.bk * r->jofs + r->off[d.part] +
+                       (int64_t)(item % g.bk) * r->L;
+            };
+            using Acc = typename std::conditional<std::is_same<T, double>::value, long long, float>::type;
+            Acc V[WC];
+#pragma unroll
+            for (int c = 0; c < WC; c++) V[c] = 0;
+            for (int q = 0; q < nch; q++, ch++) {
+                if (!(ok = __all_sync(0xffffffffu, bar_wait(&accf[h], ch & 1, &quit)))) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int c0 = 0; c0 < WC; c0 += 8) {
+                    float D[F::kSums][8];
+#pragma unroll
+                    for (int s = 0; s < F::kSums; s++) tmem_ld8(tacc + s * W + c0, D[s]);
+                    tmem_wait_ld();
+                    if (c0 + 8 == WC) {
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        bar_arrive(&acce[h]);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 8; c++) {
+                        if constexpr (std::is_same<T, double>::value)
+                            V[c0 + c] += combine(D[0][c], D[1][c], D[2][c], D[3][c], D[4][c], D[5][c], D[6][c]);
+                        else
+                            V[c0 + c] += fmaf(fmaf(D[2][c], 0x1p-10f, D[1][c]), 0x1p-10f, D[0][c]);
+                    }
+                }
+            }
+            Acc *out = (Acc *)g.out;
+            const double inv_len = kForward ? 1.0 / (double)r->L : 0.0;
+#pragma unroll
+            for (int c0 = 0; c0 < WC; c0 += 32) {
+                int e;
+                const int64_t mine = col_base(c0 + lane, e);
+#pragma unroll
+                for (int c = 0; c < 32; c++) {
+                    if (c0 + c >= WC) break;
+                    const int64_t base = __shfl_sync(0xffffffffu, mine, c);
+                    Acc v = V[c0 + c];
+                    if constexpr (std::is_same<T, float>::value) {
+                        // doubled product of 2^-8 fixed-point operands at column scale 2^(e − 126)
+                        const int ce = __shfl_sync(0xffffffffu, e, c);
+                        v = ce == kNanColumn ? __int_as_float(0x7fc00000) : scale2(v, ce - 126 - 15);
+                    }
+                    if constexpr (kForward) {
+                        // folded points scaled by 2^(e − 1020): Σ = V 2^(e − 1020 − 53)
+                        const int ce = __shfl_sync(0xffffffffu, e, c);
+                        if (ok && live && base >= 0)
+                            ((double *)g.out)[base + m] = ce == kNanColumn ? __longlong_as_double(0x7ff8000000000000ll)
+                                                                           : fixed_to_double(v, ce + 1) * inv_len;
+                    } else {
+                        if (ok && live && base >= 0) out[base + m] = v;
+                    }
+                }
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0 && quit) *g.err = 1;
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+}
+
+// ------------------------------------------------------------ unfold
+// The four quadrant parts of one (ring, item, variant) row → its 4n points, in place
+template <typename T>
+__global__ void __launch_bounds__(128) digit_unfold_kernel(void *H, const DigitRing *rings, const int *expo, int r0,
+                                                           int nitems, int nvars, int bk, int iDim, int64_t jDim) {
+    using R = typename std::conditional<std::is_same<T, double>::value, long long, float>::type;
+    extern __shared__ __align__(16) unsigned char row_raw[];
+    R *row = reinterpret_cast<R *>(row_raw);
+    const int ring = r0 + (int)(gridDim.y - 1 - blockIdx.y);
+    const DigitRing &r = rings[ring];
+    const int n = r.n, L = r.L, shift = r.shift;
+    const int var = blockIdx.x / nitems + kDigitVariants - DigitFormat<T>::kVars, item = blockIdx.x % nitems;
+    R *h = (R *)H + ((int64_t)var * nvars + item / bk) * bk * jDim + (int64_t)bk * r.jofs + (int64_t)(item % bk) * L;
+    for (int i = threadIdx.x; i < L; i += blockDim.x) row[i] = h[i];
+    int e = 0;
+    if constexpr (std::is_same<T, double>::value) e = expo[((size_t)var * nitems + item) * iDim + ring];
+    __syncthreads();
+    auto put = [&](int p, R v) {
+        int l = p - shift;
+        if (l < 0) l += L;
+        if (l >= L) l -= L;
+        if constexpr (std::is_same<T, double>::value)
+            ((double *)h)[l] = e == kNanColumn ? __longlong_as_double(0x7ff8000000000000ll) : fixed_to_double(v, e);
+        else h[l] = v;
+    };
+    for (int m = threadIdx.x; m < n; m += blockDim.x) {
+        if (r.half == 0 && m == 0) {
+            const R a = row[0], b = row[n + 1], c = row[n], d = row[3 * n + n - 1];
+            put(0, a + b);
+            put(2 * n, a - b);
+            put(n, c + d);
+            put(3 * n, c - d);
+        } else {
+            const R ce = row[m], co = row[r.off[1] + m], se = row[r.off[2] + m - r.lo[2]], so = row[r.off[3] + m - r.lo[3]];
+            const R u = ce + co, v = ce - co, w = se + so, z = se - so;
+            const int hf = r.half;
+            put(m, u + w);
+            put(4 * n - hf - m, u - w);
+            put(2 * n - hf - m, v - z);
+            put(2 * n + m, v + z);
+        }
+    }
+}
+
+// ------------------------------------------------------------ forward split and turn
+// CTA = (ring of the span, group of 8 items).  Pass 1: a warp per item finds the
+// largest exponent of its ring; pass 2: a thread per (item, cos or sin parts, 8
+// quadrant positions) folds the four reflected points of each position in 62-bit
+// fixed point (the folded parts are below 2^(expo − 1020)) and writes both parities.
+struct FoldArgs {
+    const double *C;
+    const DigitRing *rings;
+    const int64_t *btile;
+    uint8_t *B;
+    int *expo;
+    int64_t jDim;
+    int r0, nitems, iDim, bk, col_tiles;
+};
+
+__global__ void __launch_bounds__(256, 2) digit_fold_kernel(FoldArgs S) {
+    using F = DigitFormat<double>;
+    __shared__ int ex[kDigitGroup];
+    const int ring = S.r0 + (int)(gridDim.y - 1 - blockIdx.y);
+    const DigitRing r = S.rings[ring];
+    const int grp = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto row_of = [&](int item) {
+        return S.C + (int64_t)(item / S.bk) * S.bk * S.jDim + (int64_t)S.bk * r.jofs + (int64_t)(item % S.bk) * r.L;
+    };
+    {
+        const int item = grp * kDigitGroup + warp;
+        uint32_t mx = 0;
+        if (item < S.nitems) {
+            const double2 *x = reinterpret_cast<const double2 *>(row_of(item));  // even offsets and lengths
+            for (int i = lane; i < r.L / 2; i += 32) {
+                const double2 v = x[i];
+                mx = max(mx, max(mag_bits(v.x), mag_bits(v.y)));
+            }
+        }
+        const int e = mag_expo<double>(__reduce_max_sync(0xffffffffu, mx));
+        if (lane == 0) {
+            ex[warp] = e;
+            if (item < S.nitems) S.expo[(size_t)item * S.iDim + ring] = e;
+        }
+    }
+    __syncthreads();
+    const int il = threadIdx.x & 7, item = grp * kDigitGroup + il;
+    if (item >= S.nitems) return;
+    const int sine = (threadIdx.x >> 3) & 1;
+    const double *x = row_of(item);
+    const int n = r.n, hf = r.half, L = r.L, e = ex[il];
+    const int ct = item / (2 * F::kCols), cl = item % (2 * F::kCols), h = cl / F::kCols, c = cl % F::kCols;
+    const int64_t bt = S.btile[ring] + (int64_t)ct * r.tm;
+    for (int mg = threadIdx.x >> 4; mg < 2 * r.tm; mg += 16) {
+        unsigned long long even[8], odd[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int m = mg * 8 + i;
+            long long s = 0, d = 0;
+            if (m < n + 1 - hf) {
+                auto at = [&](int p) {
+                    int l = p - r.shift;
+                    if (l < 0) l += L;
+                    if (l >= L) l -= L;
+                    return fixed_point<60>(x[l], e);
+                };
+                // the axis positions hold two points, not four: m = 0 (θ = 0, π), m = n (θ = ±π/2)
+                const bool axis0 = hf == 0 && m == 0, axis1 = hf == 0 && m == n;
+                const long long a = at(m), b = axis0 ? 0 : at(4 * n - hf - m);
+                const long long f = axis1 ? 0 : at(2 * n - hf - m), g = (axis0 || axis1) ? 0 : at(2 * n + m);
+                s = sine ? a - b : a + b;
+                d = sine ? f - g : f + g;
+            }
+            // cos: even s + d, odd s − d; sin: even s − d, odd s + d; 62 → 54 bits
+            const long long u = s + d, w = s - d;
+            even[i] = kDigitBias + (unsigned long long)(((sine ? w : u) + 128) >> 8);
+            odd[i] = kDigitBias + (unsigned long long)(((sine ? u : w) + 128) >> 8);
+        }
+        uint4 w[6];
+        const int64_t tile = bt + (int64_t)(2 * sine) * S.col_tiles * r.tm + (mg >> 1);
+        uint8_t *dst = S.B + tile * digit_b_bytes<double>() + h * digit_half_bytes<double>() + (mg & 1) * 128 + (c & 7) * 16;
+        planes8(even, w);
+#pragma unroll
+        for (int i = 0; i < 6; i++) *reinterpret_cast<uint4 *>(dst + ((i * F::kCols + c) >> 3) * 256) = w[i];
+        dst += (int64_t)S.col_tiles * r.tm * digit_b_bytes<double>();
+        planes8(odd, w);
+#pragma unroll
+        for (int i = 0; i < 6; i++) *reinterpret_cast<uint4 *>(dst + ((i * F::kCols + c) >> 3) * 256) = w[i];
+    }
+}
+
+// X_k ← X_k e^{−iδ_k}: the forward coefficients at the reference's rounded angles
+__global__ void __launch_bounds__(128) digit_turn_kernel(double *Fp, const DigitRing *rings, const int *delta, int64_t frows, int r0) {
+    const DigitRing &r = rings[r0 + blockIdx.y];
+    double *f = Fp + (int64_t)blockIdx.x * frows + r.fofs;
+    for (int k = 1 + threadIdx.x; k <= r.kmax; k += blockDim.x) {
+        const double d = (double)delta[r.dofs + k - 1] * 0x1p-70;
+        const double re = f[2 * k - 1], im = f[2 * k];
+        f[2 * k - 1] = fma(d, im, re);
+        f[2 * k] = fma(-d, re, im);
+    }
+}
+
+// ------------------------------------------------------------ host
+// Least items (variables × Chebyshev modes) of a grid the products serve: FP64 grids
+// of 3 items already run ring_inverse 4.2× (6 cells), 11.7× (37) and 3.3× (200 cells)
+// faster than the FFT kernels, so the line lies at one.
+constexpr int kDigitMinItems = 1;
+// bound of a grid's matrix digits (both directions: 4.3 GB at 200 cells, growing with
+// the cube of the ring count); larger grids keep the FFT kernels
+constexpr size_t kDigitTableBytes = (size_t)16 << 30;
+// spectra digits of one span of rings; larger grids take several spans
+constexpr int64_t kDigitScratchBytes = (int64_t)1 << 30;
+template <typename T>
+constexpr size_t digit_smem() { return (size_t)DigitFormat<T>::kStages * (digit_a_bytes<T>() + digit_b_bytes<T>()); }
+
+template <typename V>
+static bool upload(ss_grid *g, const V **dst, const std::vector<V> &src) {
+    void *p = nullptr;
+    if (cudaMalloc(&p, std::max<size_t>(src.size() * sizeof(V), 16)) != cudaSuccess) { cudaGetLastError(); return false; }
+    g->allocs.push_back(p);
+    if (!src.empty() && cudaMemcpy(p, src.data(), src.size() * sizeof(V), cudaMemcpyHostToDevice) != cudaSuccess) return false;
+    *dst = (const V *)p;
+    return true;
+}
+
+template <typename T>
+static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
+    using F = DigitFormat<T>;
+    DigitPlan &D = g->digit;
+    const int nr = (int)g->d.iDim;
+    std::vector<DigitRing> rings(nr);
+    int64_t cosn = 0, atiles = 0, aftiles = 0, dn = 0;
+    for (int i = 0; i < nr; i++) {
+        DigitRing &r = rings[i];
+        std::memset(&r, 0, sizeof r);
+        r.n = rd[i].ri + 1;
+        r.L = rd[i].L;
+        r.half = r.n & 1;
+        r.shift = r.half ? (r.n - 3) / 2 : (r.n - 2) / 2;
+        r.kmax = rd[i].kmax;
+        r.te = (r.kmax / 2 + 1 + 15) / 16;
+        r.to = std::max(1, ((r.kmax + 1) / 2 + 15) / 16);
+        const int rows = r.n + 1 - r.half;
+        r.rt = (rows + kDigitRows - 1) / kDigitRows;
+        const int n = r.n;
+        if (r.half) {
+            for (int q = 0; q < 4; q++) { r.cnt[q] = n; r.lo[q] = 0; r.off[q] = q * n; }
+        } else {
+            const int cnt[4] = {n + 1, n, n - 1, n}, lo[4] = {0, 0, 1, 1}, off[4] = {0, n + 1, 2 * n + 1, 3 * n};
+            for (int q = 0; q < 4; q++) { r.cnt[q] = cnt[q]; r.lo[q] = lo[q]; r.off[q] = off[q]; }
+        }
+        r.jofs = rd[i].jofs;
+        r.fofs = rd[i].fofs;
+        r.cosofs = cosn;
+        cosn += 2 * n + 1;
+        r.a_tile = atiles;
+        atiles += (int64_t)r.rt * 2 * (r.te + r.to);
+        r.tm = (rows + 15) / 16;
+        r.rtf = ((n + 1) / 2 + kDigitRows - 1) / kDigitRows;
+        r.af_tile = aftiles;
+        aftiles += (int64_t)4 * r.rtf * r.tm;
+        r.dofs = dn;
+        dn += rd[i].ri;
+    }
+    // δ_k = fl(k·ymin) − k·(exact ymin): the product's rounding (exact by fma) and k times ymin's own
+    std::vector<int> delta(std::max<int64_t>(dn, 1), 0);
+    for (int i = 0; i < nr; i++) {
+        const int ri = rd[i].ri, L = rd[i].L;
+        const double ymin = 0.5 * (2 * 3.14159265358979323846 / L) * (ri - 1);
+        const long double exact = 3.14159265358979323846264338327950288L * (ri - 1) / L;
+        const double dy = (double)((long double)ymin - exact);
+        for (int k = 1; k <= ri; k++) {
+            const double a = k * ymin;
+            delta[rings[i].dofs + k - 1] = (int)std::lrint(std::ldexp(k * dy - std::fma((double)k, ymin, -a), 70));
+        }
+    }
+    const int ncol = (g->nitems + kDigitGroup - 1) / kDigitGroup * kDigitGroup * F::kVars;
+    D.col_tiles = (ncol + 2 * F::kCols - 1) / (2 * F::kCols);
+    D.col_tiles_fwd = (g->nitems + 2 * F::kCols - 1) / (2 * F::kCols);
+    const size_t abytes = (size_t)atiles * digit_a_bytes<T>(), afbytes = (size_t)aftiles * digit_a_bytes<T>();
+    if (abytes + afbytes > kDigitTableBytes) return SS_OK;
+    double *cosq = nullptr;
+    const size_t mark = g->allocs.size();
+    auto give_up = [&]() {  // the device has no room for the tables: the FFT kernels serve
+        cudaGetLastError();
+        if (cosq) cudaFree(cosq);
+        while (g->allocs.size() > mark) { cudaFree(g->allocs.back()); g->allocs.pop_back(); }
+        D = DigitPlan{};
+        return SS_OK;
+    };
+    // spans of rings, largest first, whose B digits fit the scratch
+    int64_t btiles = 0;
+    auto make_set = [&](int lo, int hi, bool fwd, DigitSet &set) {
+        const int tiles = fwd ? D.col_tiles_fwd : D.col_tiles;
+        std::vector<DigitItem> items;
+        std::vector<int64_t> btile(nr, 0);
+        int r = hi;
+        while (r > lo) {
+            DigitSpan sp{0, r, (int)items.size(), 0};
+            int64_t used = 0;
+            while (r > lo) {
+                const DigitRing &q = rings[r - 1];
+                const int64_t need = (int64_t)tiles * (fwd ? 4 * q.tm : 2 * (q.te + q.to));
+                if (used > 0 && (used + need) * digit_b_bytes<T>() > kDigitScratchBytes) break;
+                r--;
+                btile[r] = used;
+                for (int part = 0; part < 4; part++)
+                    for (int ct = 0; ct < tiles; ct++)
+                        for (int rt = 0; rt < (fwd ? q.rtf : q.rt); rt++) {
+                            const int steps = fwd ? q.tm : digit_steps(q, part);
+                            DigitItem it{};
+                            if (fwd) {
+                                it.a_tile = q.af_tile + ((int64_t)part * q.rtf + rt) * steps;
+                                it.b_tile = used + ((int64_t)part * tiles + ct) * steps;
+                            } else {
+                                it.a_tile = q.a_tile + digit_part_base(q, part, q.rt) + (int64_t)rt * steps;
+                                it.b_tile = used + digit_part_base(q, part, tiles) + (int64_t)ct * steps;
+                            }
+                            it.ring = r; it.part = part; it.row_tile = rt; it.col_tile = ct; it.steps = steps;
+                            items.push_back(it);
+                        }
+                used += need;
+            }
+            sp.r0 = r;
+            sp.items = (int)items.size() - sp.item0;
+            btiles = std::max(btiles, used);
+            set.spans.push_back(sp);
+        }
+        return upload(g, &set.items, items) && upload(g, &set.btile, btile);
+    };
+    const DigitRing *dr = nullptr;
+    if (!upload(g, &dr, rings)) return give_up();
+    D.rings = const_cast<DigitRing *>(dr);
+    const int *dd = nullptr;
+    if (!upload(g, &dd, delta)) return give_up();
+    D.delta = const_cast<int *>(dd);
+    if (!make_set(0, nr, false, D.whole) || !make_set(0, nr, true, D.whole_fwd)) return give_up();
+    D.chunks.resize(g->chunk_r0.size() - 1);
+    D.chunks_fwd.resize(g->chunk_r0.size() - 1);
+    for (size_t c = 0; c + 1 < g->chunk_r0.size(); c++)
+        if (!make_set(g->chunk_r0[c], g->chunk_r0[c + 1], false, D.chunks[c]) ||
+            !make_set(g->chunk_r0[c], g->chunk_r0[c + 1], true, D.chunks_fwd[c]))
+            return give_up();
+    void *p = nullptr;
+    if (cudaMalloc(&p, afbytes) != cudaSuccess) return give_up();
+    g->allocs.push_back(p);
+    D.Af = p;
+    if (cudaMalloc(&p, abytes) != cudaSuccess) return give_up();
+    g->allocs.push_back(p);
+    D.A = p;
+    if (cudaMalloc(&p, (size_t)btiles * digit_b_bytes<T>()) != cudaSuccess) return give_up();
+    g->allocs.push_back(p);
+    D.B = p;
+    if (cudaMalloc(&p, (size_t)kDigitVariants * g->nitems * nr * sizeof(int)) != cudaSuccess) return give_up();
+    g->allocs.push_back(p);
+    D.expo = (int *)p;
+    if (cudaMalloc((void **)&cosq, (size_t)cosn * 8) != cudaSuccess) return give_up();
+    if (cudaHostAlloc((void **)&D.err, sizeof(int), cudaHostAllocMapped) != cudaSuccess) { D.err = nullptr; return give_up(); }
+    *D.err = 0;
+    digit_cos_kernel<<<nr, 128, 0, g->stream>>>(D.rings, cosq);
+    digit_matrix_kernel<T, false><<<dim3(nr, 8), 256, 0, g->stream>>>(D.rings, cosq, (uint8_t *)D.A);
+    digit_matrix_kernel<T, true><<<dim3(nr, 8), 256, 0, g->stream>>>(D.rings, cosq, (uint8_t *)D.Af);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+    cudaFree(cosq);
+    cosq = nullptr;
+    CUDA_TRY(e);
+    CUDA_TRY(cudaFuncSetAttribute(digit_gemm_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digit_smem<T>()));
+    CUDA_TRY(cudaFuncSetAttribute(digit_gemm_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digit_smem<T>()));
+    D.on = true;
+    return SS_OK;
+}
+
+int32_t digit_build(ss_grid *g, const std::vector<RingDesc> &rings) {
+    if (!g->rlz || g->tl != TL_F64) return SS_OK;
+    int least = kDigitMinItems;
+    if (const char *e = std::getenv("SS_RING_DIGITS")) {  // tuning override: the least item count, 0 for never
+        least = std::atoi(e);
+        if (least <= 0) return SS_OK;
+    }
+    if (g->nitems < least) return SS_OK;
+    // binary64 sums of a ring stay below 2^63 for n ≤ 1023 (64-bit fixed point at 2^-52 of the column scale)
+    if (rings.back().ri + 1 > (g->tl == TL_F64 ? 1023 : 2047)) return SS_OK;
+    return g->tl == TL_F64 ? build<double>(g, rings) : build<float>(g, rings);
+}
+
+void digit_free(ss_grid *g) {
+    if (g->digit.err) cudaFreeHost(g->digit.err);
+    g->digit.err = nullptr;
+}
+
+template <typename T>
+static int32_t inverse(ss_grid *g, cudaStream_t st, const DigitSet &set, int *launches) {
+    const DigitPlan &D = g->digit;
+    const ss_dims &d = g->d;
+    const int groups = (g->nitems + kDigitGroup - 1) / kDigitGroup;
+    for (const DigitSpan &sp : set.spans) {
+        const int nr = sp.r1 - sp.r0;
+        SplitArgs S{g->G, D.rings, set.btile, (uint8_t *)D.B, D.expo, D.delta, g->frows, sp.r0, g->nitems, (int)d.iDim, D.col_tiles};
+        digit_split_kernel<T><<<dim3(groups, nr), 256, 0, st>>>(S);
+        GemmDigitArgs A{(const uint8_t *)D.A, (const uint8_t *)D.B, set.items + sp.item0, sp.items, D.rings, D.expo, g->H,
+                        d.jDim, g->frows, g->nitems, (int)d.nvars, (int)d.b_kDim, (int)d.iDim, D.err};
+        digit_gemm_kernel<T, false><<<std::min(g->sms, sp.items), kDigitThreads, digit_smem<T>(), st>>>(A);
+        *launches += 2;
+        CUDA_TRY(cudaGetLastError());
+        if (D.columns.on) continue;  // digit_columns_inverse reads the parts
+        const size_t row = (size_t)4 * (sp.r1 + g->pOL + 1) * sizeof(T);
+        digit_unfold_kernel<T><<<dim3(DigitFormat<T>::kVars * g->nitems, nr), 128, row, st>>>(
+            g->H, D.rings, D.expo, sp.r0, g->nitems, (int)d.nvars, (int)d.b_kDim, (int)d.iDim, d.jDim);
+        CUDA_TRY(cudaGetLastError());
+        *launches += 1;
+    }
+    return SS_OK;
+}
+
+int32_t digit_ring_forward(ss_grid *g, cudaStream_t st, int chunk, int *launches) {
+    const DigitPlan &D = g->digit;
+    const DigitSet &set = chunk < 0 ? D.whole_fwd : D.chunks_fwd[chunk];
+    const ss_dims &d = g->d;
+    const int groups = (g->nitems + kDigitGroup - 1) / kDigitGroup;
+    for (const DigitSpan &sp : set.spans) {
+        const int nr = sp.r1 - sp.r0;
+        FoldArgs S{(const double *)g->C, D.rings, set.btile, (uint8_t *)D.B, D.expo, d.jDim, sp.r0, g->nitems, (int)d.iDim,
+                   (int)d.b_kDim, D.col_tiles_fwd};
+        digit_fold_kernel<<<dim3(groups, nr), 256, 0, st>>>(S);
+        GemmDigitArgs A{(const uint8_t *)D.Af, (const uint8_t *)D.B, set.items + sp.item0, sp.items, D.rings, D.expo, g->F,
+                        d.jDim, g->frows, g->nitems, (int)d.nvars, (int)d.b_kDim, (int)d.iDim, D.err};
+        digit_gemm_kernel<double, true><<<std::min(g->sms, sp.items), kDigitThreads, digit_smem<double>(), st>>>(A);
+        digit_turn_kernel<<<dim3(g->nitems, nr), 128, 0, st>>>((double *)g->F, D.rings, D.delta, g->frows, sp.r0);
+        CUDA_TRY(cudaGetLastError());
+        *launches += 3;
+    }
+    return SS_OK;
+}
+
+int32_t digit_ring_inverse(ss_grid *g, cudaStream_t st, int chunk, int *launches) {
+    const DigitSet &set = chunk < 0 ? g->digit.whole : g->digit.chunks[chunk];
+    return g->tl == TL_F64 ? inverse<double>(g, st, set, launches) : inverse<float>(g, st, set, launches);
+}
+
+}  // namespace ss

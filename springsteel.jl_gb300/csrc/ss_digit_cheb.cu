@@ -1,0 +1,411 @@
+// ss_digit_cheb.cu — the Chebyshev column stages of binary64 RLZ grids on the
+// tensor cores, by exact products of digit slices (ss_digit.cu).
+//
+// CA (Γ fold), the CIx recurrence and the DCT-I are linear, so an output column of
+// derivative order d is u = M_d b with M_d = IDCT·(D/dscale)^d·Γ composed on the
+// host (N × b_kDim).  The column inverse reads the ring stage's quadrant parts as
+// they are (64-bit fixed point with one exponent per ring, mode and output),
+// forms the four reflected points of each quadrant position by integer
+// additions, cuts each column into digits at its own exponent and multiplies by
+// the matrix digits, which stay in shared memory.  ∂z and ∂zz share f's digits.
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "ss_digit.h"
+#include "ss_digit_dev.cuh"
+#include "ss_grid.h"
+#include "ss_internal.h"
+
+using namespace ss;
+
+#define CUDA_TRY(expr)                                                                      \
+    do {                                                                                    \
+        cudaError_t _e = (expr);                                                            \
+        if (_e != cudaSuccess) {                                                            \
+            set_error("%s failed: %s", #expr, cudaGetErrorString(_e));                      \
+            return (_e == cudaErrorMemoryAllocation) ? SS_OUT_OF_MEMORY : SS_CUDA_ERROR;   \
+        }                                                                                   \
+    } while (0)
+
+namespace ss {
+
+constexpr int kZ = 32;                      // matrix rows (levels) of one product
+constexpr int kZStep = 6 * kZ * 32;         // bytes of a K-step of matrix digits: 6 planes × 32 rows × 16
+constexpr int kColThreads = 17 * 32;        // 8 producing, 8 draining, 1 issuing warp
+constexpr int kMaxModes = 96;               // six K-steps keep every digit sum an exact integer
+constexpr int kRowExpo = 8;                 // row-exponent slots (producers run at most 4 variants ahead)
+
+struct ColumnArgs {
+    const void *H;
+    double *phys;
+    const DigitRing *rings;
+    const int *expo;          // [variant][item][ring]
+    const uint8_t *M;         // [var][3][zblocks][steps] matrix digits
+    const int *mexpo;         // [var][3][32·zblocks]
+    const int2 *blocks;       // (ring, first quadrant position) of every 32-position block
+    int nblocks;
+    int N, bk, nvars, nitems, iDim, steps, zblocks, buffers;
+    int64_t jDim, np;
+    int *err;
+};
+
+__device__ __forceinline__ void producers_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void st_global_32B(double *p, const double (&v)[4]) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3]) : "memory");
+}
+
+// grid = (CTAs per variable, variables); a CTA walks (block of 32 quadrant
+// positions = 128 columns, ring output), outputs fastest
+__global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArgs g) {
+    extern __shared__ __align__(1024) uint8_t dsm[];
+    __shared__ __align__(8) uint64_t afull[2], aempty[2], accf[2], acce[2], drain;
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile int quit;
+    __shared__ int row_expo[kRowExpo][128];
+    __shared__ int mode_expo[kMaxModes];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int v = blockIdx.y, KS = g.steps, nb = g.buffers;
+    const int jobs_bytes = KS * kZStep;
+    uint8_t *sM = dsm;                                                   // 3 × zblocks × jobs_bytes
+    uint8_t *sA = sM + (size_t)3 * g.zblocks * jobs_bytes;               // nb × KS × 24 KB
+    long long *stage = reinterpret_cast<long long *>(sA + (size_t)nb * KS * 6 * kDigitPlane);  // bk × 128
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_slot)), "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2; i++) {
+            bar_init(&afull[i], 256);
+            bar_init(&aempty[i], 1);
+            bar_init(&accf[i], 1);
+            bar_init(&acce[i], 256);
+        }
+        bar_init(&drain, 1);
+        quit = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    {
+        const uint4 *src = reinterpret_cast<const uint4 *>(g.M + (size_t)v * 3 * g.zblocks * jobs_bytes);
+        for (int i = threadIdx.x; i < 3 * g.zblocks * jobs_bytes / 16; i += blockDim.x) reinterpret_cast<uint4 *>(sM)[i] = src[i];
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    const int nitem = blockIdx.x < g.nblocks ? ((g.nblocks - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * kDigitVariants : 0;
+
+    if (warp < 8) {
+        // ---- producers: parts → points → digits
+        const long long *H = (const long long *)g.H;
+        bool ok = true;
+        for (int it = 0; ok && it < nitem; it++) {
+            const int2 blk = g.blocks[blockIdx.x + it / kDigitVariants * gridDim.x];
+            const int var = it % kDigitVariants;
+            const DigitRing *r = g.rings + blk.x;
+            const int n = r->n, m = blk.y + lane;
+            const bool edge = r->half == 0 && m == 0, live = m < n;
+            int *rex = row_expo[it % kRowExpo];
+            // offsets of the four parts at this position (edge: Ce, Co at 0, Ce and So at π/2)
+            const int o0 = m, o1 = r->off[1] + m;
+            const int o2 = edge ? n : r->off[2] + m - r->lo[2], o3 = edge ? 4 * n - 1 : r->off[3] + m - r->lo[3];
+            const int64_t base = ((int64_t)var * g.nvars + v) * g.bk * g.jDim + (int64_t)g.bk * r->jofs;
+            const int *ex = g.expo + ((size_t)var * g.nitems + (size_t)v * g.bk) * g.iDim + blk.x;
+            if (threadIdx.x < 128) rex[threadIdx.x] = 0;
+            producers_sync();
+            int mx[4] = {0, 0, 0, 0};
+            for (int i = warp; i < g.bk; i += 8) {
+                const long long *h = H + base + (int64_t)i * r->L;
+                const int e = ex[(size_t)i * g.iDim];
+                if (lane == 0) mode_expo[i] = e;
+                long long a = 0, b = 0, c = 0, d = 0;
+                if (live) { a = h[o0]; b = h[o1]; c = h[o2]; d = h[o3]; }
+                long long p[4];
+                if (edge) {
+                    p[0] = a + b; p[2] = a - b; p[1] = c - d; p[3] = c + d;
+                } else {
+                    const long long u = a + b, w = c + d, x = a - b, z = c - d;
+                    p[0] = u + w; p[1] = u - w; p[2] = x - z; p[3] = x + z;
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    stage[(size_t)i * 128 + q * 32 + lane] = p[q];
+                    const unsigned long long mag = p[q] < 0 ? 0ull - (unsigned long long)p[q] : (unsigned long long)p[q];
+                    // |p| 2^(e − 1074) < 2^(mx − 1074)
+                    if (mag) mx[q] = max(mx[q], e == kNanColumn ? kNanColumn : e + 64 - __clzll((long long)mag));
+                    else if (e == kNanColumn) mx[q] = kNanColumn;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (mx[q]) atomicMax(&rex[q * 32 + lane], mx[q]);
+            producers_sync();
+            const int buf = it % nb;
+            if (!(ok = bar_wait(&aempty[buf], ((it / nb) & 1) ^ 1, &quit))) break;
+            uint8_t *A = sA + (size_t)buf * KS * 6 * kDigitPlane;
+            const int row = threadIdx.x & 127;
+            const int er = rex[row];
+            for (int kg = threadIdx.x >> 7; kg < 2 * KS; kg += 2) {
+                unsigned long long U[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const int mode = kg * 8 + i;
+                    long long X = 0;
+                    if (mode < g.bk && er != kNanColumn) {
+                        const long long V = stage[(size_t)mode * 128 + row];
+                        const int s = mode_expo[mode] + 54 - er;  // |V 2^s| < 2^54
+                        if (V != 0) X = s >= 0 ? V << s : (s > -63 ? ((V >> (-s - 1)) + 1) >> 1 : 0);
+                    }
+                    U[i] = kDigitBias + (unsigned long long)X;
+                }
+                uint4 w[6];
+                planes8(U, w);
+                uint8_t *dst = A + (kg >> 1) * 6 * kDigitPlane + (row >> 3) * 256 + (kg & 1) * 128 + (row & 7) * 16;
+#pragma unroll
+                for (int i = 0; i < 6; i++) *reinterpret_cast<uint4 *>(dst + i * kDigitPlane) = w[i];
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            bar_arrive(&afull[buf]);
+            producers_sync();  // the staged points are free again
+        }
+    } else if (warp == 16) {
+        // ---- issuer
+        if (lane == 0) {
+            bool ok = true;
+            uint32_t job = 0;
+            for (int it = 0; ok && it < nitem; it++) {
+                const int buf = it % nb;
+                if (!(ok = bar_wait(&afull[buf], (it / nb) & 1, &quit))) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t sa0 = smem_addr(sA) + buf * KS * 6 * kDigitPlane;
+                const int nd = it % kDigitVariants == 0 ? 3 : 1;
+                for (int q = 0; ok && q < nd * g.zblocks; q++, job++) {
+                    const int t = job & 1;
+                    if (!(ok = bar_wait(&acce[t], ((job >> 1) & 1) ^ 1, &quit))) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t tacc = tmem + t * 256;
+                    for (int k = 0; k < KS; k++) {
+                        const uint32_t sa = sa0 + k * 6 * kDigitPlane, sb = smem_addr(sM) + (q * KS + k) * kZStep;
+                        const uint64_t bd = operand_desc(sb);
+                        if (k == 0) {  // D_1..D_6, then D_0, then the rest of digit 0 (as in digit_gemm)
+                            mma_f16(tacc + kZ, operand_desc(sa + kDigitPlane), bd, mma_idesc(6 * kZ), 0u);
+                            mma_f16(tacc, operand_desc(sa), bd, mma_idesc(kZ), 0u);
+                            mma_f16(tacc + kZ, operand_desc(sa), operand_desc(sb + kZ * 32), mma_idesc(5 * kZ), 1u);
+                        } else {
+                            mma_f16(tacc, operand_desc(sa), bd, mma_idesc(6 * kZ), 1u);
+                            mma_f16(tacc + kZ, operand_desc(sa + kDigitPlane), bd, mma_idesc(6 * kZ), 1u);
+                        }
+#pragma unroll
+                        for (int i = 2; i < 6; i++)
+                            mma_f16(tacc + i * kZ, operand_desc(sa + i * kDigitPlane), bd, mma_idesc((7 - i) * kZ), 1u);
+                    }
+                    mma_commit(&accf[t]);
+                }
+                if (ok) mma_commit(&aempty[buf]);
+            }
+            if (!ok) {
+                int never = 0;
+                mma_commit(&drain);
+                bar_wait(&drain, 0, &never);
+            }
+        }
+    } else {
+        // ---- drain: thread = (column, 16 levels)
+        const int zh = ((warp >> 2) & 1) * 16;
+        const int quad = warp & 3, row = quad * 32 + lane;
+        const uint32_t lanes = (uint32_t)(quad * 32) << 16;
+        const bool vec = g.N % 4 == 0;
+        uint32_t job = 0;
+        bool ok = true;
+        for (int it = 0; ok && it < nitem; it++) {
+            const int2 blk = g.blocks[blockIdx.x + it / kDigitVariants * gridDim.x];
+            const int var = it % kDigitVariants;
+            const DigitRing *r = g.rings + blk.x;
+            const int n = r->n, L = r->L, hf = r->half, m = blk.y + lane;
+            const bool edge = hf == 0 && m == 0, live = m < n;
+            int p = quad == 0 ? m : (quad == 1 ? 4 * n - hf - m : (quad == 2 ? 2 * n - hf - m : 2 * n + m));
+            if (edge) p = quad == 0 ? 0 : (quad == 1 ? 3 * n : (quad == 2 ? 2 * n : n));
+            int l = p - r->shift;
+            if (l < 0) l += L;
+            if (l >= L) l -= L;
+            const int64_t col = r->jofs + l;
+            const int nd = var == 0 ? 3 : 1;
+            for (int d = 0; ok && d < nd; d++) {
+                const int slot = var == 0 ? (d == 0 ? 0 : 4 + d) : (var == 1 ? 3 : (var == 2 ? 4 : var - 2));
+                double *dst = g.phys + ((size_t)slot * g.nvars + v) * g.np + col * g.N;
+                for (int zb = 0; zb < g.zblocks; zb++, job++) {
+                    const int t = job & 1;
+                    if (!(ok = __all_sync(0xffffffffu, bar_wait(&accf[t], (job >> 1) & 1, &quit)))) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const int er = row_expo[it % kRowExpo][row];
+                    const int z0 = zb * kZ + zh;
+                    const int *me = g.mexpo + ((size_t)v * 3 + d) * g.zblocks * kZ + z0;
+                    const uint32_t tacc = tmem + lanes + t * 256 + zh;
+#pragma unroll
+                    for (int c0 = 0; c0 < 16; c0 += 8) {
+                        float D[7][8];
+#pragma unroll
+                        for (int s = 0; s < 7; s++) tmem_ld8(tacc + s * kZ + c0, D[s]);
+                        tmem_wait_ld();
+                        if (c0 == 8) {
+                            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                            bar_arrive(&acce[t]);
+                        }
+                        double o[8];
+#pragma unroll
+                        for (int c = 0; c < 8; c++) {
+                            const long long V = combine(D[0][c], D[1][c], D[2][c], D[3][c], D[4][c], D[5][c], D[6][c]);
+                            // V 2^(er − 1074 + mexpo − 53)
+                            o[c] = er == kNanColumn ? __longlong_as_double(0x7ff8000000000000ll)
+                                                    : fixed_to_double(V, er + me[c0 + c] - 53);
+                        }
+                        if (live) {
+                            if (vec) {
+#pragma unroll
+                                for (int c = 0; c < 8; c += 4)
+                                    if (z0 + c0 + c < g.N) {
+                                        const double q4[4] = {o[c], o[c + 1], o[c + 2], o[c + 3]};
+                                        st_global_32B(dst + z0 + c0 + c, q4);
+                                    }
+                            } else {
+#pragma unroll
+                                for (int c = 0; c < 8; c++)
+                                    if (z0 + c0 + c < g.N) dst[z0 + c0 + c] = o[c];
+                            }
+                        }
+                    }
+                }
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0 && quit) *g.err = 1;
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+}
+
+// ------------------------------------------------------------ host
+// balanced digits of x·2^(53 − e), |x| < 2^e (53-bit fixed point), most significant first
+static void host_digits(double x, int e, int (&d)[6]) {
+    long long X = std::llrint(std::ldexp(x, 53 - e));
+    for (int i = 5; i > 0; i--) {
+        long long q = ((X + 256) & 511) - 256;
+        d[i] = (int)q;
+        X = (X - q) / 512;
+    }
+    d[0] = (int)X;
+}
+
+static size_t column_smem(int steps, int zblocks, int bk, int buffers) {
+    return (size_t)3 * zblocks * steps * kZStep + (size_t)buffers * steps * 6 * kDigitPlane + (size_t)bk * 128 * 8;
+}
+
+int32_t digit_columns_build(ss_grid *g, const std::vector<ChebHost> &cheb) {
+    DigitPlan &P = g->digit;
+    if (!P.on || g->tl != TL_F64) return SS_OK;
+    const int N = (int)g->d.kDim, bk = (int)g->d.b_kDim, nv = (int)g->d.nvars;
+    DigitColumns &Q = P.columns;
+    Q.steps = (bk + 15) / 16;
+    Q.zblocks = (N + kZ - 1) / kZ;
+    if (bk > kMaxModes) return SS_OK;
+    constexpr size_t kLimit = 232448 - 8192;  // 227 KB less the static part
+    Q.buffers = column_smem(Q.steps, Q.zblocks, bk, 2) <= kLimit ? 2 : 1;
+    if (column_smem(Q.steps, Q.zblocks, bk, Q.buffers) > kLimit) return SS_OK;
+    const int job = Q.steps * kZStep;
+    std::vector<uint8_t> M((size_t)nv * 3 * Q.zblocks * job, 0);
+    std::vector<int> E((size_t)nv * 3 * Q.zblocks * kZ, 0);
+    for (int v = 0; v < nv; v++) {
+        const ChebHost &c = cheb[v];
+        const int ne = (N + 1) / 2, no = std::max(N / 2, 1);
+        std::vector<double> X((size_t)N * bk, 0.0), Y((size_t)N * bk);
+        for (int k = 0; k < N; k++)
+            for (int i = 0; i < bk; i++) {
+                double s = k == i ? 1.0 : 0.0;
+                for (int p = 0; p < c.nrank; p++) s += c.gv[(size_t)p * N + k] * c.gu[(size_t)p * bk + i];
+                X[(size_t)k * bk + i] = s;
+            }
+        for (int d = 0; d < 3; d++) {
+            if (d > 0) {
+                for (int k = 0; k < N; k++)
+                    for (int i = 0; i < bk; i++) {
+                        double s = 0.0;
+                        for (int m = k + 1; m < N; m += 2) s += 2.0 * m * X[(size_t)m * bk + i];
+                        Y[(size_t)k * bk + i] = s / c.dscale;
+                    }
+                X.swap(Y);
+            }
+            for (int z = 0; z < N; z++) {
+                const int j = std::min(z, N - 1 - z);  // inv_e, inv_o hold the first half of the levels
+                const double so = z == j ? 1.0 : -1.0;
+                std::vector<double> row(bk);
+                double top = 0.0;
+                for (int i = 0; i < bk; i++) {
+                    double a = 0.0, b = 0.0;
+                    for (int k = 0; k < N; k += 2) a += c.inv_e[(size_t)j * ne + k / 2] * X[(size_t)k * bk + i];
+                    for (int k = 1; k < N; k += 2) b += c.inv_o[(size_t)j * no + k / 2] * X[(size_t)k * bk + i];
+                    row[i] = a + so * b;
+                    top = std::max(top, std::fabs(row[i]));
+                }
+                int e = 0;
+                if (top > 0.0) std::frexp(top, &e);
+                const int zb = z / kZ, zr = z % kZ;
+                E[(((size_t)v * 3 + d) * Q.zblocks + zb) * kZ + zr] = e;
+                uint8_t *dst = M.data() + (((size_t)v * 3 + d) * Q.zblocks + zb) * job;
+                for (int i = 0; i < bk; i++) {
+                    int dg[6];
+                    host_digits(row[i], e, dg);
+                    for (int q = 0; q < 6; q++) {
+                        const __half h = __float2half_rn((float)dg[q]);
+                        const int rr = q * kZ + zr, kk = i % 16;
+                        std::memcpy(dst + (i / 16) * kZStep + (rr >> 3) * 256 + (kk >> 3) * 128 + (rr & 7) * 16 + (kk & 7) * 2, &h, 2);
+                    }
+                }
+            }
+        }
+    }
+    // blocks of 32 quadrant positions, rings ascending (a radial chunk is a contiguous run)
+    std::vector<int2> blocks;
+    Q.first.assign(1, 0);
+    for (int r = 0; r < g->d.iDim; r++) {
+        const int n = r + 1 + g->pOL + 1;
+        for (int m = 0; m < n; m += 32) blocks.push_back(make_int2(r, m));
+        Q.first.push_back((int)blocks.size());
+    }
+    auto put = [&](const void *src, size_t bytes, void **dst) {
+        if (cudaMalloc(dst, std::max<size_t>(bytes, 16)) != cudaSuccess) { cudaGetLastError(); return false; }
+        g->allocs.push_back(*dst);
+        return cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
+    };
+    void *pm = nullptr, *pe = nullptr, *pb = nullptr;
+    if (!put(M.data(), M.size(), &pm) || !put(E.data(), E.size() * 4, &pe) || !put(blocks.data(), blocks.size() * 8, &pb))
+        return SS_OK;
+    Q.M = pm; Q.mexpo = (int *)pe; Q.blocks = (int2 *)pb;
+    CUDA_TRY(cudaFuncSetAttribute(digit_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLimit));
+    Q.on = true;
+    return SS_OK;
+}
+
+int32_t digit_columns_inverse(ss_grid *g, cudaStream_t st, int chunk) {
+    const DigitPlan &P = g->digit;
+    const DigitColumns &Q = P.columns;
+    const ss_dims &d = g->d;
+    const int r0 = chunk < 0 ? 0 : g->chunk_r0[chunk], r1 = chunk < 0 ? (int)d.iDim : g->chunk_r0[chunk + 1];
+    ColumnArgs A{};
+    A.H = g->H; A.phys = (double *)g->phys; A.rings = P.rings; A.expo = P.expo;
+    A.M = (const uint8_t *)Q.M; A.mexpo = Q.mexpo; A.blocks = Q.blocks + Q.first[r0]; A.nblocks = Q.first[r1] - Q.first[r0];
+    A.N = (int)d.kDim; A.bk = (int)d.b_kDim; A.nvars = (int)d.nvars; A.nitems = g->nitems; A.iDim = (int)d.iDim;
+    A.steps = Q.steps; A.zblocks = Q.zblocks; A.buffers = Q.buffers; A.jDim = d.jDim; A.np = d.n_physical; A.err = P.err;
+    const int per = std::max(1, std::min(A.nblocks, g->sms / (int)d.nvars));
+    digit_columns_kernel<<<dim3(per, (unsigned)d.nvars), kColThreads,
+                           column_smem(Q.steps, Q.zblocks, A.bk, Q.buffers), st>>>(A);
+    CUDA_TRY(cudaGetLastError());
+    return SS_OK;
+}
+
+}  // namespace ss

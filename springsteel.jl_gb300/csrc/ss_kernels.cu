@@ -187,7 +187,7 @@ __device__ __forceinline__ void ring_inverse_body(const RingLaunch &L, const int
     __syncthreads();
     const int G = (nb + kSweepSeqs - 1) / kSweepSeqs;
 
-    for (int d = 0; d < 3; d++) {
+    for (int d = 0; d < (L.value_only ? 1 : 3); d++) {
         // FAtransform!: a_re = c br - s bi, a_im = s br + c bi (phase_filter.jl:154-190)
         for (UnitWalk uw_(nk); uw_.g < (G); uw_.next()) {
         const int k = uw_.n, g = uw_.g;
@@ -208,7 +208,7 @@ __device__ __forceinline__ void ring_inverse_body(const RingLaunch &L, const int
             }
         }
         __syncthreads();
-        const int nvar = (d == 0) ? 3 : 1;
+        const int nvar = (d == 0 && !L.value_only) ? 3 : 1;
         for (int dl = 0; dl < nvar; dl++) {
             // packed spectrum Zp_k = E_k + i O_k, k < N (HC2R of length L via a length-N
             // inverse DFT).  With N = 2(ri + 1) > 2·kmax, entry k ≤ N/2 sees only X_k and

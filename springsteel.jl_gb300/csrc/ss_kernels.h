@@ -26,6 +26,7 @@ struct RingLaunch {
     int64_t np;
     int nitems, nvars, bk, rlz;
     int ib;                    // items per CTA (≤ kRingBatchMax): one batched DFT per pass
+    int value_only;            // ring_inverse: f alone (the digit products write the derivatives)
 };
 constexpr int kRingBatchMax = 16;
 constexpr size_t kRingBatchBytes = 128 * 1024;  // shared-memory budget of one ring batch

@@ -1,0 +1,91 @@
+"""RLZ ring and column stages as digit-slice products: edges of their tiles against the
+FP64 oracle, value ranges against the FFT kernels, and the rule that chooses them."""
+import numpy as np
+import pytest
+
+import springsteel_gpu as S
+from springsteel_gpu import fields
+from test_gpu_parity import TOL64, _assert_parity, _run_both
+
+pytestmark = pytest.mark.gpu
+
+
+def _gp(cells, levels, nvars, **kw):
+    kw.setdefault("BCB", {"default": S.DirichletBC()})
+    kw.setdefault("BCT", {"default": S.NeumannBC()})
+    return S.SpringsteelGridParameters(geometry="RLZ", iMin=0.0, iMax=float(cells), num_cells=cells, kMin=0.0,
+                                       kMax=1000.0, kDim=levels, vars={"v%d" % i: i + 1 for i in range(nvars)}, **kw)
+
+
+# rings n = 2..: one K-step (n ≤ 32) to several, quadrant rows across one 128-row tile (n = 126..130 at
+# 43 cells), item counts around the groups of 8, level counts around the 32-row blocks and the 16-mode
+# steps, levels not a multiple of 4 (scalar stores), a kmax that ends inside a K-step, kmax = 0
+@pytest.mark.parametrize("cells,levels,nvars,kmax", [
+    (1, 5, 1, -1), (4, 12, 1, -1), (11, 24, 1, -1), (12, 25, 2, -1), (43, 13, 1, -1), (6, 33, 3, -1),
+    (5, 72, 1, -1), (14, 16, 1, 16), (14, 16, 1, 31), (9, 16, 2, 0)])
+def test_digit_products_match_oracle(cells, levels, nvars, kmax):
+    gp = _gp(cells, levels, nvars, max_wavenumber={"default": kmax})
+    pts = S.getGridpoints(S.createGrid(gp))
+    u = np.column_stack([fields.blob_sum(pts, seed=40 + v, nblobs=4, wmin=2.0, wmax=6.0, zmax=1000.0, noise=1e-3)
+                         for v in range(nvars)])
+    _, _, sg, so, pg, po = _run_both(gp, u)
+    _assert_parity(sg, so, pg, po, gp, tol=TOL64)
+
+
+def _round_trip(gp, u):
+    g = S.createGrid(gp)
+    g.set_physical(u, slot=1)
+    S.spectralTransform_b(g)
+    S.gridTransform_b(g)
+    g.synchronize()
+    out = g.get_spectral(), g.get_physical()
+    g.close()
+    return out
+
+
+def _field(gp, seed=3):
+    pts = S.getGridpoints(S.createGrid(gp))
+    return np.column_stack([fields.blob_sum(pts, seed=seed + v, nblobs=3, wmin=2.0, wmax=6.0, zmax=1000.0)
+                            for v in range(len(gp.vars))])
+
+
+def test_digit_products_scale_exactly():
+    """Every column has its own exponent, so a power of two commutes with the transforms bit for bit
+    down to the edge of the normal range (2^-900) and up to large values (2^700)."""
+    gp = _gp(8, 12, 2)
+    u = _field(gp)
+    spec, phys = _round_trip(gp, u)
+    for s in (-900, 700):
+        sp, ph = _round_trip(gp, np.ldexp(u, s))
+        assert np.array_equal(np.ldexp(spec, s), sp)
+        assert np.array_equal(np.ldexp(phys, s), ph)
+
+
+def test_digit_products_of_zero_and_non_finite_fields(monkeypatch):
+    gp = _gp(8, 12, 2)
+    u = _field(gp)
+    u[:, 1] = 0.0
+    _, ph = _round_trip(gp, u)
+    assert np.all(ph[:, 1, :] == 0.0) and np.all(np.isfinite(ph))
+    for bad in (np.nan, np.inf):
+        w = u.copy()
+        w[100, 0] = bad
+        _, got = _round_trip(gp, w)
+        monkeypatch.setenv("SS_RING_DIGITS", "0")
+        _, want = _round_trip(gp, w)
+        monkeypatch.delenv("SS_RING_DIGITS")
+        assert np.array_equal(np.isfinite(got), np.isfinite(want))
+        assert np.all(got[:, 1, :] == 0.0)
+
+
+@pytest.mark.parametrize("cells,levels,nvars", [(7, 9, 1), (20, 18, 2)])
+def test_digit_and_fft_kernels_agree(monkeypatch, cells, levels, nvars):
+    gp = _gp(cells, levels, nvars)
+    u = _field(gp)
+    spec, phys = _round_trip(gp, u)
+    monkeypatch.setenv("SS_RING_DIGITS", "0")
+    spec0, phys0 = _round_trip(gp, u)
+    for v in range(nvars):
+        assert np.max(np.abs(spec[:, v] - spec0[:, v])) <= TOL64 * np.max(np.abs(spec0[:, v]))
+        for s in range(7):
+            assert np.max(np.abs(phys[:, v, s] - phys0[:, v, s])) <= TOL64 * np.max(np.abs(phys0[:, v, s]))
