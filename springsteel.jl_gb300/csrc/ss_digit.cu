@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256) digit_matrix_kernel(const DigitRing *ring
             for (int i = 0; i < 8; i++)
                 U[i] = (unsigned long long)__double2ll_rn(entry(i) * 0x1p53) + kDigitBias;
             uint4 w[6];
-            planes8(U, w);
+            planes8<true>(U, w);
 #pragma unroll
             for (int i = 0; i < 6; i++) *reinterpret_cast<uint4 *>(dst + i * kDigitPlane) = w[i];
         } else {
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(kDigitThreads, 1) digit_gemm_kernel(GemmDigitA
         }
         for (int h = 0; h < 2; h++) {
             bar_init(&accf[h], 1);
-            bar_init(&acce[h], kDrainWarps * 16);
+            bar_init(&acce[h], kDrainWarps * 32);
             bar_init(&drain[h], 1);
         }
         quit = 0;
@@ -422,10 +422,11 @@ __global__ void __launch_bounds__(kDigitThreads, 1) digit_gemm_kernel(GemmDigitA
             }
         }
     } else {
-        // two warpgroups per half, each with half of its columns
-        constexpr int WC = W / 2;
-        const int h = warp >> 3, cb = ((warp >> 2) & 1) * WC;
-        const uint32_t tacc = tmem + ((uint32_t)((warp & 3) * 32) << 16) + h * 256 + cb;
+        // every draining warp owns 32 rows and a quarter of each half's columns, so a
+        // half is drained by all of them in turn and is soon free for its issuer
+        constexpr int WC = W / 4;
+        const int cb = (warp >> 2) * WC;
+        const uint32_t tacc = tmem + ((uint32_t)((warp & 3) * 32) << 16) + cb;
         uint32_t ch = 0;
         bool ok = true;
         for (int w = blockIdx.x; ok && w < g.nwork; w += gridDim.x) {
@@ -437,58 +438,63 @@ __global__ void __launch_bounds__(kDigitThreads, 1) digit_gemm_kernel(GemmDigitA
             const int k = 2 * row + (d.part & 1);
             const int m = kForward ? max(2 * k - 1 + (d.part >> 1), 0) : row - r->lo[d.part];
             const bool live = kForward ? k < r->n && (k > 0 || d.part == 0) : m >= 0 && m < r->cnt[d.part];
-            // lane c's column of this warp: its output base (−1 for padding) and exponent
+            // lane c's column of this warp (half c / WC): its output base (−1 for padding) and exponent
             auto col_base = [&](int c, int &e) -> int64_t {
                 constexpr int V0 = kDigitVariants - F::kVars;
-                const int col = (d.col_tile * 2 + h) * W + cb + c;
+                const int col = (d.col_tile * 2 + c / WC) * W + cb + c % WC;
                 const int item = col / (kDigitGroup * F::kVars) * kDigitGroup + col % kDigitGroup;
                 const int var = col / kDigitGroup % F::kVars + V0;
                 e = 0;
                 if constexpr (kForward) {
-                    if (c >= WC || col >= g.nitems) return -1;
+                    if (c >= 2 * WC || col >= g.nitems) return -1;
                     e = g.expo[(size_t)col * g.iDim + d.ring];
                     return (int64_t)col * g.frows + r->fofs;
                 }
-                if (c >= WC || item >= g.nitems) return -1;
+                if (c >= 2 * WC || item >= g.nitems) return -1;
                 e = g.expo[((size_t)var * g.nitems + item) * g.iDim + d.ring];
                 return ((int64_t)var * g.nvars + item / g.bk) * g.bk * g.jDim + (int64_t)g.bk * r->jofs + r->off[d.part] +
                        (int64_t)(item % g.bk) * r->L;
             };
-            using Acc = typename std::conditional<std::is_same<T, double>::value, long long, float>::type;
-            Acc V[WC];
+            using Acc = typename std::conditional<std::is_same<T, double>::value, unsigned long long, float>::type;
+            using Comb = Combine<false>;
+            Acc V[2 * WC];
+            const Acc start = std::is_same<T, double>::value ? (Acc)(0ull - Comb::kOffset * (unsigned)nch) : (Acc)0;
 #pragma unroll
-            for (int c = 0; c < WC; c++) V[c] = 0;
-            for (int q = 0; q < nch; q++, ch++) {
-                if (!(ok = __all_sync(0xffffffffu, bar_wait(&accf[h], ch & 1, &quit)))) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int c = 0; c < 2 * WC; c++) V[c] = start;
+            for (int q = 0; ok && q < nch; q++, ch++) {
 #pragma unroll
-                for (int c0 = 0; c0 < WC; c0 += 8) {
-                    float D[F::kSums][8];
+                for (int h = 0; h < 2; h++) {
+                    if (!(ok = ok && __all_sync(0xffffffffu, bar_wait(&accf[h], ch & 1, &quit)))) continue;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-                    for (int s = 0; s < F::kSums; s++) tmem_ld8(tacc + s * W + c0, D[s]);
-                    tmem_wait_ld();
-                    if (c0 + 8 == WC) {
-                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                        bar_arrive(&acce[h]);
-                    }
+                    for (int c0 = 0; c0 < WC; c0 += 4) {
+                        float D[F::kSums][4];
 #pragma unroll
-                    for (int c = 0; c < 8; c++) {
-                        if constexpr (std::is_same<T, double>::value)
-                            V[c0 + c] += combine(D[0][c], D[1][c], D[2][c], D[3][c], D[4][c], D[5][c], D[6][c]);
-                        else
-                            V[c0 + c] += fmaf(fmaf(D[2][c], 0x1p-10f, D[1][c]), 0x1p-10f, D[0][c]);
+                        for (int s = 0; s < F::kSums; s++) tmem_ld4(tacc + h * 256 + s * W + c0, D[s]);
+                        tmem_wait_ld();
+                        if (c0 + 4 == WC) {
+                            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                            bar_arrive(&acce[h]);
+                        }
+#pragma unroll
+                        for (int c = 0; c < 4; c++) {
+                            if constexpr (std::is_same<T, double>::value)
+                                Comb::add(V[h * WC + c0 + c], D[0][c], D[1][c], D[2][c], D[3][c], D[4][c], D[5][c], D[6][c]);
+                            else
+                                V[h * WC + c0 + c] += fmaf(fmaf(D[2][c], 0x1p-10f, D[1][c]), 0x1p-10f, D[0][c]);
+                        }
                     }
                 }
             }
             Acc *out = (Acc *)g.out;
             const double inv_len = kForward ? 1.0 / (double)r->L : 0.0;
 #pragma unroll
-            for (int c0 = 0; c0 < WC; c0 += 32) {
+            for (int c0 = 0; c0 < 2 * WC; c0 += 32) {
                 int e;
                 const int64_t mine = col_base(c0 + lane, e);
 #pragma unroll
                 for (int c = 0; c < 32; c++) {
-                    if (c0 + c >= WC) break;
+                    if (c0 + c >= 2 * WC) break;
                     const int64_t base = __shfl_sync(0xffffffffu, mine, c);
                     Acc v = V[c0 + c];
                     if constexpr (std::is_same<T, float>::value) {
@@ -501,7 +507,7 @@ __global__ void __launch_bounds__(kDigitThreads, 1) digit_gemm_kernel(GemmDigitA
                         const int ce = __shfl_sync(0xffffffffu, e, c);
                         if (ok && live && base >= 0)
                             ((double *)g.out)[base + m] = ce == kNanColumn ? __longlong_as_double(0x7ff8000000000000ll)
-                                                                           : fixed_to_double(v, ce + 1) * inv_len;
+                                                                           : fixed_to_double((long long)v, ce + 1) * inv_len;
                     } else {
                         if (ok && live && base >= 0) out[base + m] = v;
                     }

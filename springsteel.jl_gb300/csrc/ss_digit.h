@@ -100,7 +100,7 @@ struct DigitSet {
 // 32-position blocks of the quadrants
 struct DigitColumns {
     bool on = false;
-    int steps = 0, zblocks = 0, buffers = 1;
+    int steps = 0, zblocks = 0, buffers = 1, raws = 1;
     void *M = nullptr;
     int *mexpo = nullptr;
     int2 *blocks = nullptr;

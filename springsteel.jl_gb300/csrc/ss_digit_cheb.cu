@@ -8,6 +8,13 @@
 // forms the four reflected points of each quadrant position by integer
 // additions, cuts each column into digits at its own exponent and multiplies by
 // the matrix digits, which stay in shared memory.  ∂z and ∂zz share f's digits.
+//
+// Measured on the 200-cell, 32-level, 5-variable FP64 grid: 20.2 ms with FP64 FMAs
+// (94% of the FP64 matmul rate), 7.2 ms as digits with loads in line, 4.95 ms with
+// the next parts in flight (cp.async), 16 draining warps and the words of a digit
+// sum added by wide multiply-adds (shifts and logic run at half rate).  Memory
+// alone would take 1.4 ms; what is left is the integer work of cutting (8 warps
+// without it: 3.5 ms) and of rounding 64-bit fixed point to binary64.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -19,6 +26,7 @@
 #include "ss_digit_dev.cuh"
 #include "ss_grid.h"
 #include "ss_internal.h"
+#include "ss_types.cuh"
 
 using namespace ss;
 
@@ -35,9 +43,13 @@ namespace ss {
 
 constexpr int kZ = 32;                      // matrix rows (levels) of one product
 constexpr int kZStep = 6 * kZ * 32;         // bytes of a K-step of matrix digits: 6 planes × 32 rows × 16
-constexpr int kColThreads = 17 * 32;        // 8 producing, 8 draining, 1 issuing warp
+// Warps: producing, draining (half of them per accumulator), one issuing.  Measured
+// on the 200-cell FP64 grid: 8 + 16 warps 4.95 ms, 16 + 8 5.34 ms, 8 + 8 5.7 ms.
+constexpr int kProducers = 8, kDrains = 16;
+constexpr int kColThreads = (kProducers + kDrains + 1) * 32;
 constexpr int kMaxModes = 96;               // six K-steps keep every digit sum an exact integer
-constexpr int kRowExpo = 8;                 // row-exponent slots (producers run at most 4 variants ahead)
+constexpr int kMaxZBlocks = 5;              // 160 levels
+constexpr int kRowExpo = 8;                 // row-exponent slots (producers run at most 4 outputs ahead)
 
 struct ColumnArgs {
     const void *H;
@@ -48,31 +60,34 @@ struct ColumnArgs {
     const int *mexpo;         // [var][3][32·zblocks]
     const int2 *blocks;       // (ring, first quadrant position) of every 32-position block
     int nblocks;
-    int N, bk, nvars, nitems, iDim, steps, zblocks, buffers;
+    int N, bk, nvars, nitems, iDim, steps, zblocks, buffers, raws;
     int64_t jDim, np;
     int *err;
 };
 
-__device__ __forceinline__ void producers_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void producers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kProducers * 32) : "memory"); }
 __device__ __forceinline__ void st_global_32B(double *p, const double (&v)[4]) {
     asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3]) : "memory");
 }
 
 // grid = (CTAs per variable, variables); a CTA walks (block of 32 quadrant
 // positions = 128 columns, ring output), outputs fastest
+// (kSmall: at most two K-steps)
+template <bool kSmall>
 __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArgs g) {
     extern __shared__ __align__(1024) uint8_t dsm[];
     __shared__ __align__(8) uint64_t afull[2], aempty[2], accf[2], acce[2], drain;
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int quit;
     __shared__ int row_expo[kRowExpo][128];
-    __shared__ int mode_expo[kMaxModes];
+    __shared__ int mode_expo[2][kMaxModes];
+    __shared__ __align__(16) int sE[3 * kZ * kMaxZBlocks];  // row exponents of the matrices, less 53
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int v = blockIdx.y, KS = g.steps, nb = g.buffers;
     const int jobs_bytes = KS * kZStep;
     uint8_t *sM = dsm;                                                   // 3 × zblocks × jobs_bytes
     uint8_t *sA = sM + (size_t)3 * g.zblocks * jobs_bytes;               // nb × KS × 24 KB
-    long long *stage = reinterpret_cast<long long *>(sA + (size_t)nb * KS * 6 * kDigitPlane);  // bk × 128
+    long long *raw = reinterpret_cast<long long *>(sA + (size_t)nb * KS * 6 * kDigitPlane);  // raws × bk × 4 × 32
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_slot)), "r"(512)
                      : "memory");
@@ -80,10 +95,10 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
     }
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; i++) {
-            bar_init(&afull[i], 256);
+            bar_init(&afull[i], kProducers * 32);
             bar_init(&aempty[i], 1);
             bar_init(&accf[i], 1);
-            bar_init(&acce[i], 256);
+            bar_init(&acce[i], kDrains * 16);
         }
         bar_init(&drain, 1);
         quit = 0;
@@ -93,6 +108,9 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
         const uint4 *src = reinterpret_cast<const uint4 *>(g.M + (size_t)v * 3 * g.zblocks * jobs_bytes);
         for (int i = threadIdx.x; i < 3 * g.zblocks * jobs_bytes / 16; i += blockDim.x) reinterpret_cast<uint4 *>(sM)[i] = src[i];
     }
+    for (int i = threadIdx.x; i < nb * KS * 6 * kDigitPlane / 16; i += blockDim.x)
+        reinterpret_cast<uint4 *>(sA)[i] = make_uint4(0, 0, 0, 0);  // K groups of 8 without modes stay zero
+    for (int i = threadIdx.x; i < 3 * g.zblocks * kZ; i += blockDim.x) sE[i] = g.mexpo[(size_t)v * 3 * g.zblocks * kZ + i] - 53;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -100,66 +118,104 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
     const uint32_t tmem = tmem_slot;
     const int nitem = blockIdx.x < g.nblocks ? ((g.nblocks - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * kDigitVariants : 0;
 
-    if (warp < 8) {
-        // ---- producers: parts → points → digits
+    if (warp < kProducers) {
+        // ---- producers: parts → points → digits.  The parts of the next output are
+        // in flight (cp.async) while this one is cut.
         const long long *H = (const long long *)g.H;
-        bool ok = true;
-        for (int it = 0; ok && it < nitem; it++) {
-            const int2 blk = g.blocks[blockIdx.x + it / kDigitVariants * gridDim.x];
-            const int var = it % kDigitVariants;
+        struct Block {  // this thread's quadrant position: offsets of its four parts from the ring's first row
+            int64_t base;
+            int o[4], L, ring, flags;  // flags: 1 live, 2 on the axes (Ce, Co at 0 and Ce, So at π/2)
+        };
+        auto load_block = [&](int item) {
+            Block k;
+            const int2 blk = g.blocks[blockIdx.x + item * gridDim.x];
             const DigitRing *r = g.rings + blk.x;
             const int n = r->n, m = blk.y + lane;
-            const bool edge = r->half == 0 && m == 0, live = m < n;
+            const bool edge = r->half == 0 && m == 0;
+            k.o[0] = m;
+            k.o[1] = r->off[1] + m;
+            k.o[2] = edge ? n : r->off[2] + m - r->lo[2];
+            k.o[3] = edge ? 4 * n - 1 : r->off[3] + m - r->lo[3];
+            k.base = (int64_t)g.bk * r->jofs;
+            k.L = r->L;
+            k.ring = blk.x;
+            k.flags = (m < n ? 1 : 0) | (edge ? 2 : 0);
+            return k;
+        };
+        auto fetch = [&](const Block &k, int var, int slot) {
+            const long long *h = H + ((int64_t)var * g.nvars + v) * g.bk * g.jDim + k.base;
+            long long *dst = raw + (size_t)slot * g.bk * 128 + lane;
+            if (k.flags & 1)
+                for (int i = warp; i < g.bk; i += kProducers)
+#pragma unroll
+                    for (int q = 0; q < 4; q++) cp_async<8>(dst + (i * 4 + q) * 32, h + (int64_t)i * k.L + k.o[q]);
+            for (int i = threadIdx.x; i < g.bk; i += kProducers * 32)
+                cp_async<4>(&mode_expo[slot][i], g.expo + ((size_t)var * g.nitems + (size_t)v * g.bk + i) * g.iDim + k.ring);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        bool ok = true;
+        Block cur, next;
+        if (nitem > 0) {
+            next = load_block(0);
+            fetch(next, 0, 0);
+        }
+        const int nr = g.raws;
+        for (int it = 0; ok && it < nitem; it++) {
+            const int var = it % kDigitVariants, slot = it % nr;
+            if (var == 0) {
+                cur = next;
+                if (it + kDigitVariants < nitem) next = load_block(it / kDigitVariants + 1);
+            }
             int *rex = row_expo[it % kRowExpo];
-            // offsets of the four parts at this position (edge: Ce, Co at 0, Ce and So at π/2)
-            const int o0 = m, o1 = r->off[1] + m;
-            const int o2 = edge ? n : r->off[2] + m - r->lo[2], o3 = edge ? 4 * n - 1 : r->off[3] + m - r->lo[3];
-            const int64_t base = ((int64_t)var * g.nvars + v) * g.bk * g.jDim + (int64_t)g.bk * r->jofs;
-            const int *ex = g.expo + ((size_t)var * g.nitems + (size_t)v * g.bk) * g.iDim + blk.x;
             if (threadIdx.x < 128) rex[threadIdx.x] = 0;
+            const bool more = it + 1 < nitem;
+            if (more && nr == 2) {
+                if (var + 1 < kDigitVariants) fetch(cur, var + 1, slot ^ 1);
+                else fetch(next, 0, slot ^ 1);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
             producers_sync();
+            long long *pts = raw + (size_t)slot * g.bk * 128;
             int mx[4] = {0, 0, 0, 0};
-            for (int i = warp; i < g.bk; i += 8) {
-                const long long *h = H + base + (int64_t)i * r->L;
-                const int e = ex[(size_t)i * g.iDim];
-                if (lane == 0) mode_expo[i] = e;
-                long long a = 0, b = 0, c = 0, d = 0;
-                if (live) { a = h[o0]; b = h[o1]; c = h[o2]; d = h[o3]; }
-                long long p[4];
-                if (edge) {
-                    p[0] = a + b; p[2] = a - b; p[1] = c - d; p[3] = c + d;
-                } else {
+            for (int i = warp; i < g.bk; i += kProducers) {
+                long long *h = pts + i * 128 + lane;
+                const int e = mode_expo[slot][i];
+                long long p[4] = {0, 0, 0, 0};
+                if (cur.flags & 1) {
+                    const long long a = h[0], b = h[32], c = h[64], d = h[96];
                     const long long u = a + b, w = c + d, x = a - b, z = c - d;
                     p[0] = u + w; p[1] = u - w; p[2] = x - z; p[3] = x + z;
+                    if (cur.flags & 2) { p[0] = u; p[1] = z; p[2] = x; p[3] = w; }
                 }
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    stage[(size_t)i * 128 + q * 32 + lane] = p[q];
-                    const unsigned long long mag = p[q] < 0 ? 0ull - (unsigned long long)p[q] : (unsigned long long)p[q];
-                    // |p| 2^(e − 1074) < 2^(mx − 1074)
-                    if (mag) mx[q] = max(mx[q], e == kNanColumn ? kNanColumn : e + 64 - __clzll((long long)mag));
-                    else if (e == kNanColumn) mx[q] = kNanColumn;
+                    h[q * 32] = p[q];
+                    // |p| ≤ 2^b, |p| 2^(e − 1074) ≤ 2^(mx − 1074)
+                    const int hi = (int)(p[q] >> 32) ^ (int)(p[q] >> 63);
+                    const int b = hi ? 64 - __clz(hi) : 32;
+                    mx[q] = max(mx[q], e == kNanColumn ? kNanColumn : e + b);
                 }
             }
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (mx[q]) atomicMax(&rex[q * 32 + lane], mx[q]);
+            for (int q = 0; q < 4; q++) atomicMax(&rex[q * 32 + lane], mx[q]);
             producers_sync();
             const int buf = it % nb;
             if (!(ok = bar_wait(&aempty[buf], ((it / nb) & 1) ^ 1, &quit))) break;
             uint8_t *A = sA + (size_t)buf * KS * 6 * kDigitPlane;
             const int row = threadIdx.x & 127;
             const int er = rex[row];
-            for (int kg = threadIdx.x >> 7; kg < 2 * KS; kg += 2) {
+            for (int kg = threadIdx.x >> 7; kg < (g.bk + 7) / 8; kg += kProducers / 4) {
                 unsigned long long U[8];
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
                     const int mode = kg * 8 + i;
                     long long X = 0;
                     if (mode < g.bk && er != kNanColumn) {
-                        const long long V = stage[(size_t)mode * 128 + row];
-                        const int s = mode_expo[mode] + 54 - er;  // |V 2^s| < 2^54
-                        if (V != 0) X = s >= 0 ? V << s : (s > -63 ? ((V >> (-s - 1)) + 1) >> 1 : 0);
+                        const long long V = pts[mode * 128 + row];
+                        const int s = mode_expo[slot][mode] + 54 - er;  // |V 2^s| ≤ 2^54
+                        X = s >= 0 ? V << min(s, 63) : (s > -63 ? ((V >> (-s - 1)) + 1) >> 1 : 0);
                     }
                     U[i] = kDigitBias + (unsigned long long)X;
                 }
@@ -171,9 +227,14 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             bar_arrive(&afull[buf]);
-            producers_sync();  // the staged points are free again
+            producers_sync();  // these points may be overwritten
+            if (more && nr == 1) {
+                if (var + 1 < kDigitVariants) fetch(cur, var + 1, 0);
+                else fetch(next, 0, 0);
+            }
         }
-    } else if (warp == 16) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    } else if (warp == kProducers + kDrains) {
         // ---- issuer
         if (lane == 0) {
             bool ok = true;
@@ -215,16 +276,17 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
             }
         }
     } else {
-        // ---- drain: thread = (column, 16 levels)
+        // ---- drain: eight warps per accumulator; thread = (column, 16 levels)
+        const int mine = (warp - kProducers) >> 3;  // the accumulator, i.e. the parity of the jobs
         const int zh = ((warp >> 2) & 1) * 16;
         const int quad = warp & 3, row = quad * 32 + lane;
-        const uint32_t lanes = (uint32_t)(quad * 32) << 16;
+        const uint32_t tacc = tmem + ((uint32_t)(quad * 32) << 16) + mine * 256 + zh;
         const bool vec = g.N % 4 == 0;
         uint32_t job = 0;
         bool ok = true;
         for (int it = 0; ok && it < nitem; it++) {
+            const int var = it % kDigitVariants, nd = var == 0 ? 3 : 1;
             const int2 blk = g.blocks[blockIdx.x + it / kDigitVariants * gridDim.x];
-            const int var = it % kDigitVariants;
             const DigitRing *r = g.rings + blk.x;
             const int n = r->n, L = r->L, hf = r->half, m = blk.y + lane;
             const bool edge = hf == 0 && m == 0, live = m < n;
@@ -233,50 +295,44 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
             int l = p - r->shift;
             if (l < 0) l += L;
             if (l >= L) l -= L;
-            const int64_t col = r->jofs + l;
-            const int nd = var == 0 ? 3 : 1;
-            for (int d = 0; ok && d < nd; d++) {
+            double *const col = g.phys + (size_t)v * g.np + (r->jofs + l) * g.N;
+            for (int q = 0; ok && q < nd * g.zblocks; q++, job++) {
+                if ((int)(job & 1) != mine) continue;
+                const int d = q / g.zblocks, z0 = (q - d * g.zblocks) * kZ + zh;
                 const int slot = var == 0 ? (d == 0 ? 0 : 4 + d) : (var == 1 ? 3 : (var == 2 ? 4 : var - 2));
-                double *dst = g.phys + ((size_t)slot * g.nvars + v) * g.np + col * g.N;
-                for (int zb = 0; zb < g.zblocks; zb++, job++) {
-                    const int t = job & 1;
-                    if (!(ok = __all_sync(0xffffffffu, bar_wait(&accf[t], (job >> 1) & 1, &quit)))) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const int er = row_expo[it % kRowExpo][row];
-                    const int z0 = zb * kZ + zh;
-                    const int *me = g.mexpo + ((size_t)v * 3 + d) * g.zblocks * kZ + z0;
-                    const uint32_t tacc = tmem + lanes + t * 256 + zh;
+                double *dst = col + (size_t)slot * g.nvars * g.np + z0;
+                if (!(ok = __all_sync(0xffffffffu, bar_wait(&accf[mine], (job >> 1) & 1, &quit)))) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const int er = row_expo[it % kRowExpo][row];
+                const int *me = sE + q * kZ + zh;
+                // rolled: the instruction cache serves all three roles
+#pragma unroll 1
+                for (int c0 = 0; c0 < 16; c0 += 4) {
+                    float D[7][4];
 #pragma unroll
-                    for (int c0 = 0; c0 < 16; c0 += 8) {
-                        float D[7][8];
+                    for (int s = 0; s < 7; s++) tmem_ld4(tacc + s * kZ + c0, D[s]);
+                    const int4 e4 = *reinterpret_cast<const int4 *>(me + c0);
+                    tmem_wait_ld();
+                    if (c0 == 12) {
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        bar_arrive(&acce[mine]);
+                    }
+                    const int ze[4] = {e4.x, e4.y, e4.z, e4.w};
+                    double o[4];
 #pragma unroll
-                        for (int s = 0; s < 7; s++) tmem_ld8(tacc + s * kZ + c0, D[s]);
-                        tmem_wait_ld();
-                        if (c0 == 8) {
-                            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                            bar_arrive(&acce[t]);
-                        }
-                        double o[8];
+                    for (int c = 0; c < 4; c++) {
+                        unsigned long long V = 0ull - Combine<kSmall>::kOffset;
+                        Combine<kSmall>::add(V, D[0][c], D[1][c], D[2][c], D[3][c], D[4][c], D[5][c], D[6][c]);
+                        o[c] = fixed_to_double((long long)V, er + ze[c]);  // V 2^(er − 1074 + mexpo − 53)
+                        if (er == kNanColumn) o[c] = __longlong_as_double(0x7ff8000000000000ll);
+                    }
+                    if (live) {
+                        if (vec) {
+                            if (z0 + c0 < g.N) st_global_32B(dst + c0, o);
+                        } else {
 #pragma unroll
-                        for (int c = 0; c < 8; c++) {
-                            const long long V = combine(D[0][c], D[1][c], D[2][c], D[3][c], D[4][c], D[5][c], D[6][c]);
-                            // V 2^(er − 1074 + mexpo − 53)
-                            o[c] = er == kNanColumn ? __longlong_as_double(0x7ff8000000000000ll)
-                                                    : fixed_to_double(V, er + me[c0 + c] - 53);
-                        }
-                        if (live) {
-                            if (vec) {
-#pragma unroll
-                                for (int c = 0; c < 8; c += 4)
-                                    if (z0 + c0 + c < g.N) {
-                                        const double q4[4] = {o[c], o[c + 1], o[c + 2], o[c + 3]};
-                                        st_global_32B(dst + z0 + c0 + c, q4);
-                                    }
-                            } else {
-#pragma unroll
-                                for (int c = 0; c < 8; c++)
-                                    if (z0 + c0 + c < g.N) dst[z0 + c0 + c] = o[c];
-                            }
+                            for (int c = 0; c < 4; c++)
+                                if (z0 + c0 + c < g.N) dst[c0 + c] = o[c];
                         }
                     }
                 }
@@ -302,8 +358,8 @@ static void host_digits(double x, int e, int (&d)[6]) {
     d[0] = (int)X;
 }
 
-static size_t column_smem(int steps, int zblocks, int bk, int buffers) {
-    return (size_t)3 * zblocks * steps * kZStep + (size_t)buffers * steps * 6 * kDigitPlane + (size_t)bk * 128 * 8;
+static size_t column_smem(int steps, int zblocks, int bk, int buffers, int raws) {
+    return (size_t)3 * zblocks * steps * kZStep + (size_t)buffers * steps * 6 * kDigitPlane + (size_t)raws * bk * 128 * 8;
 }
 
 int32_t digit_columns_build(ss_grid *g, const std::vector<ChebHost> &cheb) {
@@ -313,10 +369,14 @@ int32_t digit_columns_build(ss_grid *g, const std::vector<ChebHost> &cheb) {
     DigitColumns &Q = P.columns;
     Q.steps = (bk + 15) / 16;
     Q.zblocks = (N + kZ - 1) / kZ;
-    if (bk > kMaxModes) return SS_OK;
+    if (bk > kMaxModes || Q.zblocks > kMaxZBlocks) return SS_OK;
     constexpr size_t kLimit = 232448 - 8192;  // 227 KB less the static part
-    Q.buffers = column_smem(Q.steps, Q.zblocks, bk, 2) <= kLimit ? 2 : 1;
-    if (column_smem(Q.steps, Q.zblocks, bk, Q.buffers) > kLimit) return SS_OK;
+    // two operand buffers and two input buffers where they fit, then fewer
+    const int shapes[4][2] = {{2, 2}, {1, 2}, {2, 1}, {1, 1}};
+    Q.buffers = 0;
+    for (const auto &s : shapes)
+        if (!Q.buffers && column_smem(Q.steps, Q.zblocks, bk, s[0], s[1]) <= kLimit) { Q.buffers = s[0]; Q.raws = s[1]; }
+    if (!Q.buffers) return SS_OK;
     const int job = Q.steps * kZStep;
     std::vector<uint8_t> M((size_t)nv * 3 * Q.zblocks * job, 0);
     std::vector<int> E((size_t)nv * 3 * Q.zblocks * kZ, 0);
@@ -386,7 +446,7 @@ int32_t digit_columns_build(ss_grid *g, const std::vector<ChebHost> &cheb) {
     if (!put(M.data(), M.size(), &pm) || !put(E.data(), E.size() * 4, &pe) || !put(blocks.data(), blocks.size() * 8, &pb))
         return SS_OK;
     Q.M = pm; Q.mexpo = (int *)pe; Q.blocks = (int2 *)pb;
-    CUDA_TRY(cudaFuncSetAttribute(digit_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLimit));
+    CUDA_TRY(cudaFuncSetAttribute(Q.steps <= 2 ? digit_columns_kernel<true> : digit_columns_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLimit));
     Q.on = true;
     return SS_OK;
 }
@@ -400,10 +460,12 @@ int32_t digit_columns_inverse(ss_grid *g, cudaStream_t st, int chunk) {
     A.H = g->H; A.phys = (double *)g->phys; A.rings = P.rings; A.expo = P.expo;
     A.M = (const uint8_t *)Q.M; A.mexpo = Q.mexpo; A.blocks = Q.blocks + Q.first[r0]; A.nblocks = Q.first[r1] - Q.first[r0];
     A.N = (int)d.kDim; A.bk = (int)d.b_kDim; A.nvars = (int)d.nvars; A.nitems = g->nitems; A.iDim = (int)d.iDim;
-    A.steps = Q.steps; A.zblocks = Q.zblocks; A.buffers = Q.buffers; A.jDim = d.jDim; A.np = d.n_physical; A.err = P.err;
+    A.steps = Q.steps; A.zblocks = Q.zblocks; A.buffers = Q.buffers; A.raws = Q.raws; A.jDim = d.jDim; A.np = d.n_physical; A.err = P.err;
     const int per = std::max(1, std::min(A.nblocks, g->sms / (int)d.nvars));
-    digit_columns_kernel<<<dim3(per, (unsigned)d.nvars), kColThreads,
-                           column_smem(Q.steps, Q.zblocks, A.bk, Q.buffers), st>>>(A);
+    const size_t smem = column_smem(Q.steps, Q.zblocks, A.bk, Q.buffers, Q.raws);
+    const dim3 grid(per, (unsigned)d.nvars);
+    if (Q.steps <= 2) digit_columns_kernel<true><<<grid, kColThreads, smem, st>>>(A);
+    else digit_columns_kernel<false><<<grid, kColThreads, smem, st>>>(A);
     CUDA_TRY(cudaGetLastError());
     return SS_OK;
 }

@@ -13,10 +13,15 @@
 namespace ss {
 
 // ------------------------------------------------------------ digits
-// two unsigned fields of at most 1024 minus `bias`, exactly, as a half2
+// Two unsigned fields of at most 1024 minus `bias` as a half2, exactly.  A matrix
+// digit is the integer itself (1024 + field, less 1024 + bias); a data digit is
+// its 2^-24 multiple: the field read as a binary16 subnormal, which needs no
+// exponent bits set.
+template <bool kMatrix>
 __device__ __forceinline__ uint32_t half_pair(uint32_t a, uint32_t b, uint32_t bias) {
-    const uint32_t v = 0x64006400u + a + (b << 16);  // 1024 + field in each half
-    const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&v), *reinterpret_cast<const __half2 *>(&bias));
+    const uint32_t off = kMatrix ? 0x64006400u : 0u;
+    const uint32_t v = off + __byte_perm(a, b, 0x5410), w = off + bias;
+    const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&v), *reinterpret_cast<const __half2 *>(&w));
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 // X + bias, |X| ≤ 2^54: five low fields of 9 bits are the balanced digits + 256,
@@ -36,6 +41,7 @@ __device__ __forceinline__ long long fixed_point(double x, int emax) {
     return (long long)u < 0 ? -(long long)m : (long long)m;
 }
 // digit planes of 8 consecutive K entries: out[i] = 16 bytes of plane i, most significant first
+template <bool kMatrix = false>
 __device__ __forceinline__ void planes8(const unsigned long long (&U)[8], uint4 (&out)[6]) {
 #pragma unroll
     for (int i = 0; i < 6; i++) {
@@ -45,7 +51,7 @@ __device__ __forceinline__ void planes8(const unsigned long long (&U)[8], uint4 
         for (int q = 0; q < 4; q++) {
             uint32_t a = (uint32_t)(U[2 * q] >> sh), b = (uint32_t)(U[2 * q + 1] >> sh);
             if (i > 0) { a &= 511u; b &= 511u; }
-            w[q] = half_pair(a, b, i > 0 ? 0x65006500u : 0x66006600u);  // 1024 + 256 or 512
+            w[q] = half_pair<kMatrix>(a, b, i > 0 ? 0x01000100u : 0x02000200u);
         }
         out[i] = make_uint4(w[0], w[1], w[2], w[3]);
     }
@@ -142,42 +148,69 @@ __device__ __forceinline__ void tmem_ld8(uint32_t addr, float (&v)[8]) {
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
 }
+__device__ __forceinline__ void tmem_ld4(uint32_t addr, float (&v)[4]) {
+    uint32_t r[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] = __uint_as_float(r[i]);
+}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// Σ_s D_s 2^(36−9s) (D_5, D_6 rounded): the D_s are integers of up to 2^26; each is
-// cut at 2^9 by a fused multiply-add with 1.5·2^23 (which leaves an integer in the
-// low mantissa bits), the high part joining the next sum, so that every word is
-// far inside the 23-bit range
-__device__ __forceinline__ long long combine(const float D0, const float D1, const float D2, const float D3,
-                                             const float D4, const float D5, const float D6) {
-    constexpr float M = 12582912.f;
-    constexpr int C = 0x4B400000;
-    const float b5 = fmaf(fmaf(D6, 0x1p-9f, D5), 0x1p-9f, M);
-    const float m4 = fmaf(D4, 0x1p-9f, M), b4 = fmaf(m4 - M, -512.f, D4) + b5;
-    const float m3 = fmaf(D3, 0x1p-9f, M), b3 = fmaf(m3 - M, -512.f, D3) + m4;
-    const float m2 = fmaf(D2, 0x1p-9f, M), b2 = fmaf(m2 - M, -512.f, D2) + m3;
-    const float m1 = fmaf(D1, 0x1p-9f, M), b1 = fmaf(m1 - M, -512.f, D1) + m2;
-    const float m0 = fmaf(D0, 0x1p-9f, M), b0 = fmaf(m0 - M, -512.f, D0) + m1;
-    const int u0 = (__float_as_int(b0) - C) * 512 + (__float_as_int(b1) - C);
-    const int u1 = (__float_as_int(b2) - C) * 512 + (__float_as_int(b3) - C);
-    return ((long long)(__float_as_int(m0) - C) << 45) + ((long long)u0 << 27) + ((long long)u1 << 9) +
-           (long long)(__float_as_int(b4) - C);
-}
-
-// binary64 V·2^(expo − 1074), rounded to nearest even; V = 0 gives 0
-__device__ __forceinline__ double fixed_to_double(long long V, int expo) {
-    if (V == 0) return 0.0;
-    const unsigned long long a = V < 0 ? 0ull - (unsigned long long)V : (unsigned long long)V;
-    const int lz = __clzll((long long)a);
-    const int ef = expo + 12 - lz;
-    if (ef < 1 || ef > 2045) {  // leaves the normal range: two exact factors
-        const int s = expo - 1074, h = s / 2;
-        return scalbn(scalbn((double)V, h), s - h);
+// acc += Σ_s D_s 2^(36−9s) + kOffset (D_5, D_6 rounded).  The D_s arrive as 2^-24
+// multiples (data digits) of integers of up to 2^26; each is cut at 2^9 by a fused
+// multiply-add with 1.5·2^23, which leaves an integer in the low mantissa bits,
+// the high part joining the next sum, so that every word is far inside the 23-bit
+// range.  The words are added as raw bits (32-bit wide multiply-adds run at full
+// rate here, shifts and logic at half): the constant they carry is kOffset, taken
+// off once per result.  kSmall: |D_0| ≤ 2^22 (at most 32 products) needs no cut.
+template <bool kSmall>
+struct Combine {
+    static constexpr unsigned long long kMagic = 0x4B400000ull;  // bits of 1.5·2^23
+    static constexpr unsigned long long kOffset =
+        kMagic * (1ull + (1ull << 9) + (1ull << 18) + (1ull << 27) + (1ull << 36) + (kSmall ? 0ull : 1ull << 45));
+    static __device__ __forceinline__ void add(unsigned long long &acc, const float D0, const float D1, const float D2,
+                                               const float D3, const float D4, const float D5, const float D6) {
+        constexpr float M = 12582912.f, up = 0x1p24f, cut = 0x1p15f, back = -0x1p-15f;
+        const float b5 = fmaf(fmaf(D6, 0x1p-9f, D5), cut, M);
+        const float m4 = fmaf(D4, cut, M), b4 = fmaf(fmaf(m4 - M, back, D4), up, b5);
+        const float m3 = fmaf(D3, cut, M), b3 = fmaf(fmaf(m3 - M, back, D3), up, m4);
+        const float m2 = fmaf(D2, cut, M), b2 = fmaf(fmaf(m2 - M, back, D2), up, m3);
+        const float m1 = fmaf(D1, cut, M), b1 = fmaf(fmaf(m1 - M, back, D1), up, m2);
+        long long a = (long long)acc;
+        a += (long long)__float_as_int(b4);
+        a += (long long)__float_as_int(b3) * (1 << 9);
+        a += (long long)__float_as_int(b2) * (1 << 18);
+        a += (long long)__float_as_int(b1) * (1 << 27);
+        uint32_t hi;
+        if (kSmall) {
+            hi = (uint32_t)__float_as_int(fmaf(D0, up, m1)) * 16u;
+        } else {
+            const float m0 = fmaf(D0, cut, M), b0 = fmaf(fmaf(m0 - M, back, D0), up, m1);
+            hi = (uint32_t)__float_as_int(b0) * 16u + (uint32_t)__float_as_int(m0) * 8192u;
+        }
+        acc = (unsigned long long)a + ((unsigned long long)hi << 32);
     }
-    const unsigned long long n = a << lz;
-    const unsigned long long mant = (n >> 11) + (((n & 0x7ffull) + ((n >> 11) & 1ull)) > 0x400ull ? 1ull : 0ull);
-    const unsigned long long bits = ((unsigned long long)(ef - 1) << 52) + mant;
-    return __longlong_as_double((long long)(V < 0 ? bits | 0x8000000000000000ull : bits));
+};
+
+// binary64 V·2^(expo − 1074), rounded to nearest (a tie away from zero)
+__device__ __forceinline__ double fixed_to_double(long long V, int expo) {
+    const uint32_t sign = (uint32_t)(V >> 32) & 0x80000000u;
+    const unsigned long long a = V < 0 ? 0ull - (unsigned long long)V : (unsigned long long)V;
+    const uint32_t ahi = (uint32_t)(a >> 32);
+    int lz = __clz((int)ahi);
+    if (ahi == 0) lz = 32 + __clz((int)(uint32_t)a);  // small against the column's scale: rare
+    const int ef = expo + 12 - lz;
+    const unsigned long long n = a << (lz & 63);  // leading one at bit 63; V = 0 is set below
+    const unsigned long long mant = (n >> 11) + ((uint32_t)(n >> 10) & 1u);
+    const unsigned long long bits = mant + ((unsigned long long)((uint32_t)(ef - 1) * 1048576u + sign) << 32);
+    double out = __longlong_as_double((long long)bits);
+    if ((unsigned)(ef - 1) > 2044u || lz == 64) {  // outside the normal range, or zero: two exact factors
+        const int s = expo - 1074, h = s / 2;
+        out = V == 0 ? 0.0 : scalbn(scalbn((double)V, h), s - h);
+    }
+    return out;
 }
 
 }  // namespace ss
