@@ -197,6 +197,17 @@ static int32_t build_grid(ss_grid *g) {
         for (int i = 0; i < sh.Min; i++) dinv[i] = 1.0 / sh.L4[size_t(i) * 4];
         if ((st = upload_vec(g, &sd.L4, sh.L4))) return st;
         if ((st = upload_vec(g, &sd.dinv, dinv))) return st;
+        if (!sh.periodic) {
+            const SplineFixed f = spline_ldl(sh);
+            double *m = nullptr;
+            int *q = nullptr;
+            if ((st = upload_vec(g, &m, f.ldl))) return st;
+            if ((st = upload_vec(g, &q, f.limbs))) return st;
+            sd.ldl = m;
+            sd.fix = q;
+            g->spl_host[v].fixed_ok = f.ok;
+            sd.fix_m_up = f.m_up; sd.fix_d_up = f.d_up; sd.fix_bits = f.bits;
+        }
         if ((st = upload_vec(g, &sd.PQb, sh.PQb))) return st;
         std::vector<float> l4f(sh.L4.size()), dinvf(dinv.size());
         for (size_t i = 0; i < l4f.size(); i++) l4f[i] = (float)sh.L4[i];
@@ -551,6 +562,12 @@ SaLaunch sa_record(const ss_grid *g, int coeffs, size_t *smem_generic) {
     if (smem_generic) *smem_generic = smem;
     return A;
 }
+bool sa_band_serves(const ss_grid *g) {
+    if (g->tl == TL_DF64 || sa_band_smem((int)g->d.b_iDim) > kSaBandSmemMax) return false;
+    for (auto &sh : g->spl_host)
+        if (sh.periodic || (g->tl == TL_F32 && !sh.fixed_ok)) return false;
+    return true;
+}
 }  // namespace ss
 
 template <typename P, typename T>
@@ -596,6 +613,13 @@ static int32_t inv_sa(ss_grid *g, cudaStream_t st, int coeffs, const void *spec_
     StageScope sc(g, SS_STAGE_SA_SI, st);
     bool periodic = false;
     for (auto &sh : g->spl_host) periodic |= sh.periodic != 0;
+    if constexpr (std::is_same<P, T>::value) {
+        if (!aout && sa_band_serves(g)) {
+            CUDA_TRY(launch_sa_band<T>(A, g->nitems, st));
+            g->launches[SS_STAGE_SA_SI]++;
+            return SS_OK;
+        }
+    }
     if constexpr (std::is_same<P, float>::value && std::is_same<T, float>::value) {
         // the slot-parallel binary32 kernel has no dense-tail solve: periodic splines
         // (and the coefficient output of splineTransform!) take the tiled kernel

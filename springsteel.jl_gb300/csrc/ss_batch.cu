@@ -27,7 +27,7 @@ using namespace ss;
 // ====================================================================== batch
 // One launch of a fused batch: the CTAs of many grids' records of one stage
 // (one shared-memory class), each CTA running the record its work entry names.
-enum { FK_RING_FWD = 0, FK_SB = 1, FK_SA = 2, FK_SA_F32 = 3, FK_RING_INV = 4 };
+enum { FK_RING_FWD = 0, FK_SB = 1, FK_SA = 2, FK_SA_F32 = 3, FK_RING_INV = 4, FK_SA_BAND = 5 };
 struct FusedLaunch {
     int kind, tl;
     size_t smem;
@@ -49,7 +49,7 @@ struct ss_batch {
     bool fused = false;
     int ib_scale = 1;                   // items per ring CTA × this (autotuned)
     std::vector<FusedLaunch> fwd, inv;  // in launch order
-    std::vector<ss_grid *> unfused;     // RLZ grids: their own launch sequences
+    std::vector<ss_grid *> unfused;     // RLZ grids and grids of digit products: their own launch sequences
     std::vector<void *> fused_mem;
     std::vector<uint64_t> fused_gen;    // generations the records were built from
 };
@@ -226,10 +226,15 @@ static int32_t plan_sa(ss_batch *bt, const std::vector<ss_grid *> &gs, int tl, s
             if (sh.periodic) return true;
         return false;
     };
+    std::vector<char> band(gs.size());
+    for (size_t i = 0; i < gs.size(); i++) {
+        band[i] = sa_band_serves(gs[i]);
+        if (band[i]) smem[i] = sa_band_smem(L[i].b);
+    }
     if (tl == TL_F32) {
         std::vector<BatchWork> work;
         for (int i = 0; i < (int)gs.size(); i++)
-            if (!periodic(i))
+            if (!periodic(i) && !band[i])
                 for (int by = 0; by < gs[i]->nitems; by++)
                     for (int bx = 0; bx < (L[i].nslots_z + 127) / 128; bx++) work.push_back({i, bx, by, 0});
         if (!work.empty()) {
@@ -238,12 +243,13 @@ static int32_t plan_sa(ss_batch *bt, const std::vector<ss_grid *> &gs, int tl, s
             out.push_back({FK_SA_F32, tl, 0, 128, (int)work.size(), d_recs, (const BatchWork *)w});
         }
     }
-    for (int c = 0; c < 7; c++) {
+    for (int c = 0; c < 14; c++) {  // classes of the banded, then of the tiled kernel
         std::vector<BatchWork> work;
         size_t sm = 0;
         for (int i = 0; i < (int)gs.size(); i++) {
-            if (tl == TL_F32 && !periodic(i)) continue;
-            if (smem_class(smem[i]) != c) continue;
+            if (band[i] != (c < 7)) continue;
+            if (tl == TL_F32 && !periodic(i) && !band[i]) continue;
+            if (smem_class(smem[i]) != c % 7) continue;
             sm = std::max(sm, smem[i]);
             for (int by = 0; by < gs[i]->nitems; by++)
                 for (int bx = 0; bx < (L[i].nslots_z + 31) / 32; bx++) work.push_back({i, bx, by, 0});
@@ -251,7 +257,7 @@ static int32_t plan_sa(ss_batch *bt, const std::vector<ss_grid *> &gs, int tl, s
         if (work.empty()) continue;
         const void *w = nullptr;
         if ((rc = upload(bt, work, &w))) return rc;
-        out.push_back({FK_SA, tl, sm, 128, (int)work.size(), d_recs, (const BatchWork *)w});
+        out.push_back({c < 7 ? FK_SA_BAND : FK_SA, tl, sm, 128, (int)work.size(), d_recs, (const BatchWork *)w});
     }
     for (size_t i = 0; i < smem.size(); i++)
         if (smem_class(smem[i]) < 0) {
@@ -267,7 +273,7 @@ static int32_t build_fused(ss_batch *bt) {
     for (int tl : {TL_F64, TL_DF64, TL_F32}) {
         std::vector<ss_grid *> gs;
         for (ss_grid *g : bt->grids)
-            if (!g->rlz && g->tl == tl) gs.push_back(g);
+            if (!g->rlz && !g->digit.on && g->tl == tl) gs.push_back(g);
         if (gs.empty()) continue;
         int32_t rc = plan_rings(bt, gs, tl, false, bt->fwd);
         if (!rc) rc = plan_sb(bt, gs, tl, bt->fwd);
@@ -276,7 +282,7 @@ static int32_t build_fused(ss_batch *bt) {
         if (rc) { free_fused(bt); return rc; }
     }
     for (ss_grid *g : bt->grids)
-        if (g->rlz) bt->unfused.push_back(g);
+        if (g->rlz || g->digit.on) bt->unfused.push_back(g);
     bt->fused_gen = generations(bt);
     return SS_OK;
 }
@@ -290,6 +296,10 @@ static cudaError_t fused_launch(const FusedLaunch &f, cudaStream_t st) {
         return launch_ring_inverse_fused<P, T>((const RingLaunch *)f.recs, f.work, f.nwork, f.smem, f.threads, st);
     case FK_SB: return launch_sb_project_fused<P, T>((const SbLaunch *)f.recs, f.work, f.nwork, st);
     case FK_SA: return launch_sa_si_fused<P, T>((const SaLaunch *)f.recs, f.work, f.nwork, f.smem, st);
+    case FK_SA_BAND:
+        if constexpr (std::is_same<P, T>::value)
+            return launch_sa_band_fused<T>((const SaLaunch *)f.recs, f.work, f.nwork, f.smem, st);
+        return cudaErrorInvalidValue;
     default:
         if constexpr (std::is_same<P, float>::value)
             return launch_sa_si_f32_fused<P>((const SaLaunch *)f.recs, f.work, f.nwork, st);
@@ -306,10 +316,19 @@ static int32_t enqueue_fused(ss_batch *bt, int what, cudaStream_t st) {
                                               : fused_launch<float, float>(f, st);
             CUDA_TRY(e);
         }
-        for (ss_grid *g : bt->unfused) {
-            int32_t r = run_direction(g, dir, st);
-            if (r) return r;
-        }
+    }
+    // the other grids' sequences, round-robin over the side streams
+    const int nside = std::min((int)bt->side.size(), (int)bt->unfused.size());
+    if (nside == 0) return SS_OK;
+    CUDA_TRY(cudaEventRecord(bt->ev[0], st));
+    for (int i = 0; i < nside; i++) CUDA_TRY(cudaStreamWaitEvent(bt->side[i], bt->ev[0], 0));
+    for (size_t i = 0; i < bt->unfused.size(); i++) {
+        int32_t r = run_direction(bt->unfused[i], what, bt->side[i % nside]);
+        if (r) return r;
+    }
+    for (int i = 0; i < nside; i++) {
+        CUDA_TRY(cudaEventRecord(bt->ev[1 + i], bt->side[i]));
+        CUDA_TRY(cudaStreamWaitEvent(st, bt->ev[1 + i], 0));
     }
     return SS_OK;
 }

@@ -364,7 +364,7 @@ static size_t column_smem(int steps, int zblocks, int bk, int buffers, int raws)
 
 int32_t digit_columns_build(ss_grid *g, const std::vector<ChebHost> &cheb) {
     DigitPlan &P = g->digit;
-    if (!P.on || g->tl != TL_F64) return SS_OK;
+    if (!P.on || !g->rlz || g->tl != TL_F64) return SS_OK;
     const int N = (int)g->d.kDim, bk = (int)g->d.b_kDim, nv = (int)g->d.nvars;
     DigitColumns &Q = P.columns;
     Q.steps = (bk + 15) / 16;

@@ -129,4 +129,5 @@ RingLaunch ring_record(const ss_grid *g, bool inverse);
 size_t ring_item_smem(const ss_grid *g, const RingBucket &bkt, bool inverse);
 SbLaunch sb_record(const ss_grid *g);
 SaLaunch sa_record(const ss_grid *g, int coeffs, size_t *smem_generic);
+bool sa_band_serves(const ss_grid *g);
 }  // namespace ss

@@ -156,7 +156,15 @@ template <typename P, typename T>
 cudaError_t launch_sb_project(const SbLaunch &S, int nitems, cudaStream_t st);
 template <typename P, typename T>
 cudaError_t launch_sa_si(const SaLaunch &A, int nitems, size_t smem, cudaStream_t st);
-// binary32 grids: slot-parallel solve over the scratch arrays X, Y, each
+// binary64 and binary32 grids without a periodic spline whose 32 slots of b rows fit
+// the shared memory of a CTA (ss_sa.cu)
+size_t sa_band_smem(int b);
+constexpr size_t kSaBandSmemMax = 224 * 1024;
+template <typename T>
+cudaError_t launch_sa_band(const SaLaunch &A, int nitems, cudaStream_t st);
+template <typename T>
+cudaError_t launch_sa_band_fused(const SaLaunch *recs, const BatchWork *work, int nwork, size_t smem, cudaStream_t st);
+// binary32 grids beyond that: slot-parallel solve over the scratch arrays X, Y, each
 // nitems × b × nslots_z floats (ss_sa_f32.cu)
 template <typename P>
 cudaError_t launch_sa_si_f32(const SaLaunch &A, int nitems, float *X, float *Y, cudaStream_t st);
