@@ -163,7 +163,7 @@ struct SplitArgs {
     const int64_t *btile;
     uint8_t *B;
     int *expo;
-    const int *delta;
+    const int *delta, *cap;   // cap: largest wavenumber of every item (per-variable kmax of RL grids)
     int64_t frows;
     int r0, nitems, iDim, col_tiles;
 };
@@ -196,7 +196,8 @@ __global__ void __launch_bounds__(256, 2) digit_split_kernel(SplitArgs S) {
         uint32_t mx[kDigitVariants] = {0, 0, 0, 0, 0};
         if (item < S.nitems) {
             const T *g0 = G + (size_t)item * S.frows + r.fofs;
-            for (int s = lane; s < 1 + 2 * r.kmax; s += 32) {
+            const int kmax = min(r.kmax, S.cap[item]);
+            for (int s = lane; s < 1 + 2 * kmax; s += 32) {
                 const T k = (T)((s + 1) >> 1);
                 const T v = g0[s];
                 mx[0] = max(mx[0], mag_bits(v));
@@ -224,6 +225,7 @@ __global__ void __launch_bounds__(256, 2) digit_split_kernel(SplitArgs S) {
     const int par = (threadIdx.x >> 3) & 1, imag = (threadIdx.x >> 4) & 1;
     const int64_t bt = S.btile[ring];
     const T *g = G + (size_t)item * S.frows + r.fofs;
+    const int kmax = min(r.kmax, S.cap[item]);
     const int steps = par ? r.to : r.te;
     for (int kg = warp; kg < 2 * r.te; kg += 8) {
         const bool store = real && kg < 2 * steps;
@@ -233,7 +235,7 @@ __global__ void __launch_bounds__(256, 2) digit_split_kernel(SplitArgs S) {
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 const int k = k0 + 2 * i;
-                dk[i] = (k > 0 && k <= r.kmax) ? S.delta[r.dofs + k - 1] : 0;
+                dk[i] = (k > 0 && k <= kmax) ? S.delta[r.dofs + k - 1] : 0;
             }
         }
 #pragma unroll 1
@@ -242,7 +244,7 @@ __global__ void __launch_bounds__(256, 2) digit_split_kernel(SplitArgs S) {
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 const int k = k0 + 2 * i;
-                x[i] = (k <= r.kmax && (k > 0 || !imag)) ? g[d * plane + (k > 0 ? 2 * k - 1 + imag : 0)] : T(0);
+                x[i] = (k <= kmax && (k > 0 || !imag)) ? g[d * plane + (k > 0 ? 2 * k - 1 + imag : 0)] : T(0);
             }
 #pragma unroll 1
             for (int dl = 0; dl < (d == 0 ? 3 : 1); dl++) {
@@ -523,9 +525,10 @@ __global__ void __launch_bounds__(kDigitThreads, 1) digit_gemm_kernel(GemmDigitA
 }
 
 // ------------------------------------------------------------ unfold
-// The four quadrant parts of one (ring, item, variant) row → its 4n points, in place
+// The four quadrant parts of one (ring, item, variant) row → its 4n points: in place
+// (RLZ) or into the physical slot (RL, `phys` set)
 template <typename T>
-__global__ void __launch_bounds__(128) digit_unfold_kernel(void *H, const DigitRing *rings, const int *expo, int r0,
+__global__ void __launch_bounds__(128) digit_unfold_kernel(void *H, T *phys, const DigitRing *rings, const int *expo, int r0,
                                                            int nitems, int nvars, int bk, int iDim, int64_t jDim) {
     using R = typename std::conditional<std::is_same<T, double>::value, long long, float>::type;
     extern __shared__ __align__(16) unsigned char row_raw[];
@@ -534,7 +537,10 @@ __global__ void __launch_bounds__(128) digit_unfold_kernel(void *H, const DigitR
     const DigitRing &r = rings[ring];
     const int n = r.n, L = r.L, shift = r.shift;
     const int var = blockIdx.x / nitems + kDigitVariants - DigitFormat<T>::kVars, item = blockIdx.x % nitems;
-    R *h = (R *)H + ((int64_t)var * nvars + item / bk) * bk * jDim + (int64_t)bk * r.jofs + (int64_t)(item % bk) * L;
+    const int64_t at = (int64_t)(item / bk) * bk * jDim + (int64_t)bk * r.jofs + (int64_t)(item % bk) * L;
+    const R *h = (const R *)H + (int64_t)var * nvars * bk * jDim + at;
+    const int slot = var == 0 ? 0 : (var < 3 ? var + 2 : var - 2);  // f, ∂r, ∂rr, ∂λ, ∂λλ
+    T *dst = phys ? phys + (int64_t)slot * nvars * jDim + at : (T *)H + (int64_t)var * nvars * bk * jDim + at;
     for (int i = threadIdx.x; i < L; i += blockDim.x) row[i] = h[i];
     int e = 0;
     if constexpr (std::is_same<T, double>::value) e = expo[((size_t)var * nitems + item) * iDim + ring];
@@ -544,8 +550,8 @@ __global__ void __launch_bounds__(128) digit_unfold_kernel(void *H, const DigitR
         if (l < 0) l += L;
         if (l >= L) l -= L;
         if constexpr (std::is_same<T, double>::value)
-            ((double *)h)[l] = e == kNanColumn ? __longlong_as_double(0x7ff8000000000000ll) : fixed_to_double(v, e);
-        else h[l] = v;
+            dst[l] = e == kNanColumn ? __longlong_as_double(0x7ff8000000000000ll) : fixed_to_double(v, e);
+        else dst[l] = v;
     };
     for (int m = threadIdx.x; m < n; m += blockDim.x) {
         if (r.half == 0 && m == 0) {
@@ -652,11 +658,15 @@ __global__ void __launch_bounds__(256, 2) digit_fold_kernel(FoldArgs S) {
     }
 }
 
-// X_k ← X_k e^{−iδ_k}: the forward coefficients at the reference's rounded angles
-__global__ void __launch_bounds__(128) digit_turn_kernel(double *Fp, const DigitRing *rings, const int *delta, int64_t frows, int r0) {
+// X_k ← X_k e^{−iδ_k}: the forward coefficients at the reference's rounded angles,
+// zero above the item's own kmax
+__global__ void __launch_bounds__(128) digit_turn_kernel(double *Fp, const DigitRing *rings, const int *delta, const int *cap,
+                                                         int64_t frows, int r0) {
     const DigitRing &r = rings[r0 + blockIdx.y];
     double *f = Fp + (int64_t)blockIdx.x * frows + r.fofs;
-    for (int k = 1 + threadIdx.x; k <= r.kmax; k += blockDim.x) {
+    const int kmax = min(r.kmax, cap[blockIdx.x]);
+    for (int k = kmax + 1 + threadIdx.x; k <= r.kmax; k += blockDim.x) f[2 * k - 1] = f[2 * k] = 0.0;
+    for (int k = 1 + threadIdx.x; k <= kmax; k += blockDim.x) {
         const double d = (double)delta[r.dofs + k - 1] * 0x1p-70;
         const double re = f[2 * k - 1], im = f[2 * k];
         f[2 * k - 1] = fma(d, im, re);
@@ -672,6 +682,10 @@ constexpr int kDigitMinItems = 1;
 // bound of a grid's matrix digits (both directions: 4.3 GB at 200 cells, growing with
 // the cube of the ring count); larger grids keep the FFT kernels
 constexpr size_t kDigitTableBytes = (size_t)16 << 30;
+// RL grids hold far less data than these matrices (0.6 GB at 100 cells): up to about
+// 120 cells.  100 cells, one variable: ring_inverse 1.07 → 0.13 ms, ring_forward
+// 0.26 → 0.13 ms; 24 cells: 0.32 → 0.03 and 0.095 → 0.03 ms
+constexpr size_t kDigitTableBytesRl = (size_t)1 << 30;
 // spectra digits of one span of rings; larger grids take several spans
 constexpr int64_t kDigitScratchBytes = (int64_t)1 << 30;
 template <typename T>
@@ -702,6 +716,7 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
         r.half = r.n & 1;
         r.shift = r.half ? (r.n - 3) / 2 : (r.n - 2) / 2;
         r.kmax = rd[i].kmax;
+        for (size_t s = 1; s < rd.size() / nr; s++) r.kmax = std::max(r.kmax, rd[s * nr + i].kmax);  // RL: a set per variable
         r.te = (r.kmax / 2 + 1 + 15) / 16;
         r.to = std::max(1, ((r.kmax + 1) / 2 + 15) / 16);
         const int rows = r.n + 1 - r.half;
@@ -742,7 +757,7 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
     D.col_tiles = (ncol + 2 * F::kCols - 1) / (2 * F::kCols);
     D.col_tiles_fwd = (g->nitems + 2 * F::kCols - 1) / (2 * F::kCols);
     const size_t abytes = (size_t)atiles * digit_a_bytes<T>(), afbytes = (size_t)aftiles * digit_a_bytes<T>();
-    if (abytes + afbytes > kDigitTableBytes) return SS_OK;
+    if (abytes + afbytes > (g->rlz ? kDigitTableBytes : kDigitTableBytesRl)) return SS_OK;
     double *cosq = nullptr;
     const size_t mark = g->allocs.size();
     auto give_up = [&]() {  // the device has no room for the tables: the FFT kernels serve
@@ -798,6 +813,13 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
     const int *dd = nullptr;
     if (!upload(g, &dd, delta)) return give_up();
     D.delta = const_cast<int *>(dd);
+    std::vector<int> cap(g->nitems);
+    for (int i = 0; i < g->nitems; i++) {
+        const int km = g->rlz ? g->ring_kmax : g->kmaxv[i];
+        cap[i] = km >= 0 ? km : rd[nr - 1].ri;
+    }
+    if (!upload(g, &dd, cap)) return give_up();
+    D.cap = const_cast<int *>(dd);
     if (!make_set(0, nr, false, D.whole) || !make_set(0, nr, true, D.whole_fwd)) return give_up();
     D.chunks.resize(g->chunk_r0.size() - 1);
     D.chunks_fwd.resize(g->chunk_r0.size() - 1);
@@ -818,6 +840,11 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
     if (cudaMalloc(&p, (size_t)kDigitVariants * g->nitems * nr * sizeof(int)) != cudaSuccess) return give_up();
     g->allocs.push_back(p);
     D.expo = (int *)p;
+    if (!g->rlz) {  // quadrant parts (RLZ grids keep them in the ring outputs' buffer)
+        if (cudaMalloc(&p, (size_t)kDigitVariants * g->nitems * g->d.jDim * sizeof(T)) != cudaSuccess) return give_up();
+        g->allocs.push_back(p);
+        D.H = p;
+    }
     if (cudaMalloc((void **)&cosq, (size_t)cosn * 8) != cudaSuccess) return give_up();
     if (cudaHostAlloc((void **)&D.err, sizeof(int), cudaHostAllocMapped) != cudaSuccess) { D.err = nullptr; return give_up(); }
     *D.err = 0;
@@ -836,7 +863,7 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
 }
 
 int32_t digit_build(ss_grid *g, const std::vector<RingDesc> &rings) {
-    if (!g->rlz || g->tl != TL_F64) return SS_OK;
+    if (g->tl != TL_F64) return SS_OK;
     int least = kDigitMinItems;
     if (const char *e = std::getenv("SS_RING_DIGITS")) {  // tuning override: the least item count, 0 for never
         least = std::atoi(e);
@@ -844,7 +871,7 @@ int32_t digit_build(ss_grid *g, const std::vector<RingDesc> &rings) {
     }
     if (g->nitems < least) return SS_OK;
     // binary64 sums of a ring stay below 2^63 for n ≤ 1023 (64-bit fixed point at 2^-52 of the column scale)
-    if (rings.back().ri + 1 > (g->tl == TL_F64 ? 1023 : 2047)) return SS_OK;
+    if (rings[g->d.iDim - 1].ri + 1 > (g->tl == TL_F64 ? 1023 : 2047)) return SS_OK;
     return g->tl == TL_F64 ? build<double>(g, rings) : build<float>(g, rings);
 }
 
@@ -860,9 +887,9 @@ static int32_t inverse(ss_grid *g, cudaStream_t st, const DigitSet &set, int *la
     const int groups = (g->nitems + kDigitGroup - 1) / kDigitGroup;
     for (const DigitSpan &sp : set.spans) {
         const int nr = sp.r1 - sp.r0;
-        SplitArgs S{g->G, D.rings, set.btile, (uint8_t *)D.B, D.expo, D.delta, g->frows, sp.r0, g->nitems, (int)d.iDim, D.col_tiles};
+        SplitArgs S{g->G, D.rings, set.btile, (uint8_t *)D.B, D.expo, D.delta, D.cap, g->frows, sp.r0, g->nitems, (int)d.iDim, D.col_tiles};
         digit_split_kernel<T><<<dim3(groups, nr), 256, 0, st>>>(S);
-        GemmDigitArgs A{(const uint8_t *)D.A, (const uint8_t *)D.B, set.items + sp.item0, sp.items, D.rings, D.expo, g->H,
+        GemmDigitArgs A{(const uint8_t *)D.A, (const uint8_t *)D.B, set.items + sp.item0, sp.items, D.rings, D.expo, D.H ? D.H : g->H,
                         d.jDim, g->frows, g->nitems, (int)d.nvars, (int)d.b_kDim, (int)d.iDim, D.err};
         digit_gemm_kernel<T, false><<<std::min(g->sms, sp.items), kDigitThreads, digit_smem<T>(), st>>>(A);
         *launches += 2;
@@ -870,7 +897,8 @@ static int32_t inverse(ss_grid *g, cudaStream_t st, const DigitSet &set, int *la
         if (D.columns.on) continue;  // digit_columns_inverse reads the parts
         const size_t row = (size_t)4 * (sp.r1 + g->pOL + 1) * sizeof(T);
         digit_unfold_kernel<T><<<dim3(DigitFormat<T>::kVars * g->nitems, nr), 128, row, st>>>(
-            g->H, D.rings, D.expo, sp.r0, g->nitems, (int)d.nvars, (int)d.b_kDim, (int)d.iDim, d.jDim);
+            D.H ? D.H : g->H, g->rlz ? nullptr : (T *)g->phys, D.rings, D.expo, sp.r0, g->nitems, (int)d.nvars,
+            (int)d.b_kDim, (int)d.iDim, d.jDim);
         CUDA_TRY(cudaGetLastError());
         *launches += 1;
     }
@@ -884,13 +912,13 @@ int32_t digit_ring_forward(ss_grid *g, cudaStream_t st, int chunk, int *launches
     const int groups = (g->nitems + kDigitGroup - 1) / kDigitGroup;
     for (const DigitSpan &sp : set.spans) {
         const int nr = sp.r1 - sp.r0;
-        FoldArgs S{(const double *)g->C, D.rings, set.btile, (uint8_t *)D.B, D.expo, d.jDim, sp.r0, g->nitems, (int)d.iDim,
+        FoldArgs S{(const double *)(g->rlz ? g->C : g->phys), D.rings, set.btile, (uint8_t *)D.B, D.expo, d.jDim, sp.r0, g->nitems, (int)d.iDim,
                    (int)d.b_kDim, D.col_tiles_fwd};
         digit_fold_kernel<<<dim3(groups, nr), 256, 0, st>>>(S);
         GemmDigitArgs A{(const uint8_t *)D.Af, (const uint8_t *)D.B, set.items + sp.item0, sp.items, D.rings, D.expo, g->F,
                         d.jDim, g->frows, g->nitems, (int)d.nvars, (int)d.b_kDim, (int)d.iDim, D.err};
         digit_gemm_kernel<double, true><<<std::min(g->sms, sp.items), kDigitThreads, digit_smem<double>(), st>>>(A);
-        digit_turn_kernel<<<dim3(g->nitems, nr), 128, 0, st>>>((double *)g->F, D.rings, D.delta, g->frows, sp.r0);
+        digit_turn_kernel<<<dim3(g->nitems, nr), 128, 0, st>>>((double *)g->F, D.rings, D.delta, D.cap, g->frows, sp.r0);
         CUDA_TRY(cudaGetLastError());
         *launches += 3;
     }

@@ -1,4 +1,4 @@
-// ss_digit.h — ring DFTs of RLZ grids as tensor-core products of digit slices
+// ss_digit.h — ring DFTs as tensor-core products of digit slices
 // (ss_digit.cu): plan, device tables and launches.
 #pragma once
 
@@ -114,6 +114,8 @@ struct DigitPlan {
     void *A = nullptr;      // digit planes of the inverse DFT matrices
     void *Af = nullptr;     // and of the forward ones
     int *delta = nullptr;   // δ_k·2^70
+    int *cap = nullptr;     // per item: its variable's kmax
+    void *H = nullptr;      // RL: quadrant parts
     void *B = nullptr;      // digit planes of one span's ring spectra
     int *expo = nullptr;    // [variant][item][ring] column exponents
     int *err = nullptr;     // host-mapped: a bounded wait gave up
