@@ -505,6 +505,10 @@ static int32_t fwd_columns(ss_grid *g, cudaStream_t st, int chunk) {
     const int N = (int)d.kDim, half = (N + 1) / 2;
     size_t smem = (size_t(64) * (N | 1) + size_t(Cl.bk) * half) * sizeof(T);
     StageScope sc(g, SS_STAGE_CHEB_FWD, st);
+    if (g->digit.columns.fon) {
+        g->launches[SS_STAGE_CHEB_FWD]++;
+        return digit_columns_forward(g, st, Cl.col0, Cl.col1);
+    }
     CUDA_TRY((launch_cheb_forward<P, T>(Cl, smem, st, N)));
     g->launches[SS_STAGE_CHEB_FWD]++;
     return SS_OK;

@@ -105,6 +105,10 @@ struct DigitColumns {
     int *mexpo = nullptr;
     int2 *blocks = nullptr;
     std::vector<int> first;          // first block of every ring, their number at the end
+    bool fon = false;                // forward (binary64): K-steps of levels, blocks of 32 modes, lanes of a column
+    int fsteps = 0, fblocks = 0, fgroup = 4;
+    void *fM = nullptr;
+    int *fexpo = nullptr;
 };
 
 struct DigitPlan {
@@ -133,6 +137,8 @@ int32_t digit_ring_inverse(ss_grid *g, cudaStream_t st, int chunk, int *launches
 int32_t digit_ring_forward(ss_grid *g, cudaStream_t st, int chunk, int *launches);
 void digit_free(ss_grid *g);
 int32_t digit_columns_build(ss_grid *g, const std::vector<ChebHost> &cheb);
+// cheb_forward of the columns [col0, col1): physical slot 1 → C
+int32_t digit_columns_forward(ss_grid *g, cudaStream_t st, int64_t col0, int64_t col1);
 // cheb_inverse of the parts digit_ring_inverse left in H: H → physical
 int32_t digit_columns_inverse(ss_grid *g, cudaStream_t st, int chunk);
 

@@ -43,6 +43,7 @@ namespace ss {
 
 constexpr int kZ = 32;                      // matrix rows (levels) of one product
 constexpr int kZStep = 6 * kZ * 32;         // bytes of a K-step of matrix digits: 6 planes × 32 rows × 16
+constexpr int kAStep = 6 * kDigitPlane;     // and of column digits
 // Warps: producing, draining (half of them per accumulator), one issuing.  Measured
 // on the 200-cell FP64 grid: 8 + 16 warps 4.95 ms, 16 + 8 5.34 ms, 8 + 8 5.7 ms.
 constexpr int kProducers = 8, kDrains = 16;
@@ -68,6 +69,23 @@ struct ColumnArgs {
 __device__ __forceinline__ void producers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kProducers * 32) : "memory"); }
 __device__ __forceinline__ void st_global_32B(double *p, const double (&v)[4]) {
     asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3]) : "memory");
+}
+
+// one K-step of a product: D_1..D_6, then D_0, then the rest of digit 0 on the
+// first step (as in digit_gemm)
+__device__ __forceinline__ void issue_step64(uint32_t tacc, uint32_t sa, uint32_t sb, bool first) {
+    const uint64_t bd = operand_desc(sb);
+    if (first) {
+        mma_f16(tacc + kZ, operand_desc(sa + kDigitPlane), bd, mma_idesc(6 * kZ), 0u);
+        mma_f16(tacc, operand_desc(sa), bd, mma_idesc(kZ), 0u);
+        mma_f16(tacc + kZ, operand_desc(sa), operand_desc(sb + kZ * 32), mma_idesc(5 * kZ), 1u);
+    } else {
+        mma_f16(tacc, operand_desc(sa), bd, mma_idesc(6 * kZ), 1u);
+        mma_f16(tacc + kZ, operand_desc(sa + kDigitPlane), bd, mma_idesc(6 * kZ), 1u);
+    }
+#pragma unroll
+    for (int i = 2; i < 6; i++)
+        mma_f16(tacc + i * kZ, operand_desc(sa + i * kDigitPlane), bd, mma_idesc((7 - i) * kZ), 1u);
 }
 
 // grid = (CTAs per variable, variables); a CTA walks (block of 32 quadrant
@@ -108,7 +126,7 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
         const uint4 *src = reinterpret_cast<const uint4 *>(g.M + (size_t)v * 3 * g.zblocks * jobs_bytes);
         for (int i = threadIdx.x; i < 3 * g.zblocks * jobs_bytes / 16; i += blockDim.x) reinterpret_cast<uint4 *>(sM)[i] = src[i];
     }
-    for (int i = threadIdx.x; i < nb * KS * 6 * kDigitPlane / 16; i += blockDim.x)
+    for (int i = threadIdx.x; i < nb * KS * kAStep / 16; i += blockDim.x)
         reinterpret_cast<uint4 *>(sA)[i] = make_uint4(0, 0, 0, 0);  // K groups of 8 without modes stay zero
     for (int i = threadIdx.x; i < 3 * g.zblocks * kZ; i += blockDim.x) sE[i] = g.mexpo[(size_t)v * 3 * g.zblocks * kZ + i] - 53;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -252,18 +270,7 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
                     const uint32_t tacc = tmem + t * 256;
                     for (int k = 0; k < KS; k++) {
                         const uint32_t sa = sa0 + k * 6 * kDigitPlane, sb = smem_addr(sM) + (q * KS + k) * kZStep;
-                        const uint64_t bd = operand_desc(sb);
-                        if (k == 0) {  // D_1..D_6, then D_0, then the rest of digit 0 (as in digit_gemm)
-                            mma_f16(tacc + kZ, operand_desc(sa + kDigitPlane), bd, mma_idesc(6 * kZ), 0u);
-                            mma_f16(tacc, operand_desc(sa), bd, mma_idesc(kZ), 0u);
-                            mma_f16(tacc + kZ, operand_desc(sa), operand_desc(sb + kZ * 32), mma_idesc(5 * kZ), 1u);
-                        } else {
-                            mma_f16(tacc, operand_desc(sa), bd, mma_idesc(6 * kZ), 1u);
-                            mma_f16(tacc + kZ, operand_desc(sa + kDigitPlane), bd, mma_idesc(6 * kZ), 1u);
-                        }
-#pragma unroll
-                        for (int i = 2; i < 6; i++)
-                            mma_f16(tacc + i * kZ, operand_desc(sa + i * kDigitPlane), bd, mma_idesc((7 - i) * kZ), 1u);
+                        issue_step64(tacc, sa, sb, k == 0);
                     }
                     mma_commit(&accf[t]);
                 }
@@ -346,6 +353,195 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
 
+// ------------------------------------------------------------ forward columns
+// CBtransform! of binary64 grids: the first b_kDim modes of 128 consecutive columns
+// per tile.  A column's levels are contiguous, so G = 4..16 neighbouring lanes hold
+// 8 levels each, find the column's exponent by shuffles and cut in registers.
+// Measured: 200 cells, 32 levels, 5 variables 2.60 ms with FP64 FMAs → 0.81 ms (the bytes
+// alone take 0.23 ms), 37 cells, 20 levels, 3 variables 37 → 25 µs; bound by cutting and
+// combining.  The error against 64-bit sums is no larger than the FMA kernel's.
+struct ForwardColumnArgs {
+    const double *phys;       // slot 1
+    double *C;                // [variable][ring][mode][ring point]
+    const RingDesc *rings;
+    const int *col_ring;
+    const uint8_t *M;         // [var][mode blocks][steps] matrix digits
+    const int *mexpo;         // [var][32·mode blocks]
+    int64_t col0, col1, np, jDim;
+    int N, bk, steps, blocks, group;
+    int *err;
+};
+
+__global__ void __launch_bounds__(kColThreads, 1) digit_columns_forward_kernel(ForwardColumnArgs g) {
+    extern __shared__ __align__(1024) uint8_t dsm[];
+    __shared__ __align__(8) uint64_t afull[2], aempty[2], accf[2], acce[2], drain;
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile int quit;
+    __shared__ int row_expo[kRowExpo][128];
+    __shared__ __align__(16) int sE[kZ * kMaxZBlocks];  // row exponents of the matrix, less 1
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int v = blockIdx.y, KS = g.steps;
+    uint8_t *sM = dsm, *sA = sM + (size_t)g.blocks * KS * kZStep;  // matrix, then 2 operand buffers
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_slot)), "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2; i++) {
+            bar_init(&afull[i], kProducers * 32);
+            bar_init(&aempty[i], 1);
+            bar_init(&accf[i], 1);
+            bar_init(&acce[i], kDrains * 16);
+        }
+        bar_init(&drain, 1);
+        quit = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    {
+        const uint4 *src = reinterpret_cast<const uint4 *>(g.M + (size_t)v * g.blocks * KS * kZStep);
+        for (int i = threadIdx.x; i < g.blocks * KS * kZStep / 16; i += blockDim.x) reinterpret_cast<uint4 *>(sM)[i] = src[i];
+    }
+    for (int i = threadIdx.x; i < 2 * KS * kAStep / 16; i += blockDim.x)
+        reinterpret_cast<uint4 *>(sA)[i] = make_uint4(0, 0, 0, 0);  // levels beyond N stay zero
+    for (int i = threadIdx.x; i < g.blocks * kZ; i += blockDim.x) sE[i] = g.mexpo[(size_t)v * g.blocks * kZ + i] - 1;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    const int64_t ntile = (g.col1 - g.col0 + 127) / 128;
+    const int nitem = (int)((ntile - blockIdx.x + gridDim.x - 1) / gridDim.x);
+
+    if (warp < kProducers) {
+        const int G = g.group, per = 256 / G;  // lanes of a column, columns of a sweep
+        const int kg = threadIdx.x % G, z0 = kg * 8;
+        const bool pairs = g.N % 2 == 0;
+        auto load = [&](int64_t c, double (&x)[8]) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) x[i] = 0.0;
+            if (c >= g.col1) return;
+            const double *src = g.phys + (size_t)v * g.np + c * g.N + z0;
+            if (pairs) {
+#pragma unroll
+                for (int i = 0; i < 8; i += 2)
+                    if (z0 + i < g.N) {
+                        const double2 t = *reinterpret_cast<const double2 *>(src + i);
+                        x[i] = t.x; x[i + 1] = t.y;
+                    }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    if (z0 + i < g.N) x[i] = src[i];
+            }
+        };
+        bool ok = true;
+        double x[8], next[8];
+        load(g.col0 + blockIdx.x * 128ll + threadIdx.x / G, next);
+        for (int it = 0; ok && it < nitem; it++) {
+            const int64_t c0 = g.col0 + (blockIdx.x + (int64_t)it * gridDim.x) * 128;
+            const int buf = it & 1;
+            uint8_t *A = sA + (size_t)buf * KS * kAStep;
+            for (int r0 = 0; r0 < 128; r0 += per) {
+                const int row = r0 + threadIdx.x / G;
+#pragma unroll
+                for (int i = 0; i < 8; i++) x[i] = next[i];
+                // the next sweep's levels (of this tile or the first of the next) arrive while these are cut
+                const bool last = r0 + per >= 128;
+                const int64_t ahead = last ? (it + 1 < nitem ? c0 + 128ll * gridDim.x + threadIdx.x / G : g.col1) : c0 + row + per;
+                load(ahead, next);
+                uint32_t mx = 0;
+#pragma unroll
+                for (int i = 0; i < 8; i++) mx = max(mx, (uint32_t)__double2hiint(x[i]) & 0x7fffffffu);
+                for (int o = 1; o < G; o <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                const int eb = (int)(mx >> 20), e = eb == 0x7ff ? kNanColumn : max(eb, 1);
+                unsigned long long U[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) U[i] = kDigitBias + (unsigned long long)(e == kNanColumn ? 0ll : fixed_point<54>(x[i], e));
+                uint4 w[6];
+                planes8(U, w);
+                if (r0 == 0 && !(ok = bar_wait(&aempty[buf], ((it >> 1) & 1) ^ 1, &quit))) break;
+                if (kg == 0) row_expo[it % kRowExpo][row] = e;
+                if (kg < 2 * KS) {
+                    uint8_t *dst = A + (kg >> 1) * kAStep + (row >> 3) * 256 + (kg & 1) * 128 + (row & 7) * 16;
+#pragma unroll
+                    for (int i = 0; i < 6; i++) *reinterpret_cast<uint4 *>(dst + i * kDigitPlane) = w[i];
+                }
+            }
+            if (!ok) break;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            bar_arrive(&afull[buf]);
+        }
+    } else if (warp == kProducers + kDrains) {
+        if (lane == 0) {
+            bool ok = true;
+            uint32_t job = 0;
+            for (int it = 0; ok && it < nitem; it++) {
+                const int buf = it & 1;
+                if (!(ok = bar_wait(&afull[buf], (it >> 1) & 1, &quit))) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int q = 0; ok && q < g.blocks; q++, job++) {
+                    const int t = job & 1;
+                    if (!(ok = bar_wait(&acce[t], ((job >> 1) & 1) ^ 1, &quit))) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    for (int k = 0; k < KS; k++)
+                        issue_step64(tmem + t * 256, smem_addr(sA) + (buf * KS + k) * kAStep, smem_addr(sM) + (q * KS + k) * kZStep, k == 0);
+                    mma_commit(&accf[t]);
+                }
+                if (ok) mma_commit(&aempty[buf]);
+            }
+            if (!ok) {
+                int never = 0;
+                mma_commit(&drain);
+                bar_wait(&drain, 0, &never);
+            }
+        }
+    } else {
+        const int mine = (warp - kProducers) >> 3;
+        const int zh = ((warp >> 2) & 1) * 16;
+        const int quad = warp & 3, row = quad * 32 + lane;
+        const uint32_t tacc = tmem + ((uint32_t)(quad * 32) << 16) + mine * 256 + zh;
+        uint32_t job = 0;
+        bool ok = true;
+        for (int it = 0; ok && it < nitem; it++) {
+            const int64_t c = g.col0 + (blockIdx.x + (int64_t)it * gridDim.x) * 128 + row;
+            const bool live = c < g.col1;
+            const RingDesc *r = g.rings + (live ? g.col_ring[c] : 0);
+            const int64_t L = r->L;
+            double *const out = g.C + (size_t)v * g.bk * g.jDim + (int64_t)g.bk * r->jofs + (c - r->jofs);
+            for (int q = 0; ok && q < g.blocks; q++, job++) {
+                if ((int)(job & 1) != mine) continue;
+                if (!(ok = __all_sync(0xffffffffu, bar_wait(&accf[mine], (job >> 1) & 1, &quit)))) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const int er = row_expo[it % kRowExpo][row];
+                const int m0 = q * kZ + zh;
+#pragma unroll 1
+                for (int k0 = 0; k0 < 16 && m0 + k0 < g.bk; k0 += 4) {
+                    float D[7][4];
+#pragma unroll
+                    for (int s = 0; s < 7; s++) tmem_ld4(tacc + s * kZ + k0, D[s]);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        unsigned long long V = 0ull - Combine<false>::kOffset;
+                        Combine<false>::add(V, D[0][k], D[1][k], D[2][k], D[3][k], D[4][k], D[5][k], D[6][k]);
+                        double o = fixed_to_double((long long)V, er + sE[m0 + k0 + k]);  // V 2^(er − 1022 + mexpo − 53)
+                        if (er == kNanColumn) o = __longlong_as_double(0x7ff8000000000000ll);
+                        if (live && m0 + k0 + k < g.bk) out[(int64_t)(m0 + k0 + k) * L] = o;
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                bar_arrive(&acce[mine]);
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0 && quit) *g.err = 1;
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+}
+
 // ------------------------------------------------------------ host
 // balanced digits of x·2^(53 − e), |x| < 2^e (53-bit fixed point), most significant first
 static void host_digits(double x, int e, int (&d)[6]) {
@@ -362,9 +558,63 @@ static size_t column_smem(int steps, int zblocks, int bk, int buffers, int raws)
     return (size_t)3 * zblocks * steps * kZStep + (size_t)buffers * steps * 6 * kDigitPlane + (size_t)raws * bk * 128 * 8;
 }
 
-int32_t digit_columns_build(ss_grid *g, const std::vector<ChebHost> &cheb) {
+static size_t forward_smem(int steps, int blocks) {
+    return (size_t)blocks * steps * kZStep + (size_t)2 * steps * kAStep;
+}
+
+static int32_t build_forward(ss_grid *g, const std::vector<ChebHost> &cheb) {
+    DigitColumns &Q = g->digit.columns;
+    const int N = (int)g->d.kDim, bk = (int)g->d.b_kDim, nv = (int)g->d.nvars;
+    Q.fsteps = (N + 15) / 16;
+    Q.fblocks = (bk + kZ - 1) / kZ;
+    Q.fgroup = N <= 32 ? 4 : (N <= 64 ? 8 : 16);
+    if (Q.fsteps > 6 || Q.fblocks > kMaxZBlocks || forward_smem(Q.fsteps, Q.fblocks) > 232448 - 8192) return SS_OK;
+    const int job = Q.fsteps * kZStep;
+    std::vector<uint8_t> M((size_t)nv * Q.fblocks * job, 0);
+    std::vector<int> E((size_t)nv * Q.fblocks * kZ, 0);
+    for (int v = 0; v < nv; v++) {
+        const ChebHost &c = cheb[v];
+        for (int k = 0; k < bk; k++) {
+            std::vector<double> row(N, 0.0);
+            double top = 0.0;
+            for (int j = 0; j < c.half; j++) {  // folded over j ↔ N − 1 − j: even k +, odd k −
+                const double w = c.fwd[(size_t)k * c.half + j];
+                row[j] = w;
+                if (N - 1 - j != j) row[N - 1 - j] = k % 2 ? -w : w;
+                top = std::max(top, std::fabs(w));
+            }
+            int e = 0;
+            if (top > 0.0) std::frexp(top, &e);
+            const int kb = k / kZ, kr = k % kZ;
+            E[((size_t)v * Q.fblocks + kb) * kZ + kr] = e;
+            uint8_t *dst = M.data() + ((size_t)v * Q.fblocks + kb) * job;
+            for (int j = 0; j < N; j++) {
+                int dg[6];
+                host_digits(row[j], e, dg);
+                for (int q = 0; q < 6; q++) {
+                    const __half h = __float2half_rn((float)dg[q]);
+                    const int rr = q * kZ + kr, kk = j % 16;
+                    std::memcpy(dst + (j / 16) * kZStep + (rr >> 3) * 256 + (kk >> 3) * 128 + (rr & 7) * 16 + (kk & 7) * 2, &h, 2);
+                }
+            }
+        }
+    }
+    void *pm = nullptr, *pe = nullptr;
+    auto put = [&](const void *src, size_t bytes, void **dst) {
+        if (cudaMalloc(dst, bytes) != cudaSuccess) { cudaGetLastError(); return false; }
+        g->allocs.push_back(*dst);
+        return cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
+    };
+    if (!put(M.data(), M.size(), &pm) || !put(E.data(), E.size() * 4, &pe)) return SS_OK;
+    Q.fM = pm; Q.fexpo = (int *)pe;
+    CUDA_TRY(cudaFuncSetAttribute(digit_columns_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)forward_smem(Q.fsteps, Q.fblocks)));
+    Q.fon = true;
+    return SS_OK;
+}
+
+static int32_t build_inverse(ss_grid *g, const std::vector<ChebHost> &cheb) {
     DigitPlan &P = g->digit;
-    if (!P.on || !g->rlz || g->tl != TL_F64) return SS_OK;
     const int N = (int)g->d.kDim, bk = (int)g->d.b_kDim, nv = (int)g->d.nvars;
     DigitColumns &Q = P.columns;
     Q.steps = (bk + 15) / 16;
@@ -448,6 +698,27 @@ int32_t digit_columns_build(ss_grid *g, const std::vector<ChebHost> &cheb) {
     Q.M = pm; Q.mexpo = (int *)pe; Q.blocks = (int2 *)pb;
     CUDA_TRY(cudaFuncSetAttribute(Q.steps <= 2 ? digit_columns_kernel<true> : digit_columns_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLimit));
     Q.on = true;
+    return SS_OK;
+}
+
+int32_t digit_columns_build(ss_grid *g, const std::vector<ChebHost> &cheb) {
+    if (!g->digit.on || !g->rlz || g->tl != TL_F64) return SS_OK;
+    const int32_t rc = build_forward(g, cheb);
+    return rc ? rc : build_inverse(g, cheb);
+}
+
+int32_t digit_columns_forward(ss_grid *g, cudaStream_t st, int64_t col0, int64_t col1) {
+    if (col1 <= col0) return SS_OK;
+    const DigitColumns &Q = g->digit.columns;
+    const ss_dims &d = g->d;
+    ForwardColumnArgs A{};
+    A.phys = (const double *)g->phys; A.C = (double *)g->C; A.rings = g->d_rings; A.col_ring = g->d_col_ring;
+    A.M = (const uint8_t *)Q.fM; A.mexpo = Q.fexpo; A.col0 = col0; A.col1 = col1; A.np = d.n_physical; A.jDim = d.jDim;
+    A.N = (int)d.kDim; A.bk = (int)d.b_kDim; A.steps = Q.fsteps; A.blocks = Q.fblocks; A.group = Q.fgroup; A.err = g->digit.err;
+    const int64_t tiles = (col1 - col0 + 127) / 128;
+    const int per = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, g->sms / (int)d.nvars));
+    digit_columns_forward_kernel<<<dim3(per, (unsigned)d.nvars), kColThreads, forward_smem(Q.fsteps, Q.fblocks), st>>>(A);
+    CUDA_TRY(cudaGetLastError());
     return SS_OK;
 }
 

@@ -89,3 +89,16 @@ def test_digit_and_fft_kernels_agree(monkeypatch, cells, levels, nvars):
         assert np.max(np.abs(spec[:, v] - spec0[:, v])) <= TOL64 * np.max(np.abs(spec0[:, v]))
         for s in range(7):
             assert np.max(np.abs(phys[:, v, s] - phys0[:, v, s])) <= TOL64 * np.max(np.abs(phys0[:, v, s]))
+
+
+# forward columns: 8 levels a lane, 4, 8 or 16 lanes a column (32 and 64 levels), 16 levels a K-step,
+# 32 modes a block (48 and 50 levels keep 32 and 33 modes), the last level count with six K-steps
+@pytest.mark.parametrize("cells,levels,nvars", [(3, 6, 1), (5, 8, 2), (4, 31, 1), (7, 32, 1), (5, 48, 1), (4, 50, 2),
+                                               (6, 64, 1), (3, 65, 1), (4, 96, 1), (3, 97, 1)])
+def test_forward_columns_match_oracle(cells, levels, nvars):
+    gp = _gp(cells, levels, nvars)
+    pts = S.getGridpoints(S.createGrid(gp))
+    u = np.column_stack([fields.blob_sum(pts, seed=60 + v, nblobs=4, wmin=2.0, wmax=6.0, zmax=1000.0, noise=1e-3)
+                         for v in range(nvars)])
+    _, _, sg, so, pg, po = _run_both(gp, u)
+    _assert_parity(sg, so, pg, po, gp, tol=TOL64)
