@@ -574,6 +574,41 @@ bool sa_band_serves(const ss_grid *g) {
 }
 }  // namespace ss
 
+// Launches of the ring transforms of the whole grid; fn(list, rings, largest bucket, few).
+// A bucket joins the launch of the larger one before it when its CTAs with that
+// bucket's shared memory fill the GPU at most twice: below that the gap between two
+// launches and the emptying GPU at the end of each cost more than the lower residency
+// (30 to 600 cells, binary32 and binary64: 2 is within 5 % of the best of 0.5, 2, 3, 4,
+// 5, 8 and 20; at 20 the 600-cell grid of 12 variables runs 1.06×, of 3 variables 1.6×
+// as long); behind a launch of more than 16 fillings the gap is nothing (400 cells × 43
+// modes × 4 variables, binary32: 0.4 % of the forward transform lost by joining).
+// `few`: the threads of an item per CTA fit the GPU at once.  Such launches take one item
+// per CTA, and the inverse one output per CTA: five times the CTAs, each reading the
+// spectrum again.  Binary32, RL, both ways: 251 cells × 1 variable 115
+// against 150 µs, 120 × 3 104 / 140, but 120 × 6 193 / 145, 60 × 12 145 / 93; binary64:
+// 130 × 4 575 / 650, 251 × 4 (not few) equal.
+// Inverse rings, a launch per bucket → this rule: binary32 RL 30 cells × 3 118 → 24 µs,
+// 251 × 4 660 → 420; binary64 RL 130 × 1 1220 → 189, 400 × 4 7442 → 6612.
+template <typename Fn>
+static int32_t for_ring_launches(ss_grid *g, int chunk, bool inverse, int threads, Fn fn) {
+    if (chunk >= 0)
+        return for_ring_segments(g, chunk, [&](const int *list, int count, const RingBucket &b) { return fn(list, count, b, false); });
+    for (size_t b = 0; b < g->buckets.size();) {
+        const RingBucket &top = g->buckets[b];
+        const double per_sm = (227.0 * 1024) / (double)(ring_item_smem(g, top, inverse) + 2048);
+        int count = top.count;
+        for (b++; b < g->buckets.size(); b++) {
+            if ((double)g->buckets[b].count * g->nitems > 2.0 * per_sm * g->sms) break;
+            if ((double)count * g->nitems > 16.0 * per_sm * g->sms) break;
+            count += g->buckets[b].count;
+        }
+        const bool few = (int64_t)count * g->nitems * threads <= (int64_t)g->sms * 2048;
+        const int32_t st = fn(g->d_ring_list + top.offset, count, top, few);
+        if (st) return st;
+    }
+    return SS_OK;
+}
+
 template <typename P, typename T>
 static int32_t fwd_rings(ss_grid *g, cudaStream_t st, int chunk) {
     StageScope sc(g, SS_STAGE_RING_FWD, st);
@@ -584,10 +619,10 @@ static int32_t fwd_rings(ss_grid *g, cudaStream_t st, int chunk) {
         return rc;
     }
     RingLaunch L = ring_record(g, false);
-    return for_ring_segments(g, chunk, [&](const int *list, int count, const RingBucket &bkt) -> int32_t {
+    return for_ring_launches(g, chunk, false, g->ring_threads_fwd, [&](const int *list, int count, const RingBucket &bkt, bool few) -> int32_t {
         L.ring_list = list;
         const size_t smem = ring_item_smem(g, bkt, false);
-        L.ib = ring_batch(smem, g->nitems, count, 4 * g->sms, g->ring_threads_fwd, bkt.max_buf);
+        L.ib = few ? 1 : ring_batch(smem, g->nitems, count, 4 * g->sms, g->ring_threads_fwd, bkt.max_buf);
         CUDA_TRY((launch_ring_forward<P, T>(L, count, g->nitems, smem, g->ring_threads_fwd, st)));
         g->launches[SS_STAGE_RING_FWD]++;
         return SS_OK;
@@ -646,11 +681,12 @@ static int32_t inv_rings(ss_grid *g, cudaStream_t st, int chunk) {
         if (rc || g->tl == TL_F64) return rc;
     }
     RingLaunch L = ring_record(g, true);
-    L.value_only = g->digit.on;
-    return for_ring_segments(g, chunk, [&](const int *list, int count, const RingBucket &bkt) -> int32_t {
+    L.variant = g->digit.on ? 1 : 0;  // the digit products have written the derivatives
+    return for_ring_launches(g, chunk, true, g->ring_threads_inv, [&](const int *list, int count, const RingBucket &bkt, bool few) -> int32_t {
         L.ring_list = list;
         const size_t sm = ring_item_smem(g, bkt, true);
-        L.ib = ring_batch(sm, g->nitems, count, 4 * g->sms, g->ring_threads_inv, bkt.max_buf);
+        L.ib = few ? 1 : ring_batch(sm, g->nitems, count, 4 * g->sms, g->ring_threads_inv, bkt.max_buf);
+        L.split = few && L.variant == 0;
         CUDA_TRY((launch_ring_inverse<P, T>(L, count, g->nitems, sm, g->ring_threads_inv, st)));
         g->launches[SS_STAGE_RING_INV]++;
         return SS_OK;

@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(256, kRingMinBlocks<T>) ring_forward_kernel(Ri
 // d=2 → ∂rr.
 // ====================================================================
 template <typename P, typename T>
-__device__ __forceinline__ void ring_inverse_body(const RingLaunch &L, const int bx, const int by) {
+__device__ __forceinline__ void ring_inverse_body(const RingLaunch &L, const int bx, const int by, const int variant) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int kmx[kRingBatchMax];
     const int ring = L.ring_list[by];  // consecutive CTAs: item batches of one ring
@@ -187,7 +187,8 @@ __device__ __forceinline__ void ring_inverse_body(const RingLaunch &L, const int
     __syncthreads();
     const int G = (nb + kSweepSeqs - 1) / kSweepSeqs;
 
-    for (int d = 0; d < (L.value_only ? 1 : 3); d++) {
+    const int d0 = variant <= 3 ? 0 : variant - 3, d1 = variant == 0 ? 3 : d0 + 1;
+    for (int d = d0; d < d1; d++) {
         // FAtransform!: a_re = c br - s bi, a_im = s br + c bi (phase_filter.jl:154-190)
         for (UnitWalk uw_(nk); uw_.g < (G); uw_.next()) {
         const int k = uw_.n, g = uw_.g;
@@ -208,8 +209,9 @@ __device__ __forceinline__ void ring_inverse_body(const RingLaunch &L, const int
             }
         }
         __syncthreads();
-        const int nvar = (d == 0 && !L.value_only) ? 3 : 1;
-        for (int dl = 0; dl < nvar; dl++) {
+        const int dl0 = (d == 0 && variant > 0) ? variant - 1 : 0;
+        const int dl1 = variant > 0 ? dl0 + 1 : (d == 0 ? 3 : 1);
+        for (int dl = dl0; dl < dl1; dl++) {
             // packed spectrum Zp_k = E_k + i O_k, k < N (HC2R of length L via a length-N
             // inverse DFT).  With N = 2(ri + 1) > 2·kmax, entry k ≤ N/2 sees only X_k and
             // entry N − k only conj(X_k): for x = (iκ)^dl X_k (FIxcoefficients, κ = k)
@@ -261,7 +263,7 @@ __device__ __forceinline__ void ring_inverse_body(const RingLaunch &L, const int
 
 template <typename P, typename T>
 __global__ void __launch_bounds__(256, kRingMinBlocks<T>) ring_inverse_kernel(RingLaunch L) {
-    ring_inverse_body<P, T>(L, blockIdx.x, blockIdx.y);
+    ring_inverse_body<P, T>(L, blockIdx.x, blockIdx.y, L.split ? 1 + blockIdx.z : L.variant);
 }
 
 // ====================================================================
@@ -990,7 +992,7 @@ __global__ void __launch_bounds__(256, kRingMinBlocks<T>) ring_inverse_fused_ker
     __shared__ __align__(16) RingLaunch L;
     const BatchWork w = work[blockIdx.x];
     load_record(L, recs + w.rec);
-    ring_inverse_body<P, T>(L, w.bx, w.by);
+    ring_inverse_body<P, T>(L, w.bx, w.by, w.bz);
 }
 template <typename P, typename T>
 __global__ void __launch_bounds__(256) sb_project_fused_kernel(const SbLaunch *recs, const BatchWork *work) {
@@ -1054,7 +1056,7 @@ cudaError_t launch_ring_inverse(const RingLaunch &L0, int nrings, int nitems, si
     const size_t smem = per_item * L.ib;
     set_smem(ring_inverse_kernel<P, T>, smem);
     if (nrings > 65535) return cudaErrorInvalidConfiguration;  // rings index gridDim.y
-    ring_inverse_kernel<P, T><<<dim3((nitems + L.ib - 1) / L.ib, nrings), threads, smem, st>>>(L);
+    ring_inverse_kernel<P, T><<<dim3((nitems + L.ib - 1) / L.ib, nrings, L.split ? 5 : 1), threads, smem, st>>>(L);
     return cudaGetLastError();
 }
 template <typename P, typename T>

@@ -26,7 +26,8 @@ struct RingLaunch {
     int64_t np;
     int nitems, nvars, bk, rlz;
     int ib;                    // items per CTA (≤ kRingBatchMax): one batched DFT per pass
-    int value_only;            // ring_inverse: f alone (the digit products write the derivatives)
+    int variant;               // ring_inverse: 0 all five outputs, 1 + q the output q alone (f, ∂λ, ∂λλ, ∂r, ∂rr)
+    int split;                 // ring_inverse: gridDim.z = 5, one output per CTA
 };
 constexpr int kRingBatchMax = 16;
 constexpr size_t kRingBatchBytes = 128 * 1024;  // shared-memory budget of one ring batch

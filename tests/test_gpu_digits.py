@@ -102,3 +102,23 @@ def test_forward_columns_match_oracle(cells, levels, nvars):
                          for v in range(nvars)])
     _, _, sg, so, pg, po = _run_both(gp, u)
     _assert_parity(sg, so, pg, po, gp, tol=TOL64)
+
+
+# ring launches: buckets joined or not, an item or an output per CTA or several items, by the number
+# of (ring, item) pairs.  Each gives the same bits, so a variable's result does not depend on its company
+@pytest.mark.parametrize("geometry,precision,cells,levels", [
+    ("RL", "f32", 120, 0), ("RL", "f32", 300, 0), ("RL", "f64", 130, 0), ("RL", "f32", 5, 0), ("RLZ", "f32", 20, 8)])
+def test_ring_launches_give_the_same_bits(geometry, precision, cells, levels):
+    outs = []
+    for nvars in (1, 4, 12):
+        kw = dict(geometry=geometry, iMin=0.0, iMax=float(cells), num_cells=cells, precision=precision,
+                  vars={"v%d" % i: i + 1 for i in range(nvars)})
+        if levels:
+            kw.update(kMin=0.0, kMax=1000.0, kDim=levels)
+        gp = S.SpringsteelGridParameters(**kw)
+        n = S.getGridpoints(S.createGrid(gp)).shape[0]
+        u = np.random.default_rng(5).standard_normal((n, 12))[:, :nvars]
+        outs.append(_round_trip(gp, u))
+    for spec, phys in outs[1:]:
+        assert np.array_equal(spec[:, 0], outs[0][0][:, 0])
+        assert np.array_equal(phys[:, 0], outs[0][1][:, 0])
