@@ -706,6 +706,16 @@ static int32_t inv_columns(ss_grid *g, cudaStream_t st, int chunk) {
         g->launches[SS_STAGE_CHEB_INV]++;
         return digit_columns_inverse(g, st, chunk);
     }
+    Cl.nout = 5;
+    if (g->digit.quads.blocks) {  // binary32: the derivatives from the digit products' quadrant parts
+        const QuadBlocks &Q = g->digit.quads;
+        const int r0 = chunk < 0 ? 0 : g->chunk_r0[chunk], r1 = chunk < 0 ? (int)d.iDim : g->chunk_r0[chunk + 1];
+        Cl.nout = 1;
+        Cl.quads = Q.blocks + Q.first[r0];
+        Cl.nquads = Q.first[r1] - Q.first[r0];
+        Cl.drings = g->digit.rings;
+        g->launches[SS_STAGE_CHEB_INV]++;
+    }
     CUDA_TRY((launch_cheb_inverse<P, T>(Cl, 0, st, N)));
     g->launches[SS_STAGE_CHEB_INV]++;
     return SS_OK;

@@ -26,12 +26,16 @@
 // no larger than the FFT kernels' (9.2e-16 against 9.6e-16 of f, 3.0e-16 against
 // 3.3e-16 of the spectral array at 200 cells).
 //
+// Binary32 RLZ grids take the four derivative outputs this way (f keeps the FFT's
+// rounding, which a later ∂rr amplifies by r's spline, and so does the forward
+// direction): 400 cells, 64 levels, 4 variables ring_inverse 29.9 → 17.6 ms.
+//
 // digit_split   G (spectra at the mish points) → column exponents and digit
 //               planes in the MMA operand layout
 // digit_gemm    persistent, warp-specialised: bulk copies → 8-slot (6-slot) ring
 //               of K-steps → two issuing warps, one per accumulator half → two
 //               warpgroups drain and combine
-// digit_unfold  quadrant parts → ring points, in place
+// digit_unfold  quadrant parts → ring points (RL; RLZ columns read the parts)
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -43,6 +47,7 @@
 #include "ss_digit_dev.cuh"
 #include "ss_grid.h"
 #include "ss_internal.h"
+#include "ss_kernels.h"
 #include "ss_types.cuh"
 
 using namespace ss;
@@ -59,20 +64,21 @@ using namespace ss;
 namespace ss {
 
 // ------------------------------------------------------------ tables
-// cos(2πt/8n), t = 0..2n, of every ring
-__global__ void digit_cos_kernel(const DigitRing *rings, double *cosq) {
+// cos(2πt/8n)·2^53, t = 0..2n, of every ring
+__global__ void digit_cos_kernel(const DigitRing *rings, long long *cosq) {
     const DigitRing r = rings[blockIdx.x];
     const double inv = 1.0 / (4.0 * r.n);
     for (int t = threadIdx.x; t <= 2 * r.n; t += blockDim.x)
-        cosq[r.cosofs + t] = t <= r.n ? cospi(t * inv) : sinpi((2 * r.n - t) * inv);
+        cosq[r.cosofs + t] = __double2ll_rn((t <= r.n ? cospi(t * inv) : sinpi((2 * r.n - t) * inv)) * 0x1p53);
 }
-__device__ __forceinline__ double quarter_cos(const double *c, int n, int t) {  // cos(2πt/8n), 0 ≤ t < 8n
+__device__ __forceinline__ long long quarter_cos(const long long *c, int n, int t) {  // 0 ≤ t < 8n
     if (t > 4 * n) t = 8 * n - t;
     return t > 2 * n ? -c[4 * n - t] : c[t];
 }
-// entry of part `part` at row m, wavenumber k (half weight at k = 0: the result is doubled)
-__device__ __forceinline__ double dft_entry(const DigitRing &r, const double *c, int part, int m, int k) {
-    if (k > r.kmax || m >= r.n + 1 - r.half) return 0.0;
+// entry of part `part` at row m, wavenumber k, times 2^53 (`half`: half weight at k = 0,
+// the inverse's result is doubled)
+__device__ __forceinline__ long long dft_entry(const DigitRing &r, const long long *c, int part, int m, int k, bool half) {
+    if (k > r.kmax || m >= r.n + 1 - r.half) return 0;
     const int per = 8 * r.n;
     int t = (int)((long long)k * (2 * m + r.half) % per);
     if (part >= 2) {  // −sin = −cos(t − 2n)
@@ -80,16 +86,16 @@ __device__ __forceinline__ double dft_entry(const DigitRing &r, const double *c,
         if (t < 0) t += per;
         return -quarter_cos(c, r.n, t);
     }
-    const double v = quarter_cos(c, r.n, t);
-    return k == 0 ? 0.5 * v : v;
+    const long long v = quarter_cos(c, r.n, t);
+    return half && k == 0 ? v / 2 : v;
 }
 
 // digit planes of the inverse matrices: A tile = [digit][row group][K core][8 rows][8 k]
 // (forward: rows are wavenumbers and K the quadrant positions, without the half weight)
 template <typename T, bool kForward>
-__global__ void __launch_bounds__(256) digit_matrix_kernel(const DigitRing *rings, const double *cosq, uint8_t *A) {
+__global__ void __launch_bounds__(256) digit_matrix_kernel(const DigitRing *rings, const long long *cosq, uint8_t *A) {
     const DigitRing r = rings[blockIdx.x];
-    const double *c = cosq + r.cosofs;
+    const long long *c = cosq + r.cosofs;
     const int64_t ntile = kForward ? (int64_t)4 * r.rtf * r.tm : (int64_t)r.rt * 2 * (r.te + r.to);
     for (int64_t e = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; e < ntile * 256; e += (int64_t)gridDim.y * blockDim.x) {
         const int64_t tile = e >> 8;
@@ -107,35 +113,32 @@ __global__ void __launch_bounds__(256) digit_matrix_kernel(const DigitRing *ring
         }
         const int m = (int)(q / steps) * kDigitRows + row, j0 = (int)(q % steps) * 16 + kg * 8;
         auto entry = [&](int i) {
-            if (!kForward) return dft_entry(r, c, part, m, 2 * (j0 + i) + (part & 1));
-            const int k = 2 * m + (part & 1);
-            const double v = dft_entry(r, c, part, j0 + i, k);
-            return k == 0 ? 2.0 * v : v;
+            if (!kForward) return dft_entry(r, c, part, m, 2 * (j0 + i) + (part & 1), true);
+            return dft_entry(r, c, part, j0 + i, 2 * m + (part & 1), false);
         };
         uint8_t *dst = A + ((kForward ? r.af_tile : r.a_tile) + tile) * digit_a_bytes<T>() + (row >> 3) * 256 + kg * 128 + (row & 7) * 16;
         if constexpr (std::is_same<T, double>::value) {
             unsigned long long U[8];
 #pragma unroll
-            for (int i = 0; i < 8; i++)
-                U[i] = (unsigned long long)__double2ll_rn(entry(i) * 0x1p53) + kDigitBias;
+            for (int i = 0; i < 8; i++) U[i] = kDigitBias + (unsigned long long)entry(i);
             uint4 w[6];
             planes8<true>(U, w);
 #pragma unroll
             for (int i = 0; i < 6; i++) *reinterpret_cast<uint4 *>(dst + i * kDigitPlane) = w[i];
         } else {
-            // the digits of the binary64 entry itself, not of its binary32 rounding
+            // 28-bit fixed point, rounded from the 53 bits: a leading digit and two of base 1024
             uint32_t w[3][4];
 #pragma unroll
             for (int q2 = 0; q2 < 4; q2++) {
                 float d[3][2];
 #pragma unroll
                 for (int p = 0; p < 2; p++) {
-                    double v = entry(2 * q2 + p) * 256.0;
-                    for (int i = 0; i < 3; i++) {
-                        const double d0 = rint(v);
-                        d[i][p] = (float)d0;
-                        v = (v - d0) * 1024.0;
-                    }
+                    const int X = (int)((entry(2 * q2 + p) + (1 << 24)) >> 25);
+                    const int d2 = ((X + 512) & 1023) - 512, X1 = (X - d2) >> 10;
+                    const int d1 = ((X1 + 512) & 1023) - 512;
+                    d[2][p] = (float)d2;
+                    d[1][p] = (float)d1;
+                    d[0][p] = (float)((X1 - d1) >> 10);
                 }
 #pragma unroll
                 for (int i = 0; i < 3; i++) {
@@ -679,6 +682,13 @@ __global__ void __launch_bounds__(128) digit_turn_kernel(double *Fp, const Digit
 // of 3 items already run ring_inverse 4.2× (6 cells), 11.7× (37) and 3.3× (200 cells)
 // faster than the FFT kernels, so the line lies at one.
 constexpr int kDigitMinItems = 1;
+// Binary32 (RLZ, the four derivatives), inverse rings + columns, FFT ÷ digits.  Items:
+// 8 0.97 (100 cells), 0.88 (200), 0.83 (340); 16 1.02, 1.11, 1.05; 24 1.18, 1.24, 1.19.
+// Points: the FFT kernels hold small grids on the chip at once, 60 cells 0.94 (2.9 million),
+// 1.02 (5.3), 1.15 (11); 80 cells 1.01 (5.1); 100 cells 1.16 (4.0).  Rings: below 60 cells
+// the matrices' tiles are mostly padding, 37 cells 1.00 (81 items), 0.88 (172), 20 cells 0.75.
+constexpr int kDigitMinItemsF32 = 16, kDigitMinRingsF32 = 180;
+constexpr int64_t kDigitMinPointsF32 = 3500000;
 // bound of a grid's matrix digits (both directions: 4.3 GB at 200 cells, growing with
 // the cube of the ring count); larger grids keep the FFT kernels
 constexpr size_t kDigitTableBytes = (size_t)16 << 30;
@@ -756,9 +766,10 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
     const int ncol = (g->nitems + kDigitGroup - 1) / kDigitGroup * kDigitGroup * F::kVars;
     D.col_tiles = (ncol + 2 * F::kCols - 1) / (2 * F::kCols);
     D.col_tiles_fwd = (g->nitems + 2 * F::kCols - 1) / (2 * F::kCols);
-    const size_t abytes = (size_t)atiles * digit_a_bytes<T>(), afbytes = (size_t)aftiles * digit_a_bytes<T>();
+    constexpr bool kBoth = std::is_same<T, double>::value;  // binary32 grids keep the forward FFT's rounding
+    const size_t abytes = (size_t)atiles * digit_a_bytes<T>(), afbytes = kBoth ? (size_t)aftiles * digit_a_bytes<T>() : 0;
     if (abytes + afbytes > (g->rlz ? kDigitTableBytes : kDigitTableBytesRl)) return SS_OK;
-    double *cosq = nullptr;
+    long long *cosq = nullptr;
     const size_t mark = g->allocs.size();
     auto give_up = [&]() {  // the device has no room for the tables: the FFT kernels serve
         cudaGetLastError();
@@ -820,17 +831,19 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
     }
     if (!upload(g, &dd, cap)) return give_up();
     D.cap = const_cast<int *>(dd);
-    if (!make_set(0, nr, false, D.whole) || !make_set(0, nr, true, D.whole_fwd)) return give_up();
+    if (!make_set(0, nr, false, D.whole) || (kBoth && !make_set(0, nr, true, D.whole_fwd))) return give_up();
     D.chunks.resize(g->chunk_r0.size() - 1);
     D.chunks_fwd.resize(g->chunk_r0.size() - 1);
     for (size_t c = 0; c + 1 < g->chunk_r0.size(); c++)
         if (!make_set(g->chunk_r0[c], g->chunk_r0[c + 1], false, D.chunks[c]) ||
-            !make_set(g->chunk_r0[c], g->chunk_r0[c + 1], true, D.chunks_fwd[c]))
+            (kBoth && !make_set(g->chunk_r0[c], g->chunk_r0[c + 1], true, D.chunks_fwd[c])))
             return give_up();
     void *p = nullptr;
-    if (cudaMalloc(&p, afbytes) != cudaSuccess) return give_up();
-    g->allocs.push_back(p);
-    D.Af = p;
+    if (kBoth) {
+        if (cudaMalloc(&p, afbytes) != cudaSuccess) return give_up();
+        g->allocs.push_back(p);
+        D.Af = p;
+    }
     if (cudaMalloc(&p, abytes) != cudaSuccess) return give_up();
     g->allocs.push_back(p);
     D.A = p;
@@ -840,6 +853,17 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
     if (cudaMalloc(&p, (size_t)kDigitVariants * g->nitems * nr * sizeof(int)) != cudaSuccess) return give_up();
     g->allocs.push_back(p);
     D.expo = (int *)p;
+    if (g->tl == TL_F32 && cheb_inverse_takes_quads((int)g->d.kDim, (int)g->d.b_kDim)) {
+        std::vector<int2> blocks;
+        D.quads.first.assign(1, 0);
+        for (int r = 0; r < nr; r++) {
+            for (int m = 0; m < rings[r].n; m += 16) blocks.push_back(make_int2(r, m));
+            D.quads.first.push_back((int)blocks.size());
+        }
+        const int2 *qb = nullptr;
+        if (!upload(g, &qb, blocks)) return give_up();
+        D.quads.blocks = const_cast<int2 *>(qb);
+    }
     if (!g->rlz) {  // quadrant parts (RLZ grids keep them in the ring outputs' buffer)
         if (cudaMalloc(&p, (size_t)kDigitVariants * g->nitems * g->d.jDim * sizeof(T)) != cudaSuccess) return give_up();
         g->allocs.push_back(p);
@@ -850,24 +874,27 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
     *D.err = 0;
     digit_cos_kernel<<<nr, 128, 0, g->stream>>>(D.rings, cosq);
     digit_matrix_kernel<T, false><<<dim3(nr, 8), 256, 0, g->stream>>>(D.rings, cosq, (uint8_t *)D.A);
-    digit_matrix_kernel<T, true><<<dim3(nr, 8), 256, 0, g->stream>>>(D.rings, cosq, (uint8_t *)D.Af);
+    if constexpr (kBoth) digit_matrix_kernel<T, true><<<dim3(nr, 8), 256, 0, g->stream>>>(D.rings, cosq, (uint8_t *)D.Af);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
     cudaFree(cosq);
     cosq = nullptr;
     CUDA_TRY(e);
     CUDA_TRY(cudaFuncSetAttribute(digit_gemm_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digit_smem<T>()));
-    CUDA_TRY(cudaFuncSetAttribute(digit_gemm_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digit_smem<T>()));
+    if constexpr (kBoth)
+        CUDA_TRY(cudaFuncSetAttribute(digit_gemm_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digit_smem<T>()));
     D.on = true;
     return SS_OK;
 }
 
 int32_t digit_build(ss_grid *g, const std::vector<RingDesc> &rings) {
-    if (g->tl != TL_F64) return SS_OK;
-    int least = kDigitMinItems;
+    if (g->tl == TL_DF64 || (g->tl == TL_F32 && !g->rlz)) return SS_OK;
+    int least = g->tl == TL_F64 ? kDigitMinItems : kDigitMinItemsF32;
     if (const char *e = std::getenv("SS_RING_DIGITS")) {  // tuning override: the least item count, 0 for never
         least = std::atoi(e);
         if (least <= 0) return SS_OK;
+    } else if (g->tl == TL_F32 && (g->d.iDim < kDigitMinRingsF32 || g->d.jDim * g->nitems < kDigitMinPointsF32)) {
+        return SS_OK;
     }
     if (g->nitems < least) return SS_OK;
     // binary64 sums of a ring stay below 2^63 for n ≤ 1023 (64-bit fixed point at 2^-52 of the column scale)
@@ -894,7 +921,7 @@ static int32_t inverse(ss_grid *g, cudaStream_t st, const DigitSet &set, int *la
         digit_gemm_kernel<T, false><<<std::min(g->sms, sp.items), kDigitThreads, digit_smem<T>(), st>>>(A);
         *launches += 2;
         CUDA_TRY(cudaGetLastError());
-        if (D.columns.on) continue;  // digit_columns_inverse reads the parts
+        if (D.columns.on || D.quads.blocks) continue;  // the column stage reads the parts
         const size_t row = (size_t)4 * (sp.r1 + g->pOL + 1) * sizeof(T);
         digit_unfold_kernel<T><<<dim3(DigitFormat<T>::kVars * g->nitems, nr), 128, row, st>>>(
             D.H ? D.H : g->H, g->rlz ? nullptr : (T *)g->phys, D.rings, D.expo, sp.r0, g->nitems, (int)d.nvars,

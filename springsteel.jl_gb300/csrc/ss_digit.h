@@ -111,6 +111,13 @@ struct DigitColumns {
     int *fexpo = nullptr;
 };
 
+// Binary32 column stage: 16-position blocks of the quadrants (ring, first position) and
+// the first block of every ring
+struct QuadBlocks {
+    int2 *blocks = nullptr;
+    std::vector<int> first;
+};
+
 struct DigitPlan {
     bool on = false;
     int col_tiles = 0, col_tiles_fwd = 0;
@@ -126,6 +133,7 @@ struct DigitPlan {
     DigitSet whole, whole_fwd;
     std::vector<DigitSet> chunks, chunks_fwd;
     DigitColumns columns;
+    QuadBlocks quads;       // binary32: the column stage reads the parts
 };
 
 // Builds the plan of an RLZ grid (tables included); a grid the rule leaves to

@@ -789,6 +789,13 @@ __device__ __forceinline__ void store_run(P *dst, const P (&u)[TJ], bool vec) {
 // TC columns, consecutive threads on consecutive z, so each u[j] run and its
 // mirror u[N−1−j] leave registers as 16-byte stores covering whole sectors.
 // Summation order per output is that of cheb_inverse_m_kernel (bit-identical).
+//
+// kQuads (binary32, with the ring derivatives by digit products): the four derivative
+// outputs read the quadrant parts as digit_gemm left them.  A block is 16 quadrant
+// positions; their parts arrive by 4-byte copies as 4 × 16 columns, are turned into the 64
+// reflected ring points in shared memory, and every column is stored at its own point.
+// Measured on the 400-cell, 64-level, 4-variable grid, inverse rings + columns: FFT rings
+// 40.3 ms, digits with the parts unfolded in memory 33.4, read here 31.8.
 // ====================================================================
 // Columns per block of the persistent Chebyshev inverse.  (Measured on the
 // 400-cell binary32 grid: tiles whose parity halves sit on lane pairs joined by
@@ -797,7 +804,7 @@ __device__ __forceinline__ void store_run(P *dst, const P (&u)[TJ], bool vec) {
 template <typename T>
 __host__ __device__ constexpr int cheb_inv_cols() { return 64; }
 
-template <typename P, typename T>
+template <typename P, typename T, bool kQuads>
 __global__ void __launch_bounds__(128) cheb_inverse_p_kernel(ChebLaunch C) {
     // binary64 columns are short (kz = 32: JT = 4): 2-column tiles keep all 128
     // threads busy; binary32 (kz = 64: JT = 8) takes 4-column tiles
@@ -806,28 +813,54 @@ __global__ void __launch_bounds__(128) cheb_inverse_p_kernel(ChebLaunch C) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int64_t col_base[COLS / VEC];
     __shared__ int col_L[COLS / VEC];
+    __shared__ int64_t quad_base[2];       // kQuads: first row of the block's ring, by block parity
+    __shared__ int quad_off[2][4], quad_m[2], quad_L[2], quad_col[2][COLS];
     const int v = blockIdx.y;
     const ChebDev &cb = C.cheb[v];
     const int N = cb.N, bk = cb.bk, half = cb.half;
     const int JT = (half + TJ - 1) / TJ, JP = JT * TJ;  // JP = pad4(half), the host layout
     const int nr = cb.nrank, ke = (bk + 1) / 2, ko = bk / 2, Ke = ke + nr, Ko = ko + nr;
     const int kcap = cb.kcap;
-    T *ms = reinterpret_cast<T *>(smem_raw);    // [d][pe][kcap][JP]
-    T *xbuf = ms + (size_t)6 * kcap * JP;       // 2 × [(Ke + Ko) × COLS]: even rows, then odd rows
+    constexpr int ND = kQuads ? 2 : 6;
+    T *ms = reinterpret_cast<T *>(smem_raw);    // [d][pe][kcap][JP] (kQuads: d = 0)
+    T *xbuf = ms + (size_t)ND * kcap * JP;      // 2 × [(Ke + Ko) × COLS]: even rows, then odd rows
     const int XS = (Ke + Ko) * COLS;
-    const int64_t nblk = (C.col1 - C.col0 + COLS - 1) / COLS;
-    const int64_t nitem = ((nblk - blockIdx.x + gridDim.x - 1) / gridDim.x) * 5;  // this CTA's items
+    const int64_t nblk = kQuads ? C.nquads : (C.col1 - C.col0 + COLS - 1) / COLS;
+    const int nout = kQuads ? 4 : C.nout, var0 = kQuads ? 1 : 0;                     // ring outputs
+    const int64_t nitem = ((nblk - blockIdx.x + gridDim.x - 1) / gridDim.x) * nout;  // this CTA's items
     if (blockIdx.x >= nblk) return;
     constexpr int VP = 16 / (int)sizeof(P);
     const bool vec_ok = (N % VP) == 0 && (C.np % VP) == 0;
     {
-        const int nm = 6 * kcap * JP;  // kcap·JP is a multiple of 4 entries: 16-byte rows
+        const int nm = ND * kcap * JP;  // kcap·JP is a multiple of 4 entries: 16-byte rows
         const T *src = (const T *)cb.inv_m_t;
         for (int e = threadIdx.x * VEC; e < nm; e += blockDim.x * VEC) cp_async<16>(ms + e, src + e);
     }
     // column metadata of a block (one entry per VEC-column group: a group never
     // straddles a ring, whose starts and lengths are multiples of 4)
     auto meta = [&](int64_t blk) {
+        if constexpr (kQuads) {
+            const int2 q = C.quads[blk];
+            const DigitRing &r = C.drings[q.x];
+            const int par = (int)((blk - blockIdx.x) / gridDim.x & 1);
+            const int n = r.n, hf = r.half;
+            if (threadIdx.x == 0) {
+                quad_base[par] = (int64_t)C.bk * r.jofs;
+                quad_m[par] = q.y;
+                quad_L[par] = r.L;
+            }
+            if (threadIdx.x < 4) quad_off[par][threadIdx.x] = r.off[threadIdx.x] - r.lo[threadIdx.x];
+            for (int c = threadIdx.x; c < COLS; c += blockDim.x) {  // column = point·16 + position → ring point
+                const int m = q.y + c % 16, pt = c / 16;
+                const bool edge = hf == 0 && m == 0;
+                int p = pt == 0 ? m : (pt == 1 ? (edge ? 3 * n : 4 * n - hf - m) : (pt == 2 ? 2 * n - hf - m : (edge ? n : 2 * n + m)));
+                int l = p - r.shift;
+                if (l < 0) l += r.L;
+                if (l >= r.L) l -= r.L;
+                quad_col[par][c] = m < n ? (int)(r.jofs + l) : -1;
+            }
+            return;
+        }
         const int64_t c0 = C.col0 + blk * COLS;
         for (int g = threadIdx.x; g < COLS / VEC; g += blockDim.x) {
             const int64_t q = c0 + (int64_t)g * VEC;
@@ -839,6 +872,21 @@ __global__ void __launch_bounds__(128) cheb_inverse_p_kernel(ChebLaunch C) {
         }
     };
     auto gather = [&](int64_t blk, int var, T *xb) {
+        if constexpr (kQuads) {
+            const int par = (int)((blk - blockIdx.x) / gridDim.x & 1);
+            const int m0 = quad_m[par], L = quad_L[par], n = L / 4, hf = n & 1;
+            const T *h = (const T *)C.in + ((size_t)var * C.nvars + v) * C.bk * C.jDim + quad_base[par];
+            for (int e = threadIdx.x; e < bk * COLS; e += blockDim.x) {
+                const int zb = e / COLS, c = e % COLS, part = c / 16, m = m0 + c % 16;
+                T *dst = xb + ((zb & 1) ? (size_t)(Ke + (zb >> 1)) * COLS : (size_t)(zb >> 1) * COLS) + c;
+                // the axis position holds Ce, Co at 0 and Ce, So at π/2
+                int o = quad_off[par][part] + m;
+                if (hf == 0 && m == 0 && part >= 2) o = part == 2 ? n : 4 * n - 1;
+                if (m < n) cp_async<sizeof(T)>(dst, h + (int64_t)zb * L + o);
+                else *dst = T(0.0f);
+            }
+            return;
+        }
         const int64_t c0 = C.col0 + blk * COLS;
         const int ng = (int)(((C.col1 - c0) < COLS ? (C.col1 - c0) : COLS) / VEC);
         const T *H = (const T *)C.in + ((size_t)var * C.nvars + v) * C.bk * C.jDim;
@@ -855,15 +903,31 @@ __global__ void __launch_bounds__(128) cheb_inverse_p_kernel(ChebLaunch C) {
     };
     meta(blockIdx.x);
     __syncthreads();
-    gather(blockIdx.x, 0, xbuf);
+    gather(blockIdx.x, var0, xbuf);
     asm volatile("cp.async.commit_group;" ::: "memory");
     for (int64_t it = 0; it < nitem; it++) {
-        const int64_t blk = blockIdx.x + (it / 5) * gridDim.x;
-        const int var = (int)(it % 5);
+        const int64_t blk = blockIdx.x + (it / nout) * gridDim.x;
+        const int var = var0 + (int)(it % nout);
         T *xb = xbuf + (size_t)(it & 1) * XS;
         T *xe = xb, *xo = xb + (size_t)Ke * COLS;
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();  // item it's inputs (and, at first, the matrices) are in; item it−1 is done
+        if constexpr (kQuads) {  // parts → ring points, in place
+            const int par = (int)(it / nout & 1);
+            const bool even = (quad_L[par] / 4 & 1) == 0;
+            for (int e = threadIdx.x; e < bk * 16; e += blockDim.x) {
+                const int zb = e / 16, mm = e % 16;
+                T *x = xb + ((zb & 1) ? (size_t)(Ke + (zb >> 1)) * COLS : (size_t)(zb >> 1) * COLS) + mm;
+                const T a = x[0], b = x[16], c = x[32], d = x[48];
+                const T u = a + b, w = c + d, s = a - b, z = c - d;
+                const bool edge = even && quad_m[par] + mm == 0;
+                x[0] = edge ? u : u + w;
+                x[16] = edge ? z : u - w;
+                x[32] = edge ? s : s - z;
+                x[48] = edge ? w : s + z;
+            }
+            __syncthreads();
+        }
         // s_p = Σ_i gu[p][i] b_i (the rank term of the Γ fold), appended to both input sets
         for (int t = threadIdx.x; t < COLS * nr; t += blockDim.x) {
             const int c = t % COLS, p = t / COLS;
@@ -878,14 +942,14 @@ __global__ void __launch_bounds__(128) cheb_inverse_p_kernel(ChebLaunch C) {
             xo[(size_t)(ko + p) * COLS + c] = acc;
         }
         const bool more = it + 1 < nitem;
-        const int64_t nblk_next = blockIdx.x + ((it + 1) / 5) * gridDim.x;
+        const int64_t nblk_next = blockIdx.x + ((it + 1) / nout) * gridDim.x;
         if (more && nblk_next != blk) meta(nblk_next);
         __syncthreads();  // rank rows and the next block's metadata are visible
-        if (more) gather(nblk_next, (int)((it + 1) % 5), xbuf + (size_t)((it + 1) & 1) * XS);
+        if (more) gather(nblk_next, var0 + (int)((it + 1) % nout), xbuf + (size_t)((it + 1) & 1) * XS);
         asm volatile("cp.async.commit_group;" ::: "memory");
 
         const int64_t c0 = C.col0 + blk * COLS;
-        const int ncol = (int)((C.col1 - c0) < COLS ? (C.col1 - c0) : COLS);
+        const int ncol = kQuads ? COLS : (int)((C.col1 - c0) < COLS ? (C.col1 - c0) : COLS);
         const int nd = (var == 0) ? 3 : 1;
         for (int dd = 0; dd < nd; dd++) {
             const T *me = ms + (size_t)(2 * dd) * kcap * JP, *mo = me + (size_t)kcap * JP;
@@ -894,7 +958,8 @@ __global__ void __launch_bounds__(128) cheb_inverse_p_kernel(ChebLaunch C) {
             int slot;
             if (var == 0) slot = (dd == 0) ? 1 : (dd == 1 ? 6 : 7);
             else slot = (var == 1) ? 4 : (var == 2 ? 5 : (var == 3 ? 2 : 3));
-            P *dst = (P *)C.out + ((size_t)(slot - 1) * C.nvars + v) * C.np + c0 * N;
+            P *dst = (P *)C.out + ((size_t)(slot - 1) * C.nvars + v) * C.np + (kQuads ? 0 : c0 * N);
+            const int qpar = (int)(it / nout & 1);
             for (int t = threadIdx.x; t < JT * CT; t += blockDim.x) {
                 const int jt = t % JT, ct = t / JT;
                 const int j0 = jt * TJ, cc = ct * TC;
@@ -927,7 +992,8 @@ __global__ void __launch_bounds__(128) cheb_inverse_p_kernel(ChebLaunch C) {
 #pragma unroll
                 for (int c = 0; c < TC; c++) {
                     if (cc + c >= ncol) break;
-                    P *u = dst + (size_t)(cc + c) * N;
+                    if (kQuads && quad_col[qpar][cc + c] < 0) continue;
+                    P *u = dst + (size_t)(kQuads ? quad_col[qpar][cc + c] : cc + c) * N;
                     if (full) {
                         P lo[TJ], hi[TJ];
 #pragma unroll
@@ -954,10 +1020,10 @@ __global__ void __launch_bounds__(128) cheb_inverse_p_kernel(ChebLaunch C) {
 }
 
 template <typename T>
-size_t cheb_inverse_p_smem(int N, int bk) {  // rank of the Γ fold ≤ 2
+size_t cheb_inverse_p_smem(int N, int bk, bool quads = false) {  // rank of the Γ fold ≤ 2
     const size_t kcap = (size_t)(bk + 1) / 2 + 2, jp = (size_t)cheb_pad4((N + 1) / 2);
     const size_t kk = (size_t)(bk + 1) / 2 + bk / 2 + 4;
-    return (6 * kcap * jp + 2 * kk * cheb_inv_cols<T>()) * sizeof(T);
+    return ((quads ? 2 : 6) * kcap * jp + 2 * kk * cheb_inv_cols<T>()) * sizeof(T);
 }
 
 template <typename T>
@@ -1116,17 +1182,27 @@ cudaError_t launch_cheb_forward(const ChebLaunch &C, size_t smem, cudaStream_t s
 }
 // the register-tiled kernel; `smem` (the 64-column kernel's size) is unused.
 // N and bk are the grid's (every variable shares them).
+bool cheb_inverse_takes_quads(int N, int bk) { return cheb_inverse_p_smem<float>(N, bk) <= (size_t)227 * 1024; }
+
 template <typename P, typename T>
 cudaError_t launch_cheb_inverse(const ChebLaunch &C, size_t smem, cudaStream_t st, int N) {
     (void)smem;
     if (C.col1 <= C.col0) return cudaSuccess;
     const size_t sp = cheb_inverse_p_smem<T>(N, C.bk);
     if (sp <= (size_t)227 * 1024) {  // the three matrices stay resident: persistent CTAs
-        set_smem(cheb_inverse_p_kernel<P, T>, sp);
+        set_smem(cheb_inverse_p_kernel<P, T, false>, sp);
         constexpr int cols = cheb_inv_cols<T>();
+        if constexpr (std::is_same<T, float>::value) {
+            if (C.quads) {
+                const size_t sq = cheb_inverse_p_smem<T>(N, C.bk, true);
+                set_smem(cheb_inverse_p_kernel<P, T, true>, sq);
+                const int64_t want = std::max<int64_t>(1, (int64_t)resident_ctas(sq, 128) / std::max(C.nvars, 1));
+                cheb_inverse_p_kernel<P, T, true><<<dim3((unsigned)std::min<int64_t>(C.nquads, want), C.nvars), 128, sq, st>>>(C);
+            }
+        }
         const int64_t nblk = (C.col1 - C.col0 + cols - 1) / cols;
         const int64_t want = std::max<int64_t>(1, (int64_t)resident_ctas(sp, 128) / std::max(C.nvars, 1));
-        cheb_inverse_p_kernel<P, T><<<dim3((unsigned)std::min(nblk, want), C.nvars), 128, sp, st>>>(C);
+        cheb_inverse_p_kernel<P, T, false><<<dim3((unsigned)std::min(nblk, want), C.nvars), 128, sp, st>>>(C);
         return cudaGetLastError();
     }
     // long columns: one matrix at a time, one CTA per (block, variable, variant)

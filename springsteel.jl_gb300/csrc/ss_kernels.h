@@ -8,6 +8,7 @@
 
 #include "ss_internal.h"
 #include "ss_df64.cuh"
+#include "ss_digit.h"
 
 namespace ss {
 
@@ -104,6 +105,12 @@ struct ChebLaunch {
     int64_t jDim, np;
     int64_t col0, col1;        // columns (ring points) [col0, col1) of this launch
     int iDim, bk, nvars;
+    // cheb_inverse: `nout` ring outputs from the first; 1: f alone (with ∂z, ∂zz), 5: all; with
+    // `quads` set the other four, from their quadrant parts (ss_digit.h), in blocks of 16 positions
+    int nout;
+    const int2 *quads;
+    int nquads;
+    const DigitRing *drings;
 };
 
 // RL chain coupling (update_interface!, src/multipatch.jl:417-478)
@@ -184,6 +191,7 @@ template <typename P>
 cudaError_t launch_sa_si_f32_fused(const SaLaunch *recs, const BatchWork *work, int nwork, cudaStream_t st);
 template <typename P, typename T>
 cudaError_t launch_cheb_forward(const ChebLaunch &C, size_t smem, cudaStream_t st, int N);
+bool cheb_inverse_takes_quads(int N, int bk);  // columns of this length go to the kernel that reads `quads`
 template <typename P, typename T>
 cudaError_t launch_cheb_inverse(const ChebLaunch &C, size_t smem, cudaStream_t st, int N);
 

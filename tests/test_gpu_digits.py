@@ -104,6 +104,42 @@ def test_forward_columns_match_oracle(cells, levels, nvars):
     _assert_parity(sg, so, pg, po, gp, tol=TOL64)
 
 
+# binary32: the four derivatives by digit products, f and the forward transform by the FFT kernels.  Small
+# grids are sent there by the override: quadrants around the blocks of 16 positions (n = 2.., 43 cells:
+# n up to 130), levels not a multiple of 4, item counts around the groups of 8; 60 cells by the rule
+@pytest.mark.parametrize("cells,levels,nvars,kmax,least", [
+    (1, 5, 1, -1, "1"), (5, 13, 1, -1, "1"), (6, 33, 3, -1, "1"), (43, 16, 1, -1, "1"), (14, 16, 1, 31, "1"),
+    (9, 16, 2, 0, "1"), (60, 44, 2, -1, None)])
+def test_binary32_derivatives_by_digits(monkeypatch, cells, levels, nvars, kmax, least):
+    gp = _gp(cells, levels, nvars, max_wavenumber={"default": kmax}, precision="f32")
+    u = _field(gp)
+    if least:
+        monkeypatch.setenv("SS_RING_DIGITS", least)
+    spec, phys = _round_trip(gp, u)
+    monkeypatch.setenv("SS_RING_DIGITS", "0")
+    spec0, phys0 = _round_trip(gp, u)
+    assert np.array_equal(spec, spec0)
+    for s in (0, 5, 6):
+        assert np.array_equal(phys[:, :, s], phys0[:, :, s])
+    for v in range(nvars):
+        for s in (1, 2, 3, 4):
+            # products: 28-bit digits; FFT: 24 bits through up to log2(4n) ≤ 10 stages
+            assert np.max(np.abs(phys[:, v, s] - phys0[:, v, s])) <= 1e-5 * np.max(np.abs(phys0[:, v, s]))
+
+
+def test_binary32_digits_keep_non_finite_rings(monkeypatch):
+    gp = _gp(6, 12, 2, precision="f32")
+    u = _field(gp)
+    u[:, 1] = 0.0
+    u[50, 0] = np.inf
+    monkeypatch.setenv("SS_RING_DIGITS", "1")
+    _, got = _round_trip(gp, u)
+    monkeypatch.setenv("SS_RING_DIGITS", "0")
+    _, want = _round_trip(gp, u)
+    assert np.array_equal(np.isfinite(got), np.isfinite(want))
+    assert np.all(got[:, 1, :] == 0.0)
+
+
 # ring launches: buckets joined or not, an item or an output per CTA or several items, by the number
 # of (ring, item) pairs.  Each gives the same bits, so a variable's result does not depend on its company
 @pytest.mark.parametrize("geometry,precision,cells,levels", [
