@@ -114,6 +114,7 @@ static void free_grid(ss_grid *g) {
     for (cudaEvent_t e : g->chunk_ev) cudaEventDestroy(e);
     digit_free(g);
     for (void *p : g->allocs) cudaFree(p);
+    if (g->reg_block) cudaFree(g->reg_block);
     if (g->copy_stream) cudaStreamDestroy(g->copy_stream);
     if (g->stream) cudaStreamDestroy(g->stream);
     delete g;

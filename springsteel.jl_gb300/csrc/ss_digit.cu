@@ -35,7 +35,8 @@
 // digit_gemm    persistent, warp-specialised: bulk copies → 8-slot (6-slot) ring
 //               of K-steps → two issuing warps, one per accumulator half → two
 //               warpgroups drain and combine
-// digit_unfold  quadrant parts → ring points (RL; RLZ columns read the parts)
+// digit_unfold  quadrant parts → ring points (RL, and columns too long for the kernels that
+//               read the parts)
 #include <cuda_runtime.h>
 
 #include <algorithm>

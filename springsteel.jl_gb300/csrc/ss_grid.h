@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -79,6 +80,10 @@ struct ss_grid {
     std::vector<Mark> marks;
     int64_t launches[SS_NSTAGES] = {0, 0, 0, 0, 0, 0};
     double stage_ms[SS_NSTAGES] = {0, 0, 0, 0, 0, 0};
+    // kept device block of regularGridTransform (taken out while a call uses it)
+    std::mutex reg_mutex;
+    void *reg_block = nullptr;
+    size_t reg_bytes = 0;
 };
 
 static cudaEvent_t next_event(ss_grid *g) {

@@ -106,10 +106,11 @@ def test_forward_columns_match_oracle(cells, levels, nvars):
 
 # binary32: the four derivatives by digit products, f and the forward transform by the FFT kernels.  Small
 # grids are sent there by the override: quadrants around the blocks of 16 positions (n = 2.., 43 cells:
-# n up to 130), levels not a multiple of 4, item counts around the groups of 8; 60 cells by the rule
+# n up to 130), levels not a multiple of 4, item counts around the groups of 8, columns too long for the kernel
+# that reads quadrant parts (210 levels); 60 cells by the rule
 @pytest.mark.parametrize("cells,levels,nvars,kmax,least", [
     (1, 5, 1, -1, "1"), (5, 13, 1, -1, "1"), (6, 33, 3, -1, "1"), (43, 16, 1, -1, "1"), (14, 16, 1, 31, "1"),
-    (9, 16, 2, 0, "1"), (60, 44, 2, -1, None)])
+    (9, 16, 2, 0, "1"), (3, 210, 1, -1, "1"), (60, 44, 2, -1, None)])
 def test_binary32_derivatives_by_digits(monkeypatch, cells, levels, nvars, kmax, least):
     gp = _gp(cells, levels, nvars, max_wavenumber={"default": kmax}, precision="f32")
     u = _field(gp)

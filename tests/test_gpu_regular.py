@@ -77,3 +77,30 @@ def test_rlz_regular_grid_matches_oracle():
     print("RLZ regular errors (end levels)", ends)
     assert np.all(ends[:, :6] <= TOL64), ends
     assert np.all(ends[:, 6] <= 1e-5), ends
+
+
+def test_calls_of_several_threads_and_sizes_agree():
+    """The kept buffers are taken out by each call: two threads on one grid, larger and smaller point sets."""
+    import threading
+    gp = S.SpringsteelGridParameters(geometry="RL", iMin=0.0, iMax=20.0, num_cells=10, vars={"u": 1})
+    g = S.createGrid(gp)
+    pts = S.getGridpoints(g)
+    g.set_physical(fields.blob_sum(pts, seed=3, nblobs=4, wmin=2, wmax=6)[:, None], slot=1)
+    S.spectralTransform_b(g)
+    g.synchronize()
+    sets = [(np.linspace(0, 20, n), np.linspace(0, 6, m)) for n, m in ((3, 5), (40, 90), (7, 200), (60, 10))]
+    want = [S.regularGridTransform(g, *s) for s in sets]
+    bad = []
+
+    def work(k):
+        for i in range(40):
+            j = (i + k) % 4
+            if not np.array_equal(S.regularGridTransform(g, *sets[j]), want[j]):
+                bad.append((k, i))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
