@@ -85,37 +85,122 @@ __global__ void reg_si_kernel(const double *coef, const int *m0, const double *w
     }
 }
 
+// ---- cos(kλ), sin(kλ) tables
+// π/2 in parts of 33, 33 and 53 bits
+constexpr double kPio2a = 0x1.921fb54400000p+0, kPio2b = 0x1.0b4611a600000p-34, kPio2c = 0x1.3198a2e037073p-69;
+// cos and sin of a, |a| < 2^20: a − n·π/2 in two words (n times the first two parts is
+// exact), then the Taylor series with the leading terms in two words.  Against 64-bit
+// significands: 0.59 units of the last place at most and 0.288 rms over 4 million k·λ with
+// k ≤ 10^5, as the host library's 0.288 (cos and sin of the CUDA library: 0.36).
+__device__ __forceinline__ void cos_sin_accurate(double a, double &c, double &s) {
+    const double n = rint(a * 0.63661977236758134);
+    const double t = fma(-n, kPio2a, a);
+    const double m = n * kPio2b;
+    double h = t - m, v = t - h;
+    double l = fma(-n, kPio2c, (t - (h + v)) + (v - m));
+    const double h1 = h + l;  // renormalised
+    l = l - (h1 - h);
+    h = h1;
+    const double z = h * h, zl = fma(h, h, -z) + 2.0 * (h * l);
+    // sin: h − h³/6 + h⁵/120 − …
+    const double w = h * z, wl = fma(h, z, -w) + fma(h, zl, l * z);
+    const double k3 = 1.0 / 6.0, k3l = fma(-k3, 6.0, 1.0) / 6.0;
+    const double g = w * k3, gl = fma(w, k3, -g) + fma(w, k3l, wl * k3);
+    double p = -1.0 / 121645100408832000.0;
+    p = fma(p, z, 1.0 / 355687428096000.0);
+    p = fma(p, z, -1.0 / 1307674368000.0);
+    p = fma(p, z, 1.0 / 6227020800.0);
+    p = fma(p, z, -1.0 / 39916800.0);
+    p = fma(p, z, 1.0 / 362880.0);
+    p = fma(p, z, -1.0 / 5040.0);
+    p = fma(p, z, 1.0 / 120.0);
+    const double u = h - g;
+    const double sn = u + (((h - u) - g) + (fma(w * z, p, l - gl)));
+    // cos: 1 − h²/2 + h⁴/24 − …
+    double q = -1.0 / 6402373705728000.0;
+    q = fma(q, z, 1.0 / 20922789888000.0);
+    q = fma(q, z, -1.0 / 87178291200.0);
+    q = fma(q, z, 1.0 / 479001600.0);
+    q = fma(q, z, -1.0 / 3628800.0);
+    q = fma(q, z, 1.0 / 40320.0);
+    q = fma(q, z, -1.0 / 720.0);
+    q = fma(q, z, 1.0 / 24.0);
+    const double y = 1.0 - 0.5 * z;
+    const double cn = y + (((1.0 - y) - 0.5 * z) + fma(z * z, q, -0.5 * zl));
+    const int k = (int)n & 3;
+    const double cc = (k & 1) ? sn : cn, ss = (k & 1) ? cn : sn;
+    c = (k == 1 || k == 2) ? -cc : cc;
+    s = k >= 2 ? -ss : ss;
+}
+constexpr double kRegMaxAngle = 1e6;  // bound of kλ for the tables above
+// tc, ts[(k−1)·n_λ + j] of the rounded products kλ_j, as on the host: K = 180 × 361 points
+// took 1.2 ms there, two thirds of the time before the first launch
+__global__ void __launch_bounds__(128) reg_table_kernel(const double *lam, double *tc, double *ts, int K, int n_lam) {
+    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (e >= (int64_t)K * n_lam) return;
+    cos_sin_accurate((double)(e / n_lam + 1) * lam[e % n_lam], tc[e], ts[e]);
+}
+
 // The Fourier series at λ_j for one (item, r) per CTA row, j over threads:
 //   f = a0 + Σ_k 2 (rc cos kλ + rs sin kλ), the same with the SIx / SIxx
 //   coefficients for ∂r f / ∂rr f, ∂λ f = Σ_k 2k (−rc sin + rs cos),
 //   ∂λλ f = −Σ_k 2k² (rc cos + rs sin)   (src/transforms_cylindrical.jl:985-1005)
-// cos/sin(kλ_j) come from host tables tc/ts[(k−1)·n_λ + j].  RL writes the result
+// cos/sin(kλ_j) come from the tables tc/ts[(k−1)·n_λ + j].  RL writes the result
 // slots straight into out (rows r·n_λ + j); RLZ writes fb[variant][v][r][j][zb].
+// Bound by binary64 operations (two multiply-adds a clock and SM): the factors 2, 2k
+// and 2k² go into the coefficients as they are staged, once per CTA, which leaves ten
+// multiply-adds per (k, λ) where the sums above take sixteen operations and an integer
+// conversion.  Cosine and sine terms are summed apart: one rounding of each sum per k, as
+// many as the paired sum has (in one sum the error grows 1.4 times), and each chunk apart
+// (error of sums of 20 to 720 random terms: 0.4 of the paired sum's).  61 × 361 columns
+// of 32 modes, K = 180: 4.16 → 2.25 ms (the operations alone 2.2 ms).  A chunk is kRegChunk
+// wavenumbers, 5 KB of staged coefficients.
+constexpr int kRegChunk = 64;
 __global__ void __launch_bounds__(128) reg_fourier_kernel(const double *sr, const double *tc, const double *ts,
                                                           double *dst, int nslots_z, int K, int n_r, int n_lam,
                                                           int nitems, int rlz, int bk, int nvars) {
-    extern __shared__ __align__(16) double c[];  // [d][slot]
+    // per k: f, ∂r, ∂rr, ∂λ, ∂λλ as (factor of cos, factor of sin)
+    __shared__ __align__(16) double2 c[kRegChunk][5];
     const int r = blockIdx.y, item = blockIdx.z;
-    for (int e = threadIdx.x; e < 3 * nslots_z; e += blockDim.x) {
-        const int d = e / nslots_z, s = e - d * nslots_z;
-        c[e] = sr[(((size_t)d * nitems + item) * n_r + r) * nslots_z + s];
+    const size_t ds = (size_t)nitems * n_r * nslots_z;
+    const double *c0 = sr + ((size_t)item * n_r + r) * nslots_z, *c1 = c0 + ds, *c2 = c1 + ds;
+    const int j = blockIdx.x * blockDim.x + threadIdx.x, jj = min(j, n_lam - 1);
+    double vals[5] = {c0[0], c1[0], c2[0], 0.0, 0.0};  // variants: f, ∂r, ∂rr, ∂λ, ∂λλ
+    for (int k0 = 1; k0 <= K; k0 += kRegChunk) {
+        const int nk = min(kRegChunk, K + 1 - k0);
+        __syncthreads();
+        for (int q = threadIdx.x; q < nk; q += blockDim.x) {
+            const int k = k0 + q;
+            const double kk = 2.0 * (double)k, k2 = -(kk * (double)k);
+            const double rc = c0[2 * k - 1], rs = c0[2 * k];
+            c[q][0] = make_double2(2.0 * rc, 2.0 * rs);
+            c[q][1] = make_double2(2.0 * c1[2 * k - 1], 2.0 * c1[2 * k]);
+            c[q][2] = make_double2(2.0 * c2[2 * k - 1], 2.0 * c2[2 * k]);
+            c[q][3] = make_double2(kk * rs, -kk * rc);
+            c[q][4] = make_double2(k2 * rc, k2 * rs);
+        }
+        __syncthreads();
+        const double *pc = tc + (size_t)(k0 - 1) * n_lam + jj, *ps = ts + (size_t)(k0 - 1) * n_lam + jj;
+        if (j < n_lam) {
+            double u[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, w[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // cos and sin sums
+            for (int q = 0; q < nk; q++, pc += n_lam, ps += n_lam) {
+                const double ck = *pc, sk = *ps;
+                u[0] = fma(c[q][0].x, ck, u[0]);
+                w[0] = fma(c[q][0].y, sk, w[0]);
+                u[1] = fma(c[q][1].x, ck, u[1]);
+                w[1] = fma(c[q][1].y, sk, w[1]);
+                u[2] = fma(c[q][2].x, ck, u[2]);
+                w[2] = fma(c[q][2].y, sk, w[2]);
+                u[3] = fma(c[q][3].x, ck, u[3]);
+                w[3] = fma(c[q][3].y, sk, w[3]);
+                u[4] = fma(c[q][4].x, ck, u[4]);
+                w[4] = fma(c[q][4].y, sk, w[4]);
+            }
+#pragma unroll
+            for (int q = 0; q < 5; q++) vals[q] += u[q] + w[q];
+        }
     }
-    __syncthreads();
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n_lam) return;
-    const double *c1 = c + nslots_z, *c2 = c + 2 * nslots_z;
-    double f = c[0], fr = c1[0], frr = c2[0], fl = 0.0, fll = 0.0;
-    for (int k = 1; k <= K; k++) {
-        const double ck = tc[(size_t)(k - 1) * n_lam + j], sk = ts[(size_t)(k - 1) * n_lam + j];
-        const double rc = c[2 * k - 1], rs = c[2 * k];
-        const double kk = (double)k;
-        f += 2.0 * (rc * ck + rs * sk);
-        fr += 2.0 * (c1[2 * k - 1] * ck + c1[2 * k] * sk);
-        frr += 2.0 * (c2[2 * k - 1] * ck + c2[2 * k] * sk);
-        fl += 2.0 * kk * (-rc * sk + rs * ck);
-        fll -= 2.0 * (kk * kk) * (rc * ck + rs * sk);
-    }
-    const double vals[5] = {f, fr, frr, fl, fll};  // variants: f, ∂r, ∂rr, ∂λ, ∂λλ
     if (!rlz) {
         const size_t nrows = (size_t)n_r * n_lam, row = (size_t)r * n_lam + j;
 #pragma unroll
@@ -326,8 +411,10 @@ int32_t regular(ss_grid *g, const double *r_pts, int n_r, const double *lam_pts,
     std::vector<int> m0;
     std::vector<double> w;
     spline_point_weights(g->spl_host[0], r_pts, n_r, m0, w);  // every variable shares the radial knots
-    std::vector<double> tc(size_t(K) * n_lam), ts(size_t(K) * n_lam);
-    for (int k = 1; k <= K; k++)
+    bool dev_tables = true;  // large, infinite and NaN points: the host's tables
+    for (int j = 0; j < n_lam; j++) dev_tables &= std::fabs(lam_pts[j]) * K < kRegMaxAngle;
+    std::vector<double> tc(dev_tables ? 0 : size_t(K) * n_lam), ts(tc.size());
+    for (int k = 1; k <= K && !dev_tables; k++)
         for (int j = 0; j < n_lam; j++) {
             const double a = (double)k * lam_pts[j];
             tc[size_t(k - 1) * n_lam + j] = std::cos(a);
@@ -363,7 +450,7 @@ int32_t regular(ss_grid *g, const double *r_pts, int n_r, const double *lam_pts,
     }
     // device buffers: one block, kept by the grid for its next call
     const size_t out_elems = nrows * nv * d.nslots;
-    const size_t need[9] = {size_t(nitems) * ns * b * 8, w.size() * 8, m0.size() * 4, tc.size() * 8, ts.size() * 8,
+    const size_t need[9] = {size_t(nitems) * ns * b * 8, w.size() * 8, m0.size() * 4, (size_t(K) + 1) * n_lam * 8, size_t(K) * n_lam * 8,
                             size_t(3) * nitems * n_r * ns * 8, out_elems * 8,
                             g->rlz ? size_t(5) * nv * n_r * n_lam * bk * 8 : 0, mats.size() * 8};
     size_t off[10] = {0};
@@ -381,8 +468,16 @@ int32_t regular(ss_grid *g, const double *r_pts, int n_r, const double *lam_pts,
     auto run = [&]() -> int32_t {
         CUDA_TRY(cudaMemcpyAsync(d_w, w.data(), w.size() * 8, cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemcpyAsync(d_m0, m0.data(), m0.size() * 4, cudaMemcpyHostToDevice, st));
-        CUDA_TRY(cudaMemcpyAsync(d_tc, tc.data(), tc.size() * 8, cudaMemcpyHostToDevice, st));
-        CUDA_TRY(cudaMemcpyAsync(d_ts, ts.data(), ts.size() * 8, cudaMemcpyHostToDevice, st));
+        if (dev_tables) {
+            double *d_lam = d_tc + size_t(K) * n_lam;
+            CUDA_TRY(cudaMemcpyAsync(d_lam, lam_pts, size_t(n_lam) * 8, cudaMemcpyHostToDevice, st));
+            const int64_t ne = int64_t(K) * n_lam;
+            if (ne > 0) reg_table_kernel<<<(unsigned)((ne + 127) / 128), 128, 0, st>>>(d_lam, d_tc, d_ts, K, n_lam);
+            CUDA_TRY(cudaGetLastError());
+        } else {
+            CUDA_TRY(cudaMemcpyAsync(d_tc, tc.data(), tc.size() * 8, cudaMemcpyHostToDevice, st));
+            CUDA_TRY(cudaMemcpyAsync(d_ts, ts.data(), ts.size() * 8, cudaMemcpyHostToDevice, st));
+        }
         if (g->rlz) CUDA_TRY(cudaMemcpyAsync(d_mats, mats.data(), mats.size() * 8, cudaMemcpyHostToDevice, st));
         // SAtransform! of every slot
         int nmax = 0;
@@ -409,8 +504,7 @@ int32_t regular(ss_grid *g, const double *r_pts, int n_r, const double *lam_pts,
             set_error("regularGridTransform: %d wavenumber slots exceed shared memory", ns);
             return SS_BAD_SHAPE;
         }
-        CUDA_TRY(cudaFuncSetAttribute(reg_fourier_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm));
-        reg_fourier_kernel<<<dim3((n_lam + 127) / 128, n_r, nitems), 128, fsm, st>>>(
+        reg_fourier_kernel<<<dim3((n_lam + 127) / 128, n_r, nitems), 128, 0, st>>>(
             d_sr, d_tc, d_ts, g->rlz ? d_fb : d_out, ns, K, n_r, n_lam, nitems, g->rlz, bk, nv);
         CUDA_TRY(cudaGetLastError());
         if (g->rlz) {

@@ -79,6 +79,23 @@ def test_rlz_regular_grid_matches_oracle():
     assert np.all(ends[:, 6] <= 1e-5), ends
 
 
+# wavenumbers around the chunks of 64 (K = 3, 63, 66, 129), point counts around the 128 of a CTA, negative
+# angles, and angles beyond the device tables' range (the host's tables)
+@pytest.mark.parametrize("cells,n_lam,lo,hi", [(1, 1, 0.0, 0.0), (21, 127, -7.0, 7.0), (22, 129, 0.0, 6.2), (43, 128, 0.1, 6.3),
+                                               (21, 130, 1e5, 1e5 + 6.0)])
+def test_fourier_points_match_oracle(cells, n_lam, lo, hi):
+    gp = S.SpringsteelGridParameters(geometry="RL", iMin=0.0, iMax=float(cells), num_cells=cells, vars={"u": 1, "w": 2})
+    g = S.createGrid(gp)
+    pts = S.getGridpoints(g)
+    g.set_physical(np.column_stack([fields.blob_sum(pts, seed=50 + v, nblobs=4, wmin=1.0 + cells / 10, wmax=2.0 + cells / 5)
+                                    for v in range(2)]), slot=1)
+    S.spectralTransform_b(g)
+    r, lam = np.linspace(0.0, float(cells), 5), np.linspace(lo, hi, n_lam)
+    got = S.regularGridTransform(g, r, lam)
+    ref = O.regular_grid_transform(gp.to_abi(), g.get_spectral(), r, lam)
+    assert np.all(_slot_err(got, ref, gp) <= TOL64)
+
+
 def test_calls_of_several_threads_and_sizes_agree():
     """The kept buffers are taken out by each call: two threads on one grid, larger and smaller point sets."""
     import threading
