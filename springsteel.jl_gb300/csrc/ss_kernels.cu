@@ -809,6 +809,7 @@ __global__ void __launch_bounds__(128) cheb_inverse_p_kernel(ChebLaunch C) {
     // binary64 columns are short (kz = 32: JT = 4): 2-column tiles keep all 128
     // threads busy; binary32 (kz = 64: JT = 8) takes 4-column tiles
     constexpr int COLS = cheb_inv_cols<T>(), TJ = 4, TC = std::is_same<T, float>::value ? 4 : 2, CT = COLS / TC;
+    static_assert(!kQuads || (COLS == 64 && TC == 4), "128 threads: two rows of columns, eight of positions");
     constexpr int VEC = 16 / (int)sizeof(T);  // compute-type values per 16-byte copy
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int64_t col_base[COLS / VEC];
@@ -876,13 +877,15 @@ __global__ void __launch_bounds__(128) cheb_inverse_p_kernel(ChebLaunch C) {
             const int par = (int)((blk - blockIdx.x) / gridDim.x & 1);
             const int m0 = quad_m[par], L = quad_L[par], n = L / 4, hf = n & 1;
             const T *h = (const T *)C.in + ((size_t)var * C.nvars + v) * C.bk * C.jDim + quad_base[par];
-            for (int e = threadIdx.x; e < bk * COLS; e += blockDim.x) {
-                const int zb = e / COLS, c = e % COLS, part = c / 16, m = m0 + c % 16;
-                T *dst = xb + ((zb & 1) ? (size_t)(Ke + (zb >> 1)) * COLS : (size_t)(zb >> 1) * COLS) + c;
-                // the axis position holds Ce, Co at 0 and Ce, So at π/2
-                int o = quad_off[par][part] + m;
-                if (hf == 0 && m == 0 && part >= 2) o = part == 2 ? n : 4 * n - 1;
-                if (m < n) cp_async<sizeof(T)>(dst, h + (int64_t)zb * L + o);
+            // a thread keeps its column and its rows' parity: addresses advance by constants
+            const int c = threadIdx.x % COLS, z0 = threadIdx.x / COLS, part = c / 16, m = m0 + c % 16;
+            // the axis position holds Ce, Co at 0 and Ce, So at π/2
+            int o = quad_off[par][part] + m;
+            if (hf == 0 && m == 0 && part >= 2) o = part == 2 ? n : 4 * n - 1;
+            const T *src = h + (int64_t)z0 * L + o;
+            T *dst = xb + (z0 ? (size_t)Ke * COLS : 0) + c;
+            for (int zb = z0; zb < bk; zb += 2, src += 2 * L, dst += COLS) {
+                if (m < n) cp_async<sizeof(T)>(dst, src);
                 else *dst = T(0.0f);
             }
             return;
@@ -915,12 +918,12 @@ __global__ void __launch_bounds__(128) cheb_inverse_p_kernel(ChebLaunch C) {
         if constexpr (kQuads) {  // parts → ring points, in place
             const int par = (int)(it / nout & 1);
             const bool even = (quad_L[par] / 4 & 1) == 0;
-            for (int e = threadIdx.x; e < bk * 16; e += blockDim.x) {
-                const int zb = e / 16, mm = e % 16;
-                T *x = xb + ((zb & 1) ? (size_t)(Ke + (zb >> 1)) * COLS : (size_t)(zb >> 1) * COLS) + mm;
+            const int mm = threadIdx.x % 16, z0 = threadIdx.x / 16;
+            const bool edge = even && quad_m[par] + mm == 0;
+            T *x = xb + ((z0 & 1) ? (size_t)(Ke + (z0 >> 1)) * COLS : (size_t)(z0 >> 1) * COLS) + mm;
+            for (int zb = z0; zb < bk; zb += 8, x += 4 * COLS) {
                 const T a = x[0], b = x[16], c = x[32], d = x[48];
                 const T u = a + b, w = c + d, s = a - b, z = c - d;
-                const bool edge = even && quad_m[par] + mm == 0;
                 x[0] = edge ? u : u + w;
                 x[16] = edge ? z : u - w;
                 x[32] = edge ? s : s - z;
