@@ -890,7 +890,7 @@ static int32_t copy_out(ss_grid *g, void *host, const void *src, int32_t dtype, 
         CUDA_TRY(cudaMemcpyAsync(host, g->stage, n * hes, cudaMemcpyDeviceToHost, s));
     }
     CUDA_TRY(cudaStreamSynchronize(s));
-    return SS_OK;
+    return digit_status(g);
 }
 
 #define CHECK_GRID(g)                                         \
@@ -1061,7 +1061,7 @@ int32_t ss_grid_transform_to_host(ss_grid *g, void *host_all, int32_t dtype, voi
     if (rc) return rc;
     CUDA_TRY(cudaStreamSynchronize(g->copy_stream));
     CUDA_TRY(cudaGetLastError());
-    return SS_OK;
+    return digit_status(g);
 }
 
 int32_t ss_grid_set_filter(ss_grid *g, int32_t var, const double *fw, const double *cw) {
@@ -1140,12 +1140,7 @@ int32_t ss_grid_synchronize(ss_grid *g) {
     CHECK_GRID(g);
     CUDA_TRY(cudaStreamSynchronize(g->stream));
     CUDA_TRY(cudaGetLastError());
-    if (g->digit.err && *(volatile int *)g->digit.err) {
-        *g->digit.err = 0;
-        set_error("ring product: a bounded device wait gave up");
-        return SS_DEVICE_TIMEOUT;
-    }
-    return SS_OK;
+    return digit_status(g);
 }
 
 }  // extern "C"

@@ -480,7 +480,10 @@ extern "C" int32_t ss_batch_synchronize(ss_batch *bt) {
     if (!bt) { set_error("null batch"); return SS_BAD_ARG; }
     cudaSetDevice(bt->device);
     CUDA_TRY(cudaStreamSynchronize(bt->stream));
-    return SS_OK;
+    int32_t rc = SS_OK;
+    for (ss_grid *g : bt->grids)
+        if (const int32_t r = digit_status(g)) rc = r;
+    return rc;
 }
 
 extern "C" int32_t ss_batch_fused_launches(const ss_batch *bt, int32_t what, int32_t *launches) {

@@ -908,6 +908,14 @@ void digit_free(ss_grid *g) {
     g->digit.err = nullptr;
 }
 
+int32_t digit_status(ss_grid *g) {
+    volatile int *err = g->digit.err;
+    if (!err || !*err) return SS_OK;
+    *err = 0;
+    set_error("ring product: a bounded device wait gave up");
+    return SS_DEVICE_TIMEOUT;
+}
+
 template <typename T>
 static int32_t inverse(ss_grid *g, cudaStream_t st, const DigitSet &set, int *launches) {
     const DigitPlan &D = g->digit;

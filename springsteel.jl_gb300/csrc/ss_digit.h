@@ -144,6 +144,8 @@ int32_t digit_ring_inverse(ss_grid *g, cudaStream_t st, int chunk, int *launches
 // ring_forward likewise: C → F
 int32_t digit_ring_forward(ss_grid *g, cudaStream_t st, int chunk, int *launches);
 void digit_free(ss_grid *g);
+// after a synchronisation: SS_DEVICE_TIMEOUT once if a bounded wait of the products gave up
+int32_t digit_status(ss_grid *g);
 int32_t digit_columns_build(ss_grid *g, const std::vector<ChebHost> &cheb);
 // cheb_forward of the columns [col0, col1): physical slot 1 → C
 int32_t digit_columns_forward(ss_grid *g, cudaStream_t st, int64_t col0, int64_t col1);
