@@ -496,21 +496,21 @@ def _oracle_roundtrip(gp, slot1, threads, var_index=None):
 # one ncu capture (1-pass metrics, --clock-control none) of the full-size bench
 # workload itself: `bench.py --workload W --steps 1 --warmup 3 --no-cpu-baseline
 # --no-secondary` under `ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,
-# dram__bytes_write.sum -k regex:"ring_|cheb_|sa_si|sb_project"`, one warm-up
+# dram__bytes_write.sum -k regex:"ring_|cheb_|sa_|sb_project|digit_"`, one warm-up
 # round trip's launches.  Bytes per round trip.
 MEASURED_TRAFFIC = {
-    ("rlz200-f64", "cheb_forward"): 1.539e9,
-    ("rlz200-f64", "ring_forward"): 0.863e9,
+    ("rlz200-f64", "cheb_forward"): 1.529e9,
+    ("rlz200-f64", "ring_forward"): 6.776e9,
     ("rlz200-f64", "sb_project"): 0.493e9,
-    ("rlz200-f64", "sa_si"): 1.106e9,
-    ("rlz200-f64", "ring_inverse"): 3.903e9,
-    ("rlz200-f64", "cheb_inverse"): 9.642e9,
-    ("rlz400-f32", "cheb_forward"): 9.910e9,
+    ("rlz200-f64", "sa_si"): 1.115e9,
+    ("rlz200-f64", "ring_inverse"): 11.716e9,
+    ("rlz200-f64", "cheb_inverse"): 9.706e9,
+    ("rlz400-f32", "cheb_forward"): 9.907e9,
     ("rlz400-f32", "ring_forward"): 6.068e9,
-    ("rlz400-f32", "sb_project"): 3.279e9,
-    ("rlz400-f32", "sa_si"): 24.037e9,
-    ("rlz400-f32", "ring_inverse"): 26.665e9,
-    ("rlz400-f32", "cheb_inverse"): 64.088e9,
+    ("rlz400-f32", "sb_project"): 3.280e9,
+    ("rlz400-f32", "sa_si"): 7.244e9,
+    ("rlz400-f32", "ring_inverse"): 62.355e9,
+    ("rlz400-f32", "cheb_inverse"): 76.584e9,
 }
 
 
