@@ -513,17 +513,22 @@ __device__ __forceinline__ void load_row(const T *p, T (&v)[K]) {
 }
 
 // ====================================================================
-// cheb_forward, register-tiled: the CTA's 64 columns are staged (cp.async),
-// folded into xe[j][c] = x_j + x_{N-1-j} and xo[j][c] = x_j − x_{N-1-j}
-// (j < half; the middle point once), then out[k][c] = Σ_j FW[k][j] x{e,o}[j][c]
+// cheb_forward, register-tiled: the CTA's 64 columns are folded straight from
+// global memory into xe[j][c] = x_j + x_{N-1-j} and xo[j][c] = x_j − x_{N-1-j}
+// (j < half; the middle point once; column c of row j at c ^ 4(j mod 8), so that a
+// warp's 8 points × 4 columns and its column quads are free of bank conflicts), then out[k][c] = Σ_j FW[k][j] x{e,o}[j][c]
 // as two small GEMMs (even and odd k) with 4 × 4 register tiles; the same
 // per-output summation order (j ascending) as cheb_forward.  Results are staged
 // k-major and stored per ring row (C[r][zb][l]) with consecutive columns
-// contiguous.
+// contiguous.  Bound by instruction issue and shared-memory accesses: a staged copy
+// of the columns (4-byte cp.async, then a strided read to fold it) cost both and a CTA
+// of residency.  400 cells, 64 levels, 8 variables, binary32: staged 5.08 ms, folded
+// from global memory 4.48 ms (2.2 TB/s).
 // ====================================================================
 template <typename P, typename T>
 __global__ void __launch_bounds__(128) cheb_forward_tiled_kernel(ChebLaunch C) {
-    constexpr int COLS = 64, TK = 4, TC = 4, CT = COLS / TC;
+    constexpr int COLS = 64, TK = 4, TC = 4, CT = COLS / TC, NT = 128;
+    constexpr int FOLD = sizeof(T) == 4 ? 8 : 4;  // point pairs a thread loads at a time
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int64_t col_base[COLS];
     __shared__ int col_L[COLS];
@@ -532,13 +537,11 @@ __global__ void __launch_bounds__(128) cheb_forward_tiled_kernel(ChebLaunch C) {
     const int N = cb.N, bk = cb.bk, half = cb.half;
     const int ke = (bk + 1) / 2, ko = bk / 2;
     const int KEP = (ke + TK - 1) / TK * TK, KOP = (ko > 0 ? (ko + TK - 1) / TK : 1) * TK;
-    const int ldx = N | 1;
     T *xe = reinterpret_cast<T *>(smem_raw);      // half × COLS
     T *xo = xe + (size_t)half * COLS;              // half × COLS
     T *fe = xo + (size_t)half * COLS;              // half × KEP: FW[2i][j] at fe[j][i]
     T *fo = fe + (size_t)half * KEP;               // half × KOP: FW[2i+1][j] at fo[j][i]
-    T *xs = fo + (size_t)half * KOP;               // COLS × ldx staged columns; later bk × COLS outputs
-    T *os = xs;
+    T *os = fo + (size_t)half * KOP;               // bk × COLS outputs
     // tables once per CTA (host-transposed: coalesced)
     for (int e = threadIdx.x; e < half * KEP; e += blockDim.x) fe[e] = ld_real<T>(cb.fwd_et_t, e);
     for (int e = threadIdx.x; e < half * KOP; e += blockDim.x) fo[e] = ld_real<T>(cb.fwd_ot_t, e);
@@ -547,12 +550,6 @@ __global__ void __launch_bounds__(128) cheb_forward_tiled_kernel(ChebLaunch C) {
     const int64_t c0 = C.col0 + blk * COLS;
     const int ncol = (int)((C.col1 - c0) < COLS ? (C.col1 - c0) : COLS);
     const P *in = (const P *)C.in + (size_t)v * C.np + c0 * N;
-    // (point z, column c) walked with carries: no division per element
-    if constexpr (std::is_same<P, T>::value) {
-        for (UnitWalk u(N); u.g < ncol; u.next()) cp_async<sizeof(T)>(xs + u.g * ldx + u.n, in + u.g * N + u.n);
-    } else {
-        for (UnitWalk u(N); u.g < ncol; u.next()) xs[u.g * ldx + u.n] = to_compute<T>(in[u.g * N + u.n]);
-    }
     for (int c = threadIdx.x; c < COLS; c += blockDim.x) {
         if (c < ncol) {
             const int64_t q = c0 + c;
@@ -561,19 +558,27 @@ __global__ void __launch_bounds__(128) cheb_forward_tiled_kernel(ChebLaunch C) {
             col_L[c] = rd.L;
         }
     }
-    if constexpr (std::is_same<P, T>::value) cp_async_wait_all();
-    __syncthreads();
-    for (int e = threadIdx.x; e < half * COLS; e += blockDim.x) {
-        const int j = e / COLS, c = e % COLS;
-        T a = T(0.0f), b = T(0.0f);
-        if (c < ncol) {
-            const T *x = xs + c * ldx;
-            const int jj = N - 1 - j;
-            if (jj == j) { a = x[j]; b = x[j]; }
-            else { a = x[j] + x[jj]; b = x[j] - x[jj]; }
+    // a warp folds 8 points of 4 columns: whole 32-byte sectors in, distinct banks out
+    const int units = (half + 7) / 8 * 8 * COLS;
+    for (int e0 = threadIdx.x; e0 < units; e0 += NT * FOLD) {
+        P lo[FOLD], hi[FOLD];
+#pragma unroll
+        for (int q = 0; q < FOLD; q++) {
+            const int e = e0 + q * NT, j = e / (8 * COLS) * 8 + (e & 7), c = (e >> 3) % COLS;
+            const bool live = j < half && c < ncol;
+            lo[q] = live ? __ldg(in + (size_t)c * N + j) : P(0);
+            hi[q] = live ? __ldg(in + (size_t)c * N + N - 1 - j) : P(0);
         }
-        xe[e] = a;
-        xo[e] = b;
+#pragma unroll
+        for (int q = 0; q < FOLD; q++) {
+            const int e = e0 + q * NT, j = e / (8 * COLS) * 8 + (e & 7), c = (e >> 3) % COLS;
+            if (j >= half) continue;
+            const T a = to_compute<T>(lo[q]), b = to_compute<T>(hi[q]);
+            const bool middle = 2 * j == N - 1;
+            const int at = j * COLS + (c ^ ((j & 7) * TC));
+            xe[at] = middle ? a : a + b;
+            xo[at] = middle ? a : a - b;
+        }
     }
     __syncthreads();
     const int KT = KEP / TK + KOP / TK;
@@ -589,16 +594,16 @@ __global__ void __launch_bounds__(128) cheb_forward_tiled_kernel(ChebLaunch C) {
         for (int i = 0; i < TK; i++)
 #pragma unroll
             for (int c = 0; c < TC; c++) acc[i][c] = T(0.0f);
+#pragma unroll 8
         for (int j = 0; j < half; j++) {
             T w[TK], x[TC];
             load_row<T, TK>(ft + (size_t)j * KP + i0, w);
-            load_row<T, TC>(xt + (size_t)j * COLS + cc, x);
+            load_row<T, TC>(xt + (size_t)j * COLS + (cc ^ ((j & 7) * TC)), x);
 #pragma unroll
             for (int i = 0; i < TK; i++)
 #pragma unroll
                 for (int c = 0; c < TC; c++) acc[i][c] = acc[i][c] + w[i] * x[c];
         }
-        // os aliases xs, which only the fold pass (before the last barrier) read
 #pragma unroll
         for (int i = 0; i < TK; i++) {
             const int k = 2 * (i0 + i) + (odd ? 1 : 0);
@@ -621,8 +626,7 @@ template <typename T>
 size_t cheb_forward_tiled_smem(int N, int bk) {
     const int half = (N + 1) / 2, ke = (bk + 1) / 2, ko = bk / 2;
     const int KEP = (ke + 3) / 4 * 4, KOP = (ko > 0 ? (ko + 3) / 4 : 1) * 4;
-    const size_t stage = std::max((size_t)64 * (N | 1), (size_t)bk * 64);
-    return ((size_t)2 * half * 64 + (size_t)half * (KEP + KOP) + stage) * sizeof(T);
+    return ((size_t)2 * half * 64 + (size_t)half * (KEP + KOP) + (size_t)bk * 64) * sizeof(T);
 }
 
 // ====================================================================
