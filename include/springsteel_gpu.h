@@ -385,6 +385,11 @@ int32_t ss_spectral_transform_noalloc(const ss_grid *grid, const double *d_physi
 int32_t ss_grid_profile(ss_grid *grid, int32_t enable);
 int32_t ss_grid_profile_read(ss_grid *grid, double *ms, int64_t *launches);
 
+/* Stages of this grid that run as digit-slice products on the tensor cores (a set of
+ * SS_DIGITS_* bits; binary32 grids: the derivative outputs of the inverse rings). */
+enum { SS_DIGITS_RING_FWD = 1, SS_DIGITS_RING_INV = 2, SS_DIGITS_CHEB_FWD = 4, SS_DIGITS_CHEB_INV = 8 };
+int32_t ss_grid_digits(const ss_grid *grid, int32_t *stages);
+
 /* ---- FFT plan inspection (host only: no GPU needed) ----------------------
  * The plan grid creation builds for the complex DFT of length n (n = L/2 of a
  * ring of L = 4 + 4 ri points) in `precision`, with the same limits and tuning

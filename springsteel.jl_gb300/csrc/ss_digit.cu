@@ -216,7 +216,9 @@ __global__ void __launch_bounds__(256, 2) digit_split_kernel(SplitArgs S) {
             const int e = mag_expo<T>(__reduce_max_sync(0xffffffffu, mx[q]));
             if (lane == 0) {
                 ex[warp][q] = e;
-                if (item < S.nitems) S.expo[((size_t)q * S.nitems + item) * S.iDim + ring] = e;
+                // of the parts: one higher where the products store them halved
+                const int up = std::is_same<T, double>::value && r.n > kDigitFullRing && e != kNanColumn ? 1 : 0;
+                if (item < S.nitems) S.expo[((size_t)q * S.nitems + item) * S.iDim + ring] = e + up;
             }
         }
     }
@@ -490,6 +492,12 @@ __global__ void __launch_bounds__(kDigitThreads, 1) digit_gemm_kernel(GemmDigitA
                                 V[h * WC + c0 + c] += fmaf(fmaf(D[2][c], 0x1p-10f, D[1][c]), 0x1p-10f, D[0][c]);
                         }
                     }
+                }
+            }
+            if constexpr (!kForward && std::is_same<T, double>::value) {
+                if (r->n > kDigitFullRing) {  // headroom for the four parts' sum
+#pragma unroll
+                    for (int c = 0; c < 2 * WC; c++) V[c] = (Acc)(((long long)V[c] + 1) >> 1);
                 }
             }
             Acc *out = (Acc *)g.out;
@@ -898,8 +906,7 @@ int32_t digit_build(ss_grid *g, const std::vector<RingDesc> &rings) {
         return SS_OK;
     }
     if (g->nitems < least) return SS_OK;
-    // binary64 sums of a ring stay below 2^63 for n ≤ 1023 (64-bit fixed point at 2^-52 of the column scale)
-    if (rings[g->d.iDim - 1].ri + 1 > (g->tl == TL_F64 ? 1023 : 2047)) return SS_OK;
+    if (rings[g->d.iDim - 1].ri + 1 > (g->tl == TL_F64 ? kDigitMaxRing : kDigitMaxRingF32)) return SS_OK;
     return g->tl == TL_F64 ? build<double>(g, rings) : build<float>(g, rings);
 }
 
@@ -967,3 +974,11 @@ int32_t digit_ring_inverse(ss_grid *g, cudaStream_t st, int chunk, int *launches
 }
 
 }  // namespace ss
+
+extern "C" int32_t ss_grid_digits(const ss_grid *g, int32_t *stages) {
+    if (!g || !stages) { set_error("null argument"); return SS_BAD_ARG; }
+    const DigitPlan &D = g->digit;
+    *stages = !D.on ? 0 : (g->tl == TL_F64 ? SS_DIGITS_RING_FWD : 0) | SS_DIGITS_RING_INV |
+                              (D.columns.fon ? SS_DIGITS_CHEB_FWD : 0) | (D.columns.on ? SS_DIGITS_CHEB_INV : 0);
+    return SS_OK;
+}

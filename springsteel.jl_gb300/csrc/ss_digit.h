@@ -50,6 +50,15 @@ SS_HD constexpr int digit_b_bytes() { return 2 * digit_half_bytes<T>(); }
 constexpr int kDigitVariants = 5;   // f, ∂λ, ∂λλ, ∂r, ∂rr; a format's columns are the last kVars
 constexpr int kDigitGroup = 8;      // items whose columns are interleaved
 constexpr int kNanColumn = 0x7fffffff;  // column exponent of a column that holds an infinity or NaN
+// Headroom of the binary64 inverse sums.  A term of a ring point is below 2^53 (2^54 of
+// data × 2^53 of matrix, over 2^54) in its cosine and its sine part, so a point of a ring
+// of n = ri + 1 is below √2·n·2^53 (1.27·n·2^53 is reached where all re = ± im), which
+// passes 2^63 at n = 725.  Rings above that keep their quadrant parts (each below
+// (n/2 + 1)·2^53 < 2^63) halved, at an exponent one higher: good for n ≤ 1448.  The
+// forward sums (at most n terms below 2^53 in one part) fit for n ≤ 1023.
+constexpr int kDigitFullRing = 724;
+constexpr int kDigitMaxRing = 1023;
+constexpr int kDigitMaxRingF32 = 2047;
 
 // One ring of n = ri + 1 (L = 4n points) seen by the digit kernels.  The points
 // λ_l = 2π(l + (ri − 1)/2)/L are p = (l + shift) mod L on the grid θ_p = 2π(p + half/2)/L,
