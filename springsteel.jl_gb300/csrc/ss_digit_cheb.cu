@@ -50,6 +50,9 @@ constexpr int kProducers = 8, kDrains = 16;
 constexpr int kColThreads = (kProducers + kDrains + 1) * 32;
 constexpr int kMaxModes = 96;               // six K-steps keep every digit sum an exact integer
 constexpr int kMaxZBlocks = 5;              // 160 levels
+// Shared memory a CTA may ask for: 227 KB less the static part.  Attribute of both column
+// kernels, whatever a grid needs: it is the process's, and grids of other level counts share it.
+constexpr size_t kColumnSmem = 232448 - 8192;
 constexpr int kRowExpo = 8;                 // row-exponent slots (producers run at most 4 outputs ahead)
 
 struct ColumnArgs {
@@ -568,7 +571,7 @@ static int32_t build_forward(ss_grid *g, const std::vector<ChebHost> &cheb) {
     Q.fsteps = (N + 15) / 16;
     Q.fblocks = (bk + kZ - 1) / kZ;
     Q.fgroup = N <= 32 ? 4 : (N <= 64 ? 8 : 16);
-    if (Q.fsteps > 6 || Q.fblocks > kMaxZBlocks || forward_smem(Q.fsteps, Q.fblocks) > 232448 - 8192) return SS_OK;
+    if (Q.fsteps > 6 || Q.fblocks > kMaxZBlocks || forward_smem(Q.fsteps, Q.fblocks) > kColumnSmem) return SS_OK;
     const int job = Q.fsteps * kZStep;
     std::vector<uint8_t> M((size_t)nv * Q.fblocks * job, 0);
     std::vector<int> E((size_t)nv * Q.fblocks * kZ, 0);
@@ -607,8 +610,7 @@ static int32_t build_forward(ss_grid *g, const std::vector<ChebHost> &cheb) {
     };
     if (!put(M.data(), M.size(), &pm) || !put(E.data(), E.size() * 4, &pe)) return SS_OK;
     Q.fM = pm; Q.fexpo = (int *)pe;
-    CUDA_TRY(cudaFuncSetAttribute(digit_columns_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)forward_smem(Q.fsteps, Q.fblocks)));
+    CUDA_TRY(cudaFuncSetAttribute(digit_columns_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColumnSmem));
     Q.fon = true;
     return SS_OK;
 }
@@ -620,12 +622,11 @@ static int32_t build_inverse(ss_grid *g, const std::vector<ChebHost> &cheb) {
     Q.steps = (bk + 15) / 16;
     Q.zblocks = (N + kZ - 1) / kZ;
     if (bk > kMaxModes || Q.zblocks > kMaxZBlocks) return SS_OK;
-    constexpr size_t kLimit = 232448 - 8192;  // 227 KB less the static part
     // two operand buffers and two input buffers where they fit, then fewer
     const int shapes[4][2] = {{2, 2}, {1, 2}, {2, 1}, {1, 1}};
     Q.buffers = 0;
     for (const auto &s : shapes)
-        if (!Q.buffers && column_smem(Q.steps, Q.zblocks, bk, s[0], s[1]) <= kLimit) { Q.buffers = s[0]; Q.raws = s[1]; }
+        if (!Q.buffers && column_smem(Q.steps, Q.zblocks, bk, s[0], s[1]) <= kColumnSmem) { Q.buffers = s[0]; Q.raws = s[1]; }
     if (!Q.buffers) return SS_OK;
     const int job = Q.steps * kZStep;
     std::vector<uint8_t> M((size_t)nv * 3 * Q.zblocks * job, 0);
@@ -696,7 +697,8 @@ static int32_t build_inverse(ss_grid *g, const std::vector<ChebHost> &cheb) {
     if (!put(M.data(), M.size(), &pm) || !put(E.data(), E.size() * 4, &pe) || !put(blocks.data(), blocks.size() * 8, &pb))
         return SS_OK;
     Q.M = pm; Q.mexpo = (int *)pe; Q.blocks = (int2 *)pb;
-    CUDA_TRY(cudaFuncSetAttribute(Q.steps <= 2 ? digit_columns_kernel<true> : digit_columns_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLimit));
+    CUDA_TRY(cudaFuncSetAttribute(Q.steps <= 2 ? digit_columns_kernel<true> : digit_columns_kernel<false>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColumnSmem));
     Q.on = true;
     return SS_OK;
 }

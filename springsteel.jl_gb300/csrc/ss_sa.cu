@@ -367,7 +367,8 @@ size_t sa_band_smem(int b) { return (size_t)b * kSaLd * sizeof(double); }
 template <typename T>
 cudaError_t launch_sa_band(const SaLaunch &A, int nitems, cudaStream_t st) {
     const size_t smem = sa_band_smem(A.b);
-    const cudaError_t e = cudaFuncSetAttribute(sa_band_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the process's attribute: one value for all grids, so that launches of other threads never lower it
+    const cudaError_t e = cudaFuncSetAttribute(sa_band_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSaBandSmemMax);
     if (e != cudaSuccess) return e;
     // few CTAs: every one solves its slots again for a part of the rings only, so that
     // the evaluation (12 FP64 operations per slot and ring) spreads over idle SMs
@@ -380,7 +381,7 @@ template <typename T>
 cudaError_t launch_sa_band_fused(const SaLaunch *recs, const BatchWork *work, int nwork, size_t smem, cudaStream_t st) {
     if (nwork <= 0) return cudaSuccess;
     const cudaError_t e =
-        cudaFuncSetAttribute(sa_band_fused_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(sa_band_fused_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSaBandSmemMax);
     if (e != cudaSuccess) return e;
     sa_band_fused_kernel<T><<<nwork, kSaWarps * 32, smem, st>>>(recs, work);
     return cudaGetLastError();

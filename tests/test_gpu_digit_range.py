@@ -40,3 +40,26 @@ def test_longest_rings_keep_their_sign(monkeypatch, cells):
     assert on == 0
     for s in range(7):
         assert np.max(np.abs(got[:, 0, s] - want[:, 0, s])) <= TOL64 * np.max(np.abs(want[:, 0, s]))
+
+
+@pytest.mark.parametrize("first,second", [(32, 12), (48, 20), (12, 32)])
+def test_grids_of_other_level_counts_share_the_column_kernels(first, second):
+    """Creating a grid of fewer levels leaves the shared memory of the earlier grid's kernels alone."""
+    def grid(levels):
+        return S.createGrid(S.SpringsteelGridParameters(geometry="RLZ", iMin=0.0, iMax=6.0, num_cells=6, kMin=0.0,
+                                                        kMax=10.0, kDim=levels, vars={"u": 1}))
+
+    def transform(g):
+        g.set_physical(np.random.default_rng(2).standard_normal((g.dims["n_physical"], 1)), slot=1)
+        S.spectralTransform_b(g)
+        S.gridTransform_b(g)
+        return g.get_spectral(), g.get_physical()
+
+    a = grid(first)
+    assert digit_stages(a) == 15
+    want = transform(a)
+    b = grid(second)
+    transform(b)
+    got = transform(a)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    a.close(), b.close()
