@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
     __shared__ __align__(8) uint64_t afull[2], aempty[2], accf[2], acce[2], drain;
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int quit;
+    __shared__ volatile int halt[2];  // quit as thread 0 saw it, for all producers
     __shared__ int row_expo[kRowExpo][128];
     __shared__ int mode_expo[2][kMaxModes];
     __shared__ __align__(16) int sE[3 * kZ * kMaxZBlocks];  // row exponents of the matrices, less 53
@@ -174,14 +175,13 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
                 cp_async<4>(&mode_expo[slot][i], g.expo + ((size_t)var * g.nitems + (size_t)v * g.bk + i) * g.iDim + k.ring);
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
-        bool ok = true;
         Block cur, next;
         if (nitem > 0) {
             next = load_block(0);
             fetch(next, 0, 0);
         }
         const int nr = g.raws;
-        for (int it = 0; ok && it < nitem; it++) {
+        for (int it = 0; it < nitem; it++) {
             const int var = it % kDigitVariants, slot = it % nr;
             if (var == 0) {
                 cur = next;
@@ -221,13 +221,17 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
             }
 #pragma unroll
             for (int q = 0; q < 4; q++) atomicMax(&rex[q * 32 + lane], mx[q]);
+            // the producers leave together, on one thread's word: one that gave up waiting alone would
+            // be missed at the barrier for good
+            if (threadIdx.x == 0) halt[it & 1] = quit;
             producers_sync();
+            if (halt[it & 1]) break;
             const int buf = it % nb;
-            if (!(ok = bar_wait(&aempty[buf], ((it / nb) & 1) ^ 1, &quit))) break;
+            const bool ok = bar_wait(&aempty[buf], ((it / nb) & 1) ^ 1, &quit);  // if not: quit is set
             uint8_t *A = sA + (size_t)buf * KS * 6 * kDigitPlane;
             const int row = threadIdx.x & 127;
             const int er = rex[row];
-            for (int kg = threadIdx.x >> 7; kg < (g.bk + 7) / 8; kg += kProducers / 4) {
+            for (int kg = threadIdx.x >> 7; ok && kg < (g.bk + 7) / 8; kg += kProducers / 4) {
                 unsigned long long U[8];
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
@@ -247,7 +251,7 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
                 for (int i = 0; i < 6; i++) *reinterpret_cast<uint4 *>(dst + i * kDigitPlane) = w[i];
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            bar_arrive(&afull[buf]);
+            if (ok) bar_arrive(&afull[buf]);
             producers_sync();  // these points may be overwritten
             if (more && nr == 1) {
                 if (var + 1 < kDigitVariants) fetch(cur, var + 1, 0);
@@ -463,7 +467,8 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_forward_kernel(F
                 for (int i = 0; i < 8; i++) U[i] = kDigitBias + (unsigned long long)(e == kNanColumn ? 0ll : fixed_point<54>(x[i], e));
                 uint4 w[6];
                 planes8(U, w);
-                if (r0 == 0 && !(ok = bar_wait(&aempty[buf], ((it >> 1) & 1) ^ 1, &quit))) break;
+                // a warp decides as one: its lanes exchange values in the next sweep
+                if (r0 == 0 && !(ok = __all_sync(0xffffffffu, bar_wait(&aempty[buf], ((it >> 1) & 1) ^ 1, &quit)))) break;
                 if (kg == 0) row_expo[it % kRowExpo][row] = e;
                 if (kg < 2 * KS) {
                     uint8_t *dst = A + (kg >> 1) * kAStep + (row >> 3) * 256 + (kg & 1) * 128 + (row & 7) * 16;
