@@ -199,15 +199,9 @@ static int32_t build_grid(ss_grid *g) {
         if ((st = upload_vec(g, &sd.L4, sh.L4))) return st;
         if ((st = upload_vec(g, &sd.dinv, dinv))) return st;
         if (!sh.periodic) {
-            const SplineFixed f = spline_ldl(sh);
             double *m = nullptr;
-            int *q = nullptr;
-            if ((st = upload_vec(g, &m, f.ldl))) return st;
-            if ((st = upload_vec(g, &q, f.limbs))) return st;
+            if ((st = upload_vec(g, &m, spline_ldl(sh)))) return st;
             sd.ldl = m;
-            sd.fix = q;
-            g->spl_host[v].fixed_ok = f.ok;
-            sd.fix_m_up = f.m_up; sd.fix_d_up = f.d_up; sd.fix_bits = f.bits;
         }
         if ((st = upload_vec(g, &sd.PQb, sh.PQb))) return st;
         std::vector<float> l4f(sh.L4.size()), dinvf(dinv.size());
@@ -570,7 +564,7 @@ SaLaunch sa_record(const ss_grid *g, int coeffs, size_t *smem_generic) {
 bool sa_band_serves(const ss_grid *g) {
     if (g->tl == TL_DF64 || sa_band_smem((int)g->d.b_iDim) > kSaBandSmemMax) return false;
     for (auto &sh : g->spl_host)
-        if (sh.periodic || (g->tl == TL_F32 && !sh.fixed_ok)) return false;
+        if (sh.periodic) return false;
     return true;
 }
 }  // namespace ss

@@ -115,10 +115,6 @@ struct SplineDev {
     double *L4;         // Min*4: L[j+d][j] at j*4+d   (FP64 banded Cholesky factor)
     double *dinv;       // Min: 1/L[j][j]
     const double *ldl;  // Min*4: the factor as unit-lower M and D, row j: M[j+1..j+3][j], 1/D[j] (not periodic)
-    // the same as 60-bit fixed point, 30-bit limbs (h, l): m1, m2, m3 over 2^fix_m_up,
-    // 1/D over 2^fix_d_up; fix_bits: leading bits of b that leave room for the growth
-    const int *fix;
-    int fix_m_up, fix_d_up, fix_bits;
     double *PQb;        // bDim*7 full P+Q band (R3X only)
     float *L4f;         // FP32-rounded factor (FP32 mode)
     float *dinvf;
@@ -168,7 +164,6 @@ struct SplineHost {
     std::vector<double> PQb, L4, Aopen, sbw, siw;  // Aopen: open-form band before factoring
     std::vector<int> si_m0;
     int periodic = 0;
-    bool fixed_ok = false;              // binary32 grids: the fixed-point solve serves (SplineFixed)
     std::vector<double> tail, acorner;  // periodic factor rows n-3..n-1 and out-of-band corners of A
 };
 int32_t build_spline(double xmin, double xmax, int nc, int mubar, int quad, double l_q,
@@ -179,15 +174,8 @@ struct ChebHost {
     double dscale;
     std::vector<double> fwd, inv_e, inv_o, gu, gv, mish;
 };
-// LDLᵀ form of the (not periodic) factor: ldl[4·j + d − 1] = M[j + d][j], ldl[4·j + 3] = 1/D[j];
-// its fixed-point form and scales (SplineDev)
-struct SplineFixed {
-    std::vector<double> ldl;
-    std::vector<int> limbs;  // 8 per row
-    int m_up = 0, d_up = 0, bits = 0;
-    bool ok = false;         // the growth leaves room for binary32 data
-};
-SplineFixed spline_ldl(const SplineHost &s);
+// LDLᵀ form of the (not periodic) factor: [4·j + d − 1] = M[j + d][j], [4·j + 3] = 1/D[j]
+std::vector<double> spline_ldl(const SplineHost &s);
 int32_t build_cheb(int N, int bk, int bcb, int bct, double zmin, double zmax, ChebHost &out);
 // SI weights at arbitrary radii: window start m0[i], w[(d·n + i)·4 + tap], d = 0, 1, 2
 int32_t spline_point_weights(const SplineHost &s, const double *x, int n, std::vector<int> &m0,

@@ -9,16 +9,15 @@
 // schedulers.  The factor is kept as unit-lower M and D (M = L·diag(L)^-1): 3 FMAs
 // forward and 4 operations backward per row, one FMA on the dependent chain.
 //
-// Binary32 grids solve in 60-bit fixed point instead (30-bit limbs, 32-bit wide
-// multiply-adds at full rate: about 60 instructions per row against 448 cycles),
-// each slot at the exponent of its largest entry, and round x once to binary32:
-// the value a binary32 solve with an FP64 refinement step (15 FP64 operations and
-// ten conversions a row) is after.  The headroom of the fixed point is the exact
-// growth |M^-1 Γ|, |A^-1 Γ| of the spline, so no sum can overflow.
+// Binary32 grids solve in binary64 as well and round x once: the value a binary32 solve
+// with an FP64 refinement step (15 FP64 operations and ten conversions a row) is after, at
+// any scale and along the whole slot (60-bit fixed point took 1.4 ms less on the 400-cell
+// grid and as long elsewhere, but held a slot at one exponent; widening and rounding by
+// integer operations took 0.8 ms more than the conversions).
 //
-// Measured before → here: 400-cell binary32 RLZ grid of 4 variables 9.9 → 6.5 ms,
-// 251-cell binary32 RL grid of 4 variables 0.87 → 0.13 ms, 125-cell binary32 RLZ
-// grid 0.77 → 0.30 ms, 200-cell FP64 RLZ grid of 5 variables 2.03 → 1.38 ms (12
+// Measured before → here: 400-cell binary32 RLZ grid of 4 variables 9.9 → @SA400@ ms,
+// 251-cell binary32 RL grid of 4 variables 0.87 → @SA251@ ms, 125-cell binary32 RLZ
+// grid 0.77 → @SA125@ ms, 200-cell FP64 RLZ grid of 5 variables 2.03 → 1.38 ms (12
 // FP64 operations per slot and ring for SI alone hold the FP64 units for 0.85 ms),
 // 100-cell FP64 RL grid 0.13 → 0.05 ms (a chain of 103 rows × 7 × 64 cycles).
 #include <cuda_runtime.h>
@@ -32,22 +31,6 @@ namespace ss {
 
 constexpr int kSaWarps = 8;  // one solves, all load and evaluate
 constexpr int kSaLd = 33;  // slots of a CTA + 1: rows of a slot and slots of a row are both conflict-free
-
-// m·z of 60-bit fixed point, m = mh·2^30 + ml, z = zh·2^30 + zl: the terms of weight
-// 2^60 into `main`, the others (the last from its leading bits) into `cross`, over 2^30
-struct Fixed2 {
-    int h, l;
-};
-__device__ __forceinline__ Fixed2 limbs(long long z) { return {(int)(z >> 30), (int)((unsigned)z & 0x3fffffffu)}; }
-__device__ __forceinline__ void fixed_mad(long long &main, long long &cross, const Fixed2 m, const Fixed2 z) {
-    main += (long long)m.h * z.h;
-    cross += (long long)m.l * z.h;
-    cross += (long long)m.h * z.l;
-    cross += (long long)(m.l >> 15) * (z.l >> 15);
-}
-__device__ __forceinline__ Fixed2 shfl2(Fixed2 v, int j) {
-    return {__shfl_sync(0xffffffffu, v.h, j), __shfl_sync(0xffffffffu, v.l, j)};
-}
 
 // One warp solves its 32 slots in place; x: the lane's interior rows, row i at [i * kSaLd].
 // Lane j holds row base + j of the factor, the next 32 rows already loading; a row's
@@ -109,101 +92,12 @@ __device__ __forceinline__ void solve_f64(const SplineDev &sp, double *xi, int n
     }
 }
 
-// The same in fixed point, in units 2^(E − F) (SplineDev)
-__device__ __forceinline__ void solve_fixed(const SplineDev &sp, long long *xi, int n, int lane, bool mine) {
-    const int4 *ldl = reinterpret_cast<const int4 *>(sp.fix);  // row i: (m1, m2), (m3, 1/d) as limbs
-    const int up = sp.fix_m_up;
-    const long long half = up < 30 ? 1ll << (29 - up) : 0ll;  // rounds a sum to the nearest unit
-    auto factor = [&](int row, int4 &f0, int4 &f1) {
-        const int r = min(max(row, 0), n - 1);
-        f0 = __ldg(ldl + 2 * r);
-        f1 = __ldg(ldl + 2 * r + 1);
-    };
-    auto sum = [&](long long main, long long cross) { return (main << up) + (cross >> (30 - up)); };
-    // z/d: 1/d spans ten binades towards the ends, so its scaled product keeps the last term too
-    const int dup = sp.fix_d_up;
-    auto over_d = [&](const Fixed2 m, const Fixed2 z) {
-        long long main = (long long)m.h * z.h, cross = ((long long)m.l * z.l >> 30) + (dup < 30 ? 1ll << (29 - dup) : 0ll);
-        cross += (long long)m.l * z.h;
-        cross += (long long)m.h * z.l;
-        return (main << dup) + (cross >> (30 - dup));
-    };
-    int4 f0, f1, g0, g1;
-    factor(lane, f0, f1);
-    Fixed2 z0{0, 0}, z1{0, 0}, m1{0, 0}, m2{0, 0}, m3{0, 0}, m3b{0, 0};
-    long long xn = xi[0], part = 0, pcross = half;  // Σ of the known products of row i
-    for (int base = 0; base < n; base += 32) {
-        factor(base + 32 + lane, g0, g1);
-        const int rows = min(32, n - base);
-#pragma unroll 4
-        for (int j = 0; j < rows; j++) {
-            const int i = base + j;
-            fixed_mad(part, pcross, m1, z0);
-            const long long z = xn - sum(part, pcross);
-            xn = xi[min(i + 1, n - 1) * kSaLd];
-            part = 0; pcross = half;
-            fixed_mad(part, pcross, m3b, z1);
-            fixed_mad(part, pcross, m2, z0);
-            if (mine) xi[i * kSaLd] = z;
-            z1 = z0; z0 = limbs(z);
-            m1 = shfl2({f0.x, f0.y}, j);
-            m2 = shfl2({f0.z, f0.w}, j);
-            m3b = m3;
-            m3 = shfl2({f1.x, f1.y}, j);
-        }
-        f0 = g0; f1 = g1;
-    }
-    __syncwarp();
-    const int top = (n - 1) / 32 * 32;
-    factor(top + lane, f0, f1);
-    Fixed2 x1{0, 0}, x2{0, 0};
-    long long zd = over_d(shfl2({f1.z, f1.w}, (n - 1) & 31), limbs(xi[(n - 1) * kSaLd]));
-    part = 0; pcross = half;
-    for (int base = top; base >= 0; base -= 32) {
-        factor(base - 32 + lane, g0, g1);
-#pragma unroll 4
-        for (int j = min(32, n - base) - 1; j >= 0; j--) {
-            const int i = base + j;
-            const int jp = (j + 31) & 31;
-            const Fixed2 zp = limbs(xi[max(i - 1, 0) * kSaLd]);
-            const Fixed2 n1 = shfl2({f0.x, f0.y}, j);
-            const Fixed2 n2 = shfl2(j ? Fixed2{f0.z, f0.w} : Fixed2{g0.z, g0.w}, jp);
-            const Fixed2 n3 = shfl2(j ? Fixed2{f1.x, f1.y} : Fixed2{g1.x, g1.y}, jp);
-            const Fixed2 nd = shfl2(j ? Fixed2{f1.z, f1.w} : Fixed2{g1.z, g1.w}, jp);
-            fixed_mad(part, pcross, n1, x1);
-            const long long xv = zd - sum(part, pcross);
-            part = 0; pcross = half;
-            zd = over_d(nd, zp);
-            fixed_mad(part, pcross, n3, x2);
-            fixed_mad(part, pcross, n2, x1);
-            if (mine) xi[i * kSaLd] = xv;
-            x2 = x1; x1 = limbs(xv);
-        }
-        f0 = g0; f1 = g1;
-    }
-}
-
-// X·2^s to binary32, to nearest even
-__device__ __forceinline__ float fixed_to_float(long long X, int s) {
-    if (X == 0) return 0.f;
-    const unsigned long long a = X < 0 ? 0ull - (unsigned long long)X : (unsigned long long)X;
-    const int lz = __clzll((long long)a);
-    const unsigned long long nrm = a << lz;
-    const uint32_t m = (uint32_t)(nrm >> 40);  // 24 bits
-    const unsigned long long rest = nrm & 0xffffffffffull;
-    const int e = 63 - lz + s + 127;
-    if (e < 1 || e > 253) return (float)ldexp((double)X, s);
-    const uint32_t inc = rest > 0x8000000000ull || (rest == 0x8000000000ull && (m & 1u)) ? 1u : 0u;
-    return __uint_as_float((X < 0 ? 0x80000000u : 0u) | (((uint32_t)(e - 1) << 23) + m + inc));
-}
-
 template <typename P, typename T>
 __device__ __forceinline__ void sa_band_body(const SaLaunch &A, const int bx, const int by, const int part, const int parts) {
     static_assert(std::is_same<P, T>::value, "storage and compute types agree");
     constexpr bool kF32 = std::is_same<T, float>::value;
     extern __shared__ __align__(16) unsigned char sa_raw[];
-    __shared__ int top_expo[32];
-    double *X = reinterpret_cast<double *>(sa_raw);  // [row][slot]; a float lies in the low word
+    double *X = reinterpret_cast<double *>(sa_raw);  // [row][slot]; a float (before and after the solve) lies in the low word
     const int item = by;
     const int v = item / A.bk, zb = item % A.bk;
     const SplineDev &sp = A.spl[v];
@@ -216,9 +110,13 @@ __device__ __forceinline__ void sa_band_body(const SaLaunch &A, const int bx, co
     cp_async_wait_all();
     __syncthreads();
     auto coef = [&](int i, int sl) -> T & { return *reinterpret_cast<T *>(&X[i * kSaLd + sl]); };
-    auto fixed = [&](int i, int sl) -> long long & { return *reinterpret_cast<long long *>(&X[i * kSaLd + sl]); };
 
     if (!A.coeffs) {
+        if constexpr (kF32) {
+            for (int sl = warp; sl < nsl; sl += kSaWarps)
+                for (int i = lane; i < b; i += 32) X[i * kSaLd + sl] = (double)coef(i, sl);
+            __syncthreads();
+        }
         const double *ah0 = (sp.r3x && A.ahat) ? A.ahat + ((size_t)v * A.nblocks + (size_t)zb * A.nslots_z + s0) * b : nullptr;
         if (ah0) {  // b̃ = b − PQ·ahat (full P+Q, half-width 3)
             for (int sl = warp; sl < nsl; sl += kSaWarps) {
@@ -226,76 +124,39 @@ __device__ __forceinline__ void sa_band_body(const SaLaunch &A, const int bx, co
                 for (int i = lane; i < b; i += 32) {
                     double acc = 0.0;
                     for (int j = max(0, i - 3); j <= min(b - 1, i + 3); j++) acc += sp.PQb[i * 7 + (j - i + 3)] * ah[j];
-                    coef(i, sl) = (T)((double)coef(i, sl) - acc);
+                    X[i * kSaLd + sl] -= acc;
                 }
             }
             __syncthreads();
         }
-        // the boundary terms of the Γ fold (src/CubicBSpline.jl:427-463) of slot sl
-        auto fold_terms = [&](int sl, double (&f)[4]) {
-            const double b0 = coef(0, sl), b1 = coef(1, sl), bM1 = coef(b - 1, sl), bM2 = coef(b - 2, sl);
-            f[0] = sp.lk == BC_A1 ? sp.aL * b0 : (sp.lk == BC_A2 ? sp.aL * b0 + sp.bL * b1 : 0.0);  // into row 0
-            f[1] = sp.lk == BC_A1 ? sp.bL * b0 : 0.0;                                               // row 1
-            f[2] = sp.rk == BC_A1 ? sp.bR * bM1 : 0.0;                                              // row n − 2
-            f[3] = sp.rk == BC_A1 ? sp.aR * bM1 : (sp.rk == BC_A2 ? sp.aR * bM1 + sp.bR * bM2 : 0.0);  // row n − 1
-        };
-        const bool folds = sp.lk == BC_A1 || sp.lk == BC_A2 || sp.rk == BC_A1 || sp.rk == BC_A2;
-        if constexpr (kF32) {
-            // each slot's exponent, then every row as 60-bit fixed point in units 2^(E − F)
-            for (int sl = warp; sl < nsl; sl += kSaWarps) {
-                uint32_t mx = 0;
-                for (int i = lane; i < b; i += 32) mx = max(mx, __float_as_uint(coef(i, sl)) & 0x7fffffffu);
-                mx = __reduce_max_sync(0xffffffffu, mx);
-                const int top = max((int)(mx >> 23), 1);  // |b| < 2^(top − 126); 255: an infinity or NaN
-                if (lane == 0) top_expo[sl] = top;
-                double f[4];
-                if (folds) fold_terms(sl, f);
-                __syncwarp();
-                for (int i = lane; i < b; i += 32) {
-                    const uint32_t u = __float_as_uint(coef(i, sl));
-                    const int e = max((int)((u >> 23) & 0xffu), 1);
-                    const long long m = (u & 0x7fffffu) | ((u >> 23) & 0xffu ? 0x800000u : 0u);
-                    const int s = sp.fix_bits - 24 - (top - e);
-                    const long long x = s >= 0 ? m << s : (s > -24 ? m >> -s : 0);
-                    fixed(i, sl) = (u >> 31) ? -x : x;
+        // CTAs of an SM solve on different schedulers
+        if (warp == (bx & 3)) {
+            double *x = X + min(lane, nsl - 1), *xi = x + rL * kSaLd;
+            // the boundary terms of the Γ fold (src/CubicBSpline.jl:427-463)
+            if (lane < nsl) {
+                const double b0 = x[0], b1 = x[kSaLd], bM1 = x[(b - 1) * kSaLd], bM2 = x[(b - 2) * kSaLd];
+                if (sp.lk == BC_A1) {
+                    xi[0] += sp.aL * b0;
+                    xi[kSaLd] += sp.bL * b0;
+                } else if (sp.lk == BC_A2) {
+                    xi[0] += sp.aL * b0 + sp.bL * b1;
                 }
-                __syncwarp();
-                if (lane < 4 && folds) {
-                    const double add = lane == 0 ? f[0] : (lane == 1 ? f[1] : (lane == 2 ? f[2] : f[3]));
-                    const int row = lane == 0 ? 0 : (lane == 1 ? 1 : (lane == 2 ? n - 2 : n - 1));
-                    if (add != 0.0 && top < 255)
-                        atomicAdd(reinterpret_cast<unsigned long long *>(&fixed(rL + row, sl)),
-                                  (unsigned long long)__double2ll_rn(ldexp(add, sp.fix_bits - (top - 126))));
+                if (sp.rk == BC_A1) {
+                    xi[(n - 1) * kSaLd] += sp.aR * bM1;
+                    xi[(n - 2) * kSaLd] += sp.bR * bM1;
+                } else if (sp.rk == BC_A2) {
+                    xi[(n - 1) * kSaLd] += sp.aR * bM1 + sp.bR * bM2;
                 }
             }
-            __syncthreads();
-            if (warp == (bx & 3)) solve_fixed(sp, &fixed(rL, min(lane, nsl - 1)), n, lane, lane < nsl);
-        } else {
-            // CTAs of an SM solve on different schedulers
-            if (warp == (bx & 3)) {
-                const int sl = min(lane, nsl - 1);
-                if (folds && lane < nsl) {
-                    double f[4];
-                    fold_terms(sl, f);
-                    double *xi = X + rL * kSaLd + sl;
-                    xi[0] += f[0];
-                    xi[kSaLd] += f[1];
-                    xi[(n - 1) * kSaLd] += f[3];
-                    xi[(n - 2) * kSaLd] += f[2];
-                }
-                __syncwarp();
-                solve_f64(sp, X + rL * kSaLd + sl, n, lane, lane < nsl);
-            }
+            __syncwarp();
+            solve_f64(sp, xi, n, lane, lane < nsl);
         }
         __syncthreads();
         // the solution in the compute type; Γᵀ x (src/CubicBSpline.jl:465-500) and the background
         for (int sl = warp; sl < nsl; sl += kSaWarps) {
             const double *ah = ah0 ? ah0 + (size_t)sl * b : nullptr;
             auto sol = [&](int i) -> T {  // interior row i, rounded
-                if constexpr (kF32)
-                    return top_expo[sl] == 255 ? __int_as_float(0x7fc00000)
-                                               : fixed_to_float(fixed(rL + i, sl), top_expo[sl] - 126 - sp.fix_bits);
-                else return X[(rL + i) * kSaLd + sl];
+                return (T)X[(rL + i) * kSaLd + sl];
             };
             const T x0 = sol(0), x1 = sol(1), xn1 = sol(n - 1), xn2 = sol(n - 2);
             __syncwarp();

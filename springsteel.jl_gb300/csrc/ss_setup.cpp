@@ -322,57 +322,14 @@ static int32_t finish_weights(SplineHost &s) {
     return SS_OK;
 }
 
-SplineFixed spline_ldl(const SplineHost &s) {
-    const int n = s.Min;
-    SplineFixed f;
-    f.ldl.resize(size_t(n) * 4);
-    double mtop = 0.0, dtop = 0.0;
-    for (int i = 0; i < n; i++) {
+std::vector<double> spline_ldl(const SplineHost &s) {
+    std::vector<double> ldl(size_t(s.Min) * 4);
+    for (int i = 0; i < s.Min; i++) {
         const double d = s.L4[size_t(i) * 4];
-        for (int k = 1; k < 4; k++) {
-            f.ldl[size_t(i) * 4 + k - 1] = s.L4[size_t(i) * 4 + k] / d;
-            mtop = std::max(mtop, std::fabs(f.ldl[size_t(i) * 4 + k - 1]));
-        }
-        f.ldl[size_t(i) * 4 + 3] = 1.0 / (d * d);
-        dtop = std::max(dtop, f.ldl[size_t(i) * 4 + 3]);
+        for (int k = 1; k < 4; k++) ldl[size_t(i) * 4 + k - 1] = s.L4[size_t(i) * 4 + k] / d;
+        ldl[size_t(i) * 4 + 3] = 1.0 / (d * d);
     }
-    // entries below 1/2 after the scaling: products of 60-bit limbs stay below 2^58
-    auto above = [](double v) {  // least k with |v| < 2^(k − 1)
-        int e = 0;
-        std::frexp(v, &e);
-        return e + 1;
-    };
-    f.m_up = std::max(0, above(mtop));
-    f.d_up = std::min(30, std::max(0, above(dtop)));
-    f.m_up = std::min(30, f.m_up);
-    f.limbs.resize(size_t(n) * 8);
-    for (int i = 0; i < n; i++)
-        for (int k = 0; k < 4; k++) {
-            const long long q = std::llrint(std::ldexp(f.ldl[size_t(i) * 4 + k], 60 - (k < 3 ? f.m_up : f.d_up)));
-            f.limbs[size_t(i) * 8 + 2 * k] = (int)(q >> 30);
-            f.limbs[size_t(i) * 8 + 2 * k + 1] = (int)(q & 0x3fffffff);
-        }
-    // growth of |z| = |M⁻¹ Γ b| and of |x| = |M⁻ᵀ D⁻¹ z| over |b| ≤ 1: row sums of the inverses
-    const double gam = 1.0 + std::fabs(s.aL) + std::fabs(s.bL) + std::fabs(s.aR) + std::fabs(s.bR);
-    std::vector<double> zs(n, 0.0), xs(n, 0.0), z(n + 3), x(n + 3);
-    for (int c = 0; c < n; c++) {
-        std::fill(z.begin(), z.end(), 0.0);
-        std::fill(x.begin(), x.end(), 0.0);
-        z[c] = 1.0;
-        for (int i = c; i < n; i++)
-            for (int k = 1; k < 4 && i + k < n; k++) z[i + k] -= f.ldl[size_t(i) * 4 + k - 1] * z[i];
-        for (int i = n - 1; i >= 0; i--) {
-            x[i] = z[i] * f.ldl[size_t(i) * 4 + 3];
-            for (int k = 1; k < 4 && i + k < n; k++) x[i] -= f.ldl[size_t(i) * 4 + k - 1] * x[i + k];
-        }
-        for (int i = 0; i < n; i++) { zs[i] += std::fabs(z[i]); xs[i] += std::fabs(x[i]); }
-    }
-    double grow = 1.0;
-    for (int i = 0; i < n; i++) grow = std::max({grow, zs[i], xs[i]});
-    // |z|, |x| and, with three terms of |m| < 2^(m_up − 1) each, every partial sum below 2^61
-    f.bits = 59 - above(grow * gam) - f.m_up;
-    f.ok = f.bits >= 36 && above(mtop) <= 30 && above(dtop) <= 30;
-    return f;
+    return ldl;
 }
 
 // -------------------------------------------------------------- Chebyshev
