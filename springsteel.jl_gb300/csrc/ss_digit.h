@@ -112,6 +112,7 @@ struct DigitColumns {
     int steps = 0, zblocks = 0, buffers = 1, raws = 1;
     void *M = nullptr;
     int *mexpo = nullptr;
+    int *weight = nullptr;           // mode exponents taken from the matrices' columns into the data
     int2 *blocks = nullptr;
     std::vector<int> first;          // first block of every ring, their number at the end
     bool fon = false;                // forward (binary64): K-steps of levels, blocks of 32 modes, lanes of a column

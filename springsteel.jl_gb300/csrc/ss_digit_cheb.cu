@@ -7,7 +7,15 @@
 // they are (64-bit fixed point with one exponent per ring, mode and output),
 // forms the four reflected points of each quadrant position by integer
 // additions, cuts each column into digits at its own exponent and multiplies by
-// the matrix digits, which stay in shared memory.  ∂z and ∂zz share f's digits.
+// the matrix digits, which stay in shared memory.
+//
+// A fixed-point column is right to 2^-54 of its largest entry, which for ∂z and ∂zz must
+// be the largest contribution, not the largest mode: their matrices do not see a column's
+// mean (natural ends) and grow with the fourth power of the mode number.  So every column
+// k of M_d gives its largest exponent c_k to the data, u = (M_d 2^-c)(2^c b), and f, ∂z
+// and ∂zz are cut apart, 7 cuts for the 5 ring outputs.  One cut at f's exponent for all
+// three is faster (200 cells, 32 levels, 5 variables, the whole inverse 11.8 against 12.7 ms)
+// and loses 2^-55 of the mean, and of the low modes by the fourth power.
 //
 // Measured on the 200-cell, 32-level, 5-variable FP64 grid: 20.2 ms with FP64 FMAs
 // (94% of the FP64 matmul rate), 7.2 ms as digits with loads in line, 4.95 ms with
@@ -48,12 +56,16 @@ constexpr int kAStep = 6 * kDigitPlane;     // and of column digits
 // on the 200-cell FP64 grid: 8 + 16 warps 4.95 ms, 16 + 8 5.34 ms, 8 + 8 5.7 ms.
 constexpr int kProducers = 8, kDrains = 16;
 constexpr int kColThreads = (kProducers + kDrains + 1) * 32;
-constexpr int kMaxModes = 96;               // six K-steps keep every digit sum an exact integer
+constexpr int kMaxModes = 48;               // three K-steps: what the shared memory holds
 constexpr int kMaxZBlocks = 5;              // 160 levels
 // Shared memory a CTA may ask for: 227 KB less the static part.  Attribute of both column
 // kernels, whatever a grid needs: it is the process's, and grids of other level counts share it.
 constexpr size_t kColumnSmem = 232448 - 8192;
-constexpr int kRowExpo = 8;                 // row-exponent slots (producers run at most 4 outputs ahead)
+// Row-exponent slots: while the producers write those of cut i (at a block's first cut also
+// of i + 1 and i + 2), the drain may still read those of cut i − 2 − buffers.
+constexpr int kRowExpo = 8;
+constexpr int kCuts = kDigitVariants + 2;   // of a block: f for f, ∂z, ∂zz, then ∂λ, ∂λλ, ∂r, ∂rr
+constexpr int kUnseen = -(1 << 24);
 
 struct ColumnArgs {
     const void *H;
@@ -62,6 +74,7 @@ struct ColumnArgs {
     const int *expo;          // [variant][item][ring]
     const uint8_t *M;         // [var][3][zblocks][steps] matrix digits
     const int *mexpo;         // [var][3][32·zblocks]
+    const int *weight;        // [var][3][bk] c_k, kUnseen where M_d has no entry for the mode
     const int2 *blocks;       // (ring, first quadrant position) of every 32-position block
     int nblocks;
     int N, bk, nvars, nitems, iDim, steps, zblocks, buffers, raws;
@@ -91,8 +104,11 @@ __device__ __forceinline__ void issue_step64(uint32_t tacc, uint32_t sa, uint32_
         mma_f16(tacc + i * kZ, operand_desc(sa + i * kDigitPlane), bd, mma_idesc((7 - i) * kZ), 1u);
 }
 
+__device__ __forceinline__ int cut_output(int c) { return c < 3 ? 0 : c - 2; }
+__device__ __forceinline__ int cut_matrix(int c) { return c < 3 ? c : 0; }
+
 // grid = (CTAs per variable, variables); a CTA walks (block of 32 quadrant
-// positions = 128 columns, ring output), outputs fastest
+// positions = 128 columns, cut), cuts fastest
 // (kSmall: at most two K-steps)
 template <bool kSmall>
 __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArgs g) {
@@ -102,7 +118,8 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
     __shared__ volatile int quit;
     __shared__ volatile int halt[2];  // quit as thread 0 saw it, for all producers
     __shared__ int row_expo[kRowExpo][128];
-    __shared__ int mode_expo[2][kMaxModes];
+    __shared__ int mode_expo[2][kMaxModes], weight[3][kMaxModes];
+    __shared__ int mode_up[3][kMaxModes];  // mode exponent + c_k + 54 of the cuts of this output
     __shared__ __align__(16) int sE[3 * kZ * kMaxZBlocks];  // row exponents of the matrices, less 53
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int v = blockIdx.y, KS = g.steps, nb = g.buffers;
@@ -133,12 +150,13 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
     for (int i = threadIdx.x; i < nb * KS * kAStep / 16; i += blockDim.x)
         reinterpret_cast<uint4 *>(sA)[i] = make_uint4(0, 0, 0, 0);  // K groups of 8 without modes stay zero
     for (int i = threadIdx.x; i < 3 * g.zblocks * kZ; i += blockDim.x) sE[i] = g.mexpo[(size_t)v * 3 * g.zblocks * kZ + i] - 53;
+    for (int i = threadIdx.x; i < 3 * g.bk; i += blockDim.x) weight[i / g.bk][i % g.bk] = g.weight[(size_t)v * 3 * g.bk + i];
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
-    const int nitem = blockIdx.x < g.nblocks ? ((g.nblocks - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * kDigitVariants : 0;
+    const int nitem = blockIdx.x < g.nblocks ? ((g.nblocks - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * kCuts : 0;
 
     if (warp < kProducers) {
         // ---- producers: parts → points → digits.  The parts of the next output are
@@ -181,82 +199,102 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
             fetch(next, 0, 0);
         }
         const int nr = g.raws;
+        int out = 0;  // ring outputs so far
         for (int it = 0; it < nitem; it++) {
-            const int var = it % kDigitVariants, slot = it % nr;
-            if (var == 0) {
-                cur = next;
-                if (it + kDigitVariants < nitem) next = load_block(it / kDigitVariants + 1);
-            }
-            int *rex = row_expo[it % kRowExpo];
-            if (threadIdx.x < 128) rex[threadIdx.x] = 0;
-            const bool more = it + 1 < nitem;
-            if (more && nr == 2) {
-                if (var + 1 < kDigitVariants) fetch(cur, var + 1, slot ^ 1);
-                else fetch(next, 0, slot ^ 1);
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
-            } else {
-                asm volatile("cp.async.wait_group 0;" ::: "memory");
-            }
-            producers_sync();
+            const int cut = it % kCuts, var = cut_output(cut), md = cut_matrix(cut), slot = out % nr;
+            const bool last = cut >= 2;  // of this output
+            const bool more = it - cut + kCuts < nitem || var + 1 < kDigitVariants;
             long long *pts = raw + (size_t)slot * g.bk * 128;
-            int mx[4] = {0, 0, 0, 0};
-            for (int i = warp; i < g.bk; i += kProducers) {
-                long long *h = pts + i * 128 + lane;
-                const int e = mode_expo[slot][i];
-                long long p[4] = {0, 0, 0, 0};
-                if (cur.flags & 1) {
-                    const long long a = h[0], b = h[32], c = h[64], d = h[96];
-                    const long long u = a + b, w = c + d, x = a - b, z = c - d;
-                    p[0] = u + w; p[1] = u - w; p[2] = x - z; p[3] = x + z;
-                    if (cur.flags & 2) { p[0] = u; p[1] = z; p[2] = x; p[3] = w; }
+            if (cut == 0 || cut > 2) {
+                if (cut == 0) {
+                    cur = next;
+                    if (it + kCuts < nitem) next = load_block(it / kCuts + 1);
+                }
+                const int nd = cut == 0 ? 3 : 1;
+                if (threadIdx.x < 128)
+                    for (int d = 0; d < nd; d++) row_expo[(it + d) % kRowExpo][threadIdx.x] = 0;
+                if (more && nr == 2) {
+                    if (var + 1 < kDigitVariants) fetch(cur, var + 1, slot ^ 1);
+                    else fetch(next, 0, slot ^ 1);
+                    asm volatile("cp.async.wait_group 1;" ::: "memory");
+                } else {
+                    asm volatile("cp.async.wait_group 0;" ::: "memory");
+                }
+                producers_sync();
+                int mx[3][4] = {};
+                for (int i = warp; i < g.bk; i += kProducers) {
+                    long long *h = pts + i * 128 + lane;
+                    const int e = mode_expo[slot][i];
+                    long long p[4] = {0, 0, 0, 0};
+                    if (cur.flags & 1) {
+                        const long long a = h[0], b = h[32], c = h[64], d = h[96];
+                        const long long u = a + b, w = c + d, x = a - b, z = c - d;
+                        p[0] = u + w; p[1] = u - w; p[2] = x - z; p[3] = x + z;
+                        if (cur.flags & 2) { p[0] = u; p[1] = z; p[2] = x; p[3] = w; }
+                    }
+                    const bool nan = e == kNanColumn;
+                    if (lane < 3) mode_up[lane][i] = nan ? 0 : e + weight[lane][i] + 54;
+                    const int w0 = weight[0][i], w1 = weight[1][i], w2 = weight[2][i];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        h[q * 32] = p[q];
+                        // |p| ≤ 2^b, |p| 2^(e + c − 1074) ≤ 2^(mx − 1074)
+                        const int hi = (int)(p[q] >> 32) ^ (int)(p[q] >> 63);
+                        const int eb = (nan ? 0 : e) + (hi ? 64 - __clz(hi) : 32);
+                        mx[0][q] = max(mx[0][q], nan ? kNanColumn : eb + w0);
+                        if (cut == 0) {
+                            mx[1][q] = max(mx[1][q], nan ? kNanColumn : eb + w1);
+                            mx[2][q] = max(mx[2][q], nan ? kNanColumn : eb + w2);
+                        }
+                    }
                 }
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    h[q * 32] = p[q];
-                    // |p| ≤ 2^b, |p| 2^(e − 1074) ≤ 2^(mx − 1074)
-                    const int hi = (int)(p[q] >> 32) ^ (int)(p[q] >> 63);
-                    const int b = hi ? 64 - __clz(hi) : 32;
-                    mx[q] = max(mx[q], e == kNanColumn ? kNanColumn : e + b);
-                }
+                for (int d = 0; d < 3; d++)
+                    if (d < nd) {
+#pragma unroll
+                        for (int q = 0; q < 4; q++) atomicMax(&row_expo[(it + d) % kRowExpo][q * 32 + lane], mx[d][q]);
+                    }
+                // the producers leave together, on one thread's word: one that gave up waiting alone would
+                // be missed at the barrier for good
+                if (threadIdx.x == 0) halt[out & 1] = quit;
+                producers_sync();
+                if (halt[out & 1]) break;
             }
-#pragma unroll
-            for (int q = 0; q < 4; q++) atomicMax(&rex[q * 32 + lane], mx[q]);
-            // the producers leave together, on one thread's word: one that gave up waiting alone would
-            // be missed at the barrier for good
-            if (threadIdx.x == 0) halt[it & 1] = quit;
-            producers_sync();
-            if (halt[it & 1]) break;
             const int buf = it % nb;
             const bool ok = bar_wait(&aempty[buf], ((it / nb) & 1) ^ 1, &quit);  // if not: quit is set
             uint8_t *A = sA + (size_t)buf * KS * 6 * kDigitPlane;
             const int row = threadIdx.x & 127;
-            const int er = rex[row];
-            for (int kg = threadIdx.x >> 7; ok && kg < (g.bk + 7) / 8; kg += kProducers / 4) {
-                unsigned long long U[8];
+            const int er = min(row_expo[it % kRowExpo][row], 1 << 28);
+            // four modes at a time: 22 modes are three such cuts of every thread
+            for (int kq = threadIdx.x >> 7; ok && kq < (g.bk + 3) / 4; kq += kProducers / 4) {
+                unsigned long long U[4];
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const int mode = kg * 8 + i;
+                for (int i = 0; i < 4; i++) {
+                    const int mode = kq * 4 + i;
                     long long X = 0;
-                    if (mode < g.bk && er != kNanColumn) {
-                        const long long V = pts[mode * 128 + row];
-                        const int s = mode_expo[slot][mode] + 54 - er;  // |V 2^s| ≤ 2^54
-                        X = s >= 0 ? V << min(s, 63) : (s > -63 ? ((V >> (-s - 1)) + 1) >> 1 : 0);
+                    if (mode < g.bk) {
+                        X = pts[mode * 128 + row];
+                        const int s = mode_up[md][mode] - er;  // |V 2^s| ≤ 2^54
+                        if (s > 0) X <<= min(s, 63);
+                        else if (s < 0) X = s > -63 ? ((X >> (-s - 1)) + 1) >> 1 : 0;
                     }
                     U[i] = kDigitBias + (unsigned long long)X;
                 }
-                uint4 w[6];
-                planes8(U, w);
-                uint8_t *dst = A + (kg >> 1) * 6 * kDigitPlane + (row >> 3) * 256 + (kg & 1) * 128 + (row & 7) * 16;
+                uint2 w[6];
+                planes4(U, w);
+                uint8_t *dst = A + (kq >> 2) * 6 * kDigitPlane + (row >> 3) * 256 + ((kq >> 1) & 1) * 128 + (row & 7) * 16 + (kq & 1) * 8;
 #pragma unroll
-                for (int i = 0; i < 6; i++) *reinterpret_cast<uint4 *>(dst + i * kDigitPlane) = w[i];
+                for (int i = 0; i < 6; i++) *reinterpret_cast<uint2 *>(dst + i * kDigitPlane) = w[i];
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             if (ok) bar_arrive(&afull[buf]);
+            if (!last) continue;
             producers_sync();  // these points may be overwritten
             if (more && nr == 1) {
                 if (var + 1 < kDigitVariants) fetch(cur, var + 1, 0);
                 else fetch(next, 0, 0);
             }
+            out++;
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
     } else if (warp == kProducers + kDrains) {
@@ -269,8 +307,8 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
                 if (!(ok = bar_wait(&afull[buf], (it / nb) & 1, &quit))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t sa0 = smem_addr(sA) + buf * KS * 6 * kDigitPlane;
-                const int nd = it % kDigitVariants == 0 ? 3 : 1;
-                for (int q = 0; ok && q < nd * g.zblocks; q++, job++) {
+                const int q0 = cut_matrix(it % kCuts) * g.zblocks;
+                for (int q = q0; ok && q < q0 + g.zblocks; q++, job++) {
                     const int t = job & 1;
                     if (!(ok = bar_wait(&acce[t], ((job >> 1) & 1) ^ 1, &quit))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -299,8 +337,8 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
         uint32_t job = 0;
         bool ok = true;
         for (int it = 0; ok && it < nitem; it++) {
-            const int var = it % kDigitVariants, nd = var == 0 ? 3 : 1;
-            const int2 blk = g.blocks[blockIdx.x + it / kDigitVariants * gridDim.x];
+            const int cut = it % kCuts, var = cut_output(cut), d = cut_matrix(cut);
+            const int2 blk = g.blocks[blockIdx.x + it / kCuts * gridDim.x];
             const DigitRing *r = g.rings + blk.x;
             const int n = r->n, L = r->L, hf = r->half, m = blk.y + lane;
             const bool edge = hf == 0 && m == 0, live = m < n;
@@ -310,15 +348,15 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
             if (l < 0) l += L;
             if (l >= L) l -= L;
             double *const col = g.phys + (size_t)v * g.np + (r->jofs + l) * g.N;
-            for (int q = 0; ok && q < nd * g.zblocks; q++, job++) {
+            for (int zb = 0; ok && zb < g.zblocks; zb++, job++) {
                 if ((int)(job & 1) != mine) continue;
-                const int d = q / g.zblocks, z0 = (q - d * g.zblocks) * kZ + zh;
+                const int z0 = zb * kZ + zh;
                 const int slot = var == 0 ? (d == 0 ? 0 : 4 + d) : (var == 1 ? 3 : (var == 2 ? 4 : var - 2));
                 double *dst = col + (size_t)slot * g.nvars * g.np + z0;
                 if (!(ok = __all_sync(0xffffffffu, bar_wait(&accf[mine], (job >> 1) & 1, &quit)))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const int er = row_expo[it % kRowExpo][row];
-                const int *me = sE + q * kZ + zh;
+                const int *me = sE + (d * g.zblocks + zb) * kZ + zh;
                 // rolled: the instruction cache serves all three roles
 #pragma unroll 1
                 for (int c0 = 0; c0 < 16; c0 += 4) {
@@ -635,7 +673,7 @@ static int32_t build_inverse(ss_grid *g, const std::vector<ChebHost> &cheb) {
     if (!Q.buffers) return SS_OK;
     const int job = Q.steps * kZStep;
     std::vector<uint8_t> M((size_t)nv * 3 * Q.zblocks * job, 0);
-    std::vector<int> E((size_t)nv * 3 * Q.zblocks * kZ, 0);
+    std::vector<int> E((size_t)nv * 3 * Q.zblocks * kZ, 0), W((size_t)nv * 3 * bk, kUnseen);
     for (int v = 0; v < nv; v++) {
         const ChebHost &c = cheb[v];
         const int ne = (N + 1) / 2, no = std::max(N / 2, 1);
@@ -656,16 +694,28 @@ static int32_t build_inverse(ss_grid *g, const std::vector<ChebHost> &cheb) {
                     }
                 X.swap(Y);
             }
+            std::vector<double> M_d((size_t)N * bk);
             for (int z = 0; z < N; z++) {
                 const int j = std::min(z, N - 1 - z);  // inv_e, inv_o hold the first half of the levels
                 const double so = z == j ? 1.0 : -1.0;
-                std::vector<double> row(bk);
-                double top = 0.0;
                 for (int i = 0; i < bk; i++) {
                     double a = 0.0, b = 0.0;
                     for (int k = 0; k < N; k += 2) a += c.inv_e[(size_t)j * ne + k / 2] * X[(size_t)k * bk + i];
                     for (int k = 1; k < N; k += 2) b += c.inv_o[(size_t)j * no + k / 2] * X[(size_t)k * bk + i];
-                    row[i] = a + so * b;
+                    M_d[(size_t)z * bk + i] = a + so * b;
+                }
+            }
+            int *w = W.data() + ((size_t)v * 3 + d) * bk;
+            for (int i = 0; i < bk; i++) {
+                double top = 0.0;
+                for (int z = 0; z < N; z++) top = std::max(top, std::fabs(M_d[(size_t)z * bk + i]));
+                if (top > 0.0) std::frexp(top, &w[i]);
+            }
+            for (int z = 0; z < N; z++) {
+                double top = 0.0;
+                std::vector<double> row(bk, 0.0);
+                for (int i = 0; i < bk; i++) {
+                    if (w[i] != kUnseen) row[i] = std::ldexp(M_d[(size_t)z * bk + i], -w[i]);
                     top = std::max(top, std::fabs(row[i]));
                 }
                 int e = 0;
@@ -698,10 +748,11 @@ static int32_t build_inverse(ss_grid *g, const std::vector<ChebHost> &cheb) {
         g->allocs.push_back(*dst);
         return cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
     };
-    void *pm = nullptr, *pe = nullptr, *pb = nullptr;
-    if (!put(M.data(), M.size(), &pm) || !put(E.data(), E.size() * 4, &pe) || !put(blocks.data(), blocks.size() * 8, &pb))
+    void *pm = nullptr, *pe = nullptr, *pw = nullptr, *pb = nullptr;
+    if (!put(M.data(), M.size(), &pm) || !put(E.data(), E.size() * 4, &pe) || !put(W.data(), W.size() * 4, &pw) ||
+        !put(blocks.data(), blocks.size() * 8, &pb))
         return SS_OK;
-    Q.M = pm; Q.mexpo = (int *)pe; Q.blocks = (int2 *)pb;
+    Q.M = pm; Q.mexpo = (int *)pe; Q.weight = (int *)pw; Q.blocks = (int2 *)pb;
     CUDA_TRY(cudaFuncSetAttribute(Q.steps <= 2 ? digit_columns_kernel<true> : digit_columns_kernel<false>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColumnSmem));
     Q.on = true;
@@ -736,7 +787,7 @@ int32_t digit_columns_inverse(ss_grid *g, cudaStream_t st, int chunk) {
     const int r0 = chunk < 0 ? 0 : g->chunk_r0[chunk], r1 = chunk < 0 ? (int)d.iDim : g->chunk_r0[chunk + 1];
     ColumnArgs A{};
     A.H = g->H; A.phys = (double *)g->phys; A.rings = P.rings; A.expo = P.expo;
-    A.M = (const uint8_t *)Q.M; A.mexpo = Q.mexpo; A.blocks = Q.blocks + Q.first[r0]; A.nblocks = Q.first[r1] - Q.first[r0];
+    A.M = (const uint8_t *)Q.M; A.mexpo = Q.mexpo; A.weight = Q.weight; A.blocks = Q.blocks + Q.first[r0]; A.nblocks = Q.first[r1] - Q.first[r0];
     A.N = (int)d.kDim; A.bk = (int)d.b_kDim; A.nvars = (int)d.nvars; A.nitems = g->nitems; A.iDim = (int)d.iDim;
     A.steps = Q.steps; A.zblocks = Q.zblocks; A.buffers = Q.buffers; A.raws = Q.raws; A.jDim = d.jDim; A.np = d.n_physical; A.err = P.err;
     const int per = std::max(1, std::min(A.nblocks, g->sms / (int)d.nvars));

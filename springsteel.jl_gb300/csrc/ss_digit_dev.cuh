@@ -56,6 +56,21 @@ __device__ __forceinline__ void planes8(const unsigned long long (&U)[8], uint4 
         out[i] = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
+// and of 4
+__device__ __forceinline__ void planes4(const unsigned long long (&U)[4], uint2 (&out)[6]) {
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+        const int sh = 45 - 9 * i;
+        uint32_t w[2];
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            uint32_t a = (uint32_t)(U[2 * q] >> sh), b = (uint32_t)(U[2 * q + 1] >> sh);
+            if (i > 0) { a &= 511u; b &= 511u; }
+            w[q] = half_pair<false>(a, b, i > 0 ? 0x01000100u : 0x02000200u);
+        }
+        out[i] = make_uint2(w[0], w[1]);
+    }
+}
 // binary32: x·2^-E = (d0 + d1/1024 + d2/1024²)/256
 __device__ __forceinline__ void planes8(const float (&x)[8], uint4 (&out)[3]) {
     constexpr float M = 12582912.f;  // 1.5·2^23: adding it rounds to the nearest integer
