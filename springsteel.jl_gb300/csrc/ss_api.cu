@@ -649,7 +649,7 @@ static int32_t inv_sa(ss_grid *g, cudaStream_t st, int coeffs, const void *spec_
     for (auto &sh : g->spl_host) periodic |= sh.periodic != 0;
     if constexpr (std::is_same<P, T>::value) {
         if (!aout && sa_band_serves(g)) {
-            CUDA_TRY(launch_sa_band<T>(A, g->nitems, st));
+            CUDA_TRY(launch_sa_band<T>(A, g->nitems, g->sms, st));
             g->launches[SS_STAGE_SA_SI]++;
             return SS_OK;
         }

@@ -27,13 +27,14 @@ using namespace ss;
 // ====================================================================== batch
 // One launch of a fused batch: the CTAs of many grids' records of one stage
 // (one shared-memory class), each CTA running the record its work entry names.
-enum { FK_RING_FWD = 0, FK_SB = 1, FK_SA = 2, FK_SA_F32 = 3, FK_RING_INV = 4, FK_SA_BAND = 5 };
+enum { FK_RING_FWD = 0, FK_SB = 1, FK_SA = 2, FK_SA_F32 = 3, FK_RING_INV = 4, FK_SA_BAND = 5, FK_DIGIT = 6 };
 struct FusedLaunch {
     int kind, tl;
     size_t smem;
     int threads, nwork;
     const void *recs;       // RingLaunch / SbLaunch / SaLaunch records (device)
     const BatchWork *work;  // one entry per CTA (device)
+    DigitJoined digit = {};
 };
 
 struct ss_batch {
@@ -49,7 +50,7 @@ struct ss_batch {
     bool fused = false;
     int ib_scale = 1;                   // items per ring CTA × this (autotuned)
     std::vector<FusedLaunch> fwd, inv;  // in launch order
-    std::vector<ss_grid *> unfused;     // RLZ grids and grids of digit products: their own launch sequences
+    std::vector<ss_grid *> unfused;     // RLZ grids (and RL grids whose digits take several spans): their own launch sequences
     std::vector<void *> fused_mem;
     std::vector<uint64_t> fused_gen;    // generations the records were built from
 };
@@ -115,6 +116,30 @@ static int smem_class(size_t b) {
     return -1;
 }
 
+// The CTAs of a binary64 class join the launch of the larger class before it when, with that
+// class's shared memory, they fill the GPU at most four times: the gap between two launches
+// and the GPU emptying at the end of each cost more than the lower residency.  Behind a launch
+// of more than 16 fillings the gap is nothing.  A round trip without joining, at two fillings and
+// at four: 10 grids of 50 to 400 cells 15.65, 14.53, 14.32 ms, 4 grids of 30 to 130 cells 1.89, 1.17,
+// 1.18 ms, 64 of 50 to 400 equal.  Binary32 batches keep a launch per class: 10 grids of 76 to 358 cells
+// alone 4.02 → 3.73 ms, but several such batches on streams of their own fill each other's gaps, 3.67 → 3.77.
+struct ClassWork {
+    size_t smem = 0;
+    std::vector<BatchWork> work;
+};
+static void join_class(std::vector<ClassWork> &sets, ClassWork &&s, int tl, int sms) {
+    if (s.work.empty()) return;
+    if (!sets.empty() && tl == TL_F64) {
+        ClassWork &top = sets.back();
+        const double fill = (227.0 * 1024) / (double)(top.smem + 2048) * sms;
+        if ((double)s.work.size() <= 4.0 * fill && (double)top.work.size() <= 16.0 * fill) {
+            top.work.insert(top.work.end(), s.work.begin(), s.work.end());
+            return;
+        }
+    }
+    sets.push_back(std::move(s));
+}
+
 static void free_fused(ss_batch *bt) {
     for (void *p : bt->fused_mem) cudaFree(p);
     bt->fused_mem.clear();
@@ -168,24 +193,26 @@ static int32_t plan_rings(ss_batch *bt, const std::vector<ss_grid *> &gs, int tl
     std::vector<int> order(recs.size());
     for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return recs[a].buf > recs[b].buf; });
-    for (int c = 0; c < 7; c++)
-        for (int threads : {64, 128, 256}) {
-            std::vector<BatchWork> work;
-            size_t smem = 0;
+    for (int threads : {64, 128, 256}) {
+        std::vector<ClassWork> sets;
+        for (int c = 6; c >= 0; c--) {
+            ClassWork s;
             for (int i : order) {
                 const Rec &r = recs[i];
                 if (smem_class(r.smem) != c || r.threads != threads) continue;
-                smem = std::max(smem, r.smem);
+                s.smem = std::max(s.smem, r.smem);
                 for (int ring = 0; ring < r.nrings; ring++)
-                    for (int bx = 0; bx < r.nb; bx++) work.push_back({i, bx, ring, 0});
+                    for (int bx = 0; bx < r.nb; bx++) s.work.push_back({i, bx, ring, 0});
             }
-            if (work.empty()) continue;
-            FusedLaunch f{inverse ? FK_RING_INV : FK_RING_FWD, tl, smem, threads, (int)work.size(), d_recs, nullptr};
-            const void *w = nullptr;
-            if ((rc = upload(bt, work, &w))) return rc;
-            f.work = (const BatchWork *)w;
-            out.push_back(f);
+            join_class(sets, std::move(s), tl, gs[0]->sms);
         }
+        std::reverse(sets.begin(), sets.end());  // short rings first
+        for (const ClassWork &s : sets) {
+            const void *w = nullptr;
+            if ((rc = upload(bt, s.work, &w))) return rc;
+            out.push_back({inverse ? FK_RING_INV : FK_RING_FWD, tl, s.smem, threads, (int)s.work.size(), d_recs, (const BatchWork *)w});
+        }
+    }
     return SS_OK;
 }
 
@@ -243,21 +270,35 @@ static int32_t plan_sa(ss_batch *bt, const std::vector<ss_grid *> &gs, int tl, s
             out.push_back({FK_SA_F32, tl, 0, 128, (int)work.size(), d_recs, (const BatchWork *)w});
         }
     }
-    for (int c = 0; c < 14; c++) {  // classes of the banded, then of the tiled kernel
-        std::vector<BatchWork> work;
-        size_t sm = 0;
-        for (int i = 0; i < (int)gs.size(); i++) {
-            if (band[i] != (c < 7)) continue;
-            if (tl == TL_F32 && !periodic(i) && !band[i]) continue;
-            if (smem_class(smem[i]) != c % 7) continue;
-            sm = std::max(sm, smem[i]);
-            for (int by = 0; by < gs[i]->nitems; by++)
-                for (int bx = 0; bx < (L[i].nslots_z + 31) / 32; bx++) work.push_back({i, bx, by, 0});
+    for (int kind : {FK_SA_BAND, FK_SA}) {
+        std::vector<ClassWork> sets;
+        for (int c = 6; c >= 0; c--) {
+            ClassWork s;
+            for (int i = 0; i < (int)gs.size(); i++) {
+                if (band[i] != (kind == FK_SA_BAND)) continue;
+                if (tl == TL_F32 && !periodic(i) && !band[i]) continue;
+                if (smem_class(smem[i]) != c) continue;
+                s.smem = std::max(s.smem, smem[i]);
+                for (int by = 0; by < gs[i]->nitems; by++)
+                    for (int bx = 0; bx < (L[i].nslots_z + 31) / 32; bx++) s.work.push_back({i, bx, by, 0});
+            }
+            join_class(sets, std::move(s), tl, gs[0]->sms);
         }
-        if (work.empty()) continue;
-        const void *w = nullptr;
-        if ((rc = upload(bt, work, &w))) return rc;
-        out.push_back({c < 7 ? FK_SA_BAND : FK_SA, tl, sm, 128, (int)work.size(), d_recs, (const BatchWork *)w});
+        for (ClassWork &s : sets) {
+            if (kind == FK_SA_BAND) {  // few CTAs: parts of the rings, as launch_sa_band has them
+                const size_t ctas = s.work.size();
+                const int parts = std::max(1, std::min(8, (int)(2 * gs[0]->sms / ctas)));
+                for (size_t q = 0; q < ctas; q++) s.work[q].bz = parts;
+                for (int p = 1; p < parts; p++)
+                    for (size_t q = 0; q < ctas; q++) {
+                        s.work.push_back(s.work[q]);
+                        s.work.back().bz = p << 8 | parts;
+                    }
+            }
+            const void *w = nullptr;
+            if ((rc = upload(bt, s.work, &w))) return rc;
+            out.push_back({kind, tl, s.smem, 128, (int)s.work.size(), d_recs, (const BatchWork *)w});
+        }
     }
     for (size_t i = 0; i < smem.size(); i++)
         if (smem_class(smem[i]) < 0) {
@@ -268,21 +309,37 @@ static int32_t plan_sa(ss_batch *bt, const std::vector<ss_grid *> &gs, int tl, s
 }
 
 static std::vector<uint64_t> generations(const ss_batch *bt);
+
+// A batch gives every grid the bits that its own calls give: grids of digit products run
+// as such here too, the rings of one length as one product over all grids that have it.
+// A round trip of n equal FP64 grids of one variable, their own launches on eight streams →
+// joined (the FFT kernels' fused launches): 64 of 10 cells 1010 → 75 µs (205), 16 of 50 cells 1065
+// → 206 (609), 16 of 100 cells 3459 → 573 (2030), one of 24 cells 71 → 75 (175), of 115 cells
+// 387 → 389 (445); uneven grids: 64 of 10 to 50 cells 2477 → 523, 64 of 50 to 400 98.6 → 95.8 ms.
 static int32_t build_fused(ss_batch *bt) {
     free_fused(bt);
+    auto own = [](const ss_grid *g) { return g->rlz || (g->digit.on && !digit_joins(g)); };
     for (int tl : {TL_F64, TL_DF64, TL_F32}) {
-        std::vector<ss_grid *> gs;
-        for (ss_grid *g : bt->grids)
-            if (!g->rlz && !g->digit.on && g->tl == tl) gs.push_back(g);
+        std::vector<ss_grid *> gs, fft, digits;  // each grid once: the digit products' last step is in place
+        for (ss_grid *g : bt->grids) {
+            if (own(g) || g->tl != tl || std::find(gs.begin(), gs.end(), g) != gs.end()) continue;
+            gs.push_back(g);
+            (digit_joins(g) ? digits : fft).push_back(g);
+        }
         if (gs.empty()) continue;
-        int32_t rc = plan_rings(bt, gs, tl, false, bt->fwd);
+        int32_t rc = SS_OK;
+        if (!fft.empty()) rc = plan_rings(bt, fft, tl, false, bt->fwd);
+        std::vector<DigitJoined> joined;
+        if (!rc) rc = digit_join_plan(digits, bt->fused_mem, joined);
+        for (const DigitJoined &J : joined) bt->fwd.push_back({FK_DIGIT, tl, 0, 0, 0, nullptr, nullptr, J});
         if (!rc) rc = plan_sb(bt, gs, tl, bt->fwd);
         if (!rc) rc = plan_sa(bt, gs, tl, bt->inv);
-        if (!rc) rc = plan_rings(bt, gs, tl, true, bt->inv);
+        if (!rc && !fft.empty()) rc = plan_rings(bt, fft, tl, true, bt->inv);
+        for (const DigitJoined &J : joined) bt->inv.push_back({FK_DIGIT, tl, 0, 0, 0, nullptr, nullptr, J});
         if (rc) { free_fused(bt); return rc; }
     }
     for (ss_grid *g : bt->grids)
-        if (g->rlz || g->digit.on) bt->unfused.push_back(g);
+        if (own(g)) bt->unfused.push_back(g);
     bt->fused_gen = generations(bt);
     return SS_OK;
 }
@@ -311,7 +368,8 @@ static int32_t enqueue_fused(ss_batch *bt, int what, cudaStream_t st) {
     for (int dir = 1; dir <= 2; dir++) {
         if (!(what & dir)) continue;
         for (const FusedLaunch &f : dir == 1 ? bt->fwd : bt->inv) {
-            cudaError_t e = f.tl == TL_F64 ? fused_launch<double, double>(f, st)
+            cudaError_t e = f.kind == FK_DIGIT ? digit_join_launch(f.digit, dir == 1, st)
+                            : f.tl == TL_F64 ? fused_launch<double, double>(f, st)
                             : f.tl == TL_DF64 ? fused_launch<double, df64>(f, st)
                                               : fused_launch<float, float>(f, st);
             CUDA_TRY(e);
@@ -488,7 +546,10 @@ extern "C" int32_t ss_batch_synchronize(ss_batch *bt) {
 
 extern "C" int32_t ss_batch_fused_launches(const ss_batch *bt, int32_t what, int32_t *launches) {
     if (!bt || !launches || what < 1 || what > 3) { set_error("bad batch query"); return SS_BAD_ARG; }
-    *launches = (int32_t)(((what & 1) ? bt->fwd.size() : 0) + ((what & 2) ? bt->inv.size() : 0));
+    *launches = 0;
+    for (int dir = 1; dir <= 2; dir++)
+        if (what & dir)
+            for (const FusedLaunch &f : dir == 1 ? bt->fwd : bt->inv) *launches += f.kind == FK_DIGIT ? kDigitJoinedLaunches : 1;
     return SS_OK;
 }
 

@@ -161,6 +161,21 @@ __global__ void __launch_bounds__(256) digit_matrix_kernel(const DigitRing *ring
 // of even or odd k, writes 8 K entries of each plane as 16 bytes; the 8 items of
 // a group are the 8 rows of one core matrix, so a warp's stores are 128-byte
 // runs.  Column of (item, variant): (item / 8)·8·kVars + variant·8 + item mod 8.
+// Joined: the items of many RL grids with the same rings are the items of one product.
+// They are ordered by falling ring count, so ring r holds the first count[r] of them.
+struct DigitItemRef {
+    const double *in, *G;      // slot 1 and G of the item
+    double *F, *out;           // F; slot 1
+    long long *H;              // quadrant parts
+    int64_t gplane, hplane, oplane;  // to the next derivative of G, output of H, slot
+    int *err;
+    int cap;
+};
+struct DigitJoin {
+    const DigitItemRef *refs;
+    const int *count;
+};
+
 struct SplitArgs {
     const void *G;
     const DigitRing *rings;
@@ -170,7 +185,16 @@ struct SplitArgs {
     const int *delta, *cap;   // cap: largest wavenumber of every item (per-variable kmax of RL grids)
     int64_t frows;
     int r0, nitems, iDim, col_tiles;
+    DigitJoin join;
 };
+template <typename T>
+SS_HD constexpr int inverse_col_tiles(int items) {
+    return ((items + kDigitGroup - 1) / kDigitGroup * kDigitGroup * DigitFormat<T>::kVars + 2 * DigitFormat<T>::kCols - 1) /
+           (2 * DigitFormat<T>::kCols);
+}
+SS_HD constexpr int forward_col_tiles(int items) {
+    return (items + 2 * DigitFormat<double>::kCols - 1) / (2 * DigitFormat<double>::kCols);
+}
 
 __device__ __forceinline__ uint32_t mag_bits(double v) { return (uint32_t)__double2hiint(v) & 0x7fffffffu; }
 __device__ __forceinline__ uint32_t mag_bits(float v) { return (uint32_t)__float_as_int(v) & 0x7fffffffu; }
@@ -185,7 +209,7 @@ __device__ __forceinline__ int mag_expo(uint32_t bits) {  // biased exponent ≥
     }
 }
 
-template <typename T>
+template <typename T, bool kJoin>
 __global__ void __launch_bounds__(256, 2) digit_split_kernel(SplitArgs S) {
     using F = DigitFormat<T>;
     constexpr int V0 = kDigitVariants - F::kVars;
@@ -193,14 +217,28 @@ __global__ void __launch_bounds__(256, 2) digit_split_kernel(SplitArgs S) {
     const int ring = S.r0 + (int)(gridDim.y - 1 - blockIdx.y);  // largest rings first
     const DigitRing r = S.rings[ring];
     const int grp = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const T *G = (const T *)S.G;
-    const size_t plane = (size_t)S.nitems * S.frows;
+    const int here = kJoin ? S.join.count[ring] : S.nitems;  // items of this ring
+    if (kJoin && grp * kDigitGroup >= here) return;
+    auto row_of = [&](int item, size_t &plane, int &cap) {
+        if constexpr (kJoin) {
+            const DigitItemRef &q = S.join.refs[item];
+            plane = (size_t)q.gplane;
+            cap = q.cap;
+            return (const T *)q.G + r.fofs;
+        } else {
+            plane = (size_t)S.nitems * S.frows;
+            cap = S.cap[item];
+            return (const T *)S.G + (size_t)item * S.frows + r.fofs;
+        }
+    };
     {
         const int item = grp * kDigitGroup + warp;
         uint32_t mx[kDigitVariants] = {0, 0, 0, 0, 0};
-        if (item < S.nitems) {
-            const T *g0 = G + (size_t)item * S.frows + r.fofs;
-            const int kmax = min(r.kmax, S.cap[item]);
+        if (item < here) {
+            size_t plane;
+            int cap;
+            const T *g0 = row_of(item, plane, cap);
+            const int kmax = min(r.kmax, cap);
             for (int s = lane; s < 1 + 2 * kmax; s += 32) {
                 const T k = (T)((s + 1) >> 1);
                 const T v = g0[s];
@@ -218,7 +256,7 @@ __global__ void __launch_bounds__(256, 2) digit_split_kernel(SplitArgs S) {
                 ex[warp][q] = e;
                 // of the parts: one higher where the products store them halved
                 const int up = std::is_same<T, double>::value && r.n > kDigitFullRing && e != kNanColumn ? 1 : 0;
-                if (item < S.nitems) S.expo[((size_t)q * S.nitems + item) * S.iDim + ring] = e + up;
+                if (item < here) S.expo[((size_t)q * S.nitems + item) * S.iDim + ring] = e + up;
             }
         }
     }
@@ -226,13 +264,16 @@ __global__ void __launch_bounds__(256, 2) digit_split_kernel(SplitArgs S) {
     // warp-uniform control flow: lanes exchange values; idle ones (no such item, no
     // such odd step) read item 0 and store nothing
     const int il = threadIdx.x & 7;
-    const bool real = grp * kDigitGroup + il < S.nitems;
+    const bool real = grp * kDigitGroup + il < here;
     const int item = real ? grp * kDigitGroup + il : 0;
     const int par = (threadIdx.x >> 3) & 1, imag = (threadIdx.x >> 4) & 1;
     const int64_t bt = S.btile[ring];
-    const T *g = G + (size_t)item * S.frows + r.fofs;
-    const int kmax = min(r.kmax, S.cap[item]);
+    size_t plane;
+    int cap;
+    const T *g = row_of(item, plane, cap);
+    const int kmax = min(r.kmax, cap);
     const int steps = par ? r.to : r.te;
+    const int col_tiles = kJoin ? inverse_col_tiles<T>(here) : S.col_tiles;
     for (int kg = warp; kg < 2 * r.te; kg += 8) {
         const bool store = real && kg < 2 * steps;
         const int k0 = 16 * kg + par;
@@ -285,7 +326,7 @@ __global__ void __launch_bounds__(256, 2) digit_split_kernel(SplitArgs S) {
                     for (int i = 0; i < 8; i++) y[i] = scale2(x[i], 8 - (e - 126));
                     planes8(y, w);
                 }
-                const int64_t tile = bt + digit_part_base(r, part, S.col_tiles) + (int64_t)ct * steps + (kg >> 1);
+                const int64_t tile = bt + digit_part_base(r, part, col_tiles) + (int64_t)ct * steps + (kg >> 1);
                 uint8_t *dst = S.B + tile * digit_b_bytes<T>() + h * digit_half_bytes<T>() + (kg & 1) * 128 + (c & 7) * 16;
                 if (store)
 #pragma unroll
@@ -307,15 +348,16 @@ struct GemmDigitArgs {
     int64_t jDim, frows;
     int nitems, nvars, bk, iDim;
     int *err;
+    DigitJoin join;
 };
 
 constexpr int kDrainWarps = 16;
 constexpr int kDigitThreads = (kDrainWarps + 3) * 32;  // and 1 copying, 2 issuing warps
 
 // One CTA per SM (shared-memory ring, 2 × kSums·kCols accumulator columns).
-// Each accumulator half has its own issuing warp and warpgroup, so one half
-// computes while the other drains.
-template <typename T, bool kForward>
+// Each accumulator half has its own issuing warp, so one half computes while the
+// sixteen draining warps, which serve both, are at the other.
+template <typename T, bool kForward, bool kJoin>
 __global__ void __launch_bounds__(kDigitThreads, 1) digit_gemm_kernel(GemmDigitArgs g) {
     using F = DigitFormat<T>;
     constexpr int ND = F::kDigits, W = F::kCols, ST = F::kStages;
@@ -446,24 +488,27 @@ __global__ void __launch_bounds__(kDigitThreads, 1) digit_gemm_kernel(GemmDigitA
             const int k = 2 * row + (d.part & 1);
             const int m = kForward ? max(2 * k - 1 + (d.part >> 1), 0) : row - r->lo[d.part];
             const bool live = kForward ? k < r->n && (k > 0 || d.part == 0) : m >= 0 && m < r->cnt[d.part];
-            // lane c's column of this warp (half c / WC): its output base (−1 for padding) and exponent
-            auto col_base = [&](int c, int &e) -> int64_t {
+            const int here = kJoin ? g.join.count[d.ring] : g.nitems;
+            // lane c's column of this warp (half c / WC): its output row (null for padding) and exponent
+            using Acc = typename std::conditional<std::is_same<T, double>::value, unsigned long long, float>::type;
+            auto col_base = [&](int c, int &e) -> Acc * {
                 constexpr int V0 = kDigitVariants - F::kVars;
                 const int col = (d.col_tile * 2 + c / WC) * W + cb + c % WC;
                 const int item = col / (kDigitGroup * F::kVars) * kDigitGroup + col % kDigitGroup;
                 const int var = col / kDigitGroup % F::kVars + V0;
                 e = 0;
                 if constexpr (kForward) {
-                    if (c >= 2 * WC || col >= g.nitems) return -1;
+                    if (c >= 2 * WC || col >= here) return nullptr;
                     e = g.expo[(size_t)col * g.iDim + d.ring];
-                    return (int64_t)col * g.frows + r->fofs;
+                    if constexpr (kJoin) return (Acc *)g.join.refs[col].F + r->fofs;
+                    return (Acc *)g.out + (int64_t)col * g.frows + r->fofs;
                 }
-                if (c >= 2 * WC || item >= g.nitems) return -1;
+                if (c >= 2 * WC || item >= here) return nullptr;
                 e = g.expo[((size_t)var * g.nitems + item) * g.iDim + d.ring];
-                return ((int64_t)var * g.nvars + item / g.bk) * g.bk * g.jDim + (int64_t)g.bk * r->jofs + r->off[d.part] +
+                if constexpr (kJoin) return (Acc *)g.join.refs[item].H + var * g.join.refs[item].hplane + r->jofs + r->off[d.part];
+                return (Acc *)g.out + ((int64_t)var * g.nvars + item / g.bk) * g.bk * g.jDim + (int64_t)g.bk * r->jofs + r->off[d.part] +
                        (int64_t)(item % g.bk) * r->L;
             };
-            using Acc = typename std::conditional<std::is_same<T, double>::value, unsigned long long, float>::type;
             using Comb = Combine<false>;
             Acc V[2 * WC];
             const Acc start = std::is_same<T, double>::value ? (Acc)(0ull - Comb::kOffset * (unsigned)nch) : (Acc)0;
@@ -500,16 +545,15 @@ __global__ void __launch_bounds__(kDigitThreads, 1) digit_gemm_kernel(GemmDigitA
                     for (int c = 0; c < 2 * WC; c++) V[c] = (Acc)(((long long)V[c] + 1) >> 1);
                 }
             }
-            Acc *out = (Acc *)g.out;
             const double inv_len = kForward ? 1.0 / (double)r->L : 0.0;
 #pragma unroll
             for (int c0 = 0; c0 < 2 * WC; c0 += 32) {
                 int e;
-                const int64_t mine = col_base(c0 + lane, e);
+                const long long mine = (long long)col_base(c0 + lane, e);
 #pragma unroll
                 for (int c = 0; c < 32; c++) {
                     if (c0 + c >= 2 * WC) break;
-                    const int64_t base = __shfl_sync(0xffffffffu, mine, c);
+                    Acc *const base = (Acc *)__shfl_sync(0xffffffffu, mine, c);
                     Acc v = V[c0 + c];
                     if constexpr (std::is_same<T, float>::value) {
                         // doubled product of 2^-8 fixed-point operands at column scale 2^(e − 126)
@@ -519,11 +563,11 @@ __global__ void __launch_bounds__(kDigitThreads, 1) digit_gemm_kernel(GemmDigitA
                     if constexpr (kForward) {
                         // folded points scaled by 2^(e − 1020): Σ = V 2^(e − 1020 − 53)
                         const int ce = __shfl_sync(0xffffffffu, e, c);
-                        if (ok && live && base >= 0)
-                            ((double *)g.out)[base + m] = ce == kNanColumn ? __longlong_as_double(0x7ff8000000000000ll)
+                        if (ok && live && base)
+                            ((double *)base)[m] = ce == kNanColumn ? __longlong_as_double(0x7ff8000000000000ll)
                                                                            : fixed_to_double((long long)v, ce + 1) * inv_len;
                     } else {
-                        if (ok && live && base >= 0) out[base + m] = v;
+                        if (ok && live && base) base[m] = v;
                     }
                 }
             }
@@ -531,7 +575,11 @@ __global__ void __launch_bounds__(kDigitThreads, 1) digit_gemm_kernel(GemmDigitA
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (threadIdx.x == 0 && quit) *g.err = 1;
+    if (threadIdx.x == 0 && quit) {
+        if constexpr (kJoin)
+            for (int i = 0; i < g.nitems; i++) *g.join.refs[i].err = 1;
+        else *g.err = 1;
+    }
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
@@ -539,23 +587,40 @@ __global__ void __launch_bounds__(kDigitThreads, 1) digit_gemm_kernel(GemmDigitA
 // ------------------------------------------------------------ unfold
 // The four quadrant parts of one (ring, item, variant) row → its 4n points: in place
 // (RLZ) or into the physical slot (RL, `phys` set)
-template <typename T>
-__global__ void __launch_bounds__(128) digit_unfold_kernel(void *H, T *phys, const DigitRing *rings, const int *expo, int r0,
-                                                           int nitems, int nvars, int bk, int iDim, int64_t jDim) {
+struct UnfoldArgs {
+    void *H, *phys;
+    const DigitRing *rings;
+    const int *expo;
+    int64_t jDim;
+    int r0, nitems, nvars, bk, iDim;
+    DigitJoin join;
+};
+template <typename T, bool kJoin>
+__global__ void __launch_bounds__(128) digit_unfold_kernel(UnfoldArgs U) {
     using R = typename std::conditional<std::is_same<T, double>::value, long long, float>::type;
     extern __shared__ __align__(16) unsigned char row_raw[];
     R *row = reinterpret_cast<R *>(row_raw);
-    const int ring = r0 + (int)(gridDim.y - 1 - blockIdx.y);
-    const DigitRing &r = rings[ring];
+    const int ring = U.r0 + (int)(gridDim.y - 1 - blockIdx.y), nitems = U.nitems;
+    const DigitRing &r = U.rings[ring];
     const int n = r.n, L = r.L, shift = r.shift;
     const int var = blockIdx.x / nitems + kDigitVariants - DigitFormat<T>::kVars, item = blockIdx.x % nitems;
-    const int64_t at = (int64_t)(item / bk) * bk * jDim + (int64_t)bk * r.jofs + (int64_t)(item % bk) * L;
-    const R *h = (const R *)H + (int64_t)var * nvars * bk * jDim + at;
     const int slot = var == 0 ? 0 : (var < 3 ? var + 2 : var - 2);  // f, ∂r, ∂rr, ∂λ, ∂λλ
-    T *dst = phys ? phys + (int64_t)slot * nvars * jDim + at : (T *)H + (int64_t)var * nvars * bk * jDim + at;
+    const R *h;
+    T *dst;
+    if constexpr (kJoin) {
+        if (item >= U.join.count[ring]) return;
+        const DigitItemRef &q = U.join.refs[item];
+        h = q.H + var * q.hplane + r.jofs;
+        dst = q.out + slot * q.oplane + r.jofs;
+    } else {
+        const int64_t at = (int64_t)(item / U.bk) * U.bk * U.jDim + (int64_t)U.bk * r.jofs + (int64_t)(item % U.bk) * L;
+        const int64_t out = (int64_t)var * U.nvars * U.bk * U.jDim + at;
+        h = (const R *)U.H + out;
+        dst = U.phys ? (T *)U.phys + (int64_t)slot * U.nvars * U.jDim + at : (T *)U.H + out;
+    }
     for (int i = threadIdx.x; i < L; i += blockDim.x) row[i] = h[i];
     int e = 0;
-    if constexpr (std::is_same<T, double>::value) e = expo[((size_t)var * nitems + item) * iDim + ring];
+    if constexpr (std::is_same<T, double>::value) e = U.expo[((size_t)var * nitems + item) * U.iDim + ring];
     __syncthreads();
     auto put = [&](int p, R v) {
         int l = p - shift;
@@ -597,21 +662,26 @@ struct FoldArgs {
     int *expo;
     int64_t jDim;
     int r0, nitems, iDim, bk, col_tiles;
+    DigitJoin join;
 };
 
+template <bool kJoin>
 __global__ void __launch_bounds__(256, 2) digit_fold_kernel(FoldArgs S) {
     using F = DigitFormat<double>;
     __shared__ int ex[kDigitGroup];
     const int ring = S.r0 + (int)(gridDim.y - 1 - blockIdx.y);
     const DigitRing r = S.rings[ring];
     const int grp = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int here = kJoin ? S.join.count[ring] : S.nitems;
+    if (kJoin && grp * kDigitGroup >= here) return;
     auto row_of = [&](int item) {
+        if constexpr (kJoin) return S.join.refs[item].in + r.jofs;
         return S.C + (int64_t)(item / S.bk) * S.bk * S.jDim + (int64_t)S.bk * r.jofs + (int64_t)(item % S.bk) * r.L;
     };
     {
         const int item = grp * kDigitGroup + warp;
         uint32_t mx = 0;
-        if (item < S.nitems) {
+        if (item < here) {
             const double2 *x = reinterpret_cast<const double2 *>(row_of(item));  // even offsets and lengths
             for (int i = lane; i < r.L / 2; i += 32) {
                 const double2 v = x[i];
@@ -621,12 +691,13 @@ __global__ void __launch_bounds__(256, 2) digit_fold_kernel(FoldArgs S) {
         const int e = mag_expo<double>(__reduce_max_sync(0xffffffffu, mx));
         if (lane == 0) {
             ex[warp] = e;
-            if (item < S.nitems) S.expo[(size_t)item * S.iDim + ring] = e;
+            if (item < here) S.expo[(size_t)item * S.iDim + ring] = e;
         }
     }
     __syncthreads();
     const int il = threadIdx.x & 7, item = grp * kDigitGroup + il;
-    if (item >= S.nitems) return;
+    if (item >= here) return;
+    const int col_tiles = kJoin ? forward_col_tiles(here) : S.col_tiles;
     const int sine = (threadIdx.x >> 3) & 1;
     const double *x = row_of(item);
     const int n = r.n, hf = r.half, L = r.L, e = ex[il];
@@ -658,12 +729,12 @@ __global__ void __launch_bounds__(256, 2) digit_fold_kernel(FoldArgs S) {
             odd[i] = kDigitBias + (unsigned long long)(((sine ? u : w) + 128) >> 8);
         }
         uint4 w[6];
-        const int64_t tile = bt + (int64_t)(2 * sine) * S.col_tiles * r.tm + (mg >> 1);
+        const int64_t tile = bt + (int64_t)(2 * sine) * col_tiles * r.tm + (mg >> 1);
         uint8_t *dst = S.B + tile * digit_b_bytes<double>() + h * digit_half_bytes<double>() + (mg & 1) * 128 + (c & 7) * 16;
         planes8(even, w);
 #pragma unroll
         for (int i = 0; i < 6; i++) *reinterpret_cast<uint4 *>(dst + ((i * F::kCols + c) >> 3) * 256) = w[i];
-        dst += (int64_t)S.col_tiles * r.tm * digit_b_bytes<double>();
+        dst += (int64_t)col_tiles * r.tm * digit_b_bytes<double>();
         planes8(odd, w);
 #pragma unroll
         for (int i = 0; i < 6; i++) *reinterpret_cast<uint4 *>(dst + ((i * F::kCols + c) >> 3) * 256) = w[i];
@@ -672,11 +743,22 @@ __global__ void __launch_bounds__(256, 2) digit_fold_kernel(FoldArgs S) {
 
 // X_k ← X_k e^{−iδ_k}: the forward coefficients at the reference's rounded angles,
 // zero above the item's own kmax
-__global__ void __launch_bounds__(128) digit_turn_kernel(double *Fp, const DigitRing *rings, const int *delta, const int *cap,
-                                                         int64_t frows, int r0) {
-    const DigitRing &r = rings[r0 + blockIdx.y];
-    double *f = Fp + (int64_t)blockIdx.x * frows + r.fofs;
-    const int kmax = min(r.kmax, cap[blockIdx.x]);
+struct TurnArgs {
+    double *F;
+    const DigitRing *rings;
+    const int *delta, *cap;
+    int64_t frows;
+    int r0;
+    DigitJoin join;
+};
+template <bool kJoin>
+__global__ void __launch_bounds__(128) digit_turn_kernel(TurnArgs U) {
+    const int ring = U.r0 + blockIdx.y, item = blockIdx.x;
+    const DigitRing &r = U.rings[ring];
+    if (kJoin && item >= U.join.count[ring]) return;
+    double *f = (kJoin ? U.join.refs[item].F : U.F + (int64_t)item * U.frows) + r.fofs;
+    const int kmax = min(r.kmax, kJoin ? U.join.refs[item].cap : U.cap[item]);
+    const int *delta = U.delta;
     for (int k = kmax + 1 + threadIdx.x; k <= r.kmax; k += blockDim.x) f[2 * k - 1] = f[2 * k] = 0.0;
     for (int k = 1 + threadIdx.x; k <= kmax; k += blockDim.x) {
         const double d = (double)delta[r.dofs + k - 1] * 0x1p-70;
@@ -718,6 +800,26 @@ static bool upload(ss_grid *g, const V **dst, const std::vector<V> &src) {
     if (!src.empty() && cudaMemcpy(p, src.data(), src.size() * sizeof(V), cudaMemcpyHostToDevice) != cudaSuccess) return false;
     *dst = (const V *)p;
     return true;
+}
+
+// B tiles of a ring, and its tile products with the first B tile at `used`
+static int64_t ring_tiles(const DigitRing &q, int tiles, bool fwd) { return (int64_t)tiles * (fwd ? 4 * q.tm : 2 * (q.te + q.to)); }
+static void ring_items(const DigitRing &q, int ring, int tiles, bool fwd, int64_t used, std::vector<DigitItem> &items) {
+    for (int part = 0; part < 4; part++)
+        for (int ct = 0; ct < tiles; ct++)
+            for (int rt = 0; rt < (fwd ? q.rtf : q.rt); rt++) {
+                const int steps = fwd ? q.tm : digit_steps(q, part);
+                DigitItem it{};
+                if (fwd) {
+                    it.a_tile = q.af_tile + ((int64_t)part * q.rtf + rt) * steps;
+                    it.b_tile = used + ((int64_t)part * tiles + ct) * steps;
+                } else {
+                    it.a_tile = q.a_tile + digit_part_base(q, part, q.rt) + (int64_t)rt * steps;
+                    it.b_tile = used + digit_part_base(q, part, tiles) + (int64_t)ct * steps;
+                }
+                it.ring = ring; it.part = part; it.row_tile = rt; it.col_tile = ct; it.steps = steps;
+                items.push_back(it);
+            }
 }
 
 template <typename T>
@@ -772,9 +874,8 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
             delta[rings[i].dofs + k - 1] = (int)std::lrint(std::ldexp(k * dy - std::fma((double)k, ymin, -a), 70));
         }
     }
-    const int ncol = (g->nitems + kDigitGroup - 1) / kDigitGroup * kDigitGroup * F::kVars;
-    D.col_tiles = (ncol + 2 * F::kCols - 1) / (2 * F::kCols);
-    D.col_tiles_fwd = (g->nitems + 2 * F::kCols - 1) / (2 * F::kCols);
+    D.col_tiles = inverse_col_tiles<T>(g->nitems);
+    D.col_tiles_fwd = forward_col_tiles(g->nitems);
     constexpr bool kBoth = std::is_same<T, double>::value;  // binary32 grids keep the forward FFT's rounding
     const size_t abytes = (size_t)atiles * digit_a_bytes<T>(), afbytes = kBoth ? (size_t)aftiles * digit_a_bytes<T>() : 0;
     if (abytes + afbytes > (g->rlz ? kDigitTableBytes : kDigitTableBytesRl)) return SS_OK;
@@ -799,25 +900,11 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
             int64_t used = 0;
             while (r > lo) {
                 const DigitRing &q = rings[r - 1];
-                const int64_t need = (int64_t)tiles * (fwd ? 4 * q.tm : 2 * (q.te + q.to));
+                const int64_t need = ring_tiles(q, tiles, fwd);
                 if (used > 0 && (used + need) * digit_b_bytes<T>() > kDigitScratchBytes) break;
                 r--;
                 btile[r] = used;
-                for (int part = 0; part < 4; part++)
-                    for (int ct = 0; ct < tiles; ct++)
-                        for (int rt = 0; rt < (fwd ? q.rtf : q.rt); rt++) {
-                            const int steps = fwd ? q.tm : digit_steps(q, part);
-                            DigitItem it{};
-                            if (fwd) {
-                                it.a_tile = q.af_tile + ((int64_t)part * q.rtf + rt) * steps;
-                                it.b_tile = used + ((int64_t)part * tiles + ct) * steps;
-                            } else {
-                                it.a_tile = q.a_tile + digit_part_base(q, part, q.rt) + (int64_t)rt * steps;
-                                it.b_tile = used + digit_part_base(q, part, tiles) + (int64_t)ct * steps;
-                            }
-                            it.ring = r; it.part = part; it.row_tile = rt; it.col_tile = ct; it.steps = steps;
-                            items.push_back(it);
-                        }
+                ring_items(q, r, tiles, fwd, used, items);
                 used += need;
             }
             sp.r0 = r;
@@ -830,6 +917,7 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
     const DigitRing *dr = nullptr;
     if (!upload(g, &dr, rings)) return give_up();
     D.rings = const_cast<DigitRing *>(dr);
+    D.ring_host = rings;
     const int *dd = nullptr;
     if (!upload(g, &dd, delta)) return give_up();
     D.delta = const_cast<int *>(dd);
@@ -840,6 +928,7 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
     }
     if (!upload(g, &dd, cap)) return give_up();
     D.cap = const_cast<int *>(dd);
+    D.cap_host = cap;
     if (!make_set(0, nr, false, D.whole) || (kBoth && !make_set(0, nr, true, D.whole_fwd))) return give_up();
     D.chunks.resize(g->chunk_r0.size() - 1);
     D.chunks_fwd.resize(g->chunk_r0.size() - 1);
@@ -889,9 +978,9 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
     cudaFree(cosq);
     cosq = nullptr;
     CUDA_TRY(e);
-    CUDA_TRY(cudaFuncSetAttribute(digit_gemm_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digit_smem<T>()));
+    CUDA_TRY(cudaFuncSetAttribute(digit_gemm_kernel<T, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digit_smem<T>()));
     if constexpr (kBoth)
-        CUDA_TRY(cudaFuncSetAttribute(digit_gemm_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digit_smem<T>()));
+        CUDA_TRY(cudaFuncSetAttribute(digit_gemm_kernel<T, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digit_smem<T>()));
     D.on = true;
     return SS_OK;
 }
@@ -923,25 +1012,46 @@ int32_t digit_status(ss_grid *g) {
     return SS_DEVICE_TIMEOUT;
 }
 
+// the kernels' arguments for one span of rings
+static SplitArgs split_args(const ss_grid *g, const DigitSet &set, const DigitSpan &sp) {
+    const DigitPlan &D = g->digit;
+    return {g->G, D.rings, set.btile, (uint8_t *)D.B, D.expo, D.delta, D.cap, g->frows, sp.r0, g->nitems, (int)g->d.iDim, D.col_tiles};
+}
+static FoldArgs fold_args(const ss_grid *g, const DigitSet &set, const DigitSpan &sp) {
+    const DigitPlan &D = g->digit;
+    return {(const double *)(g->rlz ? g->C : g->phys), D.rings, set.btile, (uint8_t *)D.B, D.expo, g->d.jDim, sp.r0, g->nitems,
+            (int)g->d.iDim, (int)g->d.b_kDim, D.col_tiles_fwd};
+}
+static GemmDigitArgs gemm_args(const ss_grid *g, const DigitSet &set, const DigitSpan &sp, bool fwd) {
+    const DigitPlan &D = g->digit;
+    return {(const uint8_t *)(fwd ? D.Af : D.A), (const uint8_t *)D.B, set.items + sp.item0, sp.items, D.rings, D.expo,
+            fwd ? g->F : (D.H ? D.H : g->H), g->d.jDim, g->frows, g->nitems, (int)g->d.nvars, (int)g->d.b_kDim, (int)g->d.iDim, D.err};
+}
+static UnfoldArgs unfold_args(const ss_grid *g, const DigitSpan &sp) {
+    const DigitPlan &D = g->digit;
+    return {D.H ? D.H : g->H, g->rlz ? nullptr : g->phys, D.rings, D.expo, g->d.jDim, sp.r0, g->nitems, (int)g->d.nvars,
+            (int)g->d.b_kDim, (int)g->d.iDim};
+}
+static TurnArgs turn_args(const ss_grid *g, const DigitSpan &sp) {
+    const DigitPlan &D = g->digit;
+    return {(double *)g->F, D.rings, D.delta, D.cap, g->frows, sp.r0};
+}
+static int split_groups(const ss_grid *g) { return (g->nitems + kDigitGroup - 1) / kDigitGroup; }
+template <typename T>
+static size_t unfold_smem(const ss_grid *g, const DigitSpan &sp) { return (size_t)4 * (sp.r1 + g->pOL + 1) * sizeof(T); }
+
 template <typename T>
 static int32_t inverse(ss_grid *g, cudaStream_t st, const DigitSet &set, int *launches) {
     const DigitPlan &D = g->digit;
-    const ss_dims &d = g->d;
-    const int groups = (g->nitems + kDigitGroup - 1) / kDigitGroup;
     for (const DigitSpan &sp : set.spans) {
         const int nr = sp.r1 - sp.r0;
-        SplitArgs S{g->G, D.rings, set.btile, (uint8_t *)D.B, D.expo, D.delta, D.cap, g->frows, sp.r0, g->nitems, (int)d.iDim, D.col_tiles};
-        digit_split_kernel<T><<<dim3(groups, nr), 256, 0, st>>>(S);
-        GemmDigitArgs A{(const uint8_t *)D.A, (const uint8_t *)D.B, set.items + sp.item0, sp.items, D.rings, D.expo, D.H ? D.H : g->H,
-                        d.jDim, g->frows, g->nitems, (int)d.nvars, (int)d.b_kDim, (int)d.iDim, D.err};
-        digit_gemm_kernel<T, false><<<std::min(g->sms, sp.items), kDigitThreads, digit_smem<T>(), st>>>(A);
+        digit_split_kernel<T, false><<<dim3(split_groups(g), nr), 256, 0, st>>>(split_args(g, set, sp));
+        digit_gemm_kernel<T, false, false><<<std::min(g->sms, sp.items), kDigitThreads, digit_smem<T>(), st>>>(
+            gemm_args(g, set, sp, false));
         *launches += 2;
         CUDA_TRY(cudaGetLastError());
         if (D.columns.on || D.quads.blocks) continue;  // the column stage reads the parts
-        const size_t row = (size_t)4 * (sp.r1 + g->pOL + 1) * sizeof(T);
-        digit_unfold_kernel<T><<<dim3(DigitFormat<T>::kVars * g->nitems, nr), 128, row, st>>>(
-            D.H ? D.H : g->H, g->rlz ? nullptr : (T *)g->phys, D.rings, D.expo, sp.r0, g->nitems, (int)d.nvars,
-            (int)d.b_kDim, (int)d.iDim, d.jDim);
+        digit_unfold_kernel<T, false><<<dim3(DigitFormat<T>::kVars * g->nitems, nr), 128, unfold_smem<T>(g, sp), st>>>(unfold_args(g, sp));
         CUDA_TRY(cudaGetLastError());
         *launches += 1;
     }
@@ -949,23 +1059,127 @@ static int32_t inverse(ss_grid *g, cudaStream_t st, const DigitSet &set, int *la
 }
 
 int32_t digit_ring_forward(ss_grid *g, cudaStream_t st, int chunk, int *launches) {
-    const DigitPlan &D = g->digit;
-    const DigitSet &set = chunk < 0 ? D.whole_fwd : D.chunks_fwd[chunk];
-    const ss_dims &d = g->d;
-    const int groups = (g->nitems + kDigitGroup - 1) / kDigitGroup;
+    const DigitSet &set = chunk < 0 ? g->digit.whole_fwd : g->digit.chunks_fwd[chunk];
     for (const DigitSpan &sp : set.spans) {
         const int nr = sp.r1 - sp.r0;
-        FoldArgs S{(const double *)(g->rlz ? g->C : g->phys), D.rings, set.btile, (uint8_t *)D.B, D.expo, d.jDim, sp.r0, g->nitems, (int)d.iDim,
-                   (int)d.b_kDim, D.col_tiles_fwd};
-        digit_fold_kernel<<<dim3(groups, nr), 256, 0, st>>>(S);
-        GemmDigitArgs A{(const uint8_t *)D.Af, (const uint8_t *)D.B, set.items + sp.item0, sp.items, D.rings, D.expo, g->F,
-                        d.jDim, g->frows, g->nitems, (int)d.nvars, (int)d.b_kDim, (int)d.iDim, D.err};
-        digit_gemm_kernel<double, true><<<std::min(g->sms, sp.items), kDigitThreads, digit_smem<double>(), st>>>(A);
-        digit_turn_kernel<<<dim3(g->nitems, nr), 128, 0, st>>>((double *)g->F, D.rings, D.delta, D.cap, g->frows, sp.r0);
+        digit_fold_kernel<false><<<dim3(split_groups(g), nr), 256, 0, st>>>(fold_args(g, set, sp));
+        digit_gemm_kernel<double, true, false><<<std::min(g->sms, sp.items), kDigitThreads, digit_smem<double>(), st>>>(
+            gemm_args(g, set, sp, true));
+        digit_turn_kernel<false><<<dim3(g->nitems, nr), 128, 0, st>>>(turn_args(g, sp));
         CUDA_TRY(cudaGetLastError());
         *launches += 3;
     }
     return SS_OK;
+}
+
+// ---- joined
+bool digit_joins(const ss_grid *g) {
+    return g->digit.on && !g->rlz && g->tl == TL_F64 && g->digit.whole.spans.size() == 1 && g->digit.whole_fwd.spans.size() == 1;
+}
+
+// Grids whose common rings have the same matrices: same offset, and wavenumbers up to the
+// same cap wherever a ring reaches it
+static bool same_rings(const ss_grid *a, const ss_grid *b) {
+    const std::vector<DigitRing> &x = a->digit.ring_host, &y = b->digit.ring_host;
+    for (size_t i = 0; i < std::min(x.size(), y.size()); i++)
+        if (x[i].n != y[i].n || x[i].kmax != y[i].kmax) return false;
+    return true;
+}
+
+int32_t digit_join_plan(std::vector<ss_grid *> gs, std::vector<void *> &mem, std::vector<DigitJoined> &out) {
+    std::stable_sort(gs.begin(), gs.end(), [](const ss_grid *a, const ss_grid *b) { return a->d.iDim > b->d.iDim; });
+    auto alloc = [&](void **p, size_t bytes) -> int32_t {
+        CUDA_TRY(cudaMalloc(p, std::max<size_t>(bytes, 16)));
+        mem.push_back(*p);
+        return SS_OK;
+    };
+    auto put = [&](const auto &v, auto **dst) -> int32_t {
+        void *p = nullptr;
+        const int32_t rc = alloc(&p, v.size() * sizeof(v[0]));
+        if (rc) return rc;
+        *dst = (typename std::remove_reference<decltype(**dst)>::type *)p;
+        CUDA_TRY(cudaMemcpy(p, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice));
+        return SS_OK;
+    };
+    const int64_t most = kDigitScratchBytes / digit_b_bytes<double>();
+    while (!gs.empty()) {
+        const ss_grid *first = gs[0];  // most rings: its matrices serve the set
+        const std::vector<DigitRing> &rings = first->digit.ring_host;
+        const int nr = (int)rings.size();
+        std::vector<int> count(nr, 0);
+        auto tiles_of = [&](bool fwd) {
+            int64_t n = 0;
+            for (int r = 0; r < nr; r++) n += ring_tiles(rings[r], fwd ? forward_col_tiles(count[r]) : inverse_col_tiles<double>(count[r]), fwd);
+            return n;
+        };
+        std::vector<DigitItemRef> refs;
+        std::vector<ss_grid *> rest;
+        for (ss_grid *g : gs) {
+            for (int r = 0; r < g->d.iDim; r++) count[r] += g->nitems;
+            if (!refs.empty() && (!same_rings(first, g) || std::max(tiles_of(false), tiles_of(true)) > most)) {
+                for (int r = 0; r < g->d.iDim; r++) count[r] -= g->nitems;
+                rest.push_back(g);
+                continue;
+            }
+            for (int v = 0; v < g->nitems; v++)  // RL: items are variables
+                refs.push_back({(const double *)g->phys + v * g->d.jDim, (const double *)g->G + v * g->frows,
+                                (double *)g->F + v * g->frows, (double *)g->phys + v * g->d.jDim,
+                                (long long *)g->digit.H + v * g->d.jDim, g->nitems * g->frows, g->d.nvars * g->d.jDim,
+                                g->d.nvars * g->d.jDim, g->digit.err, g->digit.cap_host[v]});
+        }
+        DigitJoined J;
+        const DigitItemRef *dref = nullptr;
+        const int *dcount = nullptr;
+        int32_t rc = put(refs, &dref);
+        if (rc || (rc = put(count, &dcount))) return rc;
+        void *B = nullptr, *expo = nullptr;
+        if ((rc = alloc(&B, (size_t)std::max(tiles_of(false), tiles_of(true)) * digit_b_bytes<double>()))) return rc;
+        if ((rc = alloc(&expo, (size_t)kDigitVariants * refs.size() * nr * sizeof(int)))) return rc;
+        J.refs = dref; J.count = dcount; J.B = B; J.expo = (int *)expo;
+        J.owner = first; J.items = (int)refs.size();
+        for (int fwd = 0; fwd < 2; fwd++) {
+            std::vector<DigitItem> items;
+            std::vector<int64_t> btile(nr);
+            int64_t used = 0;
+            for (int r = nr - 1; r >= 0; r--) {  // longest products first: the CTAs take them in turn
+                const int tiles = fwd ? forward_col_tiles(count[r]) : inverse_col_tiles<double>(count[r]);
+                btile[r] = used;
+                ring_items(rings[r], r, tiles, fwd, used, items);
+                used += ring_tiles(rings[r], tiles, fwd);
+            }
+            if ((rc = put(items, &J.work[fwd])) || (rc = put(btile, &J.btile[fwd]))) return rc;
+            J.nwork[fwd] = (int)items.size();
+        }
+        CUDA_TRY(cudaFuncSetAttribute(digit_gemm_kernel<double, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digit_smem<double>()));
+        CUDA_TRY(cudaFuncSetAttribute(digit_gemm_kernel<double, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digit_smem<double>()));
+        out.push_back(J);
+        gs.swap(rest);
+    }
+    return SS_OK;
+}
+
+cudaError_t digit_join_launch(const DigitJoined &J, bool fwd, cudaStream_t st) {
+    const ss_grid *g = J.owner;
+    const DigitPlan &D = g->digit;
+    const DigitJoin join{(const DigitItemRef *)J.refs, J.count};
+    const int nr = (int)g->d.iDim, groups = (J.items + kDigitGroup - 1) / kDigitGroup;
+    const GemmDigitArgs A{(const uint8_t *)(fwd ? D.Af : D.A), (const uint8_t *)J.B, J.work[fwd], J.nwork[fwd], D.rings, J.expo, nullptr,
+                          0, 0, J.items, 0, 1, nr, D.err, join};
+    const int ctas = std::min(g->sms, J.nwork[fwd]);
+    if (fwd) {
+        const FoldArgs S{nullptr, D.rings, J.btile[1], (uint8_t *)J.B, J.expo, 0, 0, J.items, nr, 1, 0, join};
+        digit_fold_kernel<true><<<dim3(groups, nr), 256, 0, st>>>(S);
+        digit_gemm_kernel<double, true, true><<<ctas, kDigitThreads, digit_smem<double>(), st>>>(A);
+        digit_turn_kernel<true><<<dim3(J.items, nr), 128, 0, st>>>({nullptr, D.rings, D.delta, nullptr, 0, 0, join});
+    } else {
+        const SplitArgs S{nullptr, D.rings, J.btile[0], (uint8_t *)J.B, J.expo, D.delta, nullptr, 0, 0, J.items, nr, 0, join};
+        digit_split_kernel<double, true><<<dim3(groups, nr), 256, 0, st>>>(S);
+        digit_gemm_kernel<double, false, true><<<ctas, kDigitThreads, digit_smem<double>(), st>>>(A);
+        const size_t row = (size_t)4 * D.ring_host.back().n * sizeof(double);
+        digit_unfold_kernel<double, true><<<dim3(kDigitVariants * J.items, nr), 128, row, st>>>(
+            {nullptr, nullptr, D.rings, J.expo, 0, 0, J.items, 0, 1, nr, join});
+    }
+    return cudaGetLastError();
 }
 
 int32_t digit_ring_inverse(ss_grid *g, cudaStream_t st, int chunk, int *launches) {

@@ -132,6 +132,8 @@ struct DigitPlan {
     bool on = false;
     int col_tiles = 0, col_tiles_fwd = 0;
     DigitRing *rings = nullptr;
+    std::vector<DigitRing> ring_host;
+    std::vector<int> cap_host;
     void *A = nullptr;      // digit planes of the inverse DFT matrices
     void *Af = nullptr;     // and of the forward ones
     int *delta = nullptr;   // δ_k·2^70
@@ -153,6 +155,24 @@ int32_t digit_build(ss_grid *g, const std::vector<RingDesc> &rings);
 int32_t digit_ring_inverse(ss_grid *g, cudaStream_t st, int chunk, int *launches);
 // ring_forward likewise: C → F
 int32_t digit_ring_forward(ss_grid *g, cudaStream_t st, int chunk, int *launches);
+// The rings of many FP64 RL grids in three launches: rings of the same length share one product,
+// whose columns are the items of all grids that have it.  Bit for bit the single grids' results.
+struct DigitJoined {
+    const ss_grid *owner = nullptr;  // the grid of most rings, whose matrices serve
+    const void *refs = nullptr;
+    const int *count = nullptr;
+    void *B = nullptr;
+    int *expo = nullptr;
+    int items = 0;
+    const DigitItem *work[2] = {nullptr, nullptr};  // inverse, forward
+    const int64_t *btile[2] = {nullptr, nullptr};
+    int nwork[2] = {0, 0};
+};
+constexpr int kDigitJoinedLaunches = 3;
+bool digit_joins(const ss_grid *g);  // an RL grid whose rings are one span
+// sets of at most kDigitScratchBytes of digits; device memory goes to `mem`
+int32_t digit_join_plan(std::vector<ss_grid *> gs, std::vector<void *> &mem, std::vector<DigitJoined> &out);
+cudaError_t digit_join_launch(const DigitJoined &J, bool fwd, cudaStream_t st);
 void digit_free(ss_grid *g);
 // after a synchronisation: SS_DEVICE_TIMEOUT once if a bounded wait of the products gave up
 int32_t digit_status(ss_grid *g);

@@ -169,7 +169,7 @@ cudaError_t launch_sa_si(const SaLaunch &A, int nitems, size_t smem, cudaStream_
 size_t sa_band_smem(int b);
 constexpr size_t kSaBandSmemMax = 224 * 1024;
 template <typename T>
-cudaError_t launch_sa_band(const SaLaunch &A, int nitems, cudaStream_t st);
+cudaError_t launch_sa_band(const SaLaunch &A, int nitems, int sms, cudaStream_t st);
 template <typename T>
 cudaError_t launch_sa_band_fused(const SaLaunch *recs, const BatchWork *work, int nwork, size_t smem, cudaStream_t st);
 // binary32 grids beyond that: slot-parallel solve over the scratch arrays X, Y, each

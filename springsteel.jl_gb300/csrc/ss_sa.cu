@@ -212,7 +212,8 @@ template <typename T>
 __global__ void __launch_bounds__(kSaWarps * 32) sa_band_kernel(SaLaunch A) {
     sa_band_body<T, T>(A, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.z);
 }
-// fused multi-grid launch: CTA blockIdx.x runs work[blockIdx.x]; the record is staged in shared memory
+// fused multi-grid launch: CTA blockIdx.x runs work[blockIdx.x] (bz: part << 8 | parts); the record is
+// staged in shared memory
 template <typename T>
 __global__ void __launch_bounds__(kSaWarps * 32) sa_band_fused_kernel(const SaLaunch *recs, const BatchWork *work) {
     __shared__ __align__(16) SaLaunch A;
@@ -220,13 +221,13 @@ __global__ void __launch_bounds__(kSaWarps * 32) sa_band_fused_kernel(const SaLa
     for (int i = threadIdx.x; i < (int)(sizeof(SaLaunch) / 4); i += blockDim.x)
         reinterpret_cast<int *>(&A)[i] = __ldg(reinterpret_cast<const int *>(recs + w.rec) + i);
     __syncthreads();
-    sa_band_body<T, T>(A, w.bx, w.by, 0, 1);
+    sa_band_body<T, T>(A, w.bx, w.by, w.bz >> 8, w.bz & 255);
 }
 
 size_t sa_band_smem(int b) { return (size_t)b * kSaLd * sizeof(double); }
 
 template <typename T>
-cudaError_t launch_sa_band(const SaLaunch &A, int nitems, cudaStream_t st) {
+cudaError_t launch_sa_band(const SaLaunch &A, int nitems, int sms, cudaStream_t st) {
     const size_t smem = sa_band_smem(A.b);
     // the process's attribute: one value for all grids, so that launches of other threads never lower it
     const cudaError_t e = cudaFuncSetAttribute(sa_band_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSaBandSmemMax);
@@ -234,7 +235,7 @@ cudaError_t launch_sa_band(const SaLaunch &A, int nitems, cudaStream_t st) {
     // few CTAs: every one solves its slots again for a part of the rings only, so that
     // the evaluation (12 FP64 operations per slot and ring) spreads over idle SMs
     const int ctas = (A.nslots_z + 31) / 32 * nitems;
-    const int parts = std::max(1, std::min({8, 304 / ctas, (A.iDim + 31) / 32}));
+    const int parts = std::max(1, std::min({8, 2 * sms / ctas, (A.iDim + 31) / 32}));
     sa_band_kernel<T><<<dim3((A.nslots_z + 31) / 32, nitems, parts), kSaWarps * 32, smem, st>>>(A);
     return cudaGetLastError();
 }
@@ -247,8 +248,8 @@ cudaError_t launch_sa_band_fused(const SaLaunch *recs, const BatchWork *work, in
     sa_band_fused_kernel<T><<<nwork, kSaWarps * 32, smem, st>>>(recs, work);
     return cudaGetLastError();
 }
-template cudaError_t launch_sa_band<double>(const SaLaunch &, int, cudaStream_t);
-template cudaError_t launch_sa_band<float>(const SaLaunch &, int, cudaStream_t);
+template cudaError_t launch_sa_band<double>(const SaLaunch &, int, int, cudaStream_t);
+template cudaError_t launch_sa_band<float>(const SaLaunch &, int, int, cudaStream_t);
 template cudaError_t launch_sa_band_fused<double>(const SaLaunch *, const BatchWork *, int, size_t, cudaStream_t);
 template cudaError_t launch_sa_band_fused<float>(const SaLaunch *, const BatchWork *, int, size_t, cudaStream_t);
 
