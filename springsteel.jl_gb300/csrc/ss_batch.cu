@@ -63,6 +63,14 @@ static std::vector<uint64_t> generations(const ss_batch *bt) {
     return out;
 }
 
+// the batch's grids, each once: a grid's buffers serve one sequence of launches at a time
+static std::vector<ss_grid *> distinct(const ss_batch *bt) {
+    std::vector<ss_grid *> out;
+    for (ss_grid *g : bt->grids)
+        if (std::find(out.begin(), out.end(), g) == out.end()) out.push_back(g);
+    return out;
+}
+
 static int32_t run_direction(ss_grid *g, int what, cudaStream_t st) {
     int32_t r = SS_OK;
     if (what & 1) r = grid_forward(g, st);
@@ -320,9 +328,9 @@ static int32_t build_fused(ss_batch *bt) {
     free_fused(bt);
     auto own = [](const ss_grid *g) { return g->rlz || (g->digit.on && !digit_joins(g)); };
     for (int tl : {TL_F64, TL_DF64, TL_F32}) {
-        std::vector<ss_grid *> gs, fft, digits;  // each grid once: the digit products' last step is in place
-        for (ss_grid *g : bt->grids) {
-            if (own(g) || g->tl != tl || std::find(gs.begin(), gs.end(), g) != gs.end()) continue;
+        std::vector<ss_grid *> gs, fft, digits;
+        for (ss_grid *g : distinct(bt)) {
+            if (own(g) || g->tl != tl) continue;
             gs.push_back(g);
             (digit_joins(g) ? digits : fft).push_back(g);
         }
@@ -338,7 +346,7 @@ static int32_t build_fused(ss_batch *bt) {
         for (const DigitJoined &J : joined) bt->inv.push_back({FK_DIGIT, tl, 0, 0, 0, nullptr, nullptr, J});
         if (rc) { free_fused(bt); return rc; }
     }
-    for (ss_grid *g : bt->grids)
+    for (ss_grid *g : distinct(bt))
         if (own(g)) bt->unfused.push_back(g);
     bt->fused_gen = generations(bt);
     return SS_OK;
@@ -487,8 +495,9 @@ static int32_t enqueue_batch(ss_batch *bt, int what, cudaStream_t st) {
     const int nside = (int)bt->side.size();
     CUDA_TRY(cudaEventRecord(bt->ev[0], st));
     for (int i = 0; i < nside; i++) CUDA_TRY(cudaStreamWaitEvent(bt->side[i], bt->ev[0], 0));
-    for (size_t i = 0; i < bt->grids.size(); i++) {
-        int32_t r = run_direction(bt->grids[i], what, bt->side[i % nside]);
+    const std::vector<ss_grid *> gs = distinct(bt);
+    for (size_t i = 0; i < gs.size(); i++) {
+        int32_t r = run_direction(gs[i], what, bt->side[i % nside]);
         if (r) return r;
     }
     for (int i = 0; i < nside; i++) {

@@ -16,7 +16,7 @@ def _grid(cells, nvars, precision="f64", levels=0, kmax=-1):
         vars={"v%d" % i: i + 1 for i in range(nvars)}, max_wavenumber={"default": kmax}, **kw))
 
 
-def _run(grids, order=None):
+def _run(grids, order=None, fused=True):
     """(own calls, batch) of every grid."""
     fields = [np.random.default_rng(i).standard_normal((g.dims["n_physical"], g.dims["nvars"])) for i, g in enumerate(grids)]
     own = []
@@ -25,7 +25,7 @@ def _run(grids, order=None):
         S.spectralTransform_b(g)
         S.gridTransform_b(g)
         own.append((g.get_spectral(), g.get_physical()))
-    batch = S.Batch([grids[i] for i in order] if order else grids, autotune=False, fused=True)
+    batch = S.Batch([grids[i] for i in order] if order else grids, autotune=False, fused=fused)
     launches = batch.fused_launches(3)
     got = []
     for use_graph in (False, True):
@@ -59,5 +59,7 @@ def test_beside_grids_of_other_kinds():
     assert _run(grids) > 0
 
 
-def test_a_grid_listed_twice():
-    _run([_grid(10, 1), _grid(16, 2)], order=[0, 1, 0])
+@pytest.mark.parametrize("fused", [True, False])
+def test_a_grid_listed_twice(fused):
+    """Once a run, like any other: two streams of one grid would share its digit buffers."""
+    _run([_grid(10, 1), _grid(16, 2), _grid(5, 1, levels=12)], order=[0, 1, 2, 0, 2], fused=fused)
