@@ -43,6 +43,8 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
+#include <utility>
 
 #include "ss_digit.h"
 #include "ss_digit_dev.cuh"
@@ -792,14 +794,49 @@ constexpr int64_t kDigitScratchBytes = (int64_t)1 << 30;
 template <typename T>
 constexpr size_t digit_smem() { return (size_t)DigitFormat<T>::kStages * (digit_a_bytes<T>() + digit_b_bytes<T>()); }
 
-template <typename V>
-static bool upload(ss_grid *g, const V **dst, const std::vector<V> &src) {
-    void *p = nullptr;
-    if (cudaMalloc(&p, std::max<size_t>(src.size() * sizeof(V), 16)) != cudaSuccess) { cudaGetLastError(); return false; }
-    g->allocs.push_back(p);
-    if (!src.empty() && cudaMemcpy(p, src.data(), src.size() * sizeof(V), cudaMemcpyHostToDevice) != cudaSuccess) return false;
-    *dst = (const V *)p;
-    return true;
+// Timed-out-wait flags, host memory that the kernels write: mapping a page takes 0.11 ms and giving
+// it back 0.17, a quarter of creating a small grid, so the grids of the process share pages; a
+// page goes with its last flag.
+namespace {
+struct FlagPage {
+    int *base;
+    std::vector<char> used;
+    int live;
+};
+constexpr int kFlags = 512;
+std::mutex flag_mutex;
+std::vector<FlagPage> flag_pages;
+}  // namespace
+static int *take_flag() {
+    std::lock_guard<std::mutex> lock(flag_mutex);
+    auto page = std::find_if(flag_pages.begin(), flag_pages.end(), [](const FlagPage &p) { return p.live < kFlags; });
+    if (page == flag_pages.end()) {
+        int *base = nullptr;
+        if (cudaHostAlloc((void **)&base, kFlags * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        flag_pages.push_back({base, std::vector<char>(kFlags, 0), 0});
+        page = flag_pages.end() - 1;
+    }
+    const int i = (int)(std::find(page->used.begin(), page->used.end(), 0) - page->used.begin());
+    page->used[i] = 1;
+    page->live++;
+    page->base[i] = 0;
+    return page->base + i;
+}
+static void give_flag(int *flag) {
+    std::lock_guard<std::mutex> lock(flag_mutex);
+    for (size_t k = 0; k < flag_pages.size(); k++) {
+        FlagPage &p = flag_pages[k];
+        if (flag < p.base || flag >= p.base + kFlags) continue;
+        p.used[flag - p.base] = 0;
+        if (--p.live == 0) {
+            cudaFreeHost(p.base);
+            flag_pages.erase(flag_pages.begin() + k);
+        }
+        return;
+    }
 }
 
 // B tiles of a ring, and its tile products with the first B tile at `used`
@@ -879,11 +916,11 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
     constexpr bool kBoth = std::is_same<T, double>::value;  // binary32 grids keep the forward FFT's rounding
     const size_t abytes = (size_t)atiles * digit_a_bytes<T>(), afbytes = kBoth ? (size_t)aftiles * digit_a_bytes<T>() : 0;
     if (abytes + afbytes > (g->rlz ? kDigitTableBytes : kDigitTableBytesRl)) return SS_OK;
-    long long *cosq = nullptr;
+    DigitBlock blk;
     const size_t mark = g->allocs.size();
     auto give_up = [&]() {  // the device has no room for the tables: the FFT kernels serve
         cudaGetLastError();
-        if (cosq) cudaFree(cosq);
+        if (D.err) give_flag(D.err);
         while (g->allocs.size() > mark) { cudaFree(g->allocs.back()); g->allocs.pop_back(); }
         D = DigitPlan{};
         return SS_OK;
@@ -912,45 +949,28 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
             btiles = std::max(btiles, used);
             set.spans.push_back(sp);
         }
-        return upload(g, &set.items, items) && upload(g, &set.btile, btile);
+        blk.put(&set.items, items);
+        blk.put(&set.btile, btile);
     };
-    const DigitRing *dr = nullptr;
-    if (!upload(g, &dr, rings)) return give_up();
-    D.rings = const_cast<DigitRing *>(dr);
+    blk.put(&D.rings, rings);
     D.ring_host = rings;
-    const int *dd = nullptr;
-    if (!upload(g, &dd, delta)) return give_up();
-    D.delta = const_cast<int *>(dd);
+    blk.put(&D.delta, delta);
     std::vector<int> cap(g->nitems);
     for (int i = 0; i < g->nitems; i++) {
         const int km = g->rlz ? g->ring_kmax : g->kmaxv[i];
         cap[i] = km >= 0 ? km : rd[nr - 1].ri;
     }
-    if (!upload(g, &dd, cap)) return give_up();
-    D.cap = const_cast<int *>(dd);
+    blk.put(&D.cap, cap);
     D.cap_host = cap;
-    if (!make_set(0, nr, false, D.whole) || (kBoth && !make_set(0, nr, true, D.whole_fwd))) return give_up();
-    D.chunks.resize(g->chunk_r0.size() - 1);
-    D.chunks_fwd.resize(g->chunk_r0.size() - 1);
-    for (size_t c = 0; c + 1 < g->chunk_r0.size(); c++)
-        if (!make_set(g->chunk_r0[c], g->chunk_r0[c + 1], false, D.chunks[c]) ||
-            (kBoth && !make_set(g->chunk_r0[c], g->chunk_r0[c + 1], true, D.chunks_fwd[c])))
-            return give_up();
-    void *p = nullptr;
-    if (kBoth) {
-        if (cudaMalloc(&p, afbytes) != cudaSuccess) return give_up();
-        g->allocs.push_back(p);
-        D.Af = p;
+    make_set(0, nr, false, D.whole);
+    if (kBoth) make_set(0, nr, true, D.whole_fwd);
+    const size_t nchunk = g->chunk_r0.size() - 1;
+    D.chunks.resize(nchunk);
+    D.chunks_fwd.resize(nchunk);
+    for (size_t c = 0; c < nchunk && nchunk > 1; c++) {
+        make_set(g->chunk_r0[c], g->chunk_r0[c + 1], false, D.chunks[c]);
+        if (kBoth) make_set(g->chunk_r0[c], g->chunk_r0[c + 1], true, D.chunks_fwd[c]);
     }
-    if (cudaMalloc(&p, abytes) != cudaSuccess) return give_up();
-    g->allocs.push_back(p);
-    D.A = p;
-    if (cudaMalloc(&p, (size_t)btiles * digit_b_bytes<T>()) != cudaSuccess) return give_up();
-    g->allocs.push_back(p);
-    D.B = p;
-    if (cudaMalloc(&p, (size_t)kDigitVariants * g->nitems * nr * sizeof(int)) != cudaSuccess) return give_up();
-    g->allocs.push_back(p);
-    D.expo = (int *)p;
     if (g->tl == TL_F32 && cheb_inverse_takes_quads((int)g->d.kDim, (int)g->d.b_kDim)) {
         std::vector<int2> blocks;
         D.quads.first.assign(1, 0);
@@ -958,25 +978,29 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
             for (int m = 0; m < rings[r].n; m += 16) blocks.push_back(make_int2(r, m));
             D.quads.first.push_back((int)blocks.size());
         }
-        const int2 *qb = nullptr;
-        if (!upload(g, &qb, blocks)) return give_up();
-        D.quads.blocks = const_cast<int2 *>(qb);
+        blk.put(&D.quads.blocks, blocks);
     }
-    if (!g->rlz) {  // quadrant parts (RLZ grids keep them in the ring outputs' buffer)
-        if (cudaMalloc(&p, (size_t)kDigitVariants * g->nitems * g->d.jDim * sizeof(T)) != cudaSuccess) return give_up();
-        g->allocs.push_back(p);
-        D.H = p;
+    blk.room((void **)&D.expo, (size_t)kDigitVariants * g->nitems * nr * sizeof(int));
+    blk.room(&D.B, std::max((size_t)btiles * digit_b_bytes<T>(), (size_t)cosn * 8));
+    // quadrant parts (RLZ grids keep them in the ring outputs' buffer)
+    if (!g->rlz) blk.room(&D.H, (size_t)kDigitVariants * g->nitems * g->d.jDim * sizeof(T));
+    if (!blk.build(g->allocs)) return give_up();
+    if (nchunk == 1) {  // the only chunk is the grid
+        D.chunks[0] = D.whole;
+        D.chunks_fwd[0] = D.whole_fwd;
     }
-    if (cudaMalloc((void **)&cosq, (size_t)cosn * 8) != cudaSuccess) return give_up();
-    if (cudaHostAlloc((void **)&D.err, sizeof(int), cudaHostAllocMapped) != cudaSuccess) { D.err = nullptr; return give_up(); }
-    *D.err = 0;
+    void *p = nullptr;
+    if (cudaMalloc(&p, abytes + afbytes) != cudaSuccess) return give_up();  // whole tiles: Af is aligned
+    g->allocs.push_back(p);
+    D.A = p;
+    if (kBoth) D.Af = (uint8_t *)p + abytes;
+    if (!(D.err = take_flag())) return give_up();
+    long long *cosq = (long long *)D.B;  // scratch until the first transform
     digit_cos_kernel<<<nr, 128, 0, g->stream>>>(D.rings, cosq);
     digit_matrix_kernel<T, false><<<dim3(nr, 8), 256, 0, g->stream>>>(D.rings, cosq, (uint8_t *)D.A);
     if constexpr (kBoth) digit_matrix_kernel<T, true><<<dim3(nr, 8), 256, 0, g->stream>>>(D.rings, cosq, (uint8_t *)D.Af);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-    cudaFree(cosq);
-    cosq = nullptr;
     CUDA_TRY(e);
     CUDA_TRY(cudaFuncSetAttribute(digit_gemm_kernel<T, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digit_smem<T>()));
     if constexpr (kBoth)
@@ -1000,7 +1024,7 @@ int32_t digit_build(ss_grid *g, const std::vector<RingDesc> &rings) {
 }
 
 void digit_free(ss_grid *g) {
-    if (g->digit.err) cudaFreeHost(g->digit.err);
+    if (g->digit.err) give_flag(g->digit.err);
     g->digit.err = nullptr;
 }
 

@@ -4,7 +4,10 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
+#include <cstring>
+#include <utility>
 #include <vector>
 
 #include "ss_internal.h"
@@ -110,34 +113,34 @@ struct DigitSet {
 struct DigitColumns {
     bool on = false;
     int steps = 0, zblocks = 0, buffers = 1, raws = 1;
-    void *M = nullptr;
-    int *mexpo = nullptr;
-    int *weight = nullptr;           // mode exponents taken from the matrices' columns into the data
-    int2 *blocks = nullptr;
+    const uint8_t *M = nullptr;
+    const int *mexpo = nullptr;
+    const int *weight = nullptr;           // mode exponents taken from the matrices' columns into the data
+    const int2 *blocks = nullptr;
     std::vector<int> first;          // first block of every ring, their number at the end
     bool fon = false;                // forward (binary64): K-steps of levels, blocks of 32 modes, lanes of a column
     int fsteps = 0, fblocks = 0, fgroup = 4;
-    void *fM = nullptr;
-    int *fexpo = nullptr;
+    const uint8_t *fM = nullptr;
+    const int *fexpo = nullptr;
 };
 
 // Binary32 column stage: 16-position blocks of the quadrants (ring, first position) and
 // the first block of every ring
 struct QuadBlocks {
-    int2 *blocks = nullptr;
+    const int2 *blocks = nullptr;
     std::vector<int> first;
 };
 
 struct DigitPlan {
     bool on = false;
     int col_tiles = 0, col_tiles_fwd = 0;
-    DigitRing *rings = nullptr;
+    const DigitRing *rings = nullptr;
     std::vector<DigitRing> ring_host;
     std::vector<int> cap_host;
     void *A = nullptr;      // digit planes of the inverse DFT matrices
     void *Af = nullptr;     // and of the forward ones
-    int *delta = nullptr;   // δ_k·2^70
-    int *cap = nullptr;     // per item: its variable's kmax
+    const int *delta = nullptr;   // δ_k·2^70
+    const int *cap = nullptr;     // per item: its variable's kmax
     void *H = nullptr;      // RL: quadrant parts
     void *B = nullptr;      // digit planes of one span's ring spectra
     int *expo = nullptr;    // [variant][item][ring] column exponents
@@ -148,7 +151,36 @@ struct DigitPlan {
     QuadBlocks quads;       // binary32: the column stage reads the parts
 };
 
-// Builds the plan of an RLZ grid (tables included); a grid the rule leaves to
+// The device arrays of one plan in one allocation: host arrays are appended, then the plan's
+// other buffers, and every pointer is set once the block is there (an allocation takes 35 µs, a
+// copy 8; a small grid's plan had 17 of each)
+struct DigitBlock {
+    std::vector<unsigned char> host;
+    size_t bytes = 0;
+    std::vector<std::pair<void **, size_t>> at;
+    size_t place(size_t n, size_t align = 256) {
+        const size_t o = (bytes + align - 1) / align * align;
+        bytes = o + std::max<size_t>(n, 16);
+        return o;
+    }
+    template <typename V>
+    void put(const V **dst, const std::vector<V> &src) {
+        const size_t o = place(src.size() * sizeof(V));
+        host.resize(bytes);
+        if (!src.empty()) std::memcpy(host.data() + o, src.data(), src.size() * sizeof(V));
+        at.push_back({(void **)dst, o});
+    }
+    void room(void **dst, size_t n) { at.push_back({dst, place(n, 1024)}); }
+    bool build(std::vector<void *> &allocs) {
+        void *p = nullptr;
+        if (cudaMalloc(&p, bytes) != cudaSuccess) { cudaGetLastError(); return false; }
+        allocs.push_back(p);
+        for (const auto &q : at) *q.first = (char *)p + q.second;
+        return cudaMemcpy(p, host.data(), host.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+    }
+};
+
+// Builds the plan of a grid (tables included); a grid the rule leaves to
 // the FFT kernels, or whose tables do not fit the device, keeps on = false.
 int32_t digit_build(ss_grid *g, const std::vector<RingDesc> &rings);
 // ring_inverse of every ring (chunk < 0) or of one radial chunk: G → H

@@ -620,6 +620,11 @@ static int32_t build_forward(ss_grid *g, const std::vector<ChebHost> &cheb) {
     std::vector<int> E((size_t)nv * Q.fblocks * kZ, 0);
     for (int v = 0; v < nv; v++) {
         const ChebHost &c = cheb[v];
+        if (v > 0) {  // the forward matrix knows no ends: one for all variables
+            std::copy_n(M.begin(), (size_t)Q.fblocks * job, M.begin() + (size_t)v * Q.fblocks * job);
+            std::copy_n(E.begin(), (size_t)Q.fblocks * kZ, E.begin() + (size_t)v * Q.fblocks * kZ);
+            continue;
+        }
         for (int k = 0; k < bk; k++) {
             std::vector<double> row(N, 0.0);
             double top = 0.0;
@@ -645,14 +650,10 @@ static int32_t build_forward(ss_grid *g, const std::vector<ChebHost> &cheb) {
             }
         }
     }
-    void *pm = nullptr, *pe = nullptr;
-    auto put = [&](const void *src, size_t bytes, void **dst) {
-        if (cudaMalloc(dst, bytes) != cudaSuccess) { cudaGetLastError(); return false; }
-        g->allocs.push_back(*dst);
-        return cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
-    };
-    if (!put(M.data(), M.size(), &pm) || !put(E.data(), E.size() * 4, &pe)) return SS_OK;
-    Q.fM = pm; Q.fexpo = (int *)pe;
+    DigitBlock blk;
+    blk.put(&Q.fM, M);
+    blk.put(&Q.fexpo, E);
+    if (!blk.build(g->allocs)) return SS_OK;
     CUDA_TRY(cudaFuncSetAttribute(digit_columns_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColumnSmem));
     Q.fon = true;
     return SS_OK;
@@ -676,6 +677,15 @@ static int32_t build_inverse(ss_grid *g, const std::vector<ChebHost> &cheb) {
     std::vector<int> E((size_t)nv * 3 * Q.zblocks * kZ, 0), W((size_t)nv * 3 * bk, kUnseen);
     for (int v = 0; v < nv; v++) {
         const ChebHost &c = cheb[v];
+        int like = 0;  // the first variable with the same ends
+        while (g->bcb[like] != g->bcb[v] || g->bct[like] != g->bct[v]) like++;
+        if (like < v) {
+            const size_t m = (size_t)3 * Q.zblocks * job, e = (size_t)3 * Q.zblocks * kZ, w = (size_t)3 * bk;
+            std::copy_n(M.begin() + like * m, m, M.begin() + v * m);
+            std::copy_n(E.begin() + like * e, e, E.begin() + v * e);
+            std::copy_n(W.begin() + like * w, w, W.begin() + v * w);
+            continue;
+        }
         const int ne = (N + 1) / 2, no = std::max(N / 2, 1);
         std::vector<double> X((size_t)N * bk, 0.0), Y((size_t)N * bk);
         for (int k = 0; k < N; k++)
@@ -743,16 +753,12 @@ static int32_t build_inverse(ss_grid *g, const std::vector<ChebHost> &cheb) {
         for (int m = 0; m < n; m += 32) blocks.push_back(make_int2(r, m));
         Q.first.push_back((int)blocks.size());
     }
-    auto put = [&](const void *src, size_t bytes, void **dst) {
-        if (cudaMalloc(dst, std::max<size_t>(bytes, 16)) != cudaSuccess) { cudaGetLastError(); return false; }
-        g->allocs.push_back(*dst);
-        return cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
-    };
-    void *pm = nullptr, *pe = nullptr, *pw = nullptr, *pb = nullptr;
-    if (!put(M.data(), M.size(), &pm) || !put(E.data(), E.size() * 4, &pe) || !put(W.data(), W.size() * 4, &pw) ||
-        !put(blocks.data(), blocks.size() * 8, &pb))
-        return SS_OK;
-    Q.M = pm; Q.mexpo = (int *)pe; Q.weight = (int *)pw; Q.blocks = (int2 *)pb;
+    DigitBlock blk;
+    blk.put(&Q.M, M);
+    blk.put(&Q.mexpo, E);
+    blk.put(&Q.weight, W);
+    blk.put(&Q.blocks, blocks);
+    if (!blk.build(g->allocs)) return SS_OK;
     CUDA_TRY(cudaFuncSetAttribute(Q.steps <= 2 ? digit_columns_kernel<true> : digit_columns_kernel<false>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColumnSmem));
     Q.on = true;
@@ -771,7 +777,7 @@ int32_t digit_columns_forward(ss_grid *g, cudaStream_t st, int64_t col0, int64_t
     const ss_dims &d = g->d;
     ForwardColumnArgs A{};
     A.phys = (const double *)g->phys; A.C = (double *)g->C; A.rings = g->d_rings; A.col_ring = g->d_col_ring;
-    A.M = (const uint8_t *)Q.fM; A.mexpo = Q.fexpo; A.col0 = col0; A.col1 = col1; A.np = d.n_physical; A.jDim = d.jDim;
+    A.M = Q.fM; A.mexpo = Q.fexpo; A.col0 = col0; A.col1 = col1; A.np = d.n_physical; A.jDim = d.jDim;
     A.N = (int)d.kDim; A.bk = (int)d.b_kDim; A.steps = Q.fsteps; A.blocks = Q.fblocks; A.group = Q.fgroup; A.err = g->digit.err;
     const int64_t tiles = (col1 - col0 + 127) / 128;
     const int per = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, g->sms / (int)d.nvars));
@@ -787,7 +793,7 @@ int32_t digit_columns_inverse(ss_grid *g, cudaStream_t st, int chunk) {
     const int r0 = chunk < 0 ? 0 : g->chunk_r0[chunk], r1 = chunk < 0 ? (int)d.iDim : g->chunk_r0[chunk + 1];
     ColumnArgs A{};
     A.H = g->H; A.phys = (double *)g->phys; A.rings = P.rings; A.expo = P.expo;
-    A.M = (const uint8_t *)Q.M; A.mexpo = Q.mexpo; A.weight = Q.weight; A.blocks = Q.blocks + Q.first[r0]; A.nblocks = Q.first[r1] - Q.first[r0];
+    A.M = Q.M; A.mexpo = Q.mexpo; A.weight = Q.weight; A.blocks = Q.blocks + Q.first[r0]; A.nblocks = Q.first[r1] - Q.first[r0];
     A.N = (int)d.kDim; A.bk = (int)d.b_kDim; A.nvars = (int)d.nvars; A.nitems = g->nitems; A.iDim = (int)d.iDim;
     A.steps = Q.steps; A.zblocks = Q.zblocks; A.buffers = Q.buffers; A.raws = Q.raws; A.jDim = d.jDim; A.np = d.n_physical; A.err = P.err;
     const int per = std::max(1, std::min(A.nblocks, g->sms / (int)d.nvars));
