@@ -43,6 +43,9 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <iterator>
+#include <map>
+#include <memory>
 #include <mutex>
 #include <utility>
 
@@ -785,6 +788,9 @@ constexpr int64_t kDigitMinPointsF32 = 3500000;
 // bound of a grid's matrix digits (both directions: 4.3 GB at 200 cells, growing with
 // the cube of the ring count); larger grids keep the FFT kernels
 constexpr size_t kDigitTableBytes = (size_t)16 << 30;
+// Tables above this many bytes are built while they take at most a quarter of the device's free
+// memory, so that grids created later find room
+constexpr size_t kDigitAskBytes = (size_t)256 << 20;
 // RL grids hold far less data than these matrices (0.6 GB at 100 cells): up to about
 // 120 cells.  100 cells, one variable: ring_inverse 1.07 → 0.13 ms, ring_forward
 // 0.26 → 0.13 ms; 24 cells: 0.32 → 0.03 and 0.095 → 0.03 ms
@@ -838,6 +844,19 @@ static void give_flag(int *flag) {
         return;
     }
 }
+
+// The matrix digits depend on the ring lengths and wavenumbers alone: grids of the same rings on a device
+// share them (4.2 GB for 200 cells, 0.6 for an RL grid of 100).  They go with the last such grid.
+struct DigitTables {
+    void *A = nullptr;
+    ~DigitTables() {
+        if (A) cudaFree(A);
+    }
+};
+namespace {
+std::mutex table_mutex;
+std::map<std::vector<int>, std::weak_ptr<DigitTables>> tables;
+}  // namespace
 
 // B tiles of a ring, and its tile products with the first B tile at `used`
 static int64_t ring_tiles(const DigitRing &q, int tiles, bool fwd) { return (int64_t)tiles * (fwd ? 4 * q.tm : 2 * (q.te + q.to)); }
@@ -989,19 +1008,34 @@ static int32_t build(ss_grid *g, const std::vector<RingDesc> &rd) {
         D.chunks[0] = D.whole;
         D.chunks_fwd[0] = D.whole_fwd;
     }
-    void *p = nullptr;
-    if (cudaMalloc(&p, abytes + afbytes) != cudaSuccess) return give_up();  // whole tiles: Af is aligned
-    g->allocs.push_back(p);
-    D.A = p;
-    if (kBoth) D.Af = (uint8_t *)p + abytes;
     if (!(D.err = take_flag())) return give_up();
-    long long *cosq = (long long *)D.B;  // scratch until the first transform
-    digit_cos_kernel<<<nr, 128, 0, g->stream>>>(D.rings, cosq);
-    digit_matrix_kernel<T, false><<<dim3(nr, 8), 256, 0, g->stream>>>(D.rings, cosq, (uint8_t *)D.A);
-    if constexpr (kBoth) digit_matrix_kernel<T, true><<<dim3(nr, 8), 256, 0, g->stream>>>(D.rings, cosq, (uint8_t *)D.Af);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-    CUDA_TRY(e);
+    std::vector<int> key{g->device, g->tl};
+    for (const DigitRing &r : rings) {
+        key.push_back(r.n);
+        key.push_back(r.kmax);
+    }
+    std::lock_guard<std::mutex> lock(table_mutex);  // of two threads one builds, the other finds them complete
+    for (auto it = tables.begin(); it != tables.end();) it = it->second.expired() ? tables.erase(it) : std::next(it);
+    if (const auto found = tables.find(key); found != tables.end()) D.tables = found->second.lock();
+    if (!D.tables) {
+        size_t left = 0, total = 0;
+        if (abytes + afbytes > kDigitAskBytes &&
+            (cudaMemGetInfo(&left, &total) != cudaSuccess || abytes + afbytes > left / 4))
+            return give_up();
+        auto t = std::make_shared<DigitTables>();
+        if (cudaMalloc(&t->A, abytes + afbytes) != cudaSuccess) { t->A = nullptr; return give_up(); }
+        long long *cosq = (long long *)D.B;  // scratch until the first transform
+        uint8_t *A = (uint8_t *)t->A;        // whole tiles: Af is aligned
+        digit_cos_kernel<<<nr, 128, 0, g->stream>>>(D.rings, cosq);
+        digit_matrix_kernel<T, false><<<dim3(nr, 8), 256, 0, g->stream>>>(D.rings, cosq, A);
+        if constexpr (kBoth) digit_matrix_kernel<T, true><<<dim3(nr, 8), 256, 0, g->stream>>>(D.rings, cosq, A + abytes);
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(cudaStreamSynchronize(g->stream));
+        D.tables = t;
+        tables[key] = t;
+    }
+    D.A = D.tables->A;
+    if (kBoth) D.Af = (uint8_t *)D.A + abytes;
     CUDA_TRY(cudaFuncSetAttribute(digit_gemm_kernel<T, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digit_smem<T>()));
     if constexpr (kBoth)
         CUDA_TRY(cudaFuncSetAttribute(digit_gemm_kernel<T, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digit_smem<T>()));
@@ -1026,6 +1060,7 @@ int32_t digit_build(ss_grid *g, const std::vector<RingDesc> &rings) {
 void digit_free(ss_grid *g) {
     if (g->digit.err) give_flag(g->digit.err);
     g->digit.err = nullptr;
+    g->digit.tables.reset();
 }
 
 int32_t digit_status(ss_grid *g) {

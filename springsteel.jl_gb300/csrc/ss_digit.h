@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <memory>
 #include <utility>
 #include <vector>
 
@@ -15,6 +16,8 @@
 struct ss_grid;
 
 namespace ss {
+
+struct DigitTables;
 
 // Digit formats.  A binary64 column scaled into (-1, 1) is 54-bit fixed point (a
 // matrix entry 53-bit): a leading digit of at most 512 (256) and five balanced
@@ -137,6 +140,7 @@ struct DigitPlan {
     const DigitRing *rings = nullptr;
     std::vector<DigitRing> ring_host;
     std::vector<int> cap_host;
+    std::shared_ptr<DigitTables> tables;  // hold A and Af
     void *A = nullptr;      // digit planes of the inverse DFT matrices
     void *Af = nullptr;     // and of the forward ones
     const int *delta = nullptr;   // δ_k·2^70
