@@ -265,6 +265,8 @@ int32_t ss_grid_save(ss_grid *g, const char *path, const void *user, int64_t use
         set_error("reading the filter weights: %s", cudaGetErrorString(cudaGetLastError()));
         return SS_CUDA_ERROR;
     }
+    int32_t rc = digit_status(g);  // before the file is touched: incomplete arrays make no archive
+    if (rc) return rc;
     const std::vector<unsigned char> rec = param_record(g, fw, cw);
     FileCloser fc{fopen(path, "wb")};
     if (!fc.f) {
@@ -278,8 +280,7 @@ int32_t ss_grid_save(ss_grid *g, const char *path, const void *user, int64_t use
         return SS_BAD_ARG;
     }
     Staging sg;
-    int32_t rc = sg.init();
-    if (rc) return rc;
+    if ((rc = sg.init())) return rc;
     const size_t es = g->esz;
     if ((rc = stream_out(fc.f, g->spec, size_t(g->d.n_spectral) * nv * es, st, sg))) return rc;
     if ((rc = stream_out(fc.f, g->phys, size_t(g->d.n_physical) * nv * g->d.nslots * es, st, sg))) return rc;

@@ -531,7 +531,7 @@ int32_t regular(ss_grid *g, const double *r_pts, int n_r, const double *lam_pts,
     };
     const int32_t rc = run();
     if (rc) cudaStreamSynchronize(st);
-    return rc;
+    return rc ? rc : digit_status(g);
 }
 
 // Spline coefficients of every spectral block of `src` (FP64, [item][slot][b]) into a
@@ -674,7 +674,7 @@ int32_t unstructured(ss_grid *g, const double *pts, int64_t npts, double *out, i
         for (int64_t i = 0; i < npts; i++)
             if (mode[i] == 2)
                 for (int v = 0; v < nv; v++) out[size_t(v) * npts + i] = fill;
-    return rc;
+    return rc ? rc : digit_status(g);
 }
 
 // relocate_grid / relocate_grid! fast path (src/relocation.jl:144-439): every
@@ -770,6 +770,7 @@ extern "C" int32_t ss_relocate_grid(ss_grid *target, ss_grid *source, double dx,
     // goes), after the source's queued work has finished
     cudaStream_t st = stream ? (cudaStream_t)stream : target->stream;
     CUDA_TRY(cudaStreamSynchronize(source->stream));
+    if (const int32_t rc = digit_status(source)) return rc;
     if (source->esz == 4) return relocate<float>(target, source, dx, dy, boundary, taper_width, st);
     return relocate<double>(target, source, dx, dy, boundary, taper_width, st);
 }

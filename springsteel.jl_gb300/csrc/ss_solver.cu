@@ -1038,6 +1038,7 @@ extern "C" int32_t ss_solve(ss_problem *p, int32_t method, double tol, int32_t m
         stats->mean_iterations = sum / ns;
         stats->max_rel_residual = mx;
         stats->ms = ms;
+        return digit_status(g);
     }
     return SS_OK;
 }
@@ -1052,7 +1053,7 @@ extern "C" int32_t ss_problem_export(const ss_problem *p, double *rhs, double *x
     if (x) CUDA_TRY(cudaMemcpy(x, p->d_x, n * 8, cudaMemcpyDeviceToHost));
     if (res) CUDA_TRY(cudaMemcpy(res, p->d_res, (size_t)p->nsys * 8, cudaMemcpyDeviceToHost));
     if (iters) CUDA_TRY(cudaMemcpy(iters, p->d_iters, (size_t)p->nsys * 4, cudaMemcpyDeviceToHost));
-    return SS_OK;
+    return digit_status(p->g);
 }
 
 static int32_t check_training_args(ss_problem *p, ss_mlp *mlp) {
@@ -1108,7 +1109,7 @@ extern "C" int32_t ss_problem_collect_training(ss_problem *p, ss_mlp *mlp, const
         mlp->ds_rows += per_field;
     }
     CUDA_TRY(cudaStreamSynchronize(st));
-    return SS_OK;
+    return digit_status(g);
 }
 
 // Training pairs on random right-hand sides: `nsets` sets of one white-noise
