@@ -400,8 +400,10 @@ __global__ void __launch_bounds__(kColThreads, 1) digit_columns_kernel(ColumnArg
 
 // ------------------------------------------------------------ forward columns
 // CBtransform! of binary64 grids: the first b_kDim modes of 128 consecutive columns
-// per tile.  A column's levels are contiguous, so G = 4..16 neighbouring lanes hold
+// per tile.  A column's levels are contiguous, so 4 or 8 neighbouring lanes hold
 // 8 levels each, find the column's exponent by shuffles and cut in registers.
+// Two operand buffers of 24 KB a K-step and the matrix leave room for grids of up to 48
+// levels, and of up to 64 with at most 32 modes; longer columns keep the FMA kernel.
 // Measured: 200 cells, 32 levels, 5 variables 2.60 ms with FP64 FMAs → 0.81 ms (the bytes
 // alone take 0.23 ms), 37 cells, 20 levels, 3 variables 37 → 25 µs; bound by cutting and
 // combining.  The error against 64-bit sums is no larger than the FMA kernel's.
@@ -613,8 +615,8 @@ static int32_t build_forward(ss_grid *g, const std::vector<ChebHost> &cheb) {
     const int N = (int)g->d.kDim, bk = (int)g->d.b_kDim, nv = (int)g->d.nvars;
     Q.fsteps = (N + 15) / 16;
     Q.fblocks = (bk + kZ - 1) / kZ;
-    Q.fgroup = N <= 32 ? 4 : (N <= 64 ? 8 : 16);
-    if (Q.fsteps > 6 || Q.fblocks > kMaxZBlocks || forward_smem(Q.fsteps, Q.fblocks) > kColumnSmem) return SS_OK;
+    Q.fgroup = N <= 32 ? 4 : 8;
+    if (Q.fsteps > 4 || Q.fblocks > kMaxZBlocks || forward_smem(Q.fsteps, Q.fblocks) > kColumnSmem) return SS_OK;
     const int job = Q.fsteps * kZStep;
     std::vector<uint8_t> M((size_t)nv * Q.fblocks * job, 0);
     std::vector<int> E((size_t)nv * Q.fblocks * kZ, 0);
