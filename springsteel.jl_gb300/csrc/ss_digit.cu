@@ -1,5 +1,5 @@
-// ss_digit.cu — the ring DFTs of RLZ grids on the tensor cores, by exact
-// products of digit slices.
+// ss_digit.cu — the ring DFTs of FP64 grids (binary32 RLZ grids: four inverse outputs)
+// on the tensor cores, by products of digit slices.
 //
 // A ring of L = 4n points carries the wavenumbers k ≤ n − 1 only, and its points
 // are symmetric about 0 and π/2, so HC2R of a column folds into four real
@@ -9,13 +9,20 @@
 // SM on this GPU and the mixed-radix FFT of the arbitrary lengths 4 + 4ri spends
 // 2.3 times the conventional operations on prime factors; a binary16 tensor-core
 // product with binary32 accumulation is exact while the operands are integers
-// and the sums stay below 2^24.  So each column is scaled by the exponent of its
+// and the sums stay below 2^24 (see below).  So each column is scaled by the exponent of its
 // largest entry to a fixed-point number and cut into balanced digits (Ozaki et
 // al. 2012, error-free splitting), the matrix likewise once per grid, and
 //     Σ_k Y[m][k] X[k][c] = Σ_s 2^{−9s} D_s,   D_s = Σ_{i+j=s} Σ_k y_i x_j,
 // keeps s ≤ 6 (binary64; 26 of the 36 products, the rest is below 2^−60 of the
 // column's scale) or s ≤ 2 (binary32).  The D_s are combined as integers in
 // 64-bit fixed point (binary64) or in binary32.
+//
+// The sums are drained after at most 96 products.  Random digits then make them 2^19 (rms).
+// Data whose digits follow the signs of a matrix row's could take D_3, D_4, D_5 and D_6 to 1.15,
+// 1.30, 1.54 and 1.03 times 2^24 (computed from the cosine digits, n = 930; up to n = 193, drains of
+// 64 products, every sum stays below): such a sum loses its last bit, 2^-44, 2^-53, 2^-62 and
+// 2^-71 of the scale of one term.  Draining after 48 products excludes it for every n and costs
+// 12 % of both directions of the 200-cell grid (inverse 12.7 → 14.3 ms).
 //
 // The reference turns each coefficient by cos, sin of the Float64 product k·ymin;
 // the folded matrices hold the exact angles, and the difference δ_k (up to 1e-13)
@@ -33,8 +40,8 @@
 // digit_split   G (spectra at the mish points) → column exponents and digit
 //               planes in the MMA operand layout
 // digit_gemm    persistent, warp-specialised: bulk copies → 8-slot (6-slot) ring
-//               of K-steps → two issuing warps, one per accumulator half → two
-//               warpgroups drain and combine
+//               of K-steps → two issuing warps, one per accumulator half → sixteen
+//               warps drain and combine both
 // digit_unfold  quadrant parts → ring points (RL, and columns too long for the kernels that
 //               read the parts)
 #include <cuda_runtime.h>
@@ -785,13 +792,13 @@ constexpr int kDigitMinItems = 1;
 // the matrices' tiles are mostly padding, 37 cells 1.00 (81 items), 0.88 (172), 20 cells 0.75.
 constexpr int kDigitMinItemsF32 = 16, kDigitMinRingsF32 = 180;
 constexpr int64_t kDigitMinPointsF32 = 3500000;
-// bound of a grid's matrix digits (both directions: 4.3 GB at 200 cells, growing with
+// bound of a grid's matrix digits (both directions: 4.5 GB at 200 cells, growing with
 // the cube of the ring count); larger grids keep the FFT kernels
 constexpr size_t kDigitTableBytes = (size_t)16 << 30;
 // Tables above this many bytes are built while they take at most a quarter of the device's free
 // memory, so that grids created later find room
 constexpr size_t kDigitAskBytes = (size_t)256 << 20;
-// RL grids hold far less data than these matrices (0.6 GB at 100 cells): up to about
+// RL grids hold far less data than these matrices (0.7 GB at 100 cells): up to about
 // 120 cells.  100 cells, one variable: ring_inverse 1.07 → 0.13 ms, ring_forward
 // 0.26 → 0.13 ms; 24 cells: 0.32 → 0.03 and 0.095 → 0.03 ms
 constexpr size_t kDigitTableBytesRl = (size_t)1 << 30;
@@ -846,7 +853,7 @@ static void give_flag(int *flag) {
 }
 
 // The matrix digits depend on the ring lengths and wavenumbers alone: grids of the same rings on a device
-// share them (4.2 GB for 200 cells, 0.6 for an RL grid of 100).  They go with the last such grid.
+// share them (4.5 GB for 200 cells, 0.7 for an RL grid of 100).  They go with the last such grid.
 struct DigitTables {
     void *A = nullptr;
     ~DigitTables() {

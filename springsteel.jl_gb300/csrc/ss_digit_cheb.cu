@@ -1,5 +1,7 @@
 // ss_digit_cheb.cu — the Chebyshev column stages of binary64 RLZ grids on the
-// tensor cores, by exact products of digit slices (ss_digit.cu).
+// tensor cores, by products of digit slices (ss_digit.cu; with at most 48 modes in the
+// inverse and 64 levels in the forward direction a digit sum is below 1.31 and 1.75 times 2^24
+// for any data, 2^19 rms for random digits).
 //
 // CA (Γ fold), the CIx recurrence and the DCT-I are linear, so an output column of
 // derivative order d is u = M_d b with M_d = IDCT·(D/dscale)^d·Γ composed on the
@@ -20,9 +22,10 @@
 // Measured on the 200-cell, 32-level, 5-variable FP64 grid: 20.2 ms with FP64 FMAs
 // (94% of the FP64 matmul rate), 7.2 ms as digits with loads in line, 4.95 ms with
 // the next parts in flight (cp.async), 16 draining warps and the words of a digit
-// sum added by wide multiply-adds (shifts and logic run at half rate).  Memory
-// alone would take 1.4 ms; what is left is the integer work of cutting (8 warps
-// without it: 3.5 ms) and of rounding 64-bit fixed point to binary64.
+// sum added by wide multiply-adds (shifts and logic run at half rate); 6.1 ms with the
+// derivatives cut apart (6.7 before four modes were cut at a time).  Memory
+// alone would take 1.4 ms; what is left is the integer work of cutting (five cuts: 8 warps
+// without it 3.5 ms) and of rounding 64-bit fixed point to binary64.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -53,7 +56,8 @@ constexpr int kZ = 32;                      // matrix rows (levels) of one produ
 constexpr int kZStep = 6 * kZ * 32;         // bytes of a K-step of matrix digits: 6 planes × 32 rows × 16
 constexpr int kAStep = 6 * kDigitPlane;     // and of column digits
 // Warps: producing, draining (half of them per accumulator), one issuing.  Measured
-// on the 200-cell FP64 grid: 8 + 16 warps 4.95 ms, 16 + 8 5.34 ms, 8 + 8 5.7 ms.
+// on the 200-cell FP64 grid with five cuts: 8 + 16 warps 4.95 ms, 16 + 8 5.34 ms, 8 + 8 5.7 ms;
+// with seven, 12 + 16 is 0.1 ms slower than 8 + 16.
 constexpr int kProducers = 8, kDrains = 16;
 constexpr int kColThreads = (kProducers + kDrains + 1) * 32;
 constexpr int kMaxModes = 48;               // three K-steps: what the shared memory holds

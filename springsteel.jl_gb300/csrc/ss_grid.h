@@ -54,7 +54,7 @@ struct ss_grid {
     int64_t *d_fofs = nullptr;
     SplineDev *d_spl = nullptr;
     ChebDev *d_cheb = nullptr;
-    DigitPlan digit;                                      // RLZ rings on the tensor cores (ss_digit.cu)
+    DigitPlan digit;                                      // rings and columns on the tensor cores (ss_digit.cu)
     double *d_ahat = nullptr, *d_fw = nullptr, *d_cw = nullptr;
     int filtered = 0;
     int ring_threads_fwd = 256, ring_threads_inv = 256;  // CTA size of the ring kernels (autotuned by batches)

@@ -86,7 +86,7 @@ __global__ void reg_si_kernel(const double *coef, const int *m0, const double *w
 }
 
 // ---- cos(kλ), sin(kλ) tables
-// π/2 in parts of 33, 33 and 53 bits
+// π/2 in parts of 33, 33 and 53 bits (reduction after Cody and Waite 1980)
 constexpr double kPio2a = 0x1.921fb54400000p+0, kPio2b = 0x1.0b4611a600000p-34, kPio2c = 0x1.3198a2e037073p-69;
 // cos and sin of a, |a| < 2^20: a − n·π/2 in two words (n times the first two parts is
 // exact), then the Taylor series with the leading terms in two words.  Against 64-bit
@@ -499,7 +499,7 @@ int32_t regular(ss_grid *g, const double *r_pts, int n_r, const double *lam_pts,
         reg_si_kernel<<<dim3((ns + 127) / 128, n_r, nitems), 128, 0, st>>>(d_coef, d_m0, d_w, d_sr, b, ns, n_r,
                                                                             nitems);
         CUDA_TRY(cudaGetLastError());
-        const size_t fsm = size_t(3) * ns * 8;
+        const size_t fsm = size_t(3) * ns * 8;  // the bound of an earlier kernel that staged whole rows: kept for callers
         if (fsm > (size_t)optin) {
             set_error("regularGridTransform: %d wavenumber slots exceed shared memory", ns);
             return SS_BAD_SHAPE;

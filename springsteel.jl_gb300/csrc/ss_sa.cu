@@ -15,9 +15,9 @@
 // grid and as long elsewhere, but held a slot at one exponent; widening and rounding by
 // integer operations took 0.8 ms more than the conversions).
 //
-// Measured before → here: 400-cell binary32 RLZ grid of 4 variables 9.9 → @SA400@ ms,
-// 251-cell binary32 RL grid of 4 variables 0.87 → @SA251@ ms, 125-cell binary32 RLZ
-// grid 0.77 → @SA125@ ms, 200-cell FP64 RLZ grid of 5 variables 2.03 → 1.38 ms (12
+// Measured before → here: 400-cell, 64-level binary32 RLZ grid of 4 variables 10.0 → 8.1 ms,
+// 251-cell binary32 RL grid of 4 variables 0.88 → 0.15 ms, 125-cell, 40-level binary32 RLZ
+// grid of 2 variables 0.59 → 0.19 ms, 200-cell FP64 RLZ grid of 5 variables 2.03 → 1.39 ms (12
 // FP64 operations per slot and ring for SI alone hold the FP64 units for 0.85 ms),
 // 100-cell FP64 RL grid 0.13 → 0.05 ms (a chain of 103 rows × 7 × 64 cycles).
 #include <cuda_runtime.h>
