@@ -17,10 +17,11 @@ namespace ss {
 // digit is the integer itself (1024 + field, less 1024 + bias); a data digit is
 // its 2^-24 multiple: the field read as a binary16 subnormal, which needs no
 // exponent bits set.
+// `mask`: the fields' bits in a and b, cut from both halves at once.
 template <bool kMatrix>
-__device__ __forceinline__ uint32_t half_pair(uint32_t a, uint32_t b, uint32_t bias) {
+__device__ __forceinline__ uint32_t half_pair(uint32_t a, uint32_t b, uint32_t mask, uint32_t bias) {
     const uint32_t off = kMatrix ? 0x64006400u : 0u;
-    const uint32_t v = off + __byte_perm(a, b, 0x5410), w = off + bias;
+    const uint32_t v = off + (__byte_perm(a, b, 0x5410) & mask), w = off + bias;
     const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&v), *reinterpret_cast<const __half2 *>(&w));
     return *reinterpret_cast<const uint32_t *>(&h);
 }
@@ -49,9 +50,8 @@ __device__ __forceinline__ void planes8(const unsigned long long (&U)[8], uint4 
         uint32_t w[4];
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            uint32_t a = (uint32_t)(U[2 * q] >> sh), b = (uint32_t)(U[2 * q + 1] >> sh);
-            if (i > 0) { a &= 511u; b &= 511u; }
-            w[q] = half_pair<kMatrix>(a, b, i > 0 ? 0x01000100u : 0x02000200u);
+            w[q] = half_pair<kMatrix>((uint32_t)(U[2 * q] >> sh), (uint32_t)(U[2 * q + 1] >> sh), i > 0 ? 0x01ff01ffu : 0xffffffffu,
+                                      i > 0 ? 0x01000100u : 0x02000200u);
         }
         out[i] = make_uint4(w[0], w[1], w[2], w[3]);
     }
@@ -64,9 +64,8 @@ __device__ __forceinline__ void planes4(const unsigned long long (&U)[4], uint2 
         uint32_t w[2];
 #pragma unroll
         for (int q = 0; q < 2; q++) {
-            uint32_t a = (uint32_t)(U[2 * q] >> sh), b = (uint32_t)(U[2 * q + 1] >> sh);
-            if (i > 0) { a &= 511u; b &= 511u; }
-            w[q] = half_pair<false>(a, b, i > 0 ? 0x01000100u : 0x02000200u);
+            w[q] = half_pair<false>((uint32_t)(U[2 * q] >> sh), (uint32_t)(U[2 * q + 1] >> sh), i > 0 ? 0x01ff01ffu : 0xffffffffu,
+                                    i > 0 ? 0x01000100u : 0x02000200u);
         }
         out[i] = make_uint2(w[0], w[1]);
     }
