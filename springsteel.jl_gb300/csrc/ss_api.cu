@@ -575,7 +575,11 @@ bool sa_band_serves(const ss_grid *g) {
 // launches and the emptying GPU at the end of each cost more than the lower residency
 // (30 to 600 cells, binary32 and binary64: 2 is within 5 % of the best of 0.5, 2, 3, 4,
 // 5, 8 and 20; at 20 the 600-cell grid of 12 variables runs 1.06×, of 3 variables 1.6×
-// as long); behind a launch of more than 16 fillings the gap is nothing (400 cells × 43
+// as long); at most once when that shared memory leaves an SM fewer than three CTAs and all
+// rings would be `few`, whose CTAs are five times as many (RL, a round trip of one grid alone and
+// of eight on streams of their own, per grid, at twice → at once: binary64 300 cells × 1 variable
+// 1709 → 1502 and 1678 → 1116 µs, 200 × 1 equal, binary32 400 × 1 595 → 547 and 617 → 462; three CTAs
+// an SM and more, binary64 130 × 4 808 → 909 and equal; not few, binary32 400 × 4 1347 → 1442, 1268 → 1201); behind a launch of more than 16 fillings the gap is nothing (400 cells × 43
 // modes × 4 variables, binary32: 0.4 % of the forward transform lost by joining).
 // `few`: the threads of an item per CTA fit the GPU at once.  Such launches take one item
 // per CTA, and the inverse one output per CTA: five times the CTAs, each reading the
@@ -588,12 +592,14 @@ template <typename Fn>
 static int32_t for_ring_launches(ss_grid *g, int chunk, bool inverse, int threads, Fn fn) {
     if (chunk >= 0)
         return for_ring_segments(g, chunk, [&](const int *list, int count, const RingBucket &b) { return fn(list, count, b, false); });
+    const bool all_few = (int64_t)g->d.iDim * g->nitems * threads <= (int64_t)g->sms * 2048;
     for (size_t b = 0; b < g->buckets.size();) {
         const RingBucket &top = g->buckets[b];
         const double per_sm = (227.0 * 1024) / (double)(ring_item_smem(g, top, inverse) + 2048);
+        const double fills = all_few && per_sm < 3.0 ? 1.0 : 2.0;
         int count = top.count;
         for (b++; b < g->buckets.size(); b++) {
-            if ((double)g->buckets[b].count * g->nitems > 2.0 * per_sm * g->sms) break;
+            if ((double)g->buckets[b].count * g->nitems > fills * per_sm * g->sms) break;
             if ((double)count * g->nitems > 16.0 * per_sm * g->sms) break;
             count += g->buckets[b].count;
         }
