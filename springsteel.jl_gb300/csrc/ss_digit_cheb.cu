@@ -22,7 +22,7 @@
 // Measured on the 200-cell, 32-level, 5-variable FP64 grid: 20.2 ms with FP64 FMAs
 // (94% of the FP64 matmul rate), 7.2 ms as digits with loads in line, 4.95 ms with
 // the next parts in flight (cp.async), 16 draining warps and the words of a digit
-// sum added by wide multiply-adds (shifts and logic run at half rate); 6.1 ms with the
+// sum added by wide multiply-adds (shifts and logic run at half rate); 6.0 ms with the
 // derivatives cut apart (6.7 before four modes were cut at a time).  Memory
 // alone would take 1.4 ms; what is left is the integer work of cutting (five cuts: 8 warps
 // without it 3.5 ms) and of rounding 64-bit fixed point to binary64.
