@@ -817,8 +817,9 @@ struct FlagPage {
     int live;
 };
 constexpr int kFlags = 512;
-std::mutex flag_mutex;
-std::vector<FlagPage> flag_pages;
+// (not destroyed at exit: a grid may be closed after the library's static objects)
+std::mutex &flag_mutex = *new std::mutex;
+std::vector<FlagPage> &flag_pages = *new std::vector<FlagPage>;
 }  // namespace
 static int *take_flag() {
     std::lock_guard<std::mutex> lock(flag_mutex);
@@ -861,8 +862,8 @@ struct DigitTables {
     }
 };
 namespace {
-std::mutex table_mutex;
-std::map<std::vector<int>, std::weak_ptr<DigitTables>> tables;
+std::mutex &table_mutex = *new std::mutex;
+auto &tables = *new std::map<std::vector<int>, std::weak_ptr<DigitTables>>;
 }  // namespace
 
 // B tiles of a ring, and its tile products with the first B tile at `used`
